@@ -120,6 +120,9 @@ void free_systems(ktg_ctx *c) {
         dev_free(s.s32);
         dev_free(s.rs32);
     }
+    dev_free(c->sliced_rows);
+    dev_free(c->sliced_nnz);
+    c->sliced = ktg::SlicedSystem{};
     dev_free(c->x);
     dev_free(c->y);
     dev_free(c->ax);
@@ -153,6 +156,43 @@ int dev_grow_keep(ktg_ctx *c, T **p, int64_t keep, int64_t count) {
     return KTG_OK;
 }
 
+// The per-row scratch of the default FP64 solve, in one allocation.
+int reserve_sliced_rows(ktg_ctx *c, int64_t rows) {
+    const int64_t slices = ktg::sliced_slices(2 * rows, c->num_sms);
+    int64_t at = 0;
+    auto take = [&](int64_t bytes) {
+        const int64_t here = at;
+        at += (bytes + 255) / 256 * 256;
+        return here;
+    };
+    const int64_t vec = sizeof(double) * 2 * rows;
+    const int64_t diag = take(vec), x = take(vec), r = take(vec), z = take(vec), p = take(vec),
+                  ap = take(vec), start = take(sizeof(ktg::Start) * 2 * rows),
+                  perm = take(sizeof(int32_t) * 2 * rows), axis = take(2 * rows),
+                  lists = take(sizeof(uint2) * slices), dealt = take(sizeof(uint2) * slices),
+                  widths = take(sizeof(uint32_t) * slices), owner = take(slices),
+                  slots = take(sizeof(uint64_t) * ktg::sliced_slots(c->num_sms));
+    const int rc = dev_alloc(c, &c->sliced_rows, at);
+    if (rc) return rc;
+    char *m = c->sliced_rows;
+    ktg::SlicedSystem &s = c->sliced;
+    s.diag = reinterpret_cast<double *>(m + diag);
+    s.x = reinterpret_cast<double *>(m + x);
+    s.r = reinterpret_cast<double *>(m + r);
+    s.z = reinterpret_cast<double *>(m + z);
+    s.p = reinterpret_cast<double *>(m + p);
+    s.ap = reinterpret_cast<double *>(m + ap);
+    s.start = reinterpret_cast<ktg::Start *>(m + start);
+    s.perm = reinterpret_cast<int32_t *>(m + perm);
+    s.axis = reinterpret_cast<uint8_t *>(m + axis);
+    s.slices = reinterpret_cast<uint2 *>(m + lists);
+    s.dealt = reinterpret_cast<uint2 *>(m + dealt);
+    s.widths = reinterpret_cast<uint32_t *>(m + widths);
+    s.owner = reinterpret_cast<uint8_t *>(m + owner);
+    s.slots = reinterpret_cast<unsigned long long *>(m + slots);
+    return KTG_OK;
+}
+
 // Room for systems of `rows` rows and `nnz` entries per axis. The arrays
 // that hold a system (row pointers, columns, values, diagonal, right-hand
 // side) keep their contents when they grow, so an axis installed earlier
@@ -177,6 +217,7 @@ int reserve_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
             if ((rc = dev_alloc(c, &s.ap32, rows))) return rc;
             if ((rc = dev_alloc(c, &s.rs32, rows))) return rc;
         }
+        if ((rc = reserve_sliced_rows(c, rows))) return rc;
         if ((rc = dev_alloc(c, &c->x, rows))) return rc;
         if ((rc = dev_alloc(c, &c->y, rows))) return rc;
         if ((rc = dev_alloc(c, &c->ax, rows))) return rc;
@@ -187,11 +228,16 @@ int reserve_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
     if (nnz > c->sys_cap_nnz) {
         const int64_t old = c->sys_cap_nnz;
         for (auto &s : c->sys) {
-            if ((rc = dev_grow_keep(c, &s.col, old, nnz))) return rc;
-            if ((rc = dev_grow_keep(c, &s.val, old, nnz))) return rc;
+            // room to read the last entries four at a time
+            if ((rc = dev_grow_keep(c, &s.col, old, nnz + 3))) return rc;
+            if ((rc = dev_grow_keep(c, &s.val, old, nnz + 3))) return rc;
             if ((rc = dev_alloc(c, &s.val32, nnz))) return rc;
             if ((rc = dev_alloc(c, &s.s32, nnz))) return rc;
         }
+        const int64_t entries = ktg::sliced_entries(2 * nnz, c->num_sms);  // a multiple of 32
+        if ((rc = dev_alloc(c, &c->sliced_nnz, entries * 12))) return rc;
+        c->sliced.val = reinterpret_cast<double *>(c->sliced_nnz);
+        c->sliced.col = reinterpret_cast<int32_t *>(c->sliced.val + entries);
         c->val32_valid = false;
         c->precond_ready = false;
         c->agg_ready = false;
@@ -474,7 +520,7 @@ int ktg_upload_netlist(ktg_ctx *c, const ktg_netlist_view *nl) {
         if (var >= n) return set_error(c, KTG_ERR_ARG, "var_of_vertex out of range");
         pin_var[p] = var < 0 ? -1 : var;
     }
-    int64_t cap = 0;
+    int64_t cap = 0, range = 0;
     for (int64_t k = 0; k < N; ++k) {
         net_start32[k] = static_cast<int32_t>(nl->net_start[k]);
         const int64_t deg = nl->net_start[k + 1] - nl->net_start[k];
@@ -484,7 +530,8 @@ int ktg_upload_netlist(ktg_ctx *c, const ktg_netlist_view *nl) {
         for (int64_t p = nl->net_start[k]; p < nl->net_start[k + 1]; ++p) m += pin_var[p] >= 0;
         net_mov[k] = m;
         // Bound rows (2) get m-1 movable ends, the others at most 2 each.
-        if (m > 0) cap += 4 * static_cast<int64_t>(m);
+        if (m > 1) cap += 4 * static_cast<int64_t>(m) - 6;
+        range += 4 * static_cast<int64_t>(m);
     }
     net_start32[N] = static_cast<int32_t>(P);
     for (int64_t i = 0; i <= n; ++i) pin_start32[i] = static_cast<int32_t>(nl->pin_start[i]);
@@ -499,7 +546,7 @@ int ktg_upload_netlist(ktg_ctx *c, const ktg_netlist_view *nl) {
             const int64_t p = nl->net_start[nl->pin_net[e]] + nl->pin_q[e];
             if (pin_var[p] != i) return set_error(c, KTG_ERR_ARG, "pin_ref does not point to its cell");
         }
-    if (cap > lim) return set_error(c, KTG_ERR_RANGE, "B2B systems exceed 32-bit indices");
+    if (range > lim) return set_error(c, KTG_ERR_RANGE, "B2B systems exceed 32-bit indices");
     std::vector<double> area(n);
     double total_area = 0.0;
     for (int64_t i = 0; i < n; ++i) {

@@ -25,9 +25,33 @@ namespace ktg {
 // Bits of ktg_ctx::attr_bits.
 constexpr unsigned kAttrOccupancy = 1u;  // k_occ_accum<true> opt-in shared memory
 constexpr unsigned kAttrMixed = 2u;      // k_pcg_mixed_cg opt-in shared memory
+constexpr unsigned kAttrSliced = 4u;     // k_pcg_sliced opt-in shared memory
 
 struct AggState;  // aggregation preconditioner buffers (ktg_agg.cu)
 struct LalState;  // free space and scratch of the look-ahead legalizer (ktg_lal.cu)
+
+// The default FP64 solve's copy of the two systems (ktg_pcg_sliced.cu): rows
+// of each block's slice of [x rows | y rows] sorted by length, 32 side by
+// side; vectors in that order.
+struct Start {
+    double x;
+    int64_t pos;
+};
+struct SlicedSystem {
+    int32_t *col = nullptr;  // [sliced_entries]
+    double *val = nullptr;
+    double *diag = nullptr, *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr,
+           *ap = nullptr;                             // [2n]
+    Start *start = nullptr;                           // [2n] per row: start value, position
+    int32_t *perm = nullptr;                          // [2n] row at a position
+    uint8_t *axis = nullptr;                          // [2n]
+    // per block: its slices (first entry / 32, first position | lane shift),
+    // each slice's warp, and the slices in the order the warps take them
+    uint2 *slices = nullptr, *dealt = nullptr;
+    uint32_t *widths = nullptr;
+    uint8_t *owner = nullptr;
+    unsigned long long *slots = nullptr;              // the grid-wide sums
+};
 
 struct AxisSystem {
     int32_t *row_ptr = nullptr;  // [n+1]
@@ -92,6 +116,8 @@ struct ktg_ctx {
 
     // systems
     ktg::AxisSystem sys[2];
+    ktg::SlicedSystem sliced;  // scratch of the default FP64 solve
+    char *sliced_rows = nullptr, *sliced_nnz = nullptr;  // its two allocations
     bool have_system = false;  // both axes valid with sys_n rows
     bool axis_valid[2] = {false, false};
     bool val32_valid = false;  // sys[*].val32 mirrors sys[*].val
@@ -181,6 +207,12 @@ int launch_kraftwerk2_adjust(ktg_ctx *ctx, const double *move_weight, const doub
                              const double *toward_y, double diag_floor);
 int launch_solve(ktg_ctx *ctx, double *x, double *y, double tol, int64_t max_iter,
                  ktg_solve_info *info_dev, double *hist_x, double *hist_y, int64_t hist_cap);
+int launch_solve_sliced(ktg_ctx *ctx, double *x, double *y, double tol, int64_t max_iter,
+                        ktg_solve_info *info_dev, double *hist_x, double *hist_y,
+                        int64_t hist_cap);
+int64_t sliced_entries(int64_t nnz_both, int num_sms);
+int64_t sliced_slices(int64_t rows, int num_sms);
+int64_t sliced_slots(int num_sms);
 int launch_occupancy(ktg_ctx *ctx, const double *x, const double *y, double *occ_dev,
                      double *overflow_dev);
 int launch_solve_mixed(ktg_ctx *ctx, double *x, double *y, double tol, double inner_tol,

@@ -1017,12 +1017,10 @@ struct Variant {
 // form 0: textbook three-barrier PCG; form 1: Chronopoulos-Gear two-barrier;
 // form 2: textbook PCG with the reference's summation order everywhere
 // (bit-identical to the reference's solve); form 3: textbook PCG with A p by
-// recurrence, two barriers.
+// recurrence, two barriers (with 32 lanes, the default, it is the sliced kernel
+// of ktg_pcg_sliced.cu).
 Variant pick_variant(int form, bool smem, int lanes) {
     if (form == 3) {
-        if (lanes == 32)
-            return {smem ? k_pcg<true, 32, false, true> : k_pcg<false, 32, false, true>,
-                    kVecsPerRow};
         if (smem) return {lanes == 4 ? k_pcg<true, 4, false, true> : k_pcg<true, 1, false, true>,
                           kVecsPerRow};
         return {lanes == 4 ? k_pcg<false, 4, false, true> : k_pcg<false, 1, false, true>,
@@ -1053,6 +1051,17 @@ int pcg_form_default = 3;
 int launch_solve(ktg_ctx *c, double *x, double *y, double tol, int64_t max_iter,
                  ktg_solve_info *info_dev, double *hist_x, double *hist_y, int64_t hist_cap) {
     const int64_t nsys = c->sys_n;
+    const int lanes = c->pcg_lanes > 0 ? c->pcg_lanes : pcg_lanes_default;
+    const int form = c->pcg_form >= 0 ? c->pcg_form : pcg_form_default;
+    if (form == 3 && lanes == 32) {
+        const int rc = launch_solve_sliced(c, x, y, tol, max_iter, info_dev, hist_x, hist_y,
+                                           hist_cap);
+        if (rc) return rc;
+        k_solve_status<<<1, 1, 0, c->stream>>>(c->status, info_dev);
+        ++c->launches;
+        KTG_CUDA(c, cudaGetLastError());
+        return KTG_OK;
+    }
     PcgArgs A;
     for (int a = 0; a < 2; ++a) {
         ktg::AxisSystem &s = c->sys[a];
@@ -1066,8 +1075,6 @@ int launch_solve(ktg_ctx *c, double *x, double *y, double tol, int64_t max_iter,
     const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(c->num_sms, want)));
     A.rows_per_block = static_cast<int32_t>((A.total_rows + grid - 1) / grid);
     if (A.rows_per_block == 0) A.rows_per_block = 1;
-    const int lanes = c->pcg_lanes > 0 ? c->pcg_lanes : pcg_lanes_default;
-    const int form = c->pcg_form >= 0 ? c->pcg_form : pcg_form_default;
     // Dynamic shared memory for the vector slices: what the block may opt in
     // to, less the kernel's static arrays, capped at kPcgSmemBytes.
     size_t &bud = c->pcg_smem_budget[form][lanes_index(lanes)];  // per context (one device)

@@ -1,0 +1,96 @@
+"""The sliced FP64 solve (ktg_pcg_sliced.cu, the default form) at the sizes
+where its layout changes: rows around the lane-count limits (8, 16, 24 entries
+per lane and their doublings up to a warp per row), empty rows, blocks and
+slices that are not full, one block against several, and each choice of the
+vectors that live in shared memory.
+
+Tolerances: the solve follows the reference's iteration with other summation
+orders, so iteration counts are equal and solutions of these well-conditioned
+systems (diagonally dominant, fewer than 40 steps) agree far below the 1e-9
+that the other solve tests allow."""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+TOL, SOL_RTOL = 1e-8, 1e-11
+
+
+def random_system(n, lengths, seed):
+    """Unsymmetric pattern is enough for the products; symmetric values keep PCG
+    defined, so entry (i, j) is mirrored. lengths: wanted row lengths, cycled."""
+    rng = np.random.default_rng(seed)
+    want = np.resize(np.asarray(lengths), n) // 2
+    rows = np.repeat(np.arange(n), want)
+    cols = rng.integers(0, n, rows.shape[0])
+    keep = rows != cols
+    rows, cols = rows[keep], cols[keep]
+    v = -rng.uniform(0.1, 1.0, rows.shape[0])
+    r, c, v = np.concatenate([rows, cols]), np.concatenate([cols, rows]), np.concatenate([v, v])
+    order = np.argsort(r, kind="stable")
+    r, c, v = r[order], c[order], v[order]
+    rp = np.zeros(n + 1, np.int64)
+    np.cumsum(np.bincount(r, minlength=n), out=rp[1:])
+    diag = np.bincount(r, weights=-v, minlength=n) * 1.3 + rng.uniform(0.5, 1.0, n)
+    return dict(row_ptr=rp, col=c.astype(np.int32), val=v, diag=diag, rhs=rng.standard_normal(n))
+
+
+def check(ctx, n, lengths, seed=0):
+    sx, sy = random_system(n, lengths, seed), random_system(n, lengths[::-1], seed + 1)
+    rng = np.random.default_rng(seed + 2)
+    x0, y0 = rng.standard_normal((2, n))
+    ctx.upload_system(0, sx)
+    ctx.upload_system(1, sy)
+    got = ctx.solve(x0, y0, TOL, 1000)
+    again = ctx.solve(x0, y0, TOL, 1000)
+    ref = oracle.port_solve_both(sx, x0, sy, y0, TOL, 1000)
+    assert got["iters"] == ref["iters"]
+    for k in ("x", "y"):
+        assert np.linalg.norm(got[k] - ref[k]) <= SOL_RTOL * np.linalg.norm(ref[k])
+        assert np.array_equal(got[k], again[k])  # the same from run to run
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 300, 511, 512, 513, 640, 1021, 5003])
+def test_sizes(n, gpu_ctx, port_built):
+    check(gpu_ctx, n, [0, 2, 4, 6, 10, 20])
+
+
+@pytest.mark.parametrize("lengths", [[0], [8], [9, 7], [16, 17, 1], [24, 25, 23, 48, 49],
+                                     [96, 97, 2, 4], [190, 200, 390, 6, 6, 6], [800, 2, 0, 2, 4]])
+@pytest.mark.parametrize("n", [450, 2050])
+def test_row_lengths(n, lengths, gpu_ctx, port_built):
+    check(gpu_ctx, n, lengths, seed=7)
+
+
+@pytest.mark.parametrize("n", [40_009, 160_001, 290_003, 560_003, 1_050_001])
+def test_vector_homes(n, gpu_ctx, port_built):
+    """Wider lanes from 2,048 rows a block; 4, 2, 1 and 0 vectors in shared
+    memory (about 3.8k, 7.4k and 14.1k rows a block)."""
+    check(gpu_ctx, n, [2, 6, 2, 4, 8, 40], seed=3)
+
+
+def test_axes_apart(gpu_ctx, port_built):
+    """One axis done before the other, one that never starts (b = 0) and one
+    that is not positive definite."""
+    n = 2000
+    sx, sy = random_system(n, [4, 8], 1), random_system(n, [4, 8], 2)
+    rng = np.random.default_rng(5)
+    x0, y0 = rng.standard_normal((2, n))
+    for kind in ("zero", "solved", "indefinite"):
+        s = dict(sy)
+        y = y0.copy()
+        if kind == "zero":
+            s["rhs"] = np.zeros(n)
+        elif kind == "solved":
+            y = oracle.port_pcg_axis(sy, y0, 1e-5, 1000)["x"]
+        else:
+            s["val"] = -3.0 * sy["val"]
+        gpu_ctx.upload_system(0, sx)
+        gpu_ctx.upload_system(1, s)
+        got = gpu_ctx.solve(x0, y, TOL, 200)
+        ref = oracle.port_solve_both(sx, x0, s, y, TOL, 200)
+        assert got["iters"] == ref["iters"], kind
+        assert np.linalg.norm(got["x"] - ref["x"]) <= SOL_RTOL * np.linalg.norm(ref["x"]), kind
+        scale = max(np.linalg.norm(ref["y"]), 1e-300)
+        assert np.linalg.norm(got["y"] - ref["y"]) <= 1e-9 * scale, kind
