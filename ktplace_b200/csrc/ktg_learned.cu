@@ -124,85 +124,113 @@ __global__ void k_features(const int32_t *rp, const int32_t *col, const double *
 }
 
 // ---------------------------------------------------------------------------
-// mean aggregations over the bipartite graph (one warp per output row,
-// two channels per lane; sums in pin order: deterministic)
+// mean aggregations over the bipartite graph (half a warp per output row, four
+// channels per lane; sums in pin order: deterministic)
+//
+// A row has four pins on average, so latency bounds these kernels: the lanes
+// read up to 16 of the row's indices at once and four source rows are in flight
+// (a warp per row walking its pins one by one: 17-48 us at 60k cells, now 8-13).
 // ---------------------------------------------------------------------------
+constexpr int kAggLanes = HID / 4;
+
+// Sum over q in [b, e) of scale(index(q)) * src[index(q)], four channels per
+// lane, in the order of q; negative indices are left out. Called by the
+// kAggLanes lanes of a row.
+template <class Index, class Scale>
+__device__ __forceinline__ float4 sum_rows(int32_t b, int32_t e, const float *src, Index index,
+                                           Scale scale) {
+    const int sub = threadIdx.x & (kAggLanes - 1);
+    const unsigned mask = 0xffffu << (threadIdx.x & 16);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int32_t q = b; q < e; q += kAggLanes) {
+        const int cnt = min(kAggLanes, e - q);
+        const int32_t c = sub < cnt ? index(q + sub) : -1;
+        const float s = c >= 0 ? scale(c) : 0.f;
+        for (int j = 0; j < cnt; j += 4) {
+            int32_t cj[4];
+            float sj[4];
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                cj[u] = __shfl_sync(mask, c, j + u, kAggLanes);
+                sj[u] = __shfl_sync(mask, s, j + u, kAggLanes);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (cj[u] >= 0)
+                    v[u] = reinterpret_cast<const float4 *>(src + static_cast<int64_t>(cj[u]) * HID)[sub];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (cj[u] >= 0) {
+                    acc.x += v[u].x * sj[u];
+                    acc.y += v[u].y * sj[u];
+                    acc.z += v[u].z * sj[u];
+                    acc.w += v[u].w * sj[u];
+                }
+        }
+    }
+    return acc;
+}
+
+__device__ __forceinline__ int32_t agg_row() {
+    return static_cast<int32_t>((blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / kAggLanes);
+}
+
+__device__ __forceinline__ float4 *agg_out(float *p, int32_t row) {
+    return reinterpret_cast<float4 *>(p + static_cast<int64_t>(row) * HID) +
+           (threadIdx.x & (kAggLanes - 1));
+}
+
 // m[k] = (1/cnt_k) sum over movable pins of net k of h[cell]
 __global__ void k_cells_to_nets(const int32_t *net_start, const int32_t *pin_var,
                                 const int32_t *net_mov, int32_t N, const float *h, float *m) {
-    const int32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const int32_t k = agg_row();
     if (k >= N) return;
-    float a0 = 0.f, a1 = 0.f;
-    for (int32_t p = net_start[k]; p < net_start[k + 1]; ++p) {
-        const int32_t c = pin_var[p];
-        if (c < 0) continue;
-        const float2 v = reinterpret_cast<const float2 *>(h + static_cast<int64_t>(c) * HID)[lane];
-        a0 += v.x;
-        a1 += v.y;
-    }
+    const float4 a = sum_rows(net_start[k], net_start[k + 1], h,
+                              [&](int32_t p) { return pin_var[p]; }, [](int32_t) { return 1.f; });
     const float inv = net_mov[k] > 0 ? 1.0f / static_cast<float>(net_mov[k]) : 0.0f;
-    reinterpret_cast<float2 *>(m + static_cast<int64_t>(k) * HID)[lane] = make_float2(a0 * inv, a1 * inv);
+    *agg_out(m, k) = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
 }
 
 // g[c] = (1/cnt_c) sum over pins of cell c of e[net]
 __global__ void k_nets_to_cells(const int32_t *pin_start, const int2 *pin_ref, int32_t n,
                                 const float *e, float *g) {
-    const int32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const int32_t c = agg_row();
     if (c >= n) return;
-    float a0 = 0.f, a1 = 0.f;
     const int32_t e0 = pin_start[c], e1 = pin_start[c + 1];
-    for (int32_t q = e0; q < e1; ++q) {
-        const int32_t k = pin_ref[q].x;
-        const float2 v = reinterpret_cast<const float2 *>(e + static_cast<int64_t>(k) * HID)[lane];
-        a0 += v.x;
-        a1 += v.y;
-    }
+    const float4 a = sum_rows(e0, e1, e, [&](int32_t q) { return pin_ref[q].x; },
+                              [](int32_t) { return 1.f; });
     const float inv = e1 > e0 ? 1.0f / static_cast<float>(e1 - e0) : 0.0f;
-    reinterpret_cast<float2 *>(g + static_cast<int64_t>(c) * HID)[lane] = make_float2(a0 * inv, a1 * inv);
+    *agg_out(g, c) = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
 }
 
 // dh[c] (+)= sum over pins of cell c of dm[net] / cnt_net   (transpose of cells->nets)
 __global__ void k_cells_to_nets_T(const int32_t *pin_start, const int2 *pin_ref,
                                   const int32_t *net_mov, int32_t n, const float *dm, float *dh,
                                   int accumulate) {
-    const int32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const int32_t c = agg_row();
     if (c >= n) return;
-    float a0 = 0.f, a1 = 0.f;
-    for (int32_t q = pin_start[c]; q < pin_start[c + 1]; ++q) {
-        const int32_t k = pin_ref[q].x;
-        const float inv = 1.0f / static_cast<float>(net_mov[k]);
-        const float2 v = reinterpret_cast<const float2 *>(dm + static_cast<int64_t>(k) * HID)[lane];
-        a0 += v.x * inv;
-        a1 += v.y * inv;
-    }
-    float2 *o = reinterpret_cast<float2 *>(dh + static_cast<int64_t>(c) * HID) + lane;
+    float4 a = sum_rows(pin_start[c], pin_start[c + 1], dm, [&](int32_t q) { return pin_ref[q].x; },
+                        [&](int32_t k) { return 1.0f / static_cast<float>(net_mov[k]); });
+    float4 *o = agg_out(dh, c);
     if (accumulate) {
-        const float2 old = *o;
-        a0 += old.x;
-        a1 += old.y;
+        const float4 old = *o;
+        a.x += old.x;
+        a.y += old.y;
+        a.z += old.z;
+        a.w += old.w;
     }
-    *o = make_float2(a0, a1);
+    *o = a;
 }
 
 // de[k] = sum over movable pins of net k of dg[cell] / cnt_cell   (transpose of nets->cells)
 __global__ void k_nets_to_cells_T(const int32_t *net_start, const int32_t *pin_var,
                                   const int32_t *pin_start, int32_t N, const float *dg, float *de) {
-    const int32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    const int32_t k = agg_row();
     if (k >= N) return;
-    float a0 = 0.f, a1 = 0.f;
-    for (int32_t p = net_start[k]; p < net_start[k + 1]; ++p) {
-        const int32_t c = pin_var[p];
-        if (c < 0) continue;
-        const float inv = 1.0f / static_cast<float>(pin_start[c + 1] - pin_start[c]);
-        const float2 v = reinterpret_cast<const float2 *>(dg + static_cast<int64_t>(c) * HID)[lane];
-        a0 += v.x * inv;
-        a1 += v.y * inv;
-    }
-    reinterpret_cast<float2 *>(de + static_cast<int64_t>(k) * HID)[lane] = make_float2(a0, a1);
+    *agg_out(de, k) = sum_rows(
+        net_start[k], net_start[k + 1], dg, [&](int32_t p) { return pin_var[p]; },
+        [&](int32_t c) { return 1.0f / static_cast<float>(pin_start[c + 1] - pin_start[c]); });
 }
 
 // ---------------------------------------------------------------------------
@@ -595,9 +623,131 @@ __global__ void k_dense_fp32(DenseArgs A) {
     A.y[idx] = s;
 }
 
-// Weight gradient dW[K x OUT] = X^T (dY * mask) and db = sum rows of
-// (dY * mask), per block over a strided set of 64-row chunks, written as
-// block partials; k_reduce_partials sums blocks in order (deterministic).
+// Weight gradient of the network's wide layers, dW[K x OUT] = X^T (dY * mask)
+// and db = sum rows of (dY * mask): an FP32 contraction over the rows (60k x 64
+// x 64 per layer), so FP32 FMA issue bounds it (7 us at 60k rows), not the
+// 31 MB it reads. A block takes 64-row chunks in turn (the next one loading
+// into registers behind the products); 8 x 4 outputs per thread, so a row
+// costs three 16-byte shared loads per 32 FMAs, and G groups of threads share
+// the chunk's rows. One output per thread with two shared loads per FMA (k_wgrad
+// below) took 190 us at 60k rows. Groups, then blocks are added in order.
+constexpr int kWideRows = 64;
+
+template <int K, int OUT>
+__global__ void __launch_bounds__(256) k_wgrad_wide(const float *x, const float *dy,
+                                                    const float *ymask, int32_t rows,
+                                                    float *partials) {
+    constexpr int TX = OUT / 4, NT = TX * (K / 8), G = 256 / NT;
+    constexpr int XV = kWideRows * K / 4, DV = kWideRows * OUT / 4;  // float4 per chunk
+    constexpr int XN = (XV + 255) / 256, DN = (DV + 255) / 256;
+    __shared__ float4 sm[XV + DV];
+    float4 *xs = sm, *ds = sm + XV;
+    const int tid = threadIdx.x, g = tid / NT, t = tid % NT, tx = t % TX, ty = t / TX;
+    float4 xr[XN], dr[DN];
+    auto fetch = [&](int64_t c0) {
+        const int cr = static_cast<int>(rows - c0 < kWideRows ? rows - c0 : kWideRows);
+        const float4 *xp = reinterpret_cast<const float4 *>(x + c0 * K);
+        const float4 *dp = reinterpret_cast<const float4 *>(dy + c0 * OUT);
+        const float4 *mp = reinterpret_cast<const float4 *>(ymask + c0 * OUT);
+#pragma unroll
+        for (int q = 0; q < XN; ++q) {
+            const int i = tid + q * 256;
+            xr[q] = i < cr * K / 4 ? __ldg(xp + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int q = 0; q < DN; ++q) {
+            const int i = tid + q * 256;
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (i < cr * OUT / 4) {
+                v = __ldg(dp + i);
+                if (ymask) {
+                    const float4 m = __ldg(mp + i);
+                    if (!(m.x > 0.0f)) v.x = 0.0f;
+                    if (!(m.y > 0.0f)) v.y = 0.0f;
+                    if (!(m.z > 0.0f)) v.z = 0.0f;
+                    if (!(m.w > 0.0f)) v.w = 0.0f;
+                }
+            }
+            dr[q] = v;
+        }
+    };
+    float acc[8][4], db[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * kWideRows;
+    int64_t c0 = static_cast<int64_t>(blockIdx.x) * kWideRows;
+    if (c0 < rows) fetch(c0);
+    for (; c0 < rows; c0 += step) {
+        __syncthreads();  // the chunk before is used up
+#pragma unroll
+        for (int q = 0; q < XN; ++q)
+            if (tid + q * 256 < XV) xs[tid + q * 256] = xr[q];
+#pragma unroll
+        for (int q = 0; q < DN; ++q)
+            if (tid + q * 256 < DV) ds[tid + q * 256] = dr[q];
+        __syncthreads();
+        if (c0 + step < rows) fetch(c0 + step);
+#pragma unroll 4
+        for (int r = g; r < kWideRows; r += G) {
+            const float4 xa = xs[r * (K / 4) + ty * 2], xb = xs[r * (K / 4) + ty * 2 + 1];
+            const float4 d = ds[r * TX + tx];
+            const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                acc[i][0] = __fmaf_rn(xv[i], d.x, acc[i][0]);
+                acc[i][1] = __fmaf_rn(xv[i], d.y, acc[i][1]);
+                acc[i][2] = __fmaf_rn(xv[i], d.z, acc[i][2]);
+                acc[i][3] = __fmaf_rn(xv[i], d.w, acc[i][3]);
+            }
+            if (ty == 0) {
+                db[0] += d.x;
+                db[1] += d.y;
+                db[2] += d.z;
+                db[3] += d.w;
+            }
+        }
+    }
+    // groups in order through shared memory, group 0 keeps the sums
+    float *buf = reinterpret_cast<float *>(sm);
+    static_assert((K + 1) * OUT <= 4 * (XV + DV), "");
+    for (int q = 1; q < G; ++q) {
+        __syncthreads();
+        if (g == q) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) buf[(ty * 8 + i) * OUT + tx * 4 + j] = acc[i][j];
+            if (ty == 0)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) buf[K * OUT + tx * 4 + j] = db[j];
+        }
+        __syncthreads();
+        if (g == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] += buf[(ty * 8 + i) * OUT + tx * 4 + j];
+            if (ty == 0)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) db[j] += buf[K * OUT + tx * 4 + j];
+        }
+    }
+    if (g != 0) return;
+    float *out = partials + static_cast<int64_t>(blockIdx.x) * (K + 1) * OUT;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<float4 *>(out + (ty * 8 + i) * OUT + tx * 4) =
+            make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    if (ty == 0)
+        *reinterpret_cast<float4 *>(out + K * OUT + tx * 4) =
+            make_float4(db[0], db[1], db[2], db[3]);
+}
+
+// The same for the head's layers (18 x 16 and 16 x 1), whose widths do not
+// tile, per block over a strided set of 64-row chunks; k_reduce_partials sums
+// blocks in order (deterministic).
 __global__ void __launch_bounds__(256) k_wgrad(const float *x, int32_t k, const float *dy,
                                                 const float *ymask, int32_t out, int32_t rows,
                                                 float *partials) {
@@ -647,12 +797,24 @@ __global__ void __launch_bounds__(256) k_wgrad(const float *x, int32_t k, const 
     }
 }
 
-__global__ void k_reduce_partials(const float *partials, int blocks, int nout, float *dw,
-                                  float *db, int kout) {
-    const int oi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (oi >= nout) return;
+// Adds the blocks' partials to the gradient: 32 outputs per CTA, eight groups of
+// lanes each summing every eighth block, then the groups in order (one thread
+// walking all blocks of its output took 19 us).
+__global__ void __launch_bounds__(256) k_reduce_partials(const float *partials, int blocks,
+                                                         int nout, float *dw, float *db,
+                                                         int kout) {
+    __shared__ float sums[8][32];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const int oi = blockIdx.x * 32 + lane;
     float s = 0.0f;
-    for (int b = 0; b < blocks; ++b) s += partials[static_cast<int64_t>(b) * nout + oi];
+    if (oi < nout)
+#pragma unroll 4
+        for (int b = g; b < blocks; b += 8) s += partials[static_cast<int64_t>(b) * nout + oi];
+    sums[g][lane] = s;
+    __syncthreads();
+    if (g != 0 || oi >= nout) return;
+#pragma unroll
+    for (int q = 1; q < 8; ++q) s += sums[q][lane];
     if (oi < kout)
         dw[oi] += s;
     else if (db)
@@ -1103,7 +1265,7 @@ struct ktg_learned {
 
 namespace {
 
-constexpr int kWgradBlocks = 256;
+constexpr int kWgradBlocks = 296;  // two blocks of k_wgrad_wide per SM
 
 int lerr(ktg_learned *h, int code, const std::string &m) {
     if (h) h->err = m;
@@ -1229,9 +1391,18 @@ int wgrad(ktg_learned *h, const float *x, int k, const float *dy, const float *y
     if (rows <= 0) return KTG_OK;
     const int nout = k * out + out;
     const int blocks = static_cast<int>(std::min<int64_t>(kWgradBlocks, (rows + 63) / 64));
-    ktg::learned::k_wgrad<<<blocks, 256, 0, h->stream>>>(x, k, dy, ymask, out,
-                                                         static_cast<int32_t>(rows), h->wpart);
-    ktg::learned::k_reduce_partials<<<(nout + 255) / 256, 256, 0, h->stream>>>(
+    const int32_t r = static_cast<int32_t>(rows);
+    auto aligned16 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+    const bool wide = aligned16(x) && aligned16(dy) && aligned16(ymask);
+    if (wide && k == HID && out == HID)
+        ktg::learned::k_wgrad_wide<HID, HID><<<blocks, 256, 0, h->stream>>>(x, dy, ymask, r, h->wpart);
+    else if (wide && k == NFEAT && out == HID)
+        ktg::learned::k_wgrad_wide<NFEAT, HID><<<blocks, 256, 0, h->stream>>>(x, dy, ymask, r, h->wpart);
+    else if (wide && k == HID && out == PROJ)
+        ktg::learned::k_wgrad_wide<HID, PROJ><<<blocks, 256, 0, h->stream>>>(x, dy, ymask, r, h->wpart);
+    else
+        ktg::learned::k_wgrad<<<blocks, 256, 0, h->stream>>>(x, k, dy, ymask, out, r, h->wpart);
+    ktg::learned::k_reduce_partials<<<(nout + 31) / 32, 256, 0, h->stream>>>(
         h->wpart, blocks, nout, h->g + wofs, bofs >= 0 ? h->g + bofs : nullptr, k * out);
     h->launches += 2;
     KTG_LCUDA(h, cudaGetLastError());
@@ -1262,15 +1433,15 @@ int trunk_forward(ktg_learned *h, ktg_ctx *c, int64_t n) {
     if ((rc = dense(h, h->x, NFEAT, nullptr, L.W_in, 0, L.b_in, cell_act(h, 0), n, HID, true,
                     false, false, nullptr)))
         return rc;
-    const int wpb = 8;  // warps per block for the aggregations
+    const int wpb = 16;  // rows per block of the aggregations
     for (int l = 0; l < LAYERS; ++l) {
-        ktg::learned::k_cells_to_nets<<<static_cast<int>((N + wpb - 1) / wpb), 32 * wpb, 0, h->stream>>>(
+        ktg::learned::k_cells_to_nets<<<static_cast<int>((N + wpb - 1) / wpb), ktg::learned::kAggLanes * wpb, 0, h->stream>>>(
             c->net_start, c->pin_var, c->net_mov, static_cast<int32_t>(N), cell_act(h, l),
             net_act(h, l));
         if ((rc = dense(h, net_act(h, l), HID, nullptr, L.Wa[l], 0, L.ba[l], net_act(h, 3 + l), N,
                         HID, true, false, false, nullptr)))
             return rc;
-        ktg::learned::k_nets_to_cells<<<static_cast<int>((n + wpb - 1) / wpb), 32 * wpb, 0, h->stream>>>(
+        ktg::learned::k_nets_to_cells<<<static_cast<int>((n + wpb - 1) / wpb), ktg::learned::kAggLanes * wpb, 0, h->stream>>>(
             c->pin_start, c->pin_ref, static_cast<int32_t>(n), net_act(h, 3 + l), cell_act(h, 4 + l));
         if ((rc = dense(h, cell_act(h, l), HID, cell_act(h, 4 + l), L.Wb[l], L.Wc[l], L.bb[l],
                         cell_act(h, l + 1), n, HID, true, false, false, nullptr)))
@@ -1357,7 +1528,7 @@ int trunk_backward(ktg_learned *h, ktg_ctx *c, int64_t n) {
     if ((rc = wgrad(h, cell_act(h, LAYERS), HID, h->dp, nullptr, PROJ, n, L.P, -1))) return rc;
     if ((rc = dense(h, h->dp, PROJ, nullptr, L.P, 0, -1, h->dh, n, HID, false, true, false, nullptr)))
         return rc;
-    const int wpb = 8;
+    const int wpb = 16;  // rows per block of the aggregations
     for (int l = LAYERS - 1; l >= 0; --l) {
         // h_{l+1} = relu(h_l Wb + g_l Wc + bb): dz = dh * (h_{l+1} > 0)
         const float *hout = cell_act(h, l + 1);
@@ -1371,7 +1542,7 @@ int trunk_backward(ktg_learned *h, ktg_ctx *c, int64_t n) {
                         hout)))
             return rc;
         // g = mean nets->cells (e): de = T(dg)
-        ktg::learned::k_nets_to_cells_T<<<static_cast<int>((N + wpb - 1) / wpb), 32 * wpb, 0, h->stream>>>(
+        ktg::learned::k_nets_to_cells_T<<<static_cast<int>((N + wpb - 1) / wpb), ktg::learned::kAggLanes * wpb, 0, h->stream>>>(
             c->net_start, c->pin_var, c->pin_start, static_cast<int32_t>(N), h->dg, h->de);
         ++h->launches;
         // e = relu(m Wa + ba): dza = de * (e > 0)
@@ -1381,7 +1552,7 @@ int trunk_backward(ktg_learned *h, ktg_ctx *c, int64_t n) {
                         eout)))
             return rc;
         // m = mean cells->nets (h_l): dh_prev += T(dm)
-        ktg::learned::k_cells_to_nets_T<<<static_cast<int>((n + wpb - 1) / wpb), 32 * wpb, 0, h->stream>>>(
+        ktg::learned::k_cells_to_nets_T<<<static_cast<int>((n + wpb - 1) / wpb), ktg::learned::kAggLanes * wpb, 0, h->stream>>>(
             c->pin_start, c->pin_ref, c->net_mov, static_cast<int32_t>(n), h->dm, h->dh2, 1);
         ++h->launches;
         std::swap(h->dh, h->dh2);

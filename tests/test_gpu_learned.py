@@ -237,3 +237,33 @@ def true_resid_of(s, v):
     av = s["diag"] * v
     np.add.at(av, rows, s["val"] * v[s["col"]])
     return np.linalg.norm(s["rhs"] - av) / np.linalg.norm(s["rhs"])
+
+
+@pytest.mark.parametrize("cells,nets", [(40, 64), (64, 63), (129, 130), (18945, 18943)])
+def test_wide_gradients_and_aggregations_at_tile_edges(cells, nets, gpu_ctx, port_built):
+    """Weight gradients by 64-row chunks (fewer rows than one, exact chunks, one
+    row more, and one more than every block takes at once) and half-warp
+    aggregations (nets of more than 16 pins) against the float64 oracle, FP32
+    layers: the 2e-3 of the gradient test above."""
+    from ktplace_b200 import netlist, synth
+    from ktplace_b200.learned import Learned
+    raw = synth.generate(synth.spec_tiny(seed=cells, cells=cells, nets=nets, pads=16, rows=12))
+    nl = netlist.flatten(raw)
+    assert nl.num_nets < 100 or np.diff(nl.net_start).max() > 16
+    x, y = synth.seed_positions(raw, nl.num_movable, 3)
+    gpu_ctx.upload_netlist(nl)
+    fx, fy = nl.floors()
+    gpu_ctx.build_b2b(x, y, 0.0, None, None, fx, fy)
+    params = lr.init_params(7)
+    params["P"] *= 20.0
+    flat = lr.flatten(params).astype(np.float32)
+    learned = Learned(0, seed=1)
+    learned.set_params(flat)
+    learned.set_option("probes", 2)
+    learned.set_option("tensor_cores", 0)
+    p64 = lr.unflatten(flat.astype(np.float64))
+    L_ref, g_ref, _ = lr.loss_and_grad(p64, gpu_ctx.system(0), nl, k=2, seed=11)
+    L_gpu, g_gpu = learned.loss_grad(gpu_ctx, 0, seed=11)
+    learned.close()
+    assert abs(L_gpu - L_ref) <= 1e-4 * abs(L_ref)
+    assert rel(g_gpu.astype(np.float64), lr.flatten(g_ref)) <= 2e-3
