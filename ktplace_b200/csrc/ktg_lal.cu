@@ -750,104 +750,435 @@ struct Stripes {
 
 // ---- one CTA per block (or half) for the level-by-level path ------------------------
 //
-// Blocks too large for the one-CTA subtree have die-sized boxes: their row
-// loops are split over the CTA's threads and the profile is built by thread 0
-// from chunks staged in shared memory (the order of its sums is the
-// reference's).
+// Blocks too large for the one-CTA subtree have die-sized boxes: tens of
+// thousands of profile steps and hundreds of obstacles. Latency bounds these
+// kernels (a level has one or a few blocks), so everything that may run in any
+// order runs on all threads; what keeps the reference's order is one addition
+// per profile edge, a chain of thread 0 through shared memory. With the whole
+// walk (heights, edge tests, stores to global memory), the obstacle list and
+// the stripe loop on thread 0, the two kernels took 470 + 140 us a level on the
+// 211k-cell design.
 
-constexpr int kStage = 1024;
+constexpr int kWideT = 512;                   // threads of the per-block kernels
+constexpr int kPer = 8;                       // profile steps per thread and round
+constexpr int kRound = kWideT * kPer;         // and so edges per round at most
+constexpr int kProfSmem = 6144;               // profile edges kept in shared memory
+constexpr int kCutSmem = 4096;                // obstacle cuts sorted there
+// profile (edges, prefix), and a round's stage (three arrays) or the cuts, their
+// input order, their prefix and the stripe counts
+constexpr size_t kCtaStage = sizeof(double) * 3 * kRound;
+constexpr size_t kHalfStripesSmem = sizeof(double) * 2 * kProfSmem + kCtaStage;
+static_assert(kCtaStage >= (2 * sizeof(double) + 2 * sizeof(int32_t)) * kCutSmem, "");
 
-// Builds the profile of `box` into e/p (global). Returns the edge count on
-// thread 0.
+template <typename T, class Op>
+__device__ T cta_excl(T v, T zero, T &total, Op op) {
+    __shared__ T ws[kWideT / 32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    T inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const T t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc = op(t, inc);
+    }
+    T exc = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane == 0) exc = zero;
+    if (lane == 31) ws[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+        T w = lane < nw ? ws[lane] : zero;
+        for (int o = 1; o < 32; o <<= 1) {
+            const T t = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w = op(t, w);
+        }
+        if (lane < nw) ws[lane] = w;
+    }
+    __syncthreads();
+    total = ws[nw - 1];
+    const T before = wid > 0 ? ws[wid - 1] : zero;
+    __syncthreads();
+    return op(before, exc);
+}
+
+// Running sums of area[0, cnt) onto sum in order, in place; one thread. The
+// next eight terms load behind the additions.
+__device__ double chain_sums(double *area, int cnt, double sum) {
+    double2 *v = reinterpret_cast<double2 *>(area);  // 16-byte aligned
+    const int whole = cnt >> 3;
+    double2 n0, n1, n2, n3;
+    if (whole) n0 = v[0], n1 = v[1], n2 = v[2], n3 = v[3];
+    for (int i = 0; i < whole; ++i, v += 4) {
+        double2 c0 = n0, c1 = n1, c2 = n2, c3 = n3;
+        if (i + 1 < whole) n0 = v[4], n1 = v[5], n2 = v[6], n3 = v[7];
+        c0.x = sum = sum + c0.x;
+        c0.y = sum = sum + c0.y;
+        c1.x = sum = sum + c1.x;
+        c1.y = sum = sum + c1.y;
+        c2.x = sum = sum + c2.x;
+        c2.y = sum = sum + c2.y;
+        c3.x = sum = sum + c3.x;
+        c3.y = sum = sum + c3.y;
+        v[0] = c0, v[1] = c1, v[2] = c2, v[3] = c3;
+    }
+    for (int i = whole * 8; i < cnt; ++i) area[i] = sum = sum + area[i];
+    return sum;
+}
+
+// Exponent of the lowest set bit of a nonzero finite double.
+__device__ __forceinline__ int low_bit(double v) {
+    const unsigned long long u = static_cast<unsigned long long>(__double_as_longlong(v));
+    const int ex = static_cast<int>((u >> 52) & 0x7ff);
+    const unsigned long long m = (u & 0xfffffffffffffull) | (ex ? 0x10000000000000ull : 0ull);
+    return (ex ? ex : 1) - 1075 + __ffsll(static_cast<long long>(m)) - 1;
+}
+
+// Edges and areas of a round, staged; writes them out with running prefixes.
+// n: edges so far; plast: the last prefix (thread 0).
+__device__ void cta_flush_edges(const double *se, double *sa, int cnt, int64_t &n, double &plast,
+                                double *e, double *p) {
+    __syncthreads();
+    if (threadIdx.x == 0) plast = chain_sums(sa, cnt, plast);
+    __syncthreads();
+    for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+        e[n + i] = se[i];
+        p[n + i] = sa[i];
+    }
+    n += cnt;
+    __syncthreads();
+}
+
+// Vertical profile: the heights before each step are prefix sums of the dh.
+// Exact: every dh is a multiple of 2^g and no partial sum needs more than 53
+// bits above 2^g, so the reference's sequential double sums round nowhere and
+// 64-bit integer sums, in any order, are the same values; checked on every
+// partial sum. False (nothing usable written) when the check fails; with
+// Exact = false thread 0 adds the heights in order.
+template <bool Exact>
+__device__ bool cta_profile_steps(double lo, const Key *steps, int64_t nsteps, int g, double *stage,
+                                  int64_t &n, double &plast, double &elast, double *e, double *p) {
+    double *se = stage, *sa = stage + kRound, *sh = stage + 2 * kRound;
+    const double scale = Exact ? ldexp(1.0, -g) : 1.0, unit = Exact ? ldexp(1.0, g) : 1.0;
+    long long carry = 0;
+    double height = 0.0;  // Exact = false, thread 0
+    for (int64_t c0 = 0; c0 < nsteps; c0 += kRound) {
+        const int64_t k0 = c0 + static_cast<int64_t>(threadIdx.x) * kPer;
+        double at[kPer], dh[kPer];
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const Key q = k0 + u < nsteps ? steps[k0 + u] : Key{0ull, 0ull};
+            at[u] = unord(q.a);
+            dh[u] = k0 + u < nsteps ? unord(q.b) : 0.0;
+        }
+        double prev = k0 > 0 && k0 < nsteps ? unord(steps[k0 - 1].a) : lo;
+        bool bad = false;
+        long long run = 0;
+        if constexpr (Exact) {
+            long long local = 0, total;
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) local += __double2ll_rn(dh[u] * scale);
+            run = carry + cta_excl<long long>(local, 0ll, total,
+                                              [](long long x, long long y) { return x + y; });
+            carry += total;
+        } else {
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) sh[threadIdx.x * kPer + u] = dh[u];
+            __syncthreads();
+            if (threadIdx.x == 0)
+                for (int i = 0; i < kRound; ++i) {
+                    const double d = sh[i];
+                    sh[i] = height;
+                    height += d;
+                }
+            __syncthreads();
+        }
+        int cnt = 0;
+        double ar[kPer];
+        unsigned take = 0;
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            if (k0 + u < nsteps) {
+                const double h = Exact ? static_cast<double>(run) * unit : sh[threadIdx.x * kPer + u];
+                if (at[u] > prev) {
+                    ar[u] = h * (at[u] - prev);
+                    take |= 1u << u;
+                    ++cnt;
+                }
+                prev = at[u];
+                if constexpr (Exact) {
+                    run += __double2ll_rn(dh[u] * scale);
+                    bad = bad || run > (1ll << 53) || run < -(1ll << 53);
+                }
+            }
+        }
+        int total_cnt;
+        int at_edge = cta_excl<int>(cnt, 0, total_cnt, [](int x, int y) { return x + y; });
+        if (Exact && __syncthreads_or(bad)) return false;
+#pragma unroll
+        for (int u = 0; u < kPer; ++u)
+            if ((take >> u) & 1u) {
+                se[at_edge] = at[u];
+                sa[at_edge] = ar[u];
+                ++at_edge;
+            }
+        cta_flush_edges(se, sa, total_cnt, n, plast, e, p);
+    }
+    if (nsteps > 0) elast = ref_max(lo, unord(steps[nsteps - 1].a));
+    return true;
+}
+
+// Builds the profile of `box` into e/p (global), as build_profile_from does.
+// Returns the edge count to every thread.
 __device__ int64_t cta_build_profile(const Free &F, const double *box, bool v, const Key *steps,
                                      int64_t nsteps, double *e, double *p, double *stage) {
     const double lx = box[0], ly = box[1], ux = box[2], uy = box[3];
     const double lo = v ? lx : ly, hi = v ? ux : uy;
     const int tid = threadIdx.x, nt = blockDim.x;
     int64_t n = 1;
-    double elast = lo, plast = 0.0, height = 0.0;
-    auto extend = [&](double to, double area) {
-        if (to > elast) {
-            plast = plast + area;
-            elast = to;
-            e[n] = to;
-            p[n] = plast;
-            ++n;
-        }
-    };
+    double elast = lo, plast = 0.0;
     if (tid == 0) {
         e[0] = lo;
         p[0] = 0.0;
     }
     if (v) {
-        // chunk c + 1 is loaded into registers while thread 0 walks chunk c
-        constexpr int kPer = kStage / kT;
-        Key nxt[kPer];
-        auto fetch = [&](int64_t c0) {
-#pragma unroll
-            for (int u = 0; u < kPer; ++u) {
-                const int64_t k = c0 + u * nt + tid;
-                nxt[u] = k < nsteps ? steps[k] : Key{0ull, 0ull};
-            }
-        };
-        fetch(0);
-        for (int64_t c0 = 0; c0 < nsteps; c0 += kStage) {
-            const int cnt = static_cast<int>(nsteps - c0 < kStage ? nsteps - c0 : kStage);
-            __syncthreads();  // the previous chunk is consumed
-#pragma unroll
-            for (int u = 0; u < kPer; ++u) {
-                const int i = u * nt + tid;
-                if (i < cnt) {
-                    stage[2 * i] = unord(nxt[u].a);
-                    stage[2 * i + 1] = unord(nxt[u].b);
-                }
-            }
-            __syncthreads();
-            fetch(c0 + kStage);
-            if (tid == 0)
-                for (int i = 0; i < cnt; ++i) {
-                    const double at = stage[2 * i], dh = stage[2 * i + 1];
-                    extend(at, height * (at - elast));
-                    height += dh;
-                }
+        // the steps' granularity and size
+        int g = 2000;
+        double big = 0.0;
+        for (int64_t k = tid; k < nsteps; k += nt) {
+            const double dh = unord(steps[k].b);
+            if (dh != 0.0) g = min(g, low_bit(dh));
+            big = fmax(big, fabs(dh));
         }
-        __syncthreads();
+        cta_excl<int>(g, 2000, g, [](int x, int y) { return min(x, y); });
+        cta_excl<double>(big, 0.0, big, [](double x, double y) { return fmax(x, y); });
+        bool done = false;
+        if (g > -1000 && g < 1000 && ldexp(big, -g) * static_cast<double>(nsteps) < 4.0e18)
+            done = cta_profile_steps<true>(lo, steps, nsteps, g, stage, n, plast, elast, e, p);
+        if (!done) {
+            n = 1;
+            plast = 0.0;
+            cta_profile_steps<false>(lo, steps, nsteps, 0, stage, n, plast, elast, e, p);
+        }
     } else {
+        double *se = stage, *sa = stage + kRound;
         int32_t r0, r1;
         box_rows(F, box, r0, r1);
-        for (int32_t c0 = r0; c0 < r1; c0 += kStage) {
-            const int cnt = min(kStage, r1 - c0);
-            for (int i = tid; i < cnt; i += nt) {  // Row::getLength(b.getX())
-                const int32_t r = c0 + i;
-                double total = 0.0;
+        for (int32_t c0 = r0; c0 < r1; c0 += nt) {
+            const int32_t r = c0 + tid;
+            bool on = false;
+            double a = 0.0, z = 0.0, total = 0.0;
+            if (r < r1) {
+                a = ref_max(lo, F.rowy[2 * r]);
+                z = ref_min(hi, F.rowy[2 * r + 1]);
+                on = z > a;
+                // Row::getLength(b.getX())
                 const int64_t end = F.rowspan[r + 1];
-                for (int64_t q = first_span(F, r, lx); q < end && F.spans[2 * q] < ux; ++q)
-                    total += ref_max(0.0, ref_min(ux, F.spans[2 * q + 1]) - ref_max(lx, F.spans[2 * q]));
-                stage[i] = total;
+                if (on)
+                    for (int64_t q = first_span(F, r, lx); q < end && F.spans[2 * q] < ux; ++q)
+                        total += ref_max(0.0, ref_min(ux, F.spans[2 * q + 1]) -
+                                                  ref_max(lx, F.spans[2 * q]));
             }
-            __syncthreads();
-            if (tid == 0)
-                for (int i = 0; i < cnt; ++i) {
-                    const int32_t r = c0 + i;
-                    const double a = ref_max(lo, F.rowy[2 * r]);
-                    const double z = ref_min(hi, F.rowy[2 * r + 1]);
-                    if (z > a) {
-                        extend(a, 0.0);
-                        extend(z, stage[i] * (z - a));
-                    }
-                }
-            __syncthreads();
+            // a row extends the profile where it lies above all before it
+            double top;
+            double last = cta_excl<double>(on ? z : elast, elast, top,
+                                           [](double x, double y) { return y > x ? y : x; });
+            last = last > elast ? last : elast;
+            const bool ta = on && a > last;
+            if (ta) last = a;
+            const bool tz = on && z > last;
+            int cnt;
+            int at = cta_excl<int>((ta ? 1 : 0) + (tz ? 1 : 0), 0, cnt,
+                                   [](int x, int y) { return x + y; });
+            if (ta) {
+                se[at] = a;
+                sa[at++] = 0.0;
+            }
+            if (tz) {
+                se[at] = z;
+                sa[at] = total * (z - a);
+            }
+            if (top > elast) elast = top;
+            cta_flush_edges(se, sa, cnt, n, plast, e, p);
         }
     }
+    const bool more = hi > elast;
     if (tid == 0) {
-        extend(hi, 0.0);
-        if (n == 1) {
+        if (more) {
+            e[n] = hi;
+            p[n] = plast + 0.0;
+        } else if (n == 1) {
             e[1] = hi;
             p[1] = 0.0;
-            n = 2;
         }
     }
+    if (more || n == 1) ++n;
+    __syncthreads();
     return n;
+}
+
+// make_stripes with a CTA: the cuts gathered and sorted by all threads, each
+// interval between two cuts (independent of the others) split by one thread,
+// once to count its stripes and once to write them. Up to kCutSmem cuts.
+// Returns the number of stripes, or -1 as make_stripes does; -2 for too many
+// cuts (the caller runs make_stripes).
+__device__ int64_t cta_make_stripes(const Prof &room, const double *box, bool v, double cell_area,
+                                    double region_room, double frac, double limit_density,
+                                    const double *obst, int32_t K, double cutline, bool below,
+                                    double *stage, int64_t cap, double *sa, double *sb,
+                                    double *scap) {
+    constexpr int kDepth = 64;
+    __shared__ int s_nc;
+    double *c = stage, *before = stage + kCutSmem;
+    int32_t *idx = reinterpret_cast<int32_t *>(before + kCutSmem);
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const double lo = v ? box[0] : box[1], hi = v ? box[2] : box[3];
+    __syncthreads();
+    if (tid == 0) {
+        c[0] = lo;
+        c[1] = hi;
+        idx[0] = 0;
+        idx[1] = 1;
+        s_nc = 2;
+    }
+    __syncthreads();
+    for (int32_t o = tid; o < K; o += nt) {
+        const double *ob = obst + 4 * o;
+        if (ob[2] <= box[0] || ob[0] >= box[2] || ob[3] <= box[1] || ob[1] >= box[3]) continue;
+        for (int k = 0; k < 2; ++k) {
+            const double x = ob[(v ? 0 : 1) + 2 * k];
+            if (!(x > lo && x < hi)) continue;
+            const int q = atomicAdd(&s_nc, 1);
+            if (q < kCutSmem) {
+                c[q] = x;
+                idx[q] = 2 + 2 * o + k;
+            }
+        }
+    }
+    __syncthreads();
+    int nc = s_nc;
+    if (nc > kCutSmem) return -2;
+    // sort by (value, input order), as the stable insertion sort leaves them
+    int P = 2;
+    while (P < nc) P <<= 1;
+    for (int i = nc + tid; i < P; i += nt) {
+        c[i] = INFINITY;
+        idx[i] = 0x7fffffff;
+    }
+    __syncthreads();
+    for (int k = 2; k <= P; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int t = tid; t < (P >> 1); t += nt) {
+                const int i = 2 * j * (t / j) + (t % j), q = i + j;
+                const double x = c[i], y = c[q];
+                const int32_t xi = idx[i], yi = idx[q];
+                const bool gt = y < x || (y == x && yi < xi);
+                if (gt == ((i & k) == 0)) {
+                    c[i] = y;
+                    c[q] = x;
+                    idx[i] = yi;
+                    idx[q] = xi;
+                }
+            }
+            __syncthreads();
+        }
+    // unique, in place: kPer consecutive entries per thread
+    {
+        const int per = (nc + nt - 1) / nt;
+        const int b = min(tid * per, nc), e = min(b + per, nc);
+        double keep[kCutSmem / kWideT];
+        int cnt = 0;
+        for (int i = b; i < e; ++i)
+            if (i == 0 || !(c[i - 1] == c[i])) keep[cnt++] = c[i];
+        int total;
+        const int at = cta_excl<int>(cnt, 0, total, [](int x, int y) { return x + y; });
+        for (int i = 0; i < cnt; ++i) c[at + i] = keep[i];
+        nc = total;
+        __syncthreads();
+    }
+    for (int i = tid; i < nc; i += nt) before[i] = room.before(c[i]);
+    const double whole = room.total();
+    const double limit = frac * (region_room > 0.0 ? region_room : whole);
+    const double fill = whole > 0.0 ? ref_min(limit_density, cell_area / whole) : limit_density;
+    __syncthreads();
+    // The stripes of interval i (between cuts i - 1 and i), in order, to
+    // put(index, start, end, room); the count, or -1 when cap is exceeded
+    // with `first` stripes before them.
+    auto interval = [&](int i, int64_t first, auto put) -> int64_t {
+        double a = c[i - 1], ba = before[i - 1];
+        double stk[kDepth], stkb[kDepth];
+        int top = 0;
+        int64_t ns = first;
+        stk[top] = c[i];
+        stkb[top] = before[i];
+        ++top;
+        while (top > 0) {
+            const double b = stk[top - 1], bb = stkb[top - 1];
+            const double here = bb - ba;
+            double mid = 0.0;
+            bool cut = here > limit;
+            if (cut) {
+                mid = room.coordinate_at(ba + 0.5 * here);
+                cut = mid > a && mid < b;
+            }
+            if (cut) {
+                if (top == kDepth || ns + top + 1 > cap) return -1;
+                stk[top] = mid;
+                stkb[top] = room.before(mid);
+                ++top;
+            } else {
+                if (ns >= cap) return -1;
+                put(ns, a, b, here);
+                ++ns;
+                --top;
+                a = b;
+                ba = bb;
+            }
+        }
+        return ns - first;
+    };
+    const int per = (nc - 1 + nt - 1) / nt;
+    const int b = 1 + min(tid * per, nc - 1), e = min(b + per, nc);
+    int cnt = 0;
+    bool bad = false;
+    for (int i = b; i < e && !bad; ++i) {
+        const int64_t k = interval(i, 0, [](int64_t, double, double, double) {});
+        if (k < 0) bad = true;
+        else cnt += static_cast<int>(k);
+    }
+    int total;
+    int64_t at = cta_excl<int>(cnt, 0, total, [](int x, int y) { return x + y; });
+    if (!bad)
+        for (int i = b; i < e && !bad; ++i) {
+            const int64_t k = interval(i, at, [&](int64_t q, double x, double y, double here) {
+                sa[q] = x;
+                sb[q] = y;
+                scap[q] = fill * here;
+            });
+            if (k < 0) bad = true;
+            else at += k;
+        }
+    if (__syncthreads_or(bad)) return -1;
+    const int64_t ns = total;
+    if (!below) {
+        auto swap_at = [&](int64_t i, int64_t j) {
+            double t = sa[i]; sa[i] = sa[j]; sa[j] = t;
+            t = sb[i]; sb[i] = sb[j]; sb[j] = t;
+            t = scap[i]; scap[i] = scap[j]; scap[j] = t;
+        };
+        for (int64_t i = tid; i < ns / 2; i += nt) swap_at(i, ns - 1 - i);
+        __syncthreads();
+        // restore the original order inside each run of equal distance
+        auto from = [&](int64_t i) { return 0.5 * (sa[i] + sb[i]) - cutline; };
+        bool run = false;
+        for (int64_t i = tid; i + 1 < ns; i += nt) run = run || from(i) == from(i + 1);
+        if (__syncthreads_or(run) && tid == 0)
+            for (int64_t r = 0; r < ns;) {
+                const double f = from(r);
+                int64_t q = r + 1;
+                while (q < ns && from(q) == f) ++q;
+                for (int64_t i = r, j = q - 1; i < j; ++i, --j) swap_at(i, j);
+                r = q;
+            }
+        __syncthreads();
+    }
+    return ns;
 }
 
 // Profile steps of each block (half = 0) or half box (half = 1), one CTA
@@ -875,16 +1206,18 @@ __global__ void __launch_bounds__(kT) k_steps_cta(Level L, Free F, int half, con
 }
 
 // One CTA per block: profile, cutline, half boxes, half bounds.
-__global__ void __launch_bounds__(kT) k_block_cut_cta(Level L, Free F, const int64_t *soff,
-                                                      const Key *steps, const int64_t *nsteps,
-                                                      const int64_t *eoff, double *pe, double *pp,
-                                                      int64_t *hbound) {
-    __shared__ double stage[2 * kStage];
+__global__ void __launch_bounds__(kWideT) k_block_cut_cta(Level L, Free F, const int64_t *soff,
+                                                         const Key *steps, const int64_t *nsteps,
+                                                         const int64_t *eoff, double *pe, double *pp,
+                                                         int64_t *hbound) {
+    extern __shared__ __align__(16) double wide_smem[];
+    __shared__ double hb[8];
     const int blk = blockIdx.x;
     const bool v = L.vert[blk] != 0;
     const double *box = L.box + 4 * blk;
     double *e = pe + eoff[blk], *p = pp + eoff[blk];
-    const int64_t n = cta_build_profile(F, box, v, steps + soff[blk], nsteps[blk], e, p, stage);
+    const int64_t n =
+        cta_build_profile(F, box, v, steps + soff[blk], nsteps[blk], e, p, wide_smem);
     if (threadIdx.x == 0) {
         const Prof room{e, p, n};
         const double cell_area = L.cut[blk];
@@ -893,55 +1226,51 @@ __global__ void __launch_bounds__(kT) k_block_cut_cta(Level L, Free F, const int
         const double cut = room.total() > 0.0 ? room.coordinate_at(share * room.total())
                                               : lo + share * (hi - lo);
         L.cut[blk] = cut;
-        double *lb = L.half_box + 8 * blk, *hb = lb + 4;
-        for (int k = 0; k < 4; ++k) lb[k] = hb[k] = box[k];
-        (v ? lb[2] : lb[3]) = cut;
-        (v ? hb[0] : hb[1]) = cut;
+        for (int k = 0; k < 4; ++k) hb[k] = hb[4 + k] = box[k];
+        hb[v ? 2 : 3] = cut;
+        hb[4 + (v ? 0 : 1)] = cut;
+        for (int k = 0; k < 8; ++k) L.half_box[8 * blk + k] = hb[k];
     }
     __syncthreads();
-    for (int side = 0; side < 2; ++side) {
-        const double *bx = L.half_box + 8 * blk + 4 * side;
-        long long k = 0;  // obstacles overlapping the half box
-        for (int32_t o = threadIdx.x; o < F.K; o += blockDim.x) {
-            const double *ob = F.obst + 4 * o;
+    int k[2] = {0, 0};  // obstacles overlapping each half box
+    for (int32_t o = threadIdx.x; o < F.K; o += blockDim.x) {
+        const double *ob = F.obst + 4 * o;
+        for (int side = 0; side < 2; ++side) {
+            const double *bx = hb + 4 * side;
             if (ob[2] <= bx[0] || ob[0] >= bx[2] || ob[3] <= bx[1] || ob[1] >= bx[3]) continue;
-            ++k;
+            ++k[side];
         }
-        long long total;
-        block_excl64(k, total);
-        if (threadIdx.x == 0) {
-            int64_t st, ed;
-            profile_bound(F, bx, v, st, ed);
-            hbound[4 * blk + 2 * side] = st;
-            hbound[4 * blk + 2 * side + 1] = ed + 2 * total + 2;  // profile edges, obstacle cuts
-        }
+    }
+    int total[2];
+    for (int side = 0; side < 2; ++side)
+        cta_excl<int>(k[side], 0, total[side], [](int x, int y) { return x + y; });
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < 64) {  // a warp per side
+        const int side = threadIdx.x >> 5;
+        int64_t st, ed;
+        profile_bound(F, hb + 4 * side, v, st, ed);
+        hbound[4 * blk + 2 * side] = st;
+        hbound[4 * blk + 2 * side + 1] = ed + 2 * total[side] + 2;  // profile edges, obstacle cuts
     }
 }
 
 // One CTA per half: profile, stripes (getStripes), fill state. A profile of
-// up to kProfSmem edges is copied to shared memory before the stripe loop,
+// up to kProfSmem edges is copied to shared memory before the stripes are cut,
 // whose profile lookups are then shared-memory binary searches.
-constexpr int kProfSmem = 6144;
-constexpr size_t kHalfStripesSmem = sizeof(double) * 2 * kProfSmem;
-
-__global__ void __launch_bounds__(kT) k_half_stripes_cta(Level L, Free F, const int64_t *soff,
-                                                         const Key *steps, const int64_t *nsteps,
-                                                         const int64_t *eoff, double *pe, double *pp,
-                                                         const int64_t *cap_over, double frac,
-                                                         double limit_density, Stripes S,
-                                                         int *status) {
-    __shared__ double stage[2 * kStage];
-    __shared__ long long s_ns, s_n;
-    extern __shared__ double prof[];  // [2 * kProfSmem]
+__global__ void __launch_bounds__(kWideT) k_half_stripes_cta(Level L, Free F, const int64_t *soff,
+                                                            const Key *steps, const int64_t *nsteps,
+                                                            const int64_t *eoff, double *pe,
+                                                            double *pp, const int64_t *cap_over,
+                                                            double frac, double limit_density,
+                                                            Stripes S, int *status) {
+    extern __shared__ __align__(16) double wide_smem[];
+    __shared__ long long s_ns;
+    double *prof = wide_smem, *stage = wide_smem + 2 * kProfSmem;
     const int h = blockIdx.x;
     const int blk = h >> 1, side = h & 1;
     const bool v = L.vert[blk] != 0;
     const double *box = L.half_box + 4 * h;
     double *e = pe + eoff[h], *p = pp + eoff[h];
-    const int64_t n0 = cta_build_profile(F, box, v, steps + soff[h], nsteps[h], e, p, stage);
-    if (threadIdx.x == 0) s_n = n0;
-    __syncthreads();
-    const int64_t n = s_n;
+    const int64_t n = cta_build_profile(F, box, v, steps + soff[h], nsteps[h], e, p, stage);
     const bool local = n <= kProfSmem;
     if (local) {
         for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -951,22 +1280,26 @@ __global__ void __launch_bounds__(kT) k_half_stripes_cta(Level L, Free F, const 
         __syncthreads();
     }
     const int64_t so = S.off[h];
-    if (threadIdx.x == 0) {
-        const Prof room{local ? prof : e, local ? prof + kProfSmem : p, n};
-        const double cell_area = side ? L.high_area[blk] : L.low_area[blk];
-        // cuts live after the profile in the global scratch
-        int64_t ns = make_stripes(room, box, v, cell_area, L.room[blk], frac, limit_density,
-                                  F.obst, F.K, L.cut[blk], side == 0, p + n, cap_over[h],
-                                  S.a + so, S.b + so, S.cap + so);
-        if (ns < 0) {
-            atomicCAS(status, kStatusOk, kStatusCapacity);
-            ns = 0;
-        }
-        S.count[h] = static_cast<int32_t>(ns);
-        s_ns = ns;
+    const Prof room{local ? prof : e, local ? prof + kProfSmem : p, n};
+    const double cell_area = side ? L.high_area[blk] : L.low_area[blk];
+    int64_t ns = cta_make_stripes(room, box, v, cell_area, L.room[blk], frac, limit_density, F.obst,
+                                  F.K, L.cut[blk], side == 0, stage, cap_over[h], S.a + so,
+                                  S.b + so, S.cap + so);
+    if (ns == -2) {  // more cuts than shared memory holds
+        if (threadIdx.x == 0)
+            // cuts live after the profile in the global scratch
+            s_ns = make_stripes(room, box, v, cell_area, L.room[blk], frac, limit_density, F.obst,
+                                F.K, L.cut[blk], side == 0, p + n, cap_over[h], S.a + so, S.b + so,
+                                S.cap + so);
+        __syncthreads();
+        ns = s_ns;
     }
-    __syncthreads();
-    for (int64_t q = threadIdx.x; q < s_ns; q += blockDim.x) {
+    if (ns < 0) {
+        if (threadIdx.x == 0) atomicCAS(status, kStatusOk, kStatusCapacity);
+        ns = 0;
+    }
+    if (threadIdx.x == 0) S.count[h] = static_cast<int32_t>(ns);
+    for (int64_t q = threadIdx.x; q < ns; q += blockDim.x) {
         S.used[so + q] = 0.0;
         S.lo[so + q] = ~0ull;
         S.hi[so + q] = 0ull;
@@ -1017,7 +1350,7 @@ __global__ void k_fill(Level L, CellsDev C, const int32_t *cells, Stripes S, int
 // starts go to `sbeg`.
 __global__ void __launch_bounds__(kT) k_fill_fx(Level L, Stripes S, const long long *pre,
                                                 double inv_scale, int32_t *sbeg) {
-    __shared__ int32_t s_lo, s_hi, s_first;
+    __shared__ int32_t s_first;
     const int32_t h = blockIdx.x;
     const int32_t blk = h >> 1;
     const int32_t b = L.b[blk], e = L.e[blk], mid = b + L.m[blk];
@@ -2179,7 +2512,7 @@ struct LalState {
     DevBuf<double> sstrp;
     DevBuf<unsigned long long> sstrlh;
     bool subtree_attr = false;
-    bool half_stripes_attr = false;
+    bool wide_attr = false;
     // counters of the last ktg_lal call (ktg_lal_stats)
     double stats[16] = {};
 };
@@ -2603,8 +2936,17 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
             }
             if ((r2 = seg_sort(c, s->steps.p, s->steps_tmp.p, ssegs, s->seg))) return r2;
             // 3. profile, cutline, half boxes and bounds
-            k_block_cut_cta<<<na, kT, 0, c->stream>>>(L, F, s->soff.p, s->steps.p, s->nsteps.p,
-                                                      s->eoff.p, s->pe.p, s->pp.p, s->hbound.p);
+            if (!s->wide_attr) {
+                KTG_CUDA(c, cudaFuncSetAttribute(k_block_cut_cta,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(kCtaStage)));
+                KTG_CUDA(c, cudaFuncSetAttribute(k_half_stripes_cta,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 static_cast<int>(kHalfStripesSmem)));
+                s->wide_attr = true;
+            }
+            k_block_cut_cta<<<na, kWideT, kCtaStage, c->stream>>>(
+                L, F, s->soff.p, s->steps.p, s->nsteps.p, s->eoff.p, s->pe.p, s->pp.p, s->hbound.p);
             ++c->launches;
             std::vector<int64_t> hbound(4 * na);
             KTG_CUDA(c, cudaMemcpyAsync(hbound.data(), s->hbound.p, sizeof(int64_t) * 4 * na,
@@ -2650,13 +2992,7 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
             if ((r2 = seg_sort(c, s->steps.p, s->steps_tmp.p, ssegs, s->seg))) return r2;
             // 4. stripes per half (profile arrays: e in pe, p and the cuts in pp)
             Stripes S{s->stoff.p, s->scount.p, s->sa.p, s->sb.p, s->scap.p, s->sused.p, s->slo.p, s->shi.p};
-            if (!s->half_stripes_attr) {
-                KTG_CUDA(c, cudaFuncSetAttribute(k_half_stripes_cta,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(kHalfStripesSmem)));
-                s->half_stripes_attr = true;
-            }
-            k_half_stripes_cta<<<2 * na, kT, kHalfStripesSmem, c->stream>>>(
+            k_half_stripes_cta<<<2 * na, kWideT, kHalfStripesSmem, c->stream>>>(
                 L, F, s->hsoff.p, s->steps.p, s->hnsteps.p, s->heoff.p, s->pe.p, s->pp.p,
                 s->hbound.p, frac, c->density_limit, S, c->status);
             // 5. fill order, fill, stripe ranges, positions

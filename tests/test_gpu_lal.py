@@ -177,3 +177,43 @@ def test_simpl_mirror_legalizes_in_place(gpu_ctx):
     legalizer.legalize(px, py)
     ox, oy = run_oracle(nl, 24, 1.0, x, y)
     assert np.array_equal(px, ox) and np.array_equal(py, oy)
+
+
+@pytest.mark.parametrize("subtree", [0, 2048])
+@pytest.mark.parametrize("kind", ["uneven_rows", "many_spans", "many_obstacles"])
+def test_lal_profile_branches(kind, subtree, gpu_ctx):
+    """Free spaces that take the other branch of the level-by-level kernels:
+    rows whose heights do not sum exactly (heights added in order), more steps
+    and edges than one round of a CTA takes, more obstacle cuts than it sorts
+    in shared memory. Bit-identical positions, as everywhere."""
+    raw = synth.generate(synth.spec_tiny(seed=8, macros=2, cells=420, nets=450))
+    nl = netlist.flatten(raw)
+    x, y = clustered(raw, nl.num_movable, 31, 0.15)
+    g = grid.build_grid(nl, 8, 1.0)
+    fs = grid.build_free_space(nl)
+    rng = np.random.default_rng(4)
+    lx, ly, ux, uy = fs.die
+    if kind == "uneven_rows":
+        edge = np.concatenate([[0.0], np.cumsum(rng.uniform(11.0, 13.0, fs.row_y.shape[0]))])
+        fs.row_y = np.stack([edge[:-1], edge[1:]], 1)
+    elif kind == "many_spans":
+        cut = np.linspace(lx, ux, 421)
+        per = np.stack([cut[:-1], cut[1:] - 0.03], 1)
+        fs.spans = np.concatenate([per + 0.001 * r for r in range(fs.row_y.shape[0])])
+        fs.row_span = np.arange(fs.row_y.shape[0] + 1, dtype=np.int64) * per.shape[0]
+    else:
+        ox, oy = rng.uniform(lx, ux, 2300), rng.uniform(ly, uy, 2300)
+        fs.obstacles = np.stack([ox, oy, ox + 0.5, oy + 0.5], 1)
+    gpu_ctx.set_option("lal_subtree_cells", subtree)
+    gpu_ctx.set_option("lal_exact_sums", 1)
+    gpu_ctx.upload_netlist(nl)
+    gpu_ctx.set_grid(g)
+    gpu_ctx.set_free_space(fs)
+    gx, gy = gpu_ctx.lal(x, y)
+    gpu_ctx.set_option("lal_subtree_cells", 2048)
+    gd = dict(origin=(g.origin_x, g.origin_y), dx=g.dx, dy=g.dy, nx=g.nx, ny=g.ny, avail=g.avail)
+    L = lal_ref.LAL(nl.width, nl.height, gd, lal_ref.free_rows(fs.row_y, fs.row_span, fs.spans),
+                    fs.obstacles, fs.die, g.density_limit)
+    ox, oy = L.legalize(x, y)
+    assert np.array_equal(gx, np.array(ox)) and np.array_equal(gy, np.array(oy))
+    assert np.mean(gx != x) > 0.1
