@@ -51,7 +51,8 @@ constexpr int kBuckets = 2 + 3 * kMaxWidth;
 constexpr int kGroups = 5;                 // records a lane polls: at most 160 blocks
 constexpr int kRecord = 4;                 // words of a block's record
 constexpr int kSets = 4;
-constexpr int kSmallRows = 256;            // rows a block of a small system owns
+constexpr int kSmallRows = 256;            // rows a block of a small system owns, at least
+constexpr int kSmallBlocks = 48;           // and blocks it has, at most
 constexpr size_t kSmemBudget = 124 * 1024;
 // A partial sum that has not been written yet. Arithmetic produces only the
 // canonical NaN, and a sum that carries this pattern is replaced by it.
@@ -766,10 +767,16 @@ int launch_solve_sliced(ktg_ctx *c, double *x, double *y, double tol, int64_t ma
     A.n = static_cast<int32_t>(c->sys_n);
     const int64_t total = 2 * c->sys_n;
     // Blocks: one up to kThreads rows (its sums need no barrier: 5.1 us a step
-    // at 600 rows, 7.5 us on three blocks), else one per kSmallRows rows until
-    // every SM has one (2,000 rows: 7.0 us a step; 9.4 with 1,024 rows a block).
-    // Half the threads serve blocks that small as well.
-    const int64_t rows = total <= kThreads ? kThreads : kSmallRows;
+    // at 600 rows, 7.5 us on three blocks). Then kSmallBlocks of kSmallRows to
+    // kThreads rows (2,000 rows: 7.0 us a step with 256 rows a block, 9.4 with
+    // 1,024; 24,000 rows: 9.7 and 10.1), and beyond that kThreads rows a block:
+    // a third of the SMs serves a small system as well as all of them, and
+    // leaves room for solves on other streams.
+    const int64_t rows =
+        total <= kThreads
+            ? kThreads
+            : std::min<int64_t>(kThreads, std::max<int64_t>(kSmallRows,
+                                                            (total + kSmallBlocks - 1) / kSmallBlocks));
     const int64_t most = std::min(c->num_sms, 32 * kGroups);
     const int grid = static_cast<int>(
         std::max<int64_t>(1, std::min<int64_t>(most, (total + rows - 1) / rows)));
