@@ -39,6 +39,7 @@
 #include <array>
 #include <chrono>
 #include <cmath>
+#include <cstring>
 #include <limits>
 #include <vector>
 
@@ -1473,6 +1474,7 @@ constexpr int kSortCap = 4096;      // entries of the sort buffer (steps and pro
 constexpr int kMaxSub = 1024;       // sub-blocks of one level
 constexpr int kObstLocal = 256;     // obstacles overlapping the block
 constexpr int64_t kStripeCap = 8192;
+constexpr int kNearDesc = 12;       // sub-blocks of a level described in shared memory
 constexpr int kRowsLocal = 512;     // free-space rows staged in shared memory
 constexpr int kSpansLocal = 1280;   // and their spans
 constexpr size_t kSubSmem = sizeof(unsigned long long) * 2 * kSortCap +
@@ -1486,7 +1488,22 @@ struct SubTask {
     double box[4];
     double room;
     int32_t b, e, level, vert;
+    int32_t r0, r1;  // rows its box can meet (r1 < 0: all, to be searched)
 };
+
+// Work queue of one launch. A block of more than kHandOff cells is split once
+// and its halves go back to the queue, where idle CTAs pick them up: a batch
+// has a few blocks of up to 2,048 cells, and finishing each in one CTA left
+// the other SMs idle for ten levels. CTAs draw tickets; a ticket past the tail
+// waits (with a time limit) until its slot is filled or nothing is pending.
+struct SubQueue {
+    int32_t head, tail, pending, nfail, timeout;
+};
+constexpr int64_t kQueueHead = 64;              // bytes before the tasks
+constexpr int kHandSlots = 48;                  // queue slots per block handed in
+constexpr int kHandOff = 160;
+constexpr uint64_t kQueueTimeoutNs = 2000000000ull;
+constexpr int kLongRun = 32;                    // cells at one distance ranked by counting
 
 struct SubDesc {
     double box[4];
@@ -1499,10 +1516,13 @@ struct SubDesc {
 };
 
 struct SubArgs {
-    const SubTask *tasks;
-    int32_t ntasks;
-    int32_t *fail;           // [ntasks] 1: left for the level-by-level path
-    const int32_t *cells;    // position -> cell id
+    SubTask *tasks;          // [cap], the first ntasks filled in
+    int32_t ntasks, cap;
+    SubQueue *queue;
+    unsigned *ready;         // [cap] == epoch: slot filled
+    unsigned epoch;
+    int2 *failed;            // [cap] (task, reason) of tasks left for the level-by-level path
+    int32_t *cells;          // position -> cell id
     CellsDev C;
     Free F;
     SubDesc *desc;           // [grid * 2 * kMaxSub]
@@ -1598,6 +1618,139 @@ __device__ void sort_segments(unsigned long long *k0, unsigned long long *k1, ui
         }
     }
     __syncthreads();
+}
+
+// Where entry i of a buffer of 8- or 4-byte entries lies while it is merged: a
+// thread's four outputs are consecutive, and unswizzled its 8-byte accesses
+// would meet seven other lanes' banks.
+template <typename V>
+__device__ __forceinline__ int swizzled(int i) {
+    return sizeof(V) == 8 ? i ^ ((i >> 4) & 15) : i ^ ((i >> 5) & 31);
+}
+
+// Sorts positions [0, tot), tot <= kSub, by (tag, key, val) with the whole CTA:
+// four entries per thread sorted in registers, then merges of sorted runs, each
+// thread finding its four outputs by a binary search along the merge path. tag
+// ascends with the position, so entries move only among equal tags and every
+// position keeps its tag; without Tags it is one segment. load(p, key, val)
+// gives the entries; key and val have room for 2 kSub and end with the sorted
+// ones in [0, tot).
+template <bool Tags, typename V, class Load>
+__device__ void merge_sort(unsigned long long *key, V *val, uint32_t *tag, int tot, Load load) {
+    int P = 4, levels = 0;
+    while (P < tot) P <<= 1, ++levels;
+    int buf = levels & 1;
+    const int p0 = 4 * threadIdx.x;
+    const bool on = p0 < P;
+    auto less_eq = [&](uint32_t ti, unsigned long long ki, V vi, uint32_t tj, unsigned long long kj,
+                       V vj) {
+        const bool le = (ki < kj) | ((ki == kj) & (vi <= vj));
+        return Tags ? (ti < tj) | ((ti == tj) & le) : le;
+    };
+    if (on) {
+        unsigned long long k[4];
+        V v[4];
+        uint32_t t[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            k[u] = ~0ull;
+            v[u] = static_cast<V>(~0ull);
+            t[u] = 0u;
+            if (p0 + u < tot) load(p0 + u, k[u], v[u]);
+            else if (Tags) tag[p0 + u] = ~0u;
+            if (Tags) t[u] = tag[p0 + u];
+        }
+        auto cas = [&](int i, int j) {
+            if (t[i] == t[j] && (k[j] < k[i] || (k[j] == k[i] && v[j] < v[i]))) {
+                const unsigned long long x = k[i];
+                k[i] = k[j];
+                k[j] = x;
+                const V y = v[i];
+                v[i] = v[j];
+                v[j] = y;
+            }
+        };
+        cas(0, 1);
+        cas(2, 3);
+        cas(0, 2);
+        cas(1, 3);
+        cas(1, 2);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = p0 + u;
+            key[buf * kSub + (levels ? swizzled<unsigned long long>(i) : i)] = k[u];
+            val[buf * kSub + (levels ? swizzled<V>(i) : i)] = v[u];
+        }
+    }
+    for (int w = 4; w < P; w <<= 1, buf ^= 1) {
+        if (w >= 128) __syncthreads();  // up to there a warp merges its own entries
+        else __syncwarp();
+        if (!on) continue;
+        const unsigned long long *sk = key + buf * kSub;
+        const V *sv = val + buf * kSub;
+        unsigned long long *dk = key + (buf ^ 1) * kSub;
+        V *dv = val + (buf ^ 1) * kSub;
+        auto kat = [&](int i) { return sk[swizzled<unsigned long long>(i)]; };
+        auto vat = [&](int i) { return sv[swizzled<V>(i)]; };
+        auto tat = [&](int i) { return Tags ? tag[i] : 0u; };
+        const int base = p0 & ~(2 * w - 1), d = p0 - base;
+        int lo = max(0, d - w), hi = min(d, w);
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1, i = base + mid, j = base + w + d - 1 - mid;
+            if (less_eq(tat(i), kat(i), vat(i), tat(j), kat(j), vat(j))) lo = mid + 1;
+            else hi = mid;
+        }
+        int i = base + lo, j = base + w + d - lo;
+        const int ei = base + w, ej = base + 2 * w;
+        unsigned long long ki = 0, kj = 0;
+        V vi = 0, vj = 0;
+        uint32_t ti = 0u, tj = 0u;
+        if (i < ei) ki = kat(i), vi = vat(i), ti = tat(i);
+        if (j < ej) kj = kat(j), vj = vat(j), tj = tat(j);
+        const bool last = 2 * w == P;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool left = j >= ej || (i < ei && less_eq(ti, ki, vi, tj, kj, vj));
+            const int q = p0 + u;
+            dk[last ? q : swizzled<unsigned long long>(q)] = left ? ki : kj;
+            dv[last ? q : swizzled<V>(q)] = left ? vi : vj;
+            if (left) {
+                if (++i < ei) ki = kat(i), vi = vat(i), ti = tat(i);
+            } else {
+                if (++j < ej) kj = kat(j), vj = vat(j), tj = tat(j);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Ranks of positions [0, tot), tot <= kSubThreads, inside their segments by
+// counting: `per` threads share a position and each compares every per-th entry
+// of its segment, so short segments cost little (160 cells: 3k cycles against
+// 19k for the merges above, whose steps are chains of shared-memory reads).
+// seg(p, b, e): the segment of p, empty for positions that stay; entry q is
+// (key(q), val(q)), ties by the position. Returns the new position of *p, in
+// the first of its threads; -1 in the others.
+template <class Seg, class KeyOf, class ValOf>
+__device__ int counted_position(int tot, int &p, Seg seg, KeyOf key, ValOf val) {
+    int per = 1;
+    while (per < 32 && 2 * per * tot <= kSubThreads) per <<= 1;
+    p = threadIdx.x / per;
+    const int sub = threadIdx.x & (per - 1);
+    int b = 0, e = 0, rank = 0;
+    if (p < tot) seg(p, b, e);
+    if (e > b) {
+        const unsigned long long k = key(p);
+        const auto v = val(p);
+#pragma unroll 4
+        for (int q = b + sub; q < e; q += per) {
+            const unsigned long long kq = key(q);
+            const auto vq = val(q);
+            rank += static_cast<int>((kq < k) | ((kq == k) & ((vq < v) | ((vq == v) & (q < p)))));
+        }
+    }
+    for (int d = per >> 1; d > 0; d >>= 1) rank += __shfl_xor_sync(0xffffffffu, rank, d);
+    return p < tot && sub == 0 ? (e > b ? b + rank : p) : -1;
 }
 
 // Exclusive scan of buf[0, n) in place; returns the total to every thread.
@@ -1831,6 +1984,275 @@ __device__ int64_t team_build_profile(const Team &tm, const Free &F, const doubl
     return n;
 }
 
+// The prefix of a profile whose edges' areas are in p[1, n): one lane, the next
+// eight areas loading behind the additions.
+__device__ __forceinline__ void chain_prefix(double *p, int64_t n) {
+    double sum = 0.0, next[8];
+    int64_t i = 1;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) next[u] = i + u < n ? p[i + u] : 0.0;
+    for (; i < n; i += 8) {
+        double cur[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) cur[u] = next[u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) next[u] = i + 8 + u < n ? p[i + 8 + u] : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            sum = sum + cur[u];
+            if (i + u < n) p[i + u] = sum;
+        }
+    }
+}
+
+// team_build_profile by a whole warp: 32 steps or rows at a time, edges packed
+// by ballots, and only the prefix chained by one lane. Heights are exact
+// integer sums as in cta_profile_steps (checked before anything is
+// overwritten), else the team version takes over.
+__device__ int64_t warp_build_profile(const Team &tm, const Free &F, const double *box, bool v,
+                                      unsigned long long *k0, unsigned long long *k1, int o,
+                                      int nsteps, int len) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    double *e = reinterpret_cast<double *>(k0 + o), *p = reinterpret_cast<double *>(k1 + o);
+    const double lo = v ? box[0] : box[1], hi = v ? box[2] : box[3];
+    int64_t n = 1;
+    double elast = lo;
+    if (v) {
+        int g = 2000;
+        double big = 0.0;
+        for (int k = lane; k < nsteps; k += 32) {
+            const double dh = unord(k1[o + 2 + k]);
+            if (dh != 0.0) g = min(g, low_bit(dh));
+            big = fmax(big, fabs(dh));
+        }
+        for (int d = 16; d > 0; d >>= 1) {
+            g = min(g, __shfl_xor_sync(0xffffffffu, g, d));
+            big = fmax(big, __shfl_xor_sync(0xffffffffu, big, d));
+        }
+        bool ok = nsteps == 0 || (g > -1000 && g < 1000 &&
+                                  ldexp(big, -g) * static_cast<double>(nsteps) < 4.0e18);
+        const double scale = ok ? ldexp(1.0, -g) : 0.0, unit = ok ? ldexp(1.0, g) : 0.0;
+        auto incl = [&](long long x) {
+            for (int d = 1; d < 32; d <<= 1) {
+                const long long t = __shfl_up_sync(0xffffffffu, x, d);
+                if (lane >= d) x += t;
+            }
+            return x;
+        };
+        long long carry = 0;
+        for (int c0 = 0; ok && c0 < nsteps; c0 += 32) {
+            const int k = c0 + lane;
+            const long long s =
+                carry + incl(k < nsteps ? __double2ll_rn(unord(k1[o + 2 + k]) * scale) : 0);
+            ok = !__any_sync(0xffffffffu, s > (1ll << 53) || s < -(1ll << 53));
+            carry = __shfl_sync(0xffffffffu, s, 31);
+        }
+        if (!ok) return team_build_profile(tm, F, box, v, k0, k1, o, nsteps, len);
+        carry = 0;
+        double prev_last = lo;
+        for (int c0 = 0; c0 < nsteps; c0 += 32) {
+            const int k = c0 + lane;
+            const bool on = k < nsteps;
+            const double at = on ? unord(k0[o + 2 + k]) : 0.0;
+            const long long h = on ? __double2ll_rn(unord(k1[o + 2 + k]) * scale) : 0;
+            const long long inc = incl(h);
+            double prev = __shfl_up_sync(0xffffffffu, at, 1);
+            if (lane == 0) prev = prev_last;
+            const double area = static_cast<double>(carry + inc - h) * unit * (at - prev);
+            const unsigned m = __ballot_sync(0xffffffffu, on && at > prev);
+            if ((m >> lane) & 1u) {
+                e[n + __popc(m & below)] = at;
+                p[n + __popc(m & below)] = area;
+            }
+            n += __popc(m);
+            carry += __shfl_sync(0xffffffffu, inc, 31);
+            prev_last = __shfl_sync(0xffffffffu, at, min(31, nsteps - 1 - c0));
+            __syncwarp();
+        }
+        elast = ref_max(lo, prev_last);
+    } else {
+        const double lx = box[0], ux = box[2];
+        int32_t r0, r1;
+        box_rows(F, box, r0, r1);
+        for (int32_t c0 = r0; c0 < r1; c0 += 32) {
+            const int32_t r = c0 + lane;
+            bool on = false;
+            double a = 0.0, z = 0.0, total = 0.0;
+            if (r < r1) {
+                a = ref_max(lo, F.rowy[2 * r]);
+                z = ref_min(hi, F.rowy[2 * r + 1]);
+                on = z > a;
+                const int64_t end = F.rowspan[r + 1];
+                if (on)
+                    for (int64_t q = first_span(F, r, lx); q < end && F.spans[2 * q] < ux; ++q)
+                        total += ref_max(0.0, ref_min(ux, F.spans[2 * q + 1]) -
+                                                  ref_max(lx, F.spans[2 * q]));
+            }
+            double top = on ? z : elast;  // running maximum of the row tops
+            for (int d = 1; d < 32; d <<= 1) {
+                const double t = __shfl_up_sync(0xffffffffu, top, d);
+                if (lane >= d && t > top) top = t;
+            }
+            double last = __shfl_up_sync(0xffffffffu, top, 1);
+            if (lane == 0 || !(last > elast)) last = elast;
+            const bool ta = on && a > last;
+            if (ta) last = a;
+            const bool tz = on && z > last;
+            const unsigned ma = __ballot_sync(0xffffffffu, ta), mz = __ballot_sync(0xffffffffu, tz);
+            int64_t at = n + __popc(ma & below) + __popc(mz & below);
+            if (ta) {
+                e[at] = a;
+                p[at++] = 0.0;
+            }
+            if (tz) {
+                e[at] = z;
+                p[at] = total * (z - a);
+            }
+            n += __popc(ma) + __popc(mz);
+            const double t = __shfl_sync(0xffffffffu, top, 31);
+            if (t > elast) elast = t;
+        }
+    }
+    const bool more = hi > elast;
+    if (lane == 0) {
+        e[0] = lo;
+        p[0] = 0.0;
+        if (more || n == 1) {
+            e[n] = hi;
+            p[n] = 0.0;
+        }
+    }
+    if (more || n == 1) ++n;
+    __syncwarp();
+    if (lane == 0) chain_prefix(p, n);
+    __syncwarp();
+    return n;
+}
+
+// make_stripes by a warp for at most 32 cuts and stripes (-2: more): cuts
+// ranked, all intervals halved at once until none is above the limit. `buf`
+// holds 128 doubles of shared memory.
+__device__ int64_t warp_make_stripes(const Prof &room, const double *box, bool v, double cell_area,
+                                     double region_room, double frac, double limit_density,
+                                     const double *obst, int32_t K, double cutline, bool below,
+                                     int64_t cap, double *sa, double *sb, double *scap,
+                                     double *buf) {
+    const int lane = threadIdx.x & 31;
+    const unsigned before_me = (1u << lane) - 1u;
+    const double lo = v ? box[0] : box[1], hi = v ? box[2] : box[3];
+    int32_t *order = reinterpret_cast<int32_t *>(buf + 32);
+    int nc = 2;
+    if (lane < 2) {
+        buf[lane] = lane ? hi : lo;
+        order[lane] = lane;
+    }
+    for (int32_t o0 = 0; o0 < K; o0 += 32) {
+        const int32_t o = o0 + lane;
+        bool in = o < K;
+        const double *ob = obst + 4 * (in ? o : 0);
+        in = in && !(ob[2] <= box[0] || ob[0] >= box[2] || ob[3] <= box[1] || ob[1] >= box[3]);
+        for (int k = 0; k < 2; ++k) {
+            const double x = ob[(v ? 0 : 1) + 2 * k];
+            const bool put = in && x > lo && x < hi;
+            const unsigned m = __ballot_sync(0xffffffffu, put);
+            if (nc + __popc(m) > 32) return -2;
+            if (put) {
+                buf[nc + __popc(m & before_me)] = x;
+                order[nc + __popc(m & before_me)] = 2 + 2 * o + k;
+            }
+            nc += __popc(m);
+        }
+    }
+    __syncwarp();
+    // rank by (value, input order), drop repeats
+    double c = lane < nc ? buf[lane] : 0.0;
+    const int32_t ord_me = lane < nc ? order[lane] : 0;
+    int rank = 0;
+    for (int j = 0; j < nc; ++j) {
+        const double cj = __shfl_sync(0xffffffffu, c, j);
+        const int32_t oj = __shfl_sync(0xffffffffu, ord_me, j);
+        if (cj < c || (cj == c && oj < ord_me)) ++rank;
+    }
+    __syncwarp();
+    if (lane < nc) buf[rank] = c;
+    __syncwarp();
+    c = lane < nc ? buf[lane] : 0.0;
+    const double left = __shfl_up_sync(0xffffffffu, c, 1);
+    const unsigned keep = __ballot_sync(0xffffffffu, lane < nc && (lane == 0 || !(left == c)));
+    __syncwarp();
+    if ((keep >> lane) & 1u) buf[__popc(keep & before_me)] = c;
+    nc = __popc(keep);
+    __syncwarp();
+    c = lane < nc ? buf[lane] : 0.0;
+    const double at = lane < nc ? room.before(c) : 0.0;
+    const double whole = room.total();
+    const double limit = frac * (region_room > 0.0 ? region_room : whole);
+    const double fill = whole > 0.0 ? ref_min(limit_density, cell_area / whole) : limit_density;
+    // interval of this lane, in ascending order
+    int count = nc - 1;
+    double a = c, b = __shfl_down_sync(0xffffffffu, c, 1);
+    double ba = at, bb = __shfl_down_sync(0xffffffffu, at, 1);
+    unsigned done = 0u;
+    double *wa = buf, *wb = buf + 32, *wba = buf + 64, *wbb = buf + 96;
+    for (;;) {
+        const double here = bb - ba;
+        bool cut = lane < count && !((done >> lane) & 1u) && here > limit;
+        double mid = 0.0;
+        if (cut) {
+            mid = room.coordinate_at(ba + 0.5 * here);
+            cut = mid > a && mid < b;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, cut);
+        if (!m) break;
+        if (count + __popc(m) > 32) return -2;
+        const int to = lane + __popc(m & before_me);
+        __syncwarp();
+        if (lane < count) {
+            wa[to] = a;
+            wba[to] = ba;
+            if (cut) {
+                const double bm = room.before(mid);
+                wb[to] = wa[to + 1] = mid;
+                wbb[to] = wba[to + 1] = bm;
+                wb[to + 1] = b;
+                wbb[to + 1] = bb;
+            } else {
+                wb[to] = b;
+                wbb[to] = bb;
+            }
+        }
+        done = __reduce_or_sync(0xffffffffu, lane < count && !cut ? 1u << to : 0u);
+        count += __popc(m);
+        __syncwarp();
+        if (lane < count) {
+            a = wa[lane];
+            b = wb[lane];
+            ba = wba[lane];
+            bb = wbb[lane];
+        }
+    }
+    if (count > cap) return -1;
+    int to = lane;
+    if (!below) {  // farthest first: reversed, runs of equal distance in order
+        const double f = 0.5 * (a + b) - cutline;
+        const double pf = __shfl_up_sync(0xffffffffu, f, 1);
+        const unsigned same = __ballot_sync(0xffffffffu, lane > 0 && lane < count && pf == f);
+        const unsigned upto = 0xffffffffu >> (31 - lane);
+        const int rs = 31 - __clz(~same & upto);
+        const unsigned next = ~same & ~upto;
+        const int re = next ? min(__ffs(next) - 1, count) : count;
+        to = (count - re) + (lane - rs);
+    }
+    if (lane < count) {
+        sa[to] = a;
+        sb[to] = b;
+        scap[to] = fill * (bb - ba);
+    }
+    __syncwarp();
+    return count;
+}
+
 __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned long long *k0 = reinterpret_cast<unsigned long long *>(smem);
@@ -1842,46 +2264,118 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
     double *lrowy = obst + 4 * kObstLocal, *lspans = lrowy + 2 * kRowsLocal;
     int64_t *lrowspan = reinterpret_cast<int64_t *>(lspans + 2 * kSpansLocal);
     uint32_t *k2 = reinterpret_cast<uint32_t *>(lrowspan + kRowsLocal + 2);
+    uint32_t *v1 = reinterpret_cast<uint32_t *>(k1);  // local indices of sorted cells
     int32_t *gid = reinterpret_cast<int32_t *>(k2 + kSortCap);
     int32_t *at = gid + kSub, *sof = at + kSub, *scan = sof + kSub;
     int16_t *dof = reinterpret_cast<int16_t *>(scan + 2 * kMaxSub + 2);
     __shared__ int32_t warp_tmp[32];
     __shared__ long long w64[32];
-    __shared__ int s_fail, s_nobst, s_ncur, s_maxlen, s_maxsteps, s_c1;
+    __shared__ int s_fail, s_nobst, s_ncur, s_maxsteps, s_c1;
     const int tid = threadIdx.x, nt = blockDim.x;
-    SubDesc *const cur0 = A.desc + static_cast<size_t>(blockIdx.x) * 2 * kMaxSub;
+    __shared__ SubDesc near_desc[2][kNearDesc];  // levels of a few sub-blocks
+    __shared__ int s_task, s_slot;
+    SubDesc *const far_desc = A.desc + static_cast<size_t>(blockIdx.x) * 2 * kMaxSub;
     double *const scut = A.strp + static_cast<size_t>(blockIdx.x) * 4 * kStripeCap;
     double *const sta = scut + kStripeCap, *const stb = sta + kStripeCap;
     double *const stc = stb + kStripeCap;
-    unsigned long long *const slo = A.strlh + static_cast<size_t>(blockIdx.x) * 2 * kStripeCap;
-    unsigned long long *const shi = slo + kStripeCap;
+    unsigned long long *const glo = A.strlh + static_cast<size_t>(blockIdx.x) * 2 * kStripeCap;
+    unsigned long long *const ghi = glo + kStripeCap;
     const CellsDev &C = A.C;
-    auto centre = [&](int j, bool v) {
-        return v ? sx[j] + 0.5 * C.w[gid[j]] : sy[j] + 0.5 * C.h[gid[j]];
+    // a block of at most half the capacity keeps its cells' sizes behind their
+    // positions
+    bool near_sizes = false;
+    auto extent = [&](int j, bool v) {
+        return near_sizes ? (v ? sx : sy)[kSub / 2 + j] : v ? C.w[gid[j]] : C.h[gid[j]];
+    };
+    auto centre = [&](int j, bool v) { return (v ? sx : sy)[j] + 0.5 * extent(j, v); };
+    // the steps of regions [0, tot) by (x, dh), in place; span: a tag's steps
+    auto sort_steps = [&](int tot, auto span) {
+        int p;
+        const int to = counted_position(
+            tot, p,
+            [&](int q, int &b, int &e) {
+                span(k2[q], b, e);
+                if (q < b) b = e = 0;  // a pad stays
+            },
+            [&](int q) { return k0[q]; }, [&](int q) { return k1[q]; });
+        const unsigned long long x = to >= 0 ? k0[p] : 0ull, dh = to >= 0 ? k1[p] : 0ull;
+        __syncthreads();
+        if (to >= 0) {
+            k0[to] = x;
+            k1[to] = dh;
+        }
+        __syncthreads();
+    };
+    // profile steps in the sort buffer; a region's pads (0, 0) sort first
+    auto step_entry = [&](int p, unsigned long long &k, unsigned long long &v) {
+        k = k0[p];
+        v = k1[p];
     };
 
-    for (int task = blockIdx.x; task < A.ntasks; task += gridDim.x) {
-        const SubTask T = A.tasks[task];
-        const int size = T.e - T.b;
+    for (;;) {
+        __syncthreads();
         if (tid == 0) {
-            s_fail = size > kSub ? 1 : 0;
+            int got = -1;
+            const int t = atomicAdd(&A.queue->head, 1);
+            if (t < A.ntasks) {
+                got = t;
+            } else if (t < A.cap) {
+                const uint64_t deadline = global_timer_ns() + kQueueTimeoutNs;
+                for (;;) {
+                    if (ld_acquire_gpu(A.ready + t) == A.epoch) {
+                        got = t;
+                        break;
+                    }
+                    // nothing pending: no more slots will be filled
+                    if (ld_acquire_gpu(reinterpret_cast<unsigned *>(&A.queue->pending)) == 0u ||
+                        ld_relaxed_gpu(&A.queue->timeout) != 0)
+                        break;
+                    if (global_timer_ns() > deadline) {
+                        atomicExch(&A.queue->timeout, 1);
+                        break;
+                    }
+                    __nanosleep(100);
+                }
+            }
+            s_task = got;
+            s_fail = 0;
+            s_slot = -1;
             s_nobst = 0;
-            s_maxlen = 0;
             s_maxsteps = 0;
         }
         __syncthreads();
-        if (s_fail) {
-            if (tid == 0) A.fail[task] = 1;
-            __syncthreads();
+        const int task = s_task;
+        if (task < 0) return;
+        const SubTask T = A.tasks[task];
+        const int size = T.e - T.b;
+        if (size > kSub) {  // left alone
+            if (tid == 0) {
+                A.failed[atomicAdd(&A.queue->nfail, 1)] = make_int2(task, 1);
+                __threadfence();
+                atomicSub(&A.queue->pending, 1);
+            }
             continue;
         }
+        near_sizes = size <= kSub / 2;
+        // cells by id, so that the sorts below break ties by the local index
+        // (handed-off blocks come that way)
+        if (task < A.ntasks) {
+            merge_sort<false>(k0, v1, k2, size, [&](int p, unsigned long long &k, uint32_t &v) {
+                k = static_cast<unsigned long long>(A.cells[T.b + p]);
+                v = 0u;
+            });
+        }
         for (int j = tid; j < size; j += nt) {
-            const int32_t g = A.cells[T.b + j];
+            const int32_t g = task < A.ntasks ? static_cast<int32_t>(k0[j]) : A.cells[T.b + j];
             gid[j] = g;
             sx[j] = C.x[g];
             sy[j] = C.y[g];
             sa[j] = C.area[g];
             at[j] = j;
+            if (near_sizes) {
+                sx[kSub / 2 + j] = C.w[g];
+                sy[kSub / 2 + j] = C.h[g];
+            }
         }
         for (int o = tid; o < A.F.K; o += nt) {
             const double *ob = A.F.obst + 4 * o;
@@ -1892,7 +2386,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                 for (int q = 0; q < 4; ++q) obst[4 * k + q] = ob[q];
         }
         if (tid == 0) {
-            SubDesc &d = cur0[0];
+            SubDesc &d = near_desc[0][0];
             for (int q = 0; q < 4; ++q) d.box[q] = T.box[q];
             d.b = 0;
             d.e = size;
@@ -1901,63 +2395,65 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
             s_ncur = 1;
         }
         Free FL = A.F;
+        int32_t row0 = T.r0, rows = T.r1 - T.r0;
         {  // the rows overlapping the block, with their spans overlapping its x
-           // range, into shared memory (the only spans its sub-boxes can meet)
-            const int32_t r0 = first_row(A.F, T.box[1]);
-            int32_t lo = r0, hi = A.F.R;  // first row from r0 with y start >= uy
-            while (lo < hi) {
-                const int32_t mid = (lo + hi) >> 1;
-                if (A.F.rowy[2 * mid] < T.box[3]) lo = mid + 1;
-                else hi = mid;
+           // range, into shared memory (the only spans its sub-boxes can meet);
+           // a handed-off block takes the rows of the block it came from
+            if (T.r1 < 0) {
+                int32_t r1;
+                box_rows(A.F, T.box, row0, r1);
+                rows = r1 - row0;
             }
-            const int32_t nr = lo - r0;
-            if (nr <= kRowsLocal) {
-                for (int i = tid; i < nr; i += nt) {
-                    const int64_t f = first_span(A.F, r0 + i, T.box[0]);
-                    int64_t e = f;
-                    while (e < A.F.rowspan[r0 + i + 1] && A.F.spans[2 * e] < T.box[2]) ++e;
+            if (rows <= kRowsLocal) {
+                for (int i = tid; i < rows; i += nt) {
+                    const int64_t f = first_span(A.F, row0 + i, T.box[0]);
+                    int64_t e = f, hi = A.F.rowspan[row0 + i + 1];
+                    while (e < hi) {  // first span from f that starts at or past the box
+                        const int64_t mid = (e + hi) >> 1;
+                        if (A.F.spans[2 * mid] < T.box[2]) e = mid + 1;
+                        else hi = mid;
+                    }
                     scan[i] = static_cast<int32_t>(e - f);
                     lrowspan[i] = f;  // first span, global index (rebased below)
                 }
                 __syncthreads();
-                const int32_t ns = cta_scan(scan, nr, warp_tmp);
+                const int32_t ns = cta_scan(scan, rows, warp_tmp);
                 if (ns <= kSpansLocal) {
-                    for (int i = tid; i < nr; i += nt) {
+                    for (int i = tid; i < rows; i += nt) {
                         const int64_t f = lrowspan[i];
                         const int32_t o = scan[i];
-                        const int32_t cnt = (i + 1 < nr ? scan[i + 1] : ns) - o;
+                        const int32_t cnt = (i + 1 < rows ? scan[i + 1] : ns) - o;
                         for (int32_t q = 0; q < cnt; ++q) {
                             lspans[2 * (o + q)] = A.F.spans[2 * (f + q)];
                             lspans[2 * (o + q) + 1] = A.F.spans[2 * (f + q) + 1];
                         }
-                        lrowy[2 * i] = A.F.rowy[2 * (r0 + i)];
-                        lrowy[2 * i + 1] = A.F.rowy[2 * (r0 + i) + 1];
+                        lrowy[2 * i] = A.F.rowy[2 * (row0 + i)];
+                        lrowy[2 * i + 1] = A.F.rowy[2 * (row0 + i) + 1];
                     }
                     __syncthreads();
-                    for (int i = tid; i <= nr; i += nt) lrowspan[i] = i < nr ? scan[i] : ns;
+                    for (int i = tid; i <= rows; i += nt) lrowspan[i] = i < rows ? scan[i] : ns;
                     FL.rowy = lrowy;
                     FL.rowspan = lrowspan;
                     FL.spans = lspans;
-                    FL.R = nr;
+                    FL.R = rows;
                 }
             }
         }
         __syncthreads();
-        if (s_nobst > kObstLocal && tid == 0) s_fail = 1;  // too many obstacles
+        if (tid == 0 && s_nobst > kObstLocal) s_fail = 1;  // too many obstacles
         FL.obst = obst;
         FL.K = min(s_nobst, kObstLocal);
-        SubDesc *cur = cur0, *nxt = cur0 + kMaxSub;
-        for (;;) {
+        SubDesc *cur = near_desc[0], *nxt = near_desc[1];
+        for (int depth = 0;; ++depth) {
             __syncthreads();
             const int ncur = s_ncur;
             if (s_fail || ncur == 0) break;
-            // A. which sub-blocks split at this level, their rank, the longest
+            // A. which sub-blocks split at this level, and their rank
             for (int i = tid; i < ncur; i += nt) {
                 const int len = cur[i].e - cur[i].b;
                 const int act = cur[i].level < A.max_level && len > A.min_cells;
                 cur[i].act = act;
                 scan[i] = act;
-                if (act) atomicMax(&s_maxlen, len);
             }
             __syncthreads();
             const int nact = cta_scan(scan, ncur, warp_tmp);
@@ -1966,7 +2462,13 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                 if (tid == 0) s_fail = 2;  // too many sub-blocks
                 break;
             }
-            const int maxlen = s_maxlen;
+            int drawn = 0, filled = 0;
+            if (tid == 0) {
+                drawn = ld_relaxed_gpu(&A.queue->head);
+                filled = ld_relaxed_gpu(&A.queue->tail);
+            }
+            nxt = 2 * nact <= kNearDesc ? near_desc[(depth + 1) & 1]
+                                        : far_desc + ((depth + 1) & 1) * kMaxSub;
             for (int i = tid; i < ncur; i += nt) cur[i].rank = scan[i];
             __syncthreads();
             // the sub-blocks' starts, and ends with the split and axis flags,
@@ -1989,31 +2491,37 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                 const int ev = scan[kMaxSub + i];
                 const bool in = p >= scan[i] && p < (ev & 0x1fffffff) && ((ev >> 30) & 1);
                 dof[p] = static_cast<int16_t>(in ? i : -1);
-                const int j = at[p];
-                if (in) {
-                    k2[p] = static_cast<uint32_t>(scan[i]);
-                    k0[p] = ord(centre(j, ((ev >> 29) & 1) != 0));
-                } else {
-                    k2[p] = static_cast<uint32_t>(p);
-                    k0[p] = 0ull;
-                }
-                k1[p] = (static_cast<unsigned long long>(gid[j]) << 32) | static_cast<unsigned>(j);
+                k2[p] = static_cast<uint32_t>(in ? scan[i] : p);
             }
             __syncthreads();
-            {
-                // the active sub-blocks in rank order: nxt is free until phase L
-                for (int i = tid; i < ncur; i += nt)
-                    if (cur[i].act) {
-                        nxt[cur[i].rank].b = cur[i].b;
-                        nxt[cur[i].rank].e = cur[i].e;
-                    }
+            auto centre_key = [&](int p) {
+                const int i = dof[p];
+                return i >= 0 ? ord(centre(at[p], ((scan[kMaxSub + i] >> 29) & 1) != 0)) : 0ull;
+            };
+            if (size <= kSubThreads) {
+                for (int p = tid; p < size; p += nt) k0[p] = centre_key(p);
                 __syncthreads();
-                sort_segments(k0, k1, k2, nact, maxlen, [&](int g, int &b, int &e) {
-                    b = nxt[g].b;
-                    e = nxt[g].e;
-                });
+                int p;
+                const int to = counted_position(
+                    size, p,
+                    [&](int q, int &b, int &e) {
+                        const int i = dof[q];
+                        if (i < 0) return;
+                        b = scan[i];
+                        e = scan[kMaxSub + i] & 0x1fffffff;
+                    },
+                    [&](int q) { return k0[q]; }, [&](int q) { return at[q]; });
+                if (to >= 0) v1[to] = static_cast<uint32_t>(at[p]);
+                __syncthreads();
+            } else {
+                auto entry = [&](int p, unsigned long long &k, uint32_t &v) {
+                    k = centre_key(p);
+                    v = static_cast<uint32_t>(at[p]);
+                };
+                if (ncur == 1) merge_sort<false>(k0, v1, k2, size, entry);
+                else merge_sort<true>(k0, v1, k2, size, entry);
             }
-            for (int p = tid; p < size; p += nt) at[p] = static_cast<int32_t>(k1[p] & 0xffffffffull);
+            for (int p = tid; p < size; p += nt) at[p] = static_cast<int32_t>(v1[p]);
             __syncthreads();
             if (A.exact) cta_prefix64(at, sa, size, A.scale, pre, w64);
             // C. areas and median in sorted order; the block profile's region
@@ -2096,7 +2604,16 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                     }
                 }
                 __syncthreads();
-                sort_segments(k0, k1, k2, c1 - c0, maxsteps, [&](int g, int &b, int &e) {
+                if (maxsteps > 1 && scan[c1] - base <= kSubThreads)
+                    sort_steps(scan[c1] - base, [&](uint32_t tag, int &b, int &e) {
+                        const SubDesc &d = cur[tag];
+                        b = d.soff - base + 2;
+                        e = b + d.scnt;
+                    });
+                else if (maxsteps > 1 && scan[c1] - base <= kSub)
+                    merge_sort<true>(k0, k1, k2, scan[c1] - base, step_entry);
+                else
+                    sort_segments(k0, k1, k2, c1 - c0, maxsteps, [&](int g, int &b, int &e) {
                         const SubDesc &d = cur[c0 + g];
                         const bool on = d.act && d.vert;
                         b = on ? d.soff - base + 2 : 0;
@@ -2114,7 +2631,9 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                         }
                         const bool v = d.vert != 0;
                         const int o = d.soff - base;
-                        const int64_t n = team_build_profile(tm, FL, d.box, v, k0, k1, o, d.scnt, d.slen);
+                        const int64_t n =
+                            tm.T == 32 ? warp_build_profile(tm, FL, d.box, v, k0, k1, o, d.scnt, d.slen)
+                                       : team_build_profile(tm, FL, d.box, v, k0, k1, o, d.scnt, d.slen);
                         const Prof room{reinterpret_cast<const double *>(k0 + o),
                                         reinterpret_cast<const double *>(k1 + o), n};
                         const double share = d.cell_area > 0.0 ? d.low_area / d.cell_area : 0.5;
@@ -2213,7 +2732,16 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                     }
                 }
                 __syncthreads();
-                sort_segments(k0, k1, k2, c1 - c0, maxhsteps, [&](int g, int &b, int &e) {
+                if (maxhsteps > 1 && scan[c1] - base <= kSubThreads)
+                    sort_steps(scan[c1] - base, [&](uint32_t tag, int &b, int &e) {
+                        const SubDesc &d = cur[tag >> 1];
+                        b = d.hsoff[tag & 1] - base + 2;
+                        e = b + d.hscnt[tag & 1];
+                    });
+                else if (maxhsteps > 1 && scan[c1] - base <= kSub)
+                    merge_sort<true>(k0, k1, k2, scan[c1] - base, step_entry);
+                else
+                    sort_segments(k0, k1, k2, c1 - c0, maxhsteps, [&](int g, int &b, int &e) {
                         const int h = c0 + g;
                         const SubDesc &d = cur[h >> 1];
                         const bool on = d.act && d.vert;
@@ -2229,24 +2757,28 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                         if (!d.act) continue;
                         const bool v = d.vert != 0;
                         const int o = d.hsoff[side] - base;
-                        const int64_t n = team_build_profile(tm, FL, d.hbox + 4 * side, v, k0, k1, o,
-                                                             d.hscnt[side], d.hslen[side]);
+                        const double *bx = d.hbox + 4 * side;
+                        const int len = d.hslen[side], cnt = d.hscnt[side];
+                        const int64_t n = tm.T == 32
+                                              ? warp_build_profile(tm, FL, bx, v, k0, k1, o, cnt, len)
+                                              : team_build_profile(tm, FL, bx, v, k0, k1, o, cnt, len);
                         const int so = d.stoff[side];
-                        int64_t ns = 0;
+                        const double area = side ? d.high_area : d.low_area;
+                        const Prof room{reinterpret_cast<const double *>(k0 + o),
+                                        reinterpret_cast<const double *>(k1 + o), n};
+                        int64_t ns = -2;
+                        if (tm.T == 32)  // the tags of the step sort are used up
+                            ns = warp_make_stripes(room, bx, v, area, T.room, A.frac, A.limit_density,
+                                                   FL.obst, FL.K, d.cut, side == 0, d.stcap[side],
+                                                   sta + so, stb + so, stc + so,
+                                                   reinterpret_cast<double *>(k2) + 128 * (tid >> 5));
+                        if (ns == -2 && tm.lane == 0)
+                            ns = make_stripes(room, bx, v, area, T.room, A.frac, A.limit_density,
+                                              FL.obst, FL.K, d.cut, side == 0, scut + so,
+                                              d.stcap[side], sta + so, stb + so, stc + so);
                         if (tm.lane == 0) {
-                            const Prof room{reinterpret_cast<const double *>(k0 + o),
-                                            reinterpret_cast<const double *>(k1 + o), n};
-                            ns = make_stripes(room, d.hbox + 4 * side, v, side ? d.high_area : d.low_area,
-                                              T.room, A.frac, A.limit_density, FL.obst, FL.K, d.cut,
-                                              side == 0, scut + so, d.stcap[side], sta + so, stb + so,
-                                              stc + so);
                             if (ns < 0) atomicExch(&s_fail, 4);
                             d.stcnt[side] = static_cast<int32_t>(ns < 0 ? 0 : ns);
-                        }
-                        ns = tm.bcast(ns);
-                        for (int64_t q = tm.lane; q < ns; q += tm.T) {
-                            slo[so + q] = ~0ull;
-                            shi[so + q] = 0ull;
                         }
                     }
                 }
@@ -2255,40 +2787,81 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                 c0 = c1;
             }
             if (s_fail) break;
-            // H. cells of each half by (-distance from the cut, id)
+            // H. cells of each half by (-distance from the cut, id). The cells
+            // are in centre order, in which the distance is monotone: the low
+            // half keeps the order, the high half is reversed, and cells at
+            // the same distance go by id
             for (int p = tid; p < size; p += nt) {
                 const int i = dof[p];
-                const int j = at[p];
+                if (i < 0) continue;
+                const SubDesc &d = cur[i];
+                const double c = centre(at[p], d.vert != 0);
+                const double from = p < d.b + d.m ? d.cut - c : c - d.cut;
+                k0[p] = ord(-from);
+            }
+            __syncthreads();
+            bool unsorted = false;  // a long run out of id order
+            for (int p = tid; p < size; p += nt) {
+                const int i = dof[p];
+                int to = p;
                 if (i >= 0) {
                     const SubDesc &d = cur[i];
                     const int mid = d.b + d.m;
-                    const double c = centre(j, d.vert != 0);
-                    const double from = p < mid ? d.cut - c : c - d.cut;
-                    k2[p] = static_cast<uint32_t>(p < mid ? d.b : mid);
-                    k0[p] = ord(-from);
-                } else {
-                    k2[p] = static_cast<uint32_t>(p);
-                    k0[p] = 0ull;
-                }
-                k1[p] = (static_cast<unsigned long long>(gid[j]) << 32) | static_cast<unsigned>(j);
-            }
-            __syncthreads();
-            {
-                for (int i = tid; i < ncur; i += nt)
-                    if (cur[i].act) {
-                        nxt[cur[i].rank].b = cur[i].b;
-                        nxt[cur[i].rank].e = cur[i].e;
-                        nxt[cur[i].rank].m = cur[i].m;
+                    const int b = p < mid ? d.b : mid, e = p < mid ? mid : d.e;
+                    const unsigned long long k = k0[p];
+                    int rs = p, re = p + 1, rank = 0;
+                    while (rs > b && k0[rs - 1] == k && p - rs < kLongRun) --rs;
+                    while (re < e && k0[re] == k && re - p < kLongRun) ++re;
+                    if (p - rs == kLongRun || re - p == kLongRun) {  // all of it, by binary search
+                        int lo = b, hi = rs;
+                        while (lo < hi) {
+                            const int q = (lo + hi) >> 1;
+                            if (k0[q] == k) hi = q;
+                            else lo = q + 1;
+                        }
+                        rs = lo;
+                        hi = e;
+                        lo = re;
+                        while (lo < hi) {
+                            const int q = (lo + hi) >> 1;
+                            if (k0[q] == k) lo = q + 1;
+                            else hi = q;
+                        }
+                        re = lo;
                     }
+                    if (re - rs > kLongRun) {
+                        rank = p - rs;
+                        unsorted = unsorted || (p > rs && at[p - 1] > at[p]);
+                    } else {
+                        for (int q = rs; q < re; ++q) rank += at[q] < at[p];
+                    }
+                    to = p < mid ? rs + rank : mid + (d.e - re) + rank;
+                }
+                v1[to] = static_cast<uint32_t>(at[p]);
+            }
+            if (__syncthreads_or(unsorted)) {
+                for (int p = tid; p < size; p += nt) {
+                    const int i = dof[p];
+                    k2[p] = static_cast<uint32_t>(
+                        i < 0 ? p : (p < cur[i].b + cur[i].m ? cur[i].b : cur[i].b + cur[i].m));
+                }
                 __syncthreads();
-                sort_segments(k0, k1, k2, 2 * nact, maxlen, [&](int g, int &b, int &e) {
-                    const SubDesc &d = nxt[g >> 1];
-                    b = (g & 1) ? d.b + d.m : d.b;
-                    e = (g & 1) ? d.e : d.b + d.m;
+                merge_sort<true>(k0, v1, k2, size, [&](int p, unsigned long long &k, uint32_t &v) {
+                    k = dof[p] < 0 ? 0ull : k0[p];
+                    v = static_cast<uint32_t>(at[p]);
                 });
             }
-            for (int p = tid; p < size; p += nt) at[p] = static_cast<int32_t>(k1[p] & 0xffffffffull);
+            for (int p = tid; p < size; p += nt) at[p] = static_cast<int32_t>(v1[p]);
             __syncthreads();
+            // the stripes' starts and extreme centres, in the sort buffer when
+            // they fit (the sorted entries are used up)
+            const bool fits = stot <= kSortCap;
+            unsigned long long *const slo = fits ? k0 : glo, *const shi = fits ? k1 : ghi;
+            uint32_t *const starts = fits ? k2 : reinterpret_cast<uint32_t *>(scut);
+            for (int q = tid; q < stot; q += nt) {
+                slo[q] = ~0ull;
+                shi[q] = 0ull;
+            }
             // I. greedy fill (exact areas: stripe starts by binary search on the
             // prefix, then each position looks its stripe up; else one thread
             // per half in the reference's order)
@@ -2303,7 +2876,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                     const int ns = d.stcnt[side], so = d.stoff[side];
                     int q0 = p0;
                     for (int q = 0; q < ns; ++q) {
-                        scut[so + q] = static_cast<double>(q0);  // stripe starts
+                        starts[so + q] = static_cast<uint32_t>(q0);
                         if (q + 1 == ns) break;
                         const double cap = stc[so + q];
                         int lo = q0, hi = p1;
@@ -2327,7 +2900,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                         int lo = 0, hi = ns - 1;
                         while (lo < hi) {
                             const int k = (lo + hi + 1) >> 1;
-                            if (scut[so + k] <= static_cast<double>(p)) lo = k;
+                            if (starts[so + k] <= static_cast<uint32_t>(p)) lo = k;
                             else hi = k - 1;
                         }
                         q = so + lo;
@@ -2383,7 +2956,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                 const double lo = unord(slo[q]), hi = unord(shi[q]);
                 const double c0 = centre(j, v);
                 const double t = hi > lo ? (c0 - lo) / (hi - lo) : 0.5;
-                const double sz = v ? C.w[gid[j]] : C.h[gid[j]];
+                const double sz = extent(j, v);
                 const double a = sta[q], bb = stb[q];
                 const double c = a + t * (bb - a);
                 const double lim = ref_max(a, bb - sz);
@@ -2407,24 +2980,63 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
             }
             if (tid == 0) {
                 s_ncur = 2 * nact;
-                s_maxlen = 0;
                 s_maxsteps = 0;
+                // CTAs waiting (as of the level's start), and room for two blocks?
+                if (size > kHandOff && nact == 1 && drawn > filled) {
+                    int t = filled;
+                    while (t + 2 <= A.cap) {
+                        const int was = atomicCAS(&A.queue->tail, t, t + 2);
+                        if (was == t) {
+                            s_slot = t;
+                            break;
+                        }
+                        t = was;
+                    }
+                }
             }
-            SubDesc *t = cur;
             cur = nxt;
-            nxt = t;
+            __syncthreads();
+            if (s_slot >= 0) break;
         }
         __syncthreads();
-        if (s_fail) {
-            if (tid == 0) A.fail[task] = s_fail;
-        } else {
+        if (!s_fail) {
             for (int j = tid; j < size; j += nt) {
                 C.x[gid[j]] = sx[j];
                 C.y[gid[j]] = sy[j];
             }
-            if (tid == 0) A.fail[task] = 0;
+            if (s_slot >= 0) {  // the halves' cells, by id each
+                const int m = cur[0].e;
+                for (int p = tid; p < size; p += nt) scan[at[p]] = p < m ? 1 : 0;
+                __syncthreads();
+                for (int j = tid; j < size; j += nt) sof[j] = scan[j];
+                cta_scan(scan, size, warp_tmp);
+                for (int j = tid; j < size; j += nt)
+                    A.cells[T.b + (sof[j] ? scan[j] : m + j - scan[j])] = gid[j];
+            }
         }
         __syncthreads();
+        if (tid == 0) {
+            if (s_fail) A.failed[atomicAdd(&A.queue->nfail, 1)] = make_int2(task, s_fail);
+            if (s_slot >= 0) {
+                atomicAdd(&A.queue->pending, 2);
+                for (int q = 0; q < 2; ++q) {
+                    const SubDesc &d = cur[q];
+                    SubTask &h = A.tasks[s_slot + q];
+                    for (int k = 0; k < 4; ++k) h.box[k] = d.box[k];
+                    h.room = T.room;
+                    h.b = T.b + d.b;
+                    h.e = T.b + d.e;
+                    h.level = d.level;
+                    h.vert = d.vert;
+                    h.r0 = row0;
+                    h.r1 = rows <= kRowsLocal ? row0 + rows : -1;
+                }
+                __threadfence();
+                for (int q = 0; q < 2; ++q) atomicExch(A.ready + s_slot + q, A.epoch);
+            }
+            __threadfence();
+            atomicSub(&A.queue->pending, 1);
+        }
     }
 }
 
@@ -2506,8 +3118,10 @@ struct LalState {
     DevBuf<double> overflow;
     DevBuf<long long> pre, tile;
     DevBuf<int32_t> sbeg;
-    DevBuf<SubTask> tasks;
-    DevBuf<int32_t> tfail;
+    DevBuf<char> tasks;      // SubQueue (kQueueHead bytes), then the tasks
+    DevBuf<unsigned> ready;
+    unsigned epoch = 0;
+    DevBuf<int2> tfail;
     DevBuf<SubDesc> sdesc;
     DevBuf<double> sstrp;
     DevBuf<unsigned long long> sstrlh;
@@ -2541,6 +3155,7 @@ void free_lal(ktg_ctx *c) {
     s->sbeg.release();
     s->tasks.release();
     s->tfail.release();
+    s->ready.release();
     s->sdesc.release();
     s->sstrp.release();
     s->sstrlh.release();
@@ -2738,43 +3353,69 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
         return KTG_OK;
     };
 
-    // Blocks of at most kSub cells: one CTA each runs the rest of the
-    // bisection; failed[t] = 1 for a block left for the level-by-level path.
-    auto run_subtree = [&](const std::vector<SubTask> &tasks, std::vector<int32_t> &failed) -> int {
+    // Blocks of at most kSub cells: the subtree kernel runs the rest of the
+    // bisection; left: the blocks (given or handed off) that remain for the
+    // level-by-level path.
+    auto run_subtree = [&](const std::vector<SubTask> &tasks, std::vector<SubTask> &left) -> int {
         const int32_t nt = static_cast<int32_t>(tasks.size());
-        const int grid = std::max(1, std::min<int>(nt, c->num_sms));
+        const int32_t cap = nt * kHandSlots;
+        const int grid = std::min(c->num_sms, cap);
         const double t0 = now_ms();
         int r2;
-        if ((r2 = s->tasks.ensure(c, nt)) || (r2 = s->tfail.ensure(c, nt)) ||
+        const bool grow = s->ready.cap < cap;
+        if ((r2 = s->tasks.ensure(c, kQueueHead + sizeof(SubTask) * static_cast<int64_t>(cap))) ||
+            (r2 = s->ready.ensure(c, cap)) || (r2 = s->tfail.ensure(c, cap)) ||
             (r2 = s->sdesc.ensure(c, static_cast<int64_t>(grid) * 2 * kMaxSub)) ||
             (r2 = s->sstrp.ensure(c, static_cast<int64_t>(grid) * 4 * kStripeCap)) ||
             (r2 = s->sstrlh.ensure(c, static_cast<int64_t>(grid) * 2 * kStripeCap)))
             return r2;
+        if (grow || s->epoch == 0xffffffffu) {
+            KTG_CUDA(c, cudaMemsetAsync(s->ready.p, 0, sizeof(unsigned) * s->ready.cap, c->stream));
+            s->epoch = 0;
+        }
         if (!s->subtree_attr) {
             KTG_CUDA(c, cudaFuncSetAttribute(k_subtree, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(kSubSmem)));
             s->subtree_attr = true;
         }
-        KTG_CUDA(c, cudaMemcpyAsync(s->tasks.p, tasks.data(), sizeof(SubTask) * nt,
-                                    cudaMemcpyHostToDevice, c->stream));
-        SubArgs A{s->tasks.p, nt, s->tfail.p, s->cells.p, C, F, s->sdesc.p,
-                  s->sstrp.p, s->sstrlh.p, max_level, min_cells, stripe_extra, frac,
-                  c->density_limit, exact ? 1 : 0, scale, inv_scale};
+        std::vector<char> head(kQueueHead + sizeof(SubTask) * nt);
+        SubQueue q{0, nt, nt, 0, 0};
+        std::memcpy(head.data(), &q, sizeof(q));
+        std::memcpy(head.data() + kQueueHead, tasks.data(), sizeof(SubTask) * nt);
+        KTG_CUDA(c, cudaMemcpyAsync(s->tasks.p, head.data(), head.size(), cudaMemcpyHostToDevice,
+                                    c->stream));
+        SubTask *slots = reinterpret_cast<SubTask *>(s->tasks.p + kQueueHead);
+        SubArgs A{slots, nt, cap, reinterpret_cast<SubQueue *>(s->tasks.p), s->ready.p, ++s->epoch,
+                  s->tfail.p, s->cells.p, C, F, s->sdesc.p, s->sstrp.p, s->sstrlh.p, max_level,
+                  min_cells, stripe_extra, frac, c->density_limit, exact ? 1 : 0, scale, inv_scale};
         k_subtree<<<grid, kSubThreads, kSubSmem, c->stream>>>(A);
         ++c->launches;
         KTG_CUDA(c, cudaGetLastError());
-        failed.assign(nt, 0);
-        KTG_CUDA(c, cudaMemcpyAsync(failed.data(), s->tfail.p, sizeof(int32_t) * nt,
-                                    cudaMemcpyDeviceToHost, c->stream));
+        KTG_CUDA(c, cudaMemcpyAsync(&q, s->tasks.p, sizeof(q), cudaMemcpyDeviceToHost, c->stream));
         KTG_CUDA(c, lal_sync(c));
-        s->stats[2] += 1;
-        s->stats[4] += nt;
-        s->stats[8] += now_ms() - t0;
-        s->stats[10] += nt;
-        for (int32_t t = 0; t < nt; ++t) {
-            s->stats[11] += failed[t] != 0;
-            if (failed[t] >= 1 && failed[t] <= 4) s->stats[11 + failed[t]] += 1;
+        if (q.timeout) return set_error(c, KTG_ERR_TIMEOUT, "legalizer: the block queue timed out");
+        left.clear();
+        if (q.nfail > 0) {
+            std::vector<int2> fl(q.nfail);
+            std::vector<SubTask> all(q.tail);
+            KTG_CUDA(c, cudaMemcpyAsync(fl.data(), s->tfail.p, sizeof(int2) * q.nfail,
+                                        cudaMemcpyDeviceToHost, c->stream));
+            KTG_CUDA(c, cudaMemcpyAsync(all.data(), slots, sizeof(SubTask) * q.tail,
+                                        cudaMemcpyDeviceToHost, c->stream));
+            KTG_CUDA(c, lal_sync(c));
+            for (const int2 &f : fl) {
+                left.push_back(all[f.x]);
+                s->stats[11] += 1;
+                if (f.y >= 1 && f.y <= 4) s->stats[11 + f.y] += 1;
+            }
+            // disjoint position ranges: the level-by-level path takes them in order
+            std::sort(left.begin(), left.end(),
+                      [](const SubTask &a, const SubTask &b) { return a.b < b.b; });
         }
+        s->stats[2] += 1;
+        s->stats[4] += q.tail;
+        s->stats[8] += now_ms() - t0;
+        s->stats[10] += q.tail;
         return KTG_OK;
     };
 
@@ -2832,7 +3473,6 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
             std::vector<int32_t> ab, ae, av, al;
             std::vector<double> abox, aroom;
             std::vector<SubTask> tasks;
-            std::vector<size_t> task_src;
             auto take = [&](size_t k) {
                 ab.push_back(hb[k]);
                 ae.push_back(he[k]);
@@ -2851,17 +3491,24 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
                     t.e = he[k];
                     t.level = hl[k];
                     t.vert = hv[k];
+                    t.r0 = 0;
+                    t.r1 = -1;
                     tasks.push_back(t);
-                    task_src.push_back(k);
                 } else {
                     take(k);
                 }
             }
             if (!tasks.empty()) {
-                std::vector<int32_t> failed;
-                if ((r2 = run_subtree(tasks, failed))) return r2;
-                for (size_t t = 0; t < tasks.size(); ++t)
-                    if (failed[t]) take(task_src[t]);
+                std::vector<SubTask> left;
+                if ((r2 = run_subtree(tasks, left))) return r2;
+                for (const SubTask &t : left) {
+                    ab.push_back(t.b);
+                    ae.push_back(t.e);
+                    av.push_back(t.vert);
+                    al.push_back(t.level);
+                    for (int q = 0; q < 4; ++q) abox.push_back(t.box[q]);
+                    aroom.push_back(t.room);
+                }
             }
             const int32_t na = static_cast<int32_t>(ab.size());
             if (na == 0) break;
