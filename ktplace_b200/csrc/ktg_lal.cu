@@ -2981,8 +2981,10 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
             if (tid == 0) {
                 s_ncur = 2 * nact;
                 s_maxsteps = 0;
-                // CTAs waiting (as of the level's start), and room for two blocks?
-                if (size > kHandOff && nact == 1 && drawn > filled) {
+                // CTAs waiting (as of the level's start), and room for two
+                // blocks? Only the whole block's halves are handed off: beside a
+                // half that is done already they would not fill its positions
+                if (size > kHandOff && ncur == 1 && drawn > filled) {
                     int t = filled;
                     while (t + 2 <= A.cap) {
                         const int was = atomicCAS(&A.queue->tail, t, t + 2);

@@ -217,3 +217,22 @@ def test_lal_profile_branches(kind, subtree, gpu_ctx):
     ox, oy = L.legalize(x, y)
     assert np.array_equal(gx, np.array(ox)) and np.array_equal(gy, np.array(oy))
     assert np.mean(gx != x) > 0.1
+
+
+@pytest.mark.parametrize("cells,macros,rows,seed,spread", [(60000, 150, 400, 2, 0.05),
+                                                           (60000, 150, 400, 2, 0.2),
+                                                           (100000, 250, 500, 3, 0.25)])
+def test_lal_handed_off_blocks(cells, macros, rows, seed, spread, gpu_ctx):
+    """Blocks whose halves go to other CTAs, with macros that leave some halves
+    with too few cells to split: bit-identical to the level-by-level path,
+    whichever halves are handed off."""
+    raw = synth.generate(synth.SynthSpec(num_movable=cells, num_nets=cells + 1000, num_pads=400,
+                                         num_rows=rows, utilization=0.6, num_macros=macros,
+                                         seed=seed))
+    nl = netlist.flatten(raw)
+    x, y = clustered(raw, nl.num_movable, seed, spread)
+    bins = grid.default_bins_per_axis(nl.num_movable)
+    want = run_gpu(gpu_ctx, nl, bins, 1.0, x, y, subtree=0)
+    for _ in range(4):
+        got = run_gpu(gpu_ctx, nl, bins, 1.0, x, y)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
