@@ -1647,19 +1647,20 @@ __device__ void merge_sort(unsigned long long *key, V *val, uint32_t *tag, int t
         const bool le = (ki < kj) | ((ki == kj) & (vi <= vj));
         return Tags ? (ti < tj) | ((ti == tj) & le) : le;
     };
-    if (on) {
-        unsigned long long k[4];
-        V v[4];
-        uint32_t t[4];
+    unsigned long long k[4];
+    V v[4];
+    uint32_t t[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            k[u] = ~0ull;
-            v[u] = static_cast<V>(~0ull);
-            t[u] = 0u;
-            if (p0 + u < tot) load(p0 + u, k[u], v[u]);
-            else if (Tags) tag[p0 + u] = ~0u;
-            if (Tags) t[u] = tag[p0 + u];
-        }
+    for (int u = 0; u < 4; ++u) {
+        k[u] = ~0ull;
+        v[u] = static_cast<V>(~0ull);
+        t[u] = 0u;
+        if (p0 + u < tot) load(p0 + u, k[u], v[u]);
+        else if (Tags && on) tag[p0 + u] = ~0u;
+        if (Tags && on) t[u] = tag[p0 + u];
+    }
+    __syncwarp();  // all loaded before the first is stored: load may read key and val
+    if (on) {
         auto cas = [&](int i, int j) {
             if (t[i] == t[j] && (k[j] < k[i] || (k[j] == k[i] && v[j] < v[i]))) {
                 const unsigned long long x = k[i];
