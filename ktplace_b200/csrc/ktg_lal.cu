@@ -13,25 +13,30 @@
 //          reference's summation order over the host copy of the grid;
 //   device each batch: the regions' cells, then the recursive bisection
 //          level by level over every block of the batch at once:
-//            * cells sorted by (centre, index)          (segmented sort)
-//            * per block, in the reference's order on one thread: cell
-//              area, the area median m, the free-space profile of the box
-//              (vertical: row spans as (x, +-h) steps, segmented sort,
-//              running sums), the cutline and the two half boxes;
-//            * per half on one thread: its profile, the stripes (obstacle
-//              edges, unique, midpoint splits above stripeAreaFraction of
-//              the region's room) in the reference's distance-from-cut order;
-//            * cells sorted by (-distance from the cut, index), stripes
-//              filled greedily in that order (one thread per half);
-//            * per stripe the lowest / highest centre (exact atomics on
-//              order-preserving bits), then every cell's new position;
+//            * cells sorted by (centre, index): tiles of 2048 keys in
+//              shared memory, then merge passes;
+//            * per block: cell area and the area median m (from an exact
+//              prefix), the free-space profile of the box (vertical: row
+//              spans as sorted (x, +-h) steps, running sums), the cutline and
+//              the two half boxes;
+//            * per half: its profile, the stripes (obstacle edges, unique,
+//              midpoint splits above stripeAreaFraction of the region's room)
+//              in the reference's distance-from-cut order;
+//            * cells by (-distance from the cut, index): the centre order, or
+//              its reverse; stripes filled greedily in that order;
+//            * per stripe the lowest / highest centre, then every cell's new
+//              position;
 //            * children: the low and high cells, next axis.
+//            The host knows the boxes and the free space, so it bounds the
+//            profiles and stripes itself: one copy in and one wait per level
+//            (0.25 to 0.35 ms; it took 0.8 with six waits, 15 copies, a bitonic
+//            sort of 70 us and a second sort for the fill order).
 //          then the bins and occupancy of all cells again for the host.
 //
 // The sorts are key-only over 16-byte keys: (order bits of a double, index)
-// for cells and (order bits of x, order bits of dh) for profile steps; a
-// segment of up to kSortSmall keys is sorted by one block in shared memory,
-// a longer one by sorted chunks and merge passes.
+// for cells and (order bits of x, order bits of dh) for profile steps; tiles of
+// kSub keys are sorted by one CTA each in shared memory, longer segments by
+// merge passes over them.
 #include "ktg_common.cuh"
 #include "ktg_context.h"
 
@@ -41,6 +46,7 @@
 #include <cmath>
 #include <cstring>
 #include <limits>
+#include <utility>
 #include <vector>
 
 namespace ktg {
@@ -48,13 +54,12 @@ namespace ktg {
 namespace {
 
 constexpr int kT = 256;
-constexpr int kSortSmall = 2048;
 
 struct Key {
     unsigned long long a, b;
 };
 
-__host__ __device__ __forceinline__ bool key_lt(const Key &x, const Key &y) {
+__device__ __forceinline__ bool key_lt(const Key &x, const Key &y) {
     return x.a < y.a || (x.a == y.a && x.b < y.b);
 }
 
@@ -71,36 +76,6 @@ __device__ __forceinline__ double unord(unsigned long long u) {
 }
 
 // ---- segmented key sort ---------------------------------------------------------
-
-// One block per segment of at most kSortSmall keys: bitonic sort in shared memory.
-__global__ void __launch_bounds__(kT) k_sort_small(Key *keys, const int64_t *seg, int nseg) {
-    __shared__ Key s[kSortSmall];
-    const int sidx = blockIdx.x;
-    if (sidx >= nseg) return;
-    const int64_t b = seg[2 * sidx], e = seg[2 * sidx + 1];
-    const int len = static_cast<int>(e - b);
-    int P = 1;
-    while (P < len) P <<= 1;
-    for (int i = threadIdx.x; i < P; i += kT)
-        s[i] = i < len ? keys[b + i] : Key{~0ull, ~0ull};
-    __syncthreads();
-    for (int k = 2; k <= P; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < P; i += kT) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const Key x = s[i], y = s[ixj];
-                    if (key_lt(y, x) == ((i & k) == 0)) {
-                        s[i] = y;
-                        s[ixj] = x;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    for (int i = threadIdx.x; i < len; i += kT) keys[b + i] = s[i];
-}
 
 int blocks_for(int64_t items, int threads = kT) {
     return static_cast<int>(std::max<int64_t>(1, (items + threads - 1) / threads));
@@ -128,159 +103,6 @@ struct DevBuf {
     }
 };
 
-// Chunks [b, e) of at most kSortSmall keys, one per block, sorted in shared
-// memory; the chunk list holds (b, e) pairs.
-__global__ void __launch_bounds__(kT) k_sort_chunks_multi(Key *keys, const int64_t *chunks) {
-    __shared__ Key s[kSortSmall];
-    const int64_t c0 = chunks[2 * blockIdx.x], c1 = chunks[2 * blockIdx.x + 1];
-    const int len = static_cast<int>(c1 - c0);
-    for (int i = threadIdx.x; i < kSortSmall; i += kT)
-        s[i] = i < len ? keys[c0 + i] : Key{~0ull, ~0ull};
-    __syncthreads();
-    for (int k = 2; k <= kSortSmall; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < kSortSmall; i += kT) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const Key x = s[i], y = s[ixj];
-                    if (key_lt(y, x) == ((i & k) == 0)) {
-                        s[i] = y;
-                        s[ixj] = x;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    for (int i = threadIdx.x; i < len; i += kT) keys[c0 + i] = s[i];
-}
-
-// Segment of global position g among the segments whose lengths prefix
-// `pref` (nseg + 1 entries): the last s with pref[s] <= g.
-__device__ __forceinline__ int seg_of(const int64_t *pref, int nseg, int64_t g) {
-    int lo = 0, hi = nseg - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (pref[mid] <= g) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
-// One merge pass over every long segment at once: runs of `run` keys merged
-// pairwise (stable); a segment no longer than `run` is copied across.
-__global__ void k_merge_pass_multi(const Key *src, Key *dst, const int64_t *segs,
-                                   const int64_t *pref, int nseg, int64_t run) {
-    const int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (g >= pref[nseg]) return;
-    const int sg = seg_of(pref, nseg, g);
-    const int64_t b = segs[2 * sg], len = segs[2 * sg + 1] - b, r = g - pref[sg];
-    if (run >= len) {
-        dst[b + r] = src[b + r];
-        return;
-    }
-    const int64_t a0 = (r / (2 * run)) * 2 * run;
-    const int64_t a1 = min(a0 + run, len);
-    const int64_t b1 = min(a0 + 2 * run, len);
-    const Key k = src[b + r];
-    int64_t out;
-    if (r < a1) {  // in the first run: count second-run keys strictly below
-        int64_t lo = a1, hi = b1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (key_lt(src[b + mid], k)) lo = mid + 1;
-            else hi = mid;
-        }
-        out = a0 + (r - a0) + (lo - a1);
-    } else {  // in the second run: count first-run keys not above
-        int64_t lo = a0, hi = a1;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (!key_lt(k, src[b + mid])) lo = mid + 1;
-            else hi = mid;
-        }
-        out = a0 + (r - a1) + (lo - a0);
-    }
-    dst[b + out] = k;
-}
-
-__global__ void k_copy_multi(const Key *src, Key *dst, const int64_t *segs, const int64_t *pref,
-                             int nseg) {
-    const int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (g >= pref[nseg]) return;
-    const int sg = seg_of(pref, nseg, g);
-    const int64_t q = segs[2 * sg] + g - pref[sg];
-    dst[q] = src[q];
-}
-
-// Sorts keys[b, e) of every segment (host list of (b, e) pairs): segments of
-// up to kSortSmall keys one block each; longer ones in chunks, then merge
-// passes over all of them together. `dseg` holds the device descriptors.
-int seg_sort(ktg_ctx *c, Key *keys, Key *tmp, const std::vector<int64_t> &hseg,
-             DevBuf<int64_t> &dseg) {
-    const int nseg = static_cast<int>(hseg.size() / 2);
-    if (nseg == 0) return KTG_OK;
-    std::vector<int64_t> small, chunks, large, pref(1, 0);
-    int64_t maxlen = 0;
-    for (int s = 0; s < nseg; ++s) {
-        const int64_t b = hseg[2 * s], e = hseg[2 * s + 1];
-        if (e - b <= 1) continue;
-        if (e - b <= kSortSmall) {
-            small.push_back(b);
-            small.push_back(e);
-            continue;
-        }
-        for (int64_t q = b; q < e; q += kSortSmall) {
-            chunks.push_back(q);
-            chunks.push_back(std::min(e, q + kSortSmall));
-        }
-        large.push_back(b);
-        large.push_back(e);
-        pref.push_back(pref.back() + (e - b));
-        maxlen = std::max(maxlen, e - b);
-    }
-    // descriptors: small pairs, chunk pairs, long segments, their prefix
-    std::vector<int64_t> all;
-    all.reserve(small.size() + chunks.size() + large.size() + pref.size());
-    all.insert(all.end(), small.begin(), small.end());
-    all.insert(all.end(), chunks.begin(), chunks.end());
-    all.insert(all.end(), large.begin(), large.end());
-    all.insert(all.end(), pref.begin(), pref.end());
-    int rc;
-    if ((rc = dseg.ensure(c, static_cast<int64_t>(all.size()) + 1))) return rc;
-    KTG_CUDA(c, cudaMemcpyAsync(dseg.p, all.data(), sizeof(int64_t) * all.size(),
-                                cudaMemcpyHostToDevice, c->stream));
-    const int64_t *d_small = dseg.p;
-    const int64_t *d_chunks = d_small + small.size();
-    const int64_t *d_large = d_chunks + chunks.size();
-    const int64_t *d_pref = d_large + large.size();
-    if (!small.empty()) {
-        k_sort_small<<<static_cast<int>(small.size() / 2), kT, 0, c->stream>>>(
-            keys, d_small, static_cast<int>(small.size() / 2));
-        ++c->launches;
-    }
-    if (!large.empty()) {
-        const int nl = static_cast<int>(large.size() / 2);
-        const int64_t total = pref.back();
-        k_sort_chunks_multi<<<static_cast<int>(chunks.size() / 2), kT, 0, c->stream>>>(keys,
-                                                                                     d_chunks);
-        ++c->launches;
-        Key *src = keys, *dst = tmp;
-        for (int64_t run = kSortSmall; run < maxlen; run *= 2) {
-            k_merge_pass_multi<<<blocks_for(total), kT, 0, c->stream>>>(src, dst, d_large, d_pref,
-                                                                       nl, run);
-            ++c->launches;
-            std::swap(src, dst);
-        }
-        if (src != keys) {
-            k_copy_multi<<<blocks_for(total), kT, 0, c->stream>>>(src, keys, d_large, d_pref, nl);
-            ++c->launches;
-        }
-    }
-    KTG_CUDA(c, cudaGetLastError());
-    return KTG_OK;
-}
-
 // ---- free space -----------------------------------------------------------------
 
 struct Free {
@@ -302,24 +124,6 @@ __device__ __forceinline__ int32_t first_row(const Free &F, double ly) {
     return lo;
 }
 
-// Upper bound on a profile's step count and edge count for `box`.
-__device__ __forceinline__ void profile_bound(const Free &F, const double *box, bool vertical,
-                                              int64_t &steps, int64_t &edges) {
-    const int32_t r0 = first_row(F, box[1]);
-    int32_t lo = r0, hi = F.R;  // first row from r0 with y start >= uy
-    while (lo < hi) {
-        const int32_t mid = (lo + hi) >> 1;
-        if (F.rowy[2 * mid] < box[3]) lo = mid + 1;
-        else hi = mid;
-    }
-    const int32_t r1 = lo;
-    const int64_t sp = F.rowspan[r1] - F.rowspan[r0];
-    steps = vertical ? 2 * sp : 0;
-    edges = (vertical ? 2 * sp : 2 * static_cast<int64_t>(r1 - r0)) + 2;
-}
-
-// Vertical profile steps of `box` (unsorted), handed to sink(at, dh) in
-// row and span order; returns the count.
 // First span of row r ending after x (spans of a row ascend and are
 // disjoint, FreeSpace::build).
 __device__ __forceinline__ int64_t first_span(const Free &F, int32_t r, double x) {
@@ -387,7 +191,6 @@ struct Prof {
         const double f = (c - e[k]) / (e[k + 1] - e[k]);
         return p[k] + f * (p[k + 1] - p[k]);
     }
-    __device__ double between(double a, double b) const { return before(b) - before(a); }
     __device__ double coordinate_at(double target) const {
         if (target <= 0.0) return e[0];
         if (target >= total()) return e[n - 1];
@@ -560,6 +363,239 @@ __device__ int64_t make_stripes(const Prof &room, const double *box, bool v, dou
     return ns;
 }
 
+// ---- sorting -------------------------------------------------------------------------
+
+constexpr int kSub = 2048;         // entries a CTA sorts in shared memory
+constexpr int kSubThreads = 512;
+
+// Where entry i of a buffer of 8- or 4-byte entries lies while it is merged: a
+// thread's four outputs are consecutive, and unswizzled its 8-byte accesses
+// would meet seven other lanes' banks.
+template <typename V>
+__device__ __forceinline__ int swizzled(int i) {
+    return sizeof(V) == 8 ? i ^ ((i >> 4) & 15) : i ^ ((i >> 5) & 31);
+}
+
+// Sorts positions [0, tot), tot <= kSub, by (tag, key, val) with the whole CTA:
+// four entries per thread sorted in registers, then merges of sorted runs, each
+// thread finding its four outputs by a binary search along the merge path. tag
+// ascends with the position, so entries move only among equal tags and every
+// position keeps its tag; without Tags it is one segment. load(p, key, val)
+// gives the entries; key and val have room for 2 kSub and end with the sorted
+// ones in [0, tot).
+template <bool Tags, typename V, class Load>
+__device__ void merge_sort(unsigned long long *key, V *val, uint32_t *tag, int tot, Load load) {
+    int P = 4, levels = 0;
+    while (P < tot) P <<= 1, ++levels;
+    int buf = levels & 1;
+    const int p0 = 4 * threadIdx.x;
+    const bool on = p0 < P;
+    auto less_eq = [&](uint32_t ti, unsigned long long ki, V vi, uint32_t tj, unsigned long long kj,
+                       V vj) {
+        const bool le = (ki < kj) | ((ki == kj) & (vi <= vj));
+        return Tags ? (ti < tj) | ((ti == tj) & le) : le;
+    };
+    unsigned long long k[4];
+    V v[4];
+    uint32_t t[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        k[u] = ~0ull;
+        v[u] = static_cast<V>(~0ull);
+        t[u] = 0u;
+        if (p0 + u < tot) load(p0 + u, k[u], v[u]);
+        else if (Tags && on) tag[p0 + u] = ~0u;
+        if (Tags && on) t[u] = tag[p0 + u];
+    }
+    __syncwarp();  // all loaded before the first is stored: load may read key and val
+    if (on) {
+        auto cas = [&](int i, int j) {
+            if (t[i] == t[j] && (k[j] < k[i] || (k[j] == k[i] && v[j] < v[i]))) {
+                const unsigned long long x = k[i];
+                k[i] = k[j];
+                k[j] = x;
+                const V y = v[i];
+                v[i] = v[j];
+                v[j] = y;
+            }
+        };
+        cas(0, 1);
+        cas(2, 3);
+        cas(0, 2);
+        cas(1, 3);
+        cas(1, 2);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = p0 + u;
+            key[buf * kSub + (levels ? swizzled<unsigned long long>(i) : i)] = k[u];
+            val[buf * kSub + (levels ? swizzled<V>(i) : i)] = v[u];
+        }
+    }
+    for (int w = 4; w < P; w <<= 1, buf ^= 1) {
+        if (w >= 128) __syncthreads();  // up to there a warp merges its own entries
+        else __syncwarp();
+        if (!on) continue;
+        const unsigned long long *sk = key + buf * kSub;
+        const V *sv = val + buf * kSub;
+        unsigned long long *dk = key + (buf ^ 1) * kSub;
+        V *dv = val + (buf ^ 1) * kSub;
+        auto kat = [&](int i) { return sk[swizzled<unsigned long long>(i)]; };
+        auto vat = [&](int i) { return sv[swizzled<V>(i)]; };
+        auto tat = [&](int i) { return Tags ? tag[i] : 0u; };
+        const int base = p0 & ~(2 * w - 1), d = p0 - base;
+        int lo = max(0, d - w), hi = min(d, w);
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1, i = base + mid, j = base + w + d - 1 - mid;
+            if (less_eq(tat(i), kat(i), vat(i), tat(j), kat(j), vat(j))) lo = mid + 1;
+            else hi = mid;
+        }
+        int i = base + lo, j = base + w + d - lo;
+        const int ei = base + w, ej = base + 2 * w;
+        unsigned long long ki = 0, kj = 0;
+        V vi = 0, vj = 0;
+        uint32_t ti = 0u, tj = 0u;
+        if (i < ei) ki = kat(i), vi = vat(i), ti = tat(i);
+        if (j < ej) kj = kat(j), vj = vat(j), tj = tat(j);
+        const bool last = 2 * w == P;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool left = j >= ej || (i < ei && less_eq(ti, ki, vi, tj, kj, vj));
+            const int q = p0 + u;
+            dk[last ? q : swizzled<unsigned long long>(q)] = left ? ki : kj;
+            dv[last ? q : swizzled<V>(q)] = left ? vi : vj;
+            if (left) {
+                if (++i < ei) ki = kat(i), vi = vat(i), ti = tat(i);
+            } else {
+                if (++j < ej) kj = kat(j), vj = vat(j), tj = tat(j);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// The segments of a sort: positions [b, e) (cells) or n entries from off.
+struct Segs {
+    const int32_t *b, *e;
+    const int64_t *off, *n;
+    __device__ int64_t begin(int i) const { return b ? b[i] : off[i]; }
+    __device__ int64_t size(int i) const { return b ? e[i] - b[i] : n[i]; }
+};
+
+constexpr size_t kTileSmem = sizeof(unsigned long long) * 4 * kSub;
+
+// Sorts tiles of kSub keys of every segment, in place: 17 us a tile (a bitonic
+// network over 16-byte keys took 70).
+__global__ void __launch_bounds__(kSubThreads) k_sort_tiles(Key *keys, Segs sg, int nseg) {
+    extern __shared__ __align__(16) unsigned long long tile[];
+    for (int i = blockIdx.y; i < nseg; i += gridDim.y) {
+        const int64_t c0 = static_cast<int64_t>(blockIdx.x) * kSub, n = sg.size(i);
+        if (c0 >= n) continue;
+        Key *k = keys + sg.begin(i) + c0;
+        const int tot = static_cast<int>(n - c0 < kSub ? n - c0 : kSub);
+        unsigned long long *sa = tile, *sb = tile + 2 * kSub;
+        merge_sort<false>(sa, sb, nullptr, tot,
+                          [&](int p, unsigned long long &a, unsigned long long &b) {
+                              a = k[p].a;
+                              b = k[p].b;
+                          });
+        for (int p = threadIdx.x; p < tot; p += blockDim.x) k[p] = Key{sa[p], sb[p]};
+        __syncthreads();
+    }
+}
+
+// Entries that the first d of the merged runs A (la) and B (lb) take from A;
+// a warp, 32 probes a round.
+__device__ int64_t warp_merge_path(const Key *A, int64_t la, const Key *B, int64_t lb, int64_t d) {
+    const int lane = threadIdx.x & 31;
+    int64_t lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
+    while (lo < hi) {
+        const int64_t step = (hi - lo + 31) / 32, i = lo + lane * step;
+        const int c = __popc(__ballot_sync(0xffffffffu, i < hi && !key_lt(B[d - 1 - i], A[i])));
+        const int64_t end = lo + c * step;
+        if (c < 32 && end < hi) hi = end;
+        if (c > 0) lo += (c - 1) * step + 1;
+    }
+    return lo;
+}
+
+// One merge pass: runs of `run` keys of every segment merged pairwise, kSub
+// outputs per CTA through shared memory.
+__global__ void __launch_bounds__(kSubThreads) k_merge_tiles(const Key *src, Key *dst, Segs sg,
+                                                             int nseg, int64_t run) {
+    extern __shared__ __align__(16) unsigned long long tile[];
+    __shared__ int64_t s_split[2];
+    unsigned long long *sa = tile, *sb = tile + kSub;
+    for (int i = blockIdx.y; i < nseg; i += gridDim.y) {
+        const int64_t c0 = static_cast<int64_t>(blockIdx.x) * kSub, n = sg.size(i);
+        if (c0 >= n) continue;
+        const int64_t base = c0 / (2 * run) * (2 * run);
+        const int64_t la = n - base < run ? n - base : run;
+        const int64_t lb = n - base - la < run ? n - base - la : run;
+        const Key *A = src + sg.begin(i) + base, *B = A + la;
+        Key *out = dst + sg.begin(i) + c0;
+        const int64_t d0 = c0 - base, d1 = d0 + kSub < la + lb ? d0 + kSub : la + lb;
+        const int warp = threadIdx.x >> 5;
+        if (warp < 2) {
+            const int64_t x = warp_merge_path(A, la, B, lb, warp ? d1 : d0);
+            if ((threadIdx.x & 31) == 0) s_split[warp] = x;
+        }
+        __syncthreads();
+        const int64_t i0 = s_split[0], j0 = d0 - i0;
+        const int na = static_cast<int>(s_split[1] - i0), tot = static_cast<int>(d1 - d0);
+        auto at = [](int q) { return swizzled<unsigned long long>(q); };
+        for (int q = threadIdx.x; q < tot; q += blockDim.x) {
+            const Key k = q < na ? A[i0 + q] : B[j0 + q - na];
+            sa[at(q)] = k.a;
+            sb[at(q)] = k.b;
+        }
+        __syncthreads();
+        const int nb = tot - na, d = 4 * threadIdx.x;
+        auto key = [&](int q) { return Key{sa[at(q)], sb[at(q)]}; };
+        if (d < tot) {
+            int lo = max(0, d - nb), hi = min(d, na);
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (!key_lt(key(na + d - 1 - mid), key(mid))) lo = mid + 1;
+                else hi = mid;
+            }
+            int x = lo, y = na + d - lo;
+            Key kx = x < na ? key(x) : Key{0ull, 0ull}, ky = y < tot ? key(y) : Key{0ull, 0ull};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (d + u >= tot) break;
+                const bool left = y >= tot || (x < na && !key_lt(ky, kx));
+                out[d + u] = left ? kx : ky;
+                if (left) {
+                    if (++x < na) kx = key(x);
+                } else {
+                    if (++y < tot) ky = key(y);
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Sorts the segments (the longest of at most `maxlen` keys); the sorted keys
+// are in *sorted, keys or tmp.
+int sort_segs(ktg_ctx *c, Key *keys, Key *tmp, const Segs &sg, int nseg, int64_t maxlen,
+              Key **sorted) {
+    *sorted = keys;
+    if (nseg == 0 || maxlen <= 1) return KTG_OK;
+    const dim3 grid(static_cast<unsigned>((maxlen + kSub - 1) / kSub), std::min(nseg, 65535));
+    k_sort_tiles<<<grid, kSubThreads, kTileSmem, c->stream>>>(keys, sg, nseg);
+    ++c->launches;
+    Key *src = keys, *dst = tmp;
+    for (int64_t run = kSub; run < maxlen; run *= 2) {
+        k_merge_tiles<<<grid, kSubThreads, kTileSmem / 2, c->stream>>>(src, dst, sg, nseg, run);
+        ++c->launches;
+        std::swap(src, dst);
+    }
+    *sorted = src;
+    KTG_CUDA(c, cudaGetLastError());
+    return KTG_OK;
+}
+
 // ---- per-level kernels --------------------------------------------------------------
 
 struct CellsDev {
@@ -581,7 +617,6 @@ struct Level {
     int32_t *m;
     double *low_area, *high_area, *cut;
     double *half_box;      // [8 na]: low box, high box
-    int64_t *bound;        // [2 na] or [4 na]: steps, edges per owner
 };
 
 // The per-cell kernels below run on a 2-D grid: y strides over the active
@@ -604,8 +639,6 @@ __global__ void k_keys_to_cells(Level L, const Key *keys, int32_t *cells) {
             cells[p] = static_cast<int32_t>(keys[p].b);
 }
 
-// One thread per block: areas and median in the reference's order, and the
-// block profile's bound.
 // ---- exact area sums ------------------------------------------------------------
 //
 // When every cell area is a multiple of 2^-q and the total times 2^q stays
@@ -711,37 +744,51 @@ __device__ __forceinline__ int32_t median_fx(const long long *pre, int32_t b, in
     return lo;
 }
 
-// One thread per block: areas and median in the reference's order (or from
-// the exact prefix when `pre` is set), and the block profile's bound.
-__global__ void k_block_split(Level L, CellsDev C, Free F, const int32_t *cells,
-                              const long long *pre, double inv_scale) {
-    const int32_t blk = blockIdx.x * blockDim.x + threadIdx.x;
+// median_fx by a warp.
+__device__ int32_t warp_median_fx(const long long *pre, int32_t b, int32_t size) {
+    if (size <= 1) return 0;
+    const int lane = threadIdx.x & 31;
+    const long long first = pre[b], tot = pre[b + size] - first;
+    int32_t lo = 1, hi = size - 1;  // answer in [lo, hi]
+    while (lo < hi) {
+        const int32_t step = (hi - lo + 31) / 32, i = lo + lane * step;
+        const bool below = i < hi && 2 * (pre[b + i] - first) < tot;  // answer past i
+        const int c = __popc(__ballot_sync(0xffffffffu, below));
+        const int32_t end = lo + c * step;
+        if (c < 32 && end < hi) hi = end;
+        if (c > 0) lo += (c - 1) * step + 1;
+    }
+    return lo;
+}
+
+// Areas and median of every block: from the exact prefix by a warp (32 probes a
+// round), or in the reference's order by one thread.
+__global__ void k_block_split(Level L, CellsDev C, const int32_t *cells, const long long *pre,
+                              double inv_scale) {
+    const int32_t blk = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
     if (blk >= L.na) return;
     const int32_t b = L.b[blk], e = L.e[blk];
     const int32_t size = e - b;
     double cell_area = 0.0, low = 0.0, high = 0.0;
     int32_t m = 0;
     if (pre) {
-        m = median_fx(pre, b, size);
+        m = warp_median_fx(pre, b, size);
         cell_area = static_cast<double>(pre[e] - pre[b]) * inv_scale;
         low = static_cast<double>(pre[b + m] - pre[b]) * inv_scale;
         high = static_cast<double>(pre[e] - pre[b + m]) * inv_scale;
-    } else {
+    } else if (lane == 0) {
         for (int32_t p = b; p < e; ++p) cell_area += C.area[cells[p]];
         while (m + 1 < size && (m == 0 || low < 0.5 * cell_area)) low += C.area[cells[b + m++]];
         for (int32_t p = b + m; p < e; ++p) high += C.area[cells[p]];
     }
+    if (lane != 0) return;
     L.m[blk] = m;
     L.low_area[blk] = low;
     L.high_area[blk] = high;
     L.cut[blk] = cell_area;  // kept until the cutline replaces it
-    int64_t st, ed;
-    profile_bound(F, L.box + 4 * blk, L.vert[blk] != 0, st, ed);
-    L.bound[2 * blk] = st;
-    L.bound[2 * blk + 1] = ed;
 }
 
-// One thread per block: profile, cutline, half boxes, half bounds.
 struct Stripes {
     int64_t *off;    // [2 na] first stripe of the half (into the arrays below)
     int32_t *count;  // [2 na]
@@ -1182,76 +1229,80 @@ __device__ int64_t cta_make_stripes(const Prof &room, const double *box, bool v,
     return ns;
 }
 
-// Profile steps of each block (half = 0) or half box (half = 1), one CTA
-// each, rows split over the threads.
-__global__ void __launch_bounds__(kT) k_steps_cta(Level L, Free F, int half, const int64_t *soff,
-                                                  Key *steps, int64_t *nsteps) {
-    const int item = blockIdx.x;
+// Profile steps of each block (half = 0) or half box (half = 1), one CTA each,
+// a warp per row; in any order (they are sorted next).
+__global__ void __launch_bounds__(1024) k_steps_cta(Level L, Free F, int half, const int64_t *soff,
+                                                    Key *steps, int64_t *nsteps) {
+    __shared__ int32_t s_rows[2];
+    __shared__ unsigned s_n;
+    const int item = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int blk = half ? item >> 1 : item;
     const double *box = half ? L.half_box + 4 * item : L.box + 4 * item;
     if (!L.vert[blk]) {
         if (threadIdx.x == 0) nsteps[item] = 0;
         return;
     }
-    int32_t r0, r1;
-    box_rows(F, box, r0, r1);
-    long long c = 0;
-    for (int32_t r = r0 + threadIdx.x; r < r1; r += blockDim.x)
-        c += row_steps(F, r, box, [](int64_t, double, double) {}, 0);
-    long long total;
-    int64_t k = block_excl64(c, total);
+    if (threadIdx.x == 0) {
+        box_rows(F, box, s_rows[0], s_rows[1]);
+        s_n = 0;
+    }
+    __syncthreads();
+    const int32_t r1 = s_rows[1];
+    const double lx = box[0], ly = box[1], ux = box[2], uy = box[3];
     Key *out = steps + soff[item];
-    auto sink = [&](int64_t q, double x, double dh) { out[q] = Key{ord(x), ord(dh)}; };
-    for (int32_t r = r0 + threadIdx.x; r < r1; r += blockDim.x) k += row_steps(F, r, box, sink, k);
-    if (threadIdx.x == 0) nsteps[item] = total;
+    for (int32_t r = s_rows[0] + warp; r < r1; r += blockDim.x >> 5) {
+        const double h = ref_min(uy, F.rowy[2 * r + 1]) - ref_max(ly, F.rowy[2 * r]);
+        if (!(h > 0.0)) continue;
+        const int64_t end = F.rowspan[r + 1];
+        for (int64_t s0 = first_span(F, r, lx); s0 < end; s0 += 32) {
+            const int64_t s = s0 + lane;
+            const bool in = s < end && F.spans[2 * s] < ux;
+            double a = 0.0, z = 0.0;
+            if (in) {
+                a = ref_max(F.spans[2 * s], lx);
+                z = ref_min(F.spans[2 * s + 1], ux);
+            }
+            const bool on = in && z > a;
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (!__any_sync(0xffffffffu, in)) break;
+            if (!m) continue;
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&s_n, 2u * __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0) + 2u * __popc(m & ((1u << lane) - 1u));
+            if (on) {
+                out[at] = Key{ord(a), ord(h)};
+                out[at + 1] = Key{ord(z), ord(-h)};
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) nsteps[item] = s_n;
 }
 
-// One CTA per block: profile, cutline, half boxes, half bounds.
+// One CTA per block: profile, cutline, half boxes.
 __global__ void __launch_bounds__(kWideT) k_block_cut_cta(Level L, Free F, const int64_t *soff,
                                                          const Key *steps, const int64_t *nsteps,
-                                                         const int64_t *eoff, double *pe, double *pp,
-                                                         int64_t *hbound) {
+                                                         const int64_t *eoff, double *pe,
+                                                         double *pp) {
     extern __shared__ __align__(16) double wide_smem[];
-    __shared__ double hb[8];
     const int blk = blockIdx.x;
     const bool v = L.vert[blk] != 0;
     const double *box = L.box + 4 * blk;
     double *e = pe + eoff[blk], *p = pp + eoff[blk];
     const int64_t n =
         cta_build_profile(F, box, v, steps + soff[blk], nsteps[blk], e, p, wide_smem);
-    if (threadIdx.x == 0) {
-        const Prof room{e, p, n};
-        const double cell_area = L.cut[blk];
-        const double share = cell_area > 0.0 ? L.low_area[blk] / cell_area : 0.5;
-        const double lo = v ? box[0] : box[1], hi = v ? box[2] : box[3];
-        const double cut = room.total() > 0.0 ? room.coordinate_at(share * room.total())
-                                              : lo + share * (hi - lo);
-        L.cut[blk] = cut;
-        for (int k = 0; k < 4; ++k) hb[k] = hb[4 + k] = box[k];
-        hb[v ? 2 : 3] = cut;
-        hb[4 + (v ? 0 : 1)] = cut;
-        for (int k = 0; k < 8; ++k) L.half_box[8 * blk + k] = hb[k];
-    }
-    __syncthreads();
-    int k[2] = {0, 0};  // obstacles overlapping each half box
-    for (int32_t o = threadIdx.x; o < F.K; o += blockDim.x) {
-        const double *ob = F.obst + 4 * o;
-        for (int side = 0; side < 2; ++side) {
-            const double *bx = hb + 4 * side;
-            if (ob[2] <= bx[0] || ob[0] >= bx[2] || ob[3] <= bx[1] || ob[1] >= bx[3]) continue;
-            ++k[side];
-        }
-    }
-    int total[2];
-    for (int side = 0; side < 2; ++side)
-        cta_excl<int>(k[side], 0, total[side], [](int x, int y) { return x + y; });
-    if ((threadIdx.x & 31) == 0 && threadIdx.x < 64) {  // a warp per side
-        const int side = threadIdx.x >> 5;
-        int64_t st, ed;
-        profile_bound(F, hb + 4 * side, v, st, ed);
-        hbound[4 * blk + 2 * side] = st;
-        hbound[4 * blk + 2 * side + 1] = ed + 2 * total[side] + 2;  // profile edges, obstacle cuts
-    }
+    if (threadIdx.x != 0) return;
+    const Prof room{e, p, n};
+    const double cell_area = L.cut[blk];
+    const double share = cell_area > 0.0 ? L.low_area[blk] / cell_area : 0.5;
+    const double lo = v ? box[0] : box[1], hi = v ? box[2] : box[3];
+    const double cut = room.total() > 0.0 ? room.coordinate_at(share * room.total())
+                                          : lo + share * (hi - lo);
+    L.cut[blk] = cut;
+    double *lb = L.half_box + 8 * blk, *hb = lb + 4;
+    for (int k = 0; k < 4; ++k) lb[k] = hb[k] = box[k];
+    (v ? lb[2] : lb[3]) = cut;
+    (v ? hb[0] : hb[1]) = cut;
 }
 
 // One CTA per half: profile, stripes (getStripes), fill state. A profile of
@@ -1307,16 +1358,52 @@ __global__ void __launch_bounds__(kWideT) k_half_stripes_cta(Level L, Free F, co
     }
 }
 
-__global__ void k_fill_keys(Level L, CellsDev C, const int32_t *cells, Key *keys) {
+// Cells of each half by (-distance from the cut, id), from the keys sorted by
+// (centre, id): the distance is monotone in that order, so the low half keeps
+// it, the high half reverses it, and cells at the same (rounded) distance go by
+// id. A run of one centre is in id order already; a run of several centres is
+// ranked by counting.
+__global__ void k_fill_order(Level L, const Key *keys, int32_t *cells) {
     for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
         const int32_t b = L.b[blk], e = L.e[blk], mid = b + L.m[blk];
-        const bool v = L.vert[blk] != 0;
         const double cut = L.cut[blk];
-        for (int32_t p = b + blockIdx.x * blockDim.x + threadIdx.x; p < e; p += gridDim.x * blockDim.x) {
-            const int32_t i = cells[p];
-            const double c = centre(C, i, v);
-            const double from = p < mid ? cut - c : c - cut;
-            keys[p] = Key{ord(-from), static_cast<unsigned long long>(i)};
+        for (int32_t p = b + blockIdx.x * blockDim.x + threadIdx.x; p < e;
+             p += gridDim.x * blockDim.x) {
+            const bool low = p < mid;
+            const int32_t hb = low ? b : mid, he = low ? mid : e;
+            auto dist = [&](int32_t q) {
+                const double c = unord(keys[q].a);
+                return ord(-(low ? cut - c : c - cut));
+            };
+            const unsigned long long d = dist(p);
+            int32_t rs = p, re = p + 1;
+            while (rs > hb && p - rs < 32 && dist(rs - 1) == d) --rs;
+            while (re < he && re - p < 32 && dist(re) == d) ++re;
+            if (p - rs == 32) {
+                int32_t lo = hb, hi = rs;
+                while (lo < hi) {
+                    const int32_t q = (lo + hi) >> 1;
+                    if (dist(q) == d) hi = q;
+                    else lo = q + 1;
+                }
+                rs = lo;
+            }
+            if (re - p == 32) {
+                int32_t lo = re, hi = he;
+                while (lo < hi) {
+                    const int32_t q = (lo + hi) >> 1;
+                    if (dist(q) == d) lo = q + 1;
+                    else hi = q;
+                }
+                re = lo;
+            }
+            const unsigned long long id = keys[p].b;
+            int32_t rank = p - rs;
+            if (re - rs > 1 && keys[rs].a != keys[re - 1].a) {
+                rank = 0;
+                for (int32_t q = rs; q < re; ++q) rank += keys[q].b < id ? 1 : 0;
+            }
+            cells[low ? rs + rank : mid + (he - re) + rank] = static_cast<int32_t>(id);
         }
     }
 }
@@ -1346,74 +1433,152 @@ __global__ void k_fill(Level L, CellsDev C, const int32_t *cells, Stripes S, int
 
 // Greedy fill from the exact prefix (fill order): stripe s of a half takes
 // positions [start_s, start_{s+1}), start_{s+1} the least position whose
-// preceding area in the stripe reaches its capacity. One CTA per half; each
-// start is found by rounds of kT-way probing of the (monotone) prefix. The
-// starts go to `sbeg`.
-__global__ void __launch_bounds__(kT) k_fill_fx(Level L, Stripes S, const long long *pre,
-                                                double inv_scale, int32_t *sbeg) {
-    __shared__ int32_t s_first;
+// preceding area in the stripe reaches its capacity; the starts go to `sbeg`.
+// The starts form a chain, so latency bounds this: one CTA per half loads the
+// prefix a window at a time and a warp finds the starts in shared memory, 32
+// probes a round, comparing integers (the area scale is a power of two, so
+// used >= cap is prefix >= base + ceil(cap x scale)). 55 us a level at 211k
+// cells (84 with every probe in global memory).
+constexpr int kFillWindow = 16384;
+constexpr size_t kFillSmem = sizeof(long long) * kFillWindow;
+
+__global__ void __launch_bounds__(1024) k_fill_fx(Level L, Stripes S, const long long *pre,
+                                                  double scale, int32_t *sbeg) {
+    extern __shared__ long long win[];
+    __shared__ int32_t s_done;
+    const int lane = threadIdx.x & 31;
     const int32_t h = blockIdx.x;
     const int32_t blk = h >> 1;
     const int32_t b = L.b[blk], e = L.e[blk], mid = b + L.m[blk];
     const int32_t p0 = (h & 1) ? mid : b, p1 = (h & 1) ? e : mid;
     const int64_t so = S.off[h];
     const int32_t ns = S.count[h];
-    int32_t at = p0;
-    for (int32_t s = 0; s < ns; ++s) {
-        if (threadIdx.x == 0) sbeg[so + s] = at;
-        if (s + 1 == ns) break;
-        const double cap = S.cap[so + s];
-        const long long base = pre[at];
-        // least k in [at, p1] with used(k) >= cap, p1 counting as true
-        auto hit = [&](int32_t k) {
-            return k >= p1 || static_cast<double>(pre[k] - base) * inv_scale >= cap;
-        };
-        int32_t lo = at, hi = p1;
-        while (hi - lo + 1 > kT) {
-            const int32_t step = (hi - lo + kT) / kT;  // ceil((hi - lo + 1) / kT)
-            if (threadIdx.x == 0) s_first = kT;
-            __syncthreads();
-            const int32_t k = min(hi, lo + (threadIdx.x + 1) * step - 1);
-            if (hit(k)) atomicMin(&s_first, static_cast<int32_t>(threadIdx.x));
-            __syncthreads();
-            const int32_t f = s_first;
-            const int32_t nlo = f == 0 ? lo : min(hi, lo + f * step - 1) + 1;
-            const int32_t nhi = min(hi, lo + (f + 1) * step - 1);
-            __syncthreads();
-            lo = nlo;
-            hi = nhi;
+    if (ns == 0) return;
+    int32_t s = 0, at = p0;
+    long long base = pre[p0];
+    auto need = [&](int32_t q) {  // area that fills stripe q (none reaches it: 2^62)
+        const double cap = q < ns ? S.cap[so + q] : 0.0;
+        return cap * scale < 0x1p62 ? __double2ll_ru(cap * scale) : 1ll << 62;
+    };
+    long long mine = need(lane);  // of stripe s - s % 32 + lane
+    if (threadIdx.x == 0) {
+        sbeg[so] = p0;
+        s_done = ns == 1 ? 1 : 0;
+    }
+    __syncthreads();
+    for (int32_t w0 = p0; !s_done; w0 += kFillWindow) {
+        const int32_t w1 = min(w0 + kFillWindow, p1);  // positions [w0, w1)
+        for (int32_t k = w0 + threadIdx.x; k < w1; k += blockDim.x) win[k - w0] = pre[k];
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            for (;;) {
+                const long long full = base + __shfl_sync(0xffffffffu, mine, s & 31);
+                int32_t lo = max(at, w0), hi = max(w1, lo);  // first hit in [lo, hi), or hi
+                while (lo < hi) {
+                    const int32_t step = (hi - lo + 31) / 32, k = lo + lane * step;
+                    const int c =
+                        __popc(__ballot_sync(0xffffffffu, k < hi && win[k - w0] < full));
+                    const int32_t end = lo + c * step;
+                    if (c < 32 && end < hi) hi = end;
+                    if (c > 0) lo += (c - 1) * step + 1;
+                }
+                if (lo >= w1 && w1 < p1) break;  // not in this window
+                at = min(lo, p1);
+                base = at < w1 ? win[at - w0] : pre[at];
+                ++s;
+                if ((s & 31) == 0) mine = need(s + lane);
+                if (lane == 0) sbeg[so + s] = at;
+                if (s + 1 == ns) {
+                    if (lane == 0) s_done = 1;
+                    break;
+                }
+            }
         }
-        if (threadIdx.x == 0) s_first = hi;
-        __syncthreads();
-        if (lo + static_cast<int32_t>(threadIdx.x) <= hi && hit(lo + threadIdx.x))
-            atomicMin(&s_first, lo + static_cast<int32_t>(threadIdx.x));
-        __syncthreads();
-        at = s_first;
         __syncthreads();
     }
 }
 
-// Stripe of every position: the last stripe of its half starting at or
-// before it.
-__global__ void k_assign_fx(Level L, const int32_t *cells, Stripes S, const int32_t *sbeg,
-                            int32_t *stripe_of) {
+// Lowest and highest centre of each stripe, a warp per stripe: the centres are
+// monotone along the fill order but for cells at one rounded distance, so only
+// the runs at a stripe's ends can hold them.
+__global__ void k_stripe_ends(Level L, CellsDev C, const int32_t *cells, Stripes S,
+                              const int32_t *sbeg) {
+    const int lane = threadIdx.x & 31;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int32_t h = blockIdx.y; h < 2 * L.na; h += gridDim.y) {
+        const int32_t blk = h >> 1;
+        const int32_t p1 = (h & 1) ? L.e[blk] : L.b[blk] + L.m[blk];
+        const int64_t so = S.off[h];
+        const int32_t ns = S.count[h];
+        const bool v = L.vert[blk] != 0;
+        const double cut = L.cut[blk];
+        for (int32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < ns; q += warps) {
+            const int32_t f = sbeg[so + q], l = q + 1 < ns ? sbeg[so + q + 1] : p1;
+            if (f >= l) continue;
+            auto cen = [&](int32_t k) { return centre(C, cells[k], v); };
+            auto dist = [&](double c) { return ord(-((h & 1) ? c - cut : cut - c)); };
+            const double cf = cen(f), cl = cen(l - 1);
+            unsigned long long mn = min(ord(cf), ord(cl)), mx = max(ord(cf), ord(cl));
+            const unsigned long long ends[2] = {dist(cf), dist(cl)};
+            for (int side = 0; side < (ends[0] == ends[1] ? 1 : 2); ++side) {
+                for (int32_t k0 = 0; k0 < l - f; k0 += 32) {
+                    const int32_t k = side ? l - 1 - k0 - lane : f + k0 + lane;
+                    bool in = k >= f && k < l;
+                    const double c = in ? cen(k) : 0.0;
+                    in = in && dist(c) == ends[side];
+                    if (in) {
+                        mn = min(mn, ord(c));
+                        mx = max(mx, ord(c));
+                    }
+                    if (!__all_sync(0xffffffffu, in)) break;
+                }
+            }
+            for (int o = 16; o > 0; o >>= 1) {
+                mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            }
+            if (lane == 0) {
+                S.lo[so + q] = mn;
+                S.hi[so + q] = mx;
+            }
+        }
+    }
+}
+
+// New position of cell i in stripe s.
+__device__ __forceinline__ void place_cell(const CellsDev &C, const Stripes &S, int32_t i, int64_t s,
+                                           bool v) {
+    const double lo = unord(S.lo[s]), hi = unord(S.hi[s]);
+    const double c0 = centre(C, i, v);
+    const double t = hi > lo ? (c0 - lo) / (hi - lo) : 0.5;
+    const double size = v ? C.w[i] : C.h[i];
+    const double a = S.a[s], bb = S.b[s];
+    const double c = a + t * (bb - a);
+    const double lim = ref_max(a, bb - size);
+    double np = c - 0.5 * size;
+    np = np < a ? a : (lim < np ? lim : np);  // std::clamp
+    (v ? C.x : C.y)[i] = np;
+}
+
+// Stripe of every position (the last of its half starting at or before it) and
+// the cell's new position.
+__global__ void k_place_fx(Level L, CellsDev C, const int32_t *cells, Stripes S,
+                           const int32_t *sbeg) {
     for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
         const int32_t b = L.b[blk], e = L.e[blk], mid = b + L.m[blk];
+        const bool v = L.vert[blk] != 0;
         for (int32_t p = b + blockIdx.x * blockDim.x + threadIdx.x; p < e; p += gridDim.x * blockDim.x) {
             const int32_t h = 2 * blk + (p < mid ? 0 : 1);
             const int64_t so = S.off[h];
             const int32_t ns = S.count[h];
-            int32_t s = -1;
-            if (ns > 0) {
-                int32_t lo = 0, hi = ns - 1;  // last s with sbeg[s] <= p (sbeg[0] <= p)
-                while (lo < hi) {
-                    const int32_t k = (lo + hi + 1) >> 1;
-                    if (sbeg[so + k] <= p) lo = k;
-                    else hi = k - 1;
-                }
-                s = static_cast<int32_t>(so + lo);
+            if (ns == 0) continue;  // a half of zero width: its cells stay where they are
+            int32_t lo = 0, hi = ns - 1;  // last s with sbeg[s] <= p (sbeg[0] <= p)
+            while (lo < hi) {
+                const int32_t k = (lo + hi + 1) >> 1;
+                if (sbeg[so + k] <= p) lo = k;
+                else hi = k - 1;
             }
-            stripe_of[cells[p]] = s;
+            place_cell(C, S, cells[p], so + lo, v);
         }
     }
 }
@@ -1437,23 +1602,12 @@ __global__ void k_stripe_minmax(Level L, CellsDev C, const int32_t *cells, Strip
 __global__ void k_new_pos(Level L, CellsDev C, const int32_t *cells, Stripes S,
                           const int32_t *stripe_of) {
     for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
-    const int32_t b = L.b[blk], e = L.e[blk];
-    const bool v = L.vert[blk] != 0;
-    for (int32_t p = b + blockIdx.x * blockDim.x + threadIdx.x; p < e; p += gridDim.x * blockDim.x) {
-        const int32_t i = cells[p];
-        const int32_t s = stripe_of[i];
-        if (s < 0) continue;
-        const double lo = unord(S.lo[s]), hi = unord(S.hi[s]);
-        const double c0 = centre(C, i, v);
-        const double t = hi > lo ? (c0 - lo) / (hi - lo) : 0.5;
-        const double size = v ? C.w[i] : C.h[i];
-        const double a = S.a[s], bb = S.b[s];
-        const double c = a + t * (bb - a);
-        const double lim = ref_max(a, bb - size);
-        double np = c - 0.5 * size;
-        np = np < a ? a : (lim < np ? lim : np);  // std::clamp
-        (v ? C.x : C.y)[i] = np;
-    }
+        const int32_t b = L.b[blk], e = L.e[blk];
+        const bool v = L.vert[blk] != 0;
+        for (int32_t p = b + blockIdx.x * blockDim.x + threadIdx.x; p < e; p += gridDim.x * blockDim.x) {
+            const int32_t i = cells[p];
+            if (stripe_of[i] >= 0) place_cell(C, S, i, stripe_of[i], v);
+        }
     }
 }
 
@@ -1468,8 +1622,6 @@ __global__ void k_new_pos(Level L, CellsDev C, const int32_t *cells, Stripes S,
 // stripe slots, sub-blocks per level, local obstacles) is left untouched
 // and flagged; the caller runs it level by level instead.
 
-constexpr int kSub = 2048;
-constexpr int kSubThreads = 512;
 constexpr int kSortCap = 4096;      // entries of the sort buffer (steps and profiles)
 constexpr int kMaxSub = 1024;       // sub-blocks of one level
 constexpr int kObstLocal = 256;     // obstacles overlapping the block
@@ -1514,6 +1666,9 @@ struct SubDesc {
     int32_t hsoff[2], hscnt[2], hslen[2];         // the halves' regions
     int32_t stoff[2], stcap[2], stcnt[2];         // the halves' stripes
 };
+
+constexpr int64_t kDescBytes = 2 * kMaxSub * sizeof(SubDesc);  // of a CTA
+static_assert(sizeof(SubDesc) % 8 == 0, "");
 
 struct SubArgs {
     SubTask *tasks;          // [cap], the first ntasks filled in
@@ -1615,111 +1770,6 @@ __device__ void sort_segments(unsigned long long *k0, unsigned long long *k1, ui
             int b, e;
             seg(g, b, e);
             net_sort(k0, k1, k2, b, e - b, me, T, [mask] { __syncwarp(mask); });
-        }
-    }
-    __syncthreads();
-}
-
-// Where entry i of a buffer of 8- or 4-byte entries lies while it is merged: a
-// thread's four outputs are consecutive, and unswizzled its 8-byte accesses
-// would meet seven other lanes' banks.
-template <typename V>
-__device__ __forceinline__ int swizzled(int i) {
-    return sizeof(V) == 8 ? i ^ ((i >> 4) & 15) : i ^ ((i >> 5) & 31);
-}
-
-// Sorts positions [0, tot), tot <= kSub, by (tag, key, val) with the whole CTA:
-// four entries per thread sorted in registers, then merges of sorted runs, each
-// thread finding its four outputs by a binary search along the merge path. tag
-// ascends with the position, so entries move only among equal tags and every
-// position keeps its tag; without Tags it is one segment. load(p, key, val)
-// gives the entries; key and val have room for 2 kSub and end with the sorted
-// ones in [0, tot).
-template <bool Tags, typename V, class Load>
-__device__ void merge_sort(unsigned long long *key, V *val, uint32_t *tag, int tot, Load load) {
-    int P = 4, levels = 0;
-    while (P < tot) P <<= 1, ++levels;
-    int buf = levels & 1;
-    const int p0 = 4 * threadIdx.x;
-    const bool on = p0 < P;
-    auto less_eq = [&](uint32_t ti, unsigned long long ki, V vi, uint32_t tj, unsigned long long kj,
-                       V vj) {
-        const bool le = (ki < kj) | ((ki == kj) & (vi <= vj));
-        return Tags ? (ti < tj) | ((ti == tj) & le) : le;
-    };
-    unsigned long long k[4];
-    V v[4];
-    uint32_t t[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        k[u] = ~0ull;
-        v[u] = static_cast<V>(~0ull);
-        t[u] = 0u;
-        if (p0 + u < tot) load(p0 + u, k[u], v[u]);
-        else if (Tags && on) tag[p0 + u] = ~0u;
-        if (Tags && on) t[u] = tag[p0 + u];
-    }
-    __syncwarp();  // all loaded before the first is stored: load may read key and val
-    if (on) {
-        auto cas = [&](int i, int j) {
-            if (t[i] == t[j] && (k[j] < k[i] || (k[j] == k[i] && v[j] < v[i]))) {
-                const unsigned long long x = k[i];
-                k[i] = k[j];
-                k[j] = x;
-                const V y = v[i];
-                v[i] = v[j];
-                v[j] = y;
-            }
-        };
-        cas(0, 1);
-        cas(2, 3);
-        cas(0, 2);
-        cas(1, 3);
-        cas(1, 2);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i = p0 + u;
-            key[buf * kSub + (levels ? swizzled<unsigned long long>(i) : i)] = k[u];
-            val[buf * kSub + (levels ? swizzled<V>(i) : i)] = v[u];
-        }
-    }
-    for (int w = 4; w < P; w <<= 1, buf ^= 1) {
-        if (w >= 128) __syncthreads();  // up to there a warp merges its own entries
-        else __syncwarp();
-        if (!on) continue;
-        const unsigned long long *sk = key + buf * kSub;
-        const V *sv = val + buf * kSub;
-        unsigned long long *dk = key + (buf ^ 1) * kSub;
-        V *dv = val + (buf ^ 1) * kSub;
-        auto kat = [&](int i) { return sk[swizzled<unsigned long long>(i)]; };
-        auto vat = [&](int i) { return sv[swizzled<V>(i)]; };
-        auto tat = [&](int i) { return Tags ? tag[i] : 0u; };
-        const int base = p0 & ~(2 * w - 1), d = p0 - base;
-        int lo = max(0, d - w), hi = min(d, w);
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1, i = base + mid, j = base + w + d - 1 - mid;
-            if (less_eq(tat(i), kat(i), vat(i), tat(j), kat(j), vat(j))) lo = mid + 1;
-            else hi = mid;
-        }
-        int i = base + lo, j = base + w + d - lo;
-        const int ei = base + w, ej = base + 2 * w;
-        unsigned long long ki = 0, kj = 0;
-        V vi = 0, vj = 0;
-        uint32_t ti = 0u, tj = 0u;
-        if (i < ei) ki = kat(i), vi = vat(i), ti = tat(i);
-        if (j < ej) kj = kat(j), vj = vat(j), tj = tat(j);
-        const bool last = 2 * w == P;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const bool left = j >= ej || (i < ei && less_eq(ti, ki, vi, tj, kj, vj));
-            const int q = p0 + u;
-            dk[last ? q : swizzled<unsigned long long>(q)] = left ? ki : kj;
-            dv[last ? q : swizzled<V>(q)] = left ? vi : vj;
-            if (left) {
-                if (++i < ei) ki = kat(i), vi = vat(i), ti = tat(i);
-            } else {
-                if (++j < ej) kj = kat(j), vj = vat(j), tj = tat(j);
-            }
         }
     }
     __syncthreads();
@@ -3105,31 +3155,55 @@ __global__ void k_clamp_die(CellsDev C, int32_t n, double lx, double ly, double 
 // Free space, obstacles and die for the legalizer, and its scratch.
 struct LalState {
     std::vector<double> rowy, spans, obst;
+    std::vector<double> side[4];  // obstacles' lx, ly, ux, uy, each sorted
     std::vector<int64_t> rowspan;
     double die[4] = {0, 0, 0, 0};
     DevBuf<double> d_rowy, d_spans, d_obst;
     DevBuf<int64_t> d_rowspan;
-    DevBuf<int32_t> binof, map, cells, cnt, stripe_of, rects, lb, le, lvert, nb_, ne_, nvert;
-    DevBuf<double> occ, lbox, lroom, nbox, nroom, low_area, high_area, cut, half_box;
-    DevBuf<int32_t> m;
-    DevBuf<int64_t> bound, hbound, soff, eoff, nsteps, hsoff, heoff, hnsteps, seg, stoff;
-    DevBuf<Key> keys, keys_tmp, steps, steps_tmp;
-    DevBuf<double> pe, pp;
-    DevBuf<int32_t> scount;
-    DevBuf<double> sa, sb, scap, sused;
-    DevBuf<unsigned long long> slo, shi;
+    DevBuf<int32_t> binof, map, cells, cnt, stripe_of, rects;
+    DevBuf<double> occ;
+    DevBuf<char> level;      // everything of the level in work (launch_lal)
+    DevBuf<Key> keys, keys_tmp;
     DevBuf<double> overflow;
     DevBuf<long long> pre, tile;
-    DevBuf<int32_t> sbeg;
     DevBuf<char> tasks;      // SubQueue (kQueueHead bytes), then the tasks
     DevBuf<unsigned> ready;
     unsigned epoch = 0;
     DevBuf<int2> tfail;
-    DevBuf<SubDesc> sdesc;
-    DevBuf<double> sstrp;
-    DevBuf<unsigned long long> sstrlh;
+    DevBuf<char> swork;      // the subtree CTAs' sub-blocks and stripes
     bool subtree_attr = false;
     bool wide_attr = false;
+    // Upper bound on the obstacles that overlap `box`: the lesser of those that
+    // meet its x range and those that meet its y range.
+    int64_t obstacle_bound(const double *box) const {
+        auto meet = [&](int k) {
+            const auto past = std::lower_bound(side[k].begin(), side[k].end(), box[k + 2]);
+            const auto before = std::upper_bound(side[k + 2].begin(), side[k + 2].end(), box[k]);
+            return (past - side[k].begin()) - (before - side[k + 2].begin());
+        };
+        return std::max<int64_t>(0, std::min(meet(0), meet(1)));
+    }
+    // Upper bound on the profile's steps and edges of `box`: the rows it can
+    // meet (as box_rows) and their spans.
+    void profile_bound(const double *box, bool vertical, int64_t &steps, int64_t &edges) const {
+        const int64_t R = static_cast<int64_t>(rowy.size() / 2);
+        int64_t lo = 0, hi = R;  // first row with box.ly < y end
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (box[1] < rowy[2 * mid + 1]) hi = mid;
+            else lo = mid + 1;
+        }
+        const int64_t r0 = lo;
+        hi = R;  // first row from r0 with y start >= box.uy
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (rowy[2 * mid] < box[3]) lo = mid + 1;
+            else hi = mid;
+        }
+        const int64_t sp = R ? rowspan[lo] - rowspan[r0] : 0;
+        steps = vertical ? 2 * sp : 0;
+        edges = (vertical ? 2 * sp : 2 * (lo - r0)) + 2;
+    }
     // counters of the last ktg_lal call (ktg_lal_stats)
     double stats[16] = {};
 };
@@ -3137,31 +3211,19 @@ struct LalState {
 void free_lal(ktg_ctx *c) {
     LalState *s = c->lal;
     if (!s) return;
-    for (auto *b : {&s->binof, &s->map, &s->cells, &s->cnt, &s->stripe_of, &s->rects, &s->lb,
-                    &s->le, &s->lvert, &s->nb_, &s->ne_, &s->nvert, &s->m, &s->scount})
+    for (auto *b : {&s->binof, &s->map, &s->cells, &s->cnt, &s->stripe_of, &s->rects})
         b->release();
-    for (auto *b : {&s->d_rowy, &s->d_spans, &s->d_obst, &s->occ, &s->lbox, &s->lroom, &s->nbox,
-                    &s->nroom, &s->low_area, &s->high_area, &s->cut, &s->half_box, &s->pe, &s->pp,
-                    &s->sa, &s->sb, &s->scap, &s->sused, &s->overflow})
-        b->release();
-    for (auto *b : {&s->d_rowspan, &s->bound, &s->hbound, &s->soff, &s->eoff, &s->nsteps,
-                    &s->hsoff, &s->heoff, &s->hnsteps, &s->seg, &s->stoff})
-        b->release();
+    for (auto *b : {&s->d_rowy, &s->d_spans, &s->d_obst, &s->occ, &s->overflow}) b->release();
+    s->d_rowspan.release();
+    s->level.release();
     s->keys.release();
     s->keys_tmp.release();
-    s->steps.release();
-    s->steps_tmp.release();
-    s->slo.release();
-    s->shi.release();
     s->pre.release();
     s->tile.release();
-    s->sbeg.release();
     s->tasks.release();
     s->tfail.release();
     s->ready.release();
-    s->sdesc.release();
-    s->sstrp.release();
-    s->sstrlh.release();
+    s->swork.release();
     delete s;
     c->lal = nullptr;
 }
@@ -3175,6 +3237,13 @@ int set_free_space(ktg_ctx *c, int64_t nrows, const double *rowy, const int64_t 
     s->rowspan.assign(rowspan, rowspan + nrows + 1);
     s->spans.assign(spans, spans + 2 * S);
     s->obst.assign(obst, obst + 4 * nobst);
+    for (int k = 0; k < 4; ++k) s->side[k].clear();
+    for (int64_t o = 0; o < nobst; ++o) {
+        const double *q = obst + 4 * o;
+        if (!(q[0] <= q[2]) || !(q[1] <= q[3])) continue;  // overlaps no box
+        for (int k = 0; k < 4; ++k) s->side[k].push_back(q[k]);
+    }
+    for (int k = 0; k < 4; ++k) std::sort(s->side[k].begin(), s->side[k].end());
     std::copy(die4, die4 + 4, s->die);
     int rc;
     if ((rc = s->d_rowy.ensure(c, 2 * nrows + 2)) || (rc = s->d_rowspan.ensure(c, nrows + 2)) ||
@@ -3297,7 +3366,7 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
     const int64_t nbins = static_cast<int64_t>(nx) * ny;
     int rc;
     if ((rc = s->binof.ensure(c, n + 1)) || (rc = s->map.ensure(c, nbins)) ||
-        (rc = s->cells.ensure(c, n + 1)) || (rc = s->stripe_of.ensure(c, n + 1)) ||
+        (rc = s->cells.ensure(c, n + 1)) ||
         (rc = s->occ.ensure(c, nbins)) || (rc = s->overflow.ensure(c, 1)) ||
         (rc = s->keys.ensure(c, n + 1)) || (rc = s->keys_tmp.ensure(c, n + 1)))
         return rc;
@@ -3368,10 +3437,11 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
         const bool grow = s->ready.cap < cap;
         if ((r2 = s->tasks.ensure(c, kQueueHead + sizeof(SubTask) * static_cast<int64_t>(cap))) ||
             (r2 = s->ready.ensure(c, cap)) || (r2 = s->tfail.ensure(c, cap)) ||
-            (r2 = s->sdesc.ensure(c, static_cast<int64_t>(grid) * 2 * kMaxSub)) ||
-            (r2 = s->sstrp.ensure(c, static_cast<int64_t>(grid) * 4 * kStripeCap)) ||
-            (r2 = s->sstrlh.ensure(c, static_cast<int64_t>(grid) * 2 * kStripeCap)))
+            (r2 = s->swork.ensure(c, c->num_sms * (kDescBytes + 6 * 8 * kStripeCap))))
             return r2;
+        double *const strp = reinterpret_cast<double *>(s->swork.p + c->num_sms * kDescBytes);
+        auto *const strlh =
+            reinterpret_cast<unsigned long long *>(strp + c->num_sms * 4 * kStripeCap);
         if (grow || s->epoch == 0xffffffffu) {
             KTG_CUDA(c, cudaMemsetAsync(s->ready.p, 0, sizeof(unsigned) * s->ready.cap, c->stream));
             s->epoch = 0;
@@ -3389,8 +3459,9 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
                                     c->stream));
         SubTask *slots = reinterpret_cast<SubTask *>(s->tasks.p + kQueueHead);
         SubArgs A{slots, nt, cap, reinterpret_cast<SubQueue *>(s->tasks.p), s->ready.p, ++s->epoch,
-                  s->tfail.p, s->cells.p, C, F, s->sdesc.p, s->sstrp.p, s->sstrlh.p, max_level,
-                  min_cells, stripe_extra, frac, c->density_limit, exact ? 1 : 0, scale, inv_scale};
+                  s->tfail.p, s->cells.p, C, F, reinterpret_cast<SubDesc *>(s->swork.p), strp,
+                  strlh, max_level, min_cells, stripe_extra, frac, c->density_limit,
+                  exact ? 1 : 0, scale, inv_scale};
         k_subtree<<<grid, kSubThreads, kSubSmem, c->stream>>>(A);
         ++c->launches;
         KTG_CUDA(c, cudaGetLastError());
@@ -3459,10 +3530,6 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
             run += cnt[r];
             he[r] = run;
         }
-        if ((r2 = s->lb.ensure(c, nreg)) || (r2 = s->le.ensure(c, nreg)) ||
-            (r2 = s->lvert.ensure(c, nreg)) || (r2 = s->lbox.ensure(c, 4 * nreg)) ||
-            (r2 = s->lroom.ensure(c, nreg)))
-            return r2;
         KTG_CUDA(c, cudaMemcpyAsync(s->cnt.p, hb.data(), sizeof(int32_t) * nreg,
                                     cudaMemcpyHostToDevice, c->stream));
         k_region_place<<<blocks_for(n), kT, 0, c->stream>>>(s->binof.p, n, s->map.p, s->cnt.p,
@@ -3518,173 +3585,155 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
             s->stats[2] += 1;
             s->stats[4] += na;
             s->stats[9] += 1;
-            if ((r2 = s->lb.ensure(c, na)) || (r2 = s->le.ensure(c, na)) ||
-                (r2 = s->lvert.ensure(c, na)) || (r2 = s->lbox.ensure(c, 4 * na)) ||
-                (r2 = s->lroom.ensure(c, na)) || (r2 = s->m.ensure(c, na)) ||
-                (r2 = s->low_area.ensure(c, na)) || (r2 = s->high_area.ensure(c, na)) ||
-                (r2 = s->cut.ensure(c, na)) || (r2 = s->half_box.ensure(c, 8 * na)) ||
-                (r2 = s->bound.ensure(c, 2 * na)) || (r2 = s->hbound.ensure(c, 4 * na)) ||
-                (r2 = s->soff.ensure(c, na)) || (r2 = s->eoff.ensure(c, na)) ||
-                (r2 = s->nsteps.ensure(c, na)) || (r2 = s->hsoff.ensure(c, 2 * na)) ||
-                (r2 = s->heoff.ensure(c, 2 * na)) || (r2 = s->hnsteps.ensure(c, 2 * na)) ||
-                (r2 = s->seg.ensure(c, 4 * na + 2)) || (r2 = s->stoff.ensure(c, 2 * na)) ||
-                (r2 = s->scount.ensure(c, 2 * na)))
-                return r2;
-            KTG_CUDA(c, cudaMemcpyAsync(s->lb.p, ab.data(), sizeof(int32_t) * na, cudaMemcpyHostToDevice, c->stream));
-            KTG_CUDA(c, cudaMemcpyAsync(s->le.p, ae.data(), sizeof(int32_t) * na, cudaMemcpyHostToDevice, c->stream));
-            KTG_CUDA(c, cudaMemcpyAsync(s->lvert.p, av.data(), sizeof(int32_t) * na, cudaMemcpyHostToDevice, c->stream));
-            KTG_CUDA(c, cudaMemcpyAsync(s->lbox.p, abox.data(), sizeof(double) * 4 * na, cudaMemcpyHostToDevice, c->stream));
-            KTG_CUDA(c, cudaMemcpyAsync(s->lroom.p, aroom.data(), sizeof(double) * na, cudaMemcpyHostToDevice, c->stream));
-            Level L{na, s->lb.p, s->le.p, s->lbox.p, s->lvert.p, s->lroom.p, s->m.p, s->low_area.p,
-                    s->high_area.p, s->cut.p, s->half_box.p, s->bound.p};
+            // Room for the profiles and stripes of the blocks (steps, edges) and
+            // of their halves, which have no more each; one copy takes the
+            // level's descriptors to the device, one brings the halves back.
+            std::vector<int64_t> soff(na), eoff(na), hsoff(2 * na), heoff(2 * na), stoff(2 * na),
+                hcap(2 * na);
+            int64_t st = 0, ed = 0, hst = 0, hed = 0, stripes = 0, max_steps = 0;
             int32_t maxlen = 0;
-            std::vector<int64_t> segs(2 * na);
             for (int32_t k = 0; k < na; ++k) {
-                maxlen = std::max(maxlen, ae[k] - ab[k]);
-                segs[2 * k] = ab[k];
-                segs[2 * k + 1] = ae[k];
-            }
-            const dim3 gcell(std::min(64, blocks_for(maxlen)), std::min(na, 65535));
-            // 1. cells by centre
-            k_centre_keys<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, s->keys.p);
-            ++c->launches;
-            if ((r2 = seg_sort(c, s->keys.p, s->keys_tmp.p, segs, s->seg))) return r2;
-            k_keys_to_cells<<<gcell, kT, 0, c->stream>>>(L, s->keys.p, s->cells.p);
-            ++c->launches;
-            // 2. areas, median, block profile bounds
-            if (exact && (r2 = fx_prefix(run))) return r2;
-            k_block_split<<<blocks_for(na), kT, 0, c->stream>>>(L, C, F, s->cells.p,
-                                                              exact ? s->pre.p : nullptr, inv_scale);
-            ++c->launches;
-            std::vector<int64_t> bound(2 * na);
-            KTG_CUDA(c, cudaMemcpyAsync(bound.data(), s->bound.p, sizeof(int64_t) * 2 * na,
-                                        cudaMemcpyDeviceToHost, c->stream));
-            KTG_CUDA(c, lal_sync(c));
-            std::vector<int64_t> soff(na), eoff(na);
-            int64_t st = 0, ed = 0;
-            for (int32_t k = 0; k < na; ++k) {
+                int64_t ks, ke;
+                s->profile_bound(&abox[4 * k], av[k] != 0, ks, ke);
+                const int64_t ko = s->obstacle_bound(&abox[4 * k]);
                 soff[k] = st;
-                st += bound[2 * k];
                 eoff[k] = ed;
-                ed += bound[2 * k + 1];
+                st += ks;
+                ed += ke;
+                max_steps = std::max(max_steps, ks);
+                maxlen = std::max(maxlen, ae[k] - ab[k]);
+                for (int side = 0; side < 2; ++side) {
+                    // pe: the profile edges; pp: the prefix, then up to `edges` cuts
+                    const int64_t edges = ke + 2 * ko + 2 + stripe_extra;
+                    hsoff[2 * k + side] = hst;
+                    heoff[2 * k + side] = hed;
+                    hcap[2 * k + side] = edges;
+                    stoff[2 * k + side] = stripes;
+                    hst += ks;
+                    hed += 2 * edges;
+                    stripes += edges;
+                }
             }
-            if ((r2 = s->steps.ensure(c, st + 1)) || (r2 = s->steps_tmp.ensure(c, st + 1)) ||
-                (r2 = s->pe.ensure(c, ed + 1)) || (r2 = s->pp.ensure(c, ed + 1)))
-                return r2;
-            KTG_CUDA(c, cudaMemcpyAsync(s->soff.p, soff.data(), sizeof(int64_t) * na, cudaMemcpyHostToDevice, c->stream));
-            KTG_CUDA(c, cudaMemcpyAsync(s->eoff.p, eoff.data(), sizeof(int64_t) * na, cudaMemcpyHostToDevice, c->stream));
-            k_steps_cta<<<na, kT, 0, c->stream>>>(L, F, 0, s->soff.p, s->steps.p, s->nsteps.p);
-            ++c->launches;
-            std::vector<int64_t> nst(na);
-            KTG_CUDA(c, cudaMemcpyAsync(nst.data(), s->nsteps.p, sizeof(int64_t) * na,
-                                        cudaMemcpyDeviceToHost, c->stream));
-            KTG_CUDA(c, lal_sync(c));
-            std::vector<int64_t> ssegs;
-            for (int32_t k = 0; k < na; ++k) {
-                ssegs.push_back(soff[k]);
-                ssegs.push_back(soff[k] + nst[k]);
-            }
-            if ((r2 = seg_sort(c, s->steps.p, s->steps_tmp.p, ssegs, s->seg))) return r2;
-            // 3. profile, cutline, half boxes and bounds
+            std::vector<char> blob;
+            auto pack = [&](const void *v, size_t bytes) {
+                const size_t at = blob.size();
+                blob.resize(at + (bytes + 7) / 8 * 8);
+                std::memcpy(blob.data() + at, v, bytes);
+                return at;
+            };
+            const size_t i32 = sizeof(int32_t) * na, i64 = sizeof(int64_t) * na;
+            const size_t o_b = pack(ab.data(), i32), o_e = pack(ae.data(), i32),
+                         o_v = pack(av.data(), i32), o_box = pack(abox.data(), 4 * i64),
+                         o_room = pack(aroom.data(), i64), o_soff = pack(soff.data(), i64),
+                         o_eoff = pack(eoff.data(), i64), o_hsoff = pack(hsoff.data(), 2 * i64),
+                         o_heoff = pack(heoff.data(), 2 * i64), o_st = pack(stoff.data(), 2 * i64),
+                         o_cap = pack(hcap.data(), 2 * i64);
+            // the level's scratch, one allocation (a new context's first call at 12k
+            // cells takes 2.5 ms; with one per array it took 5.2)
+            size_t need = 0;
+            auto carve = [&](size_t bytes) {
+                const size_t at = need;
+                need += (bytes + 255) / 256 * 256;
+                return at;
+            };
+            const size_t n_steps = std::max(st, hst) + 1, n_edges = std::max(ed, hed) + 1,
+                         n_st = stripes + 1;
+            const size_t a_blob = carve(blob.size()), a_halves = carve(8 * i64 + i32),
+                         a_low = carve(i64), a_high = carve(i64), a_cut = carve(i64),
+                         a_nsteps = carve(2 * i64), a_count = carve(2 * i32),
+                         a_steps = carve(sizeof(Key) * n_steps),
+                         a_tmp = carve(sizeof(Key) * n_steps), a_pe = carve(8 * n_edges),
+                         a_pp = carve(8 * n_edges), a_sa = carve(8 * n_st), a_sb = carve(8 * n_st),
+                         a_cap = carve(8 * n_st), a_used = carve(8 * n_st), a_lo = carve(8 * n_st),
+                         a_hi = carve(8 * n_st), a_beg = carve(4 * n_st);
+            if ((r2 = s->level.ensure(c, static_cast<int64_t>(need)))) return r2;
+            char *const slab = s->level.p;
+            auto dbl = [&](size_t at) { return reinterpret_cast<double *>(slab + at); };
+            auto i32p = [&](size_t at) { return reinterpret_cast<int32_t *>(slab + at); };
+            auto i64p = [&](size_t at) { return reinterpret_cast<int64_t *>(slab + at); };
+            auto d32 = [&](size_t o) { return i32p(a_blob + o); };
+            auto d64 = [&](size_t o) { return i64p(a_blob + o); };
+            Key *const steps = reinterpret_cast<Key *>(slab + a_steps);
+            Key *const steps_tmp = reinterpret_cast<Key *>(slab + a_tmp);
+            int64_t *const nsteps = i64p(a_nsteps);
+            int32_t *const sbeg = i32p(a_beg);
             if (!s->wide_attr) {
-                KTG_CUDA(c, cudaFuncSetAttribute(k_block_cut_cta,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(kCtaStage)));
-                KTG_CUDA(c, cudaFuncSetAttribute(k_half_stripes_cta,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(kHalfStripesSmem)));
+                const std::pair<const void *, size_t> attrs[] = {
+                    {reinterpret_cast<const void *>(k_block_cut_cta), kCtaStage},
+                    {reinterpret_cast<const void *>(k_half_stripes_cta), kHalfStripesSmem},
+                    {reinterpret_cast<const void *>(k_fill_fx), kFillSmem},
+                    {reinterpret_cast<const void *>(k_sort_tiles), kTileSmem}};
+                for (const auto &a : attrs)
+                    KTG_CUDA(c, cudaFuncSetAttribute(a.first,
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     static_cast<int>(a.second)));
                 s->wide_attr = true;
             }
-            k_block_cut_cta<<<na, kWideT, kCtaStage, c->stream>>>(
-                L, F, s->soff.p, s->steps.p, s->nsteps.p, s->eoff.p, s->pe.p, s->pp.p, s->hbound.p);
-            ++c->launches;
-            std::vector<int64_t> hbound(4 * na);
-            KTG_CUDA(c, cudaMemcpyAsync(hbound.data(), s->hbound.p, sizeof(int64_t) * 4 * na,
-                                        cudaMemcpyDeviceToHost, c->stream));
-            KTG_CUDA(c, lal_sync(c));
-            std::vector<int64_t> hsoff(2 * na), heoff(2 * na), hcap(2 * na), stoff(2 * na);
-            st = ed = 0;
-            int64_t stripes = 0;
-            for (int32_t h = 0; h < 2 * na; ++h) {
-                hsoff[h] = st;
-                st += hbound[2 * h];
-                heoff[h] = ed;
-                // pe: the profile edges; pp: the prefix, then up to `edges` cuts
-                const int64_t edges = hbound[2 * h + 1] + stripe_extra;
-                hcap[h] = edges;
-                ed += 2 * edges;
-                stoff[h] = stripes;
-                stripes += edges;
-            }
-            if ((r2 = s->steps.ensure(c, st + 1)) || (r2 = s->steps_tmp.ensure(c, st + 1)) ||
-                (r2 = s->pe.ensure(c, ed + 1)) || (r2 = s->pp.ensure(c, ed + 1)) ||
-                (r2 = s->sa.ensure(c, stripes + 1)) || (r2 = s->sb.ensure(c, stripes + 1)) ||
-                (r2 = s->scap.ensure(c, stripes + 1)) || (r2 = s->sused.ensure(c, stripes + 1)) ||
-                (r2 = s->slo.ensure(c, stripes + 1)) || (r2 = s->shi.ensure(c, stripes + 1)) ||
-                (r2 = s->bound.ensure(c, 2 * na)))
+            KTG_CUDA(c, cudaMemcpyAsync(slab + a_blob, blob.data(), blob.size(),
+                                        cudaMemcpyHostToDevice, c->stream));
+            Level L{na, d32(o_b), d32(o_e), dbl(a_blob + o_box), d32(o_v), dbl(a_blob + o_room),
+                    i32p(a_halves + 8 * i64), dbl(a_low), dbl(a_high), dbl(a_cut), dbl(a_halves)};
+            const dim3 gcell(std::min(64, blocks_for(maxlen)), std::min(na, 65535));
+            // 1. cells by centre
+            Key *order, *sorted;
+            k_centre_keys<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, s->keys.p);
+            if ((r2 = sort_segs(c, s->keys.p, s->keys_tmp.p, Segs{L.b, L.e, nullptr, nullptr}, na,
+                                maxlen, &order)))
                 return r2;
-            KTG_CUDA(c, cudaMemcpyAsync(s->hsoff.p, hsoff.data(), sizeof(int64_t) * 2 * na, cudaMemcpyHostToDevice, c->stream));
-            KTG_CUDA(c, cudaMemcpyAsync(s->heoff.p, heoff.data(), sizeof(int64_t) * 2 * na, cudaMemcpyHostToDevice, c->stream));
-            KTG_CUDA(c, cudaMemcpyAsync(s->stoff.p, stoff.data(), sizeof(int64_t) * 2 * na, cudaMemcpyHostToDevice, c->stream));
-            // cut capacity per half, read by k_half_stripes_cta
-            KTG_CUDA(c, cudaMemcpyAsync(s->hbound.p, hcap.data(), sizeof(int64_t) * 2 * na, cudaMemcpyHostToDevice, c->stream));
-            k_steps_cta<<<2 * na, kT, 0, c->stream>>>(L, F, 1, s->hsoff.p, s->steps.p, s->hnsteps.p);
-            ++c->launches;
-            std::vector<int64_t> hnst(2 * na);
-            KTG_CUDA(c, cudaMemcpyAsync(hnst.data(), s->hnsteps.p, sizeof(int64_t) * 2 * na,
-                                        cudaMemcpyDeviceToHost, c->stream));
-            KTG_CUDA(c, lal_sync(c));
-            ssegs.clear();
-            for (int32_t h = 0; h < 2 * na; ++h) {
-                ssegs.push_back(hsoff[h]);
-                ssegs.push_back(hsoff[h] + hnst[h]);
-            }
-            if ((r2 = seg_sort(c, s->steps.p, s->steps_tmp.p, ssegs, s->seg))) return r2;
+            k_keys_to_cells<<<gcell, kT, 0, c->stream>>>(L, order, s->cells.p);
+            // 2. areas and median
+            if (exact && (r2 = fx_prefix(run))) return r2;
+            k_block_split<<<blocks_for(32 * static_cast<int64_t>(na)), kT, 0, c->stream>>>(
+                L, C, s->cells.p, exact ? s->pre.p : nullptr, inv_scale);
+            // 3. profile, cutline, half boxes
+            k_steps_cta<<<na, 1024, 0, c->stream>>>(L, F, 0, d64(o_soff), steps, nsteps);
+            c->launches += 4;
+            if ((r2 = sort_segs(c, steps, steps_tmp,
+                                Segs{nullptr, nullptr, d64(o_soff), nsteps}, na, max_steps,
+                                &sorted)))
+                return r2;
+            k_block_cut_cta<<<na, kWideT, kCtaStage, c->stream>>>(
+                L, F, d64(o_soff), sorted, nsteps, d64(o_eoff), dbl(a_pe), dbl(a_pp));
             // 4. stripes per half (profile arrays: e in pe, p and the cuts in pp)
-            Stripes S{s->stoff.p, s->scount.p, s->sa.p, s->sb.p, s->scap.p, s->sused.p, s->slo.p, s->shi.p};
-            k_half_stripes_cta<<<2 * na, kWideT, kHalfStripesSmem, c->stream>>>(
-                L, F, s->hsoff.p, s->steps.p, s->hnsteps.p, s->heoff.p, s->pe.p, s->pp.p,
-                s->hbound.p, frac, c->density_limit, S, c->status);
-            // 5. fill order, fill, stripe ranges, positions
-            k_fill_keys<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, s->keys.p);
+            k_steps_cta<<<2 * na, 1024, 0, c->stream>>>(L, F, 1, d64(o_hsoff), steps,
+                                                        nsteps);
             c->launches += 2;
-            std::vector<int32_t> mh(na);
-            KTG_CUDA(c, cudaMemcpyAsync(mh.data(), s->m.p, sizeof(int32_t) * na,
-                                        cudaMemcpyDeviceToHost, c->stream));
-            std::vector<double> cuth(na);
-            KTG_CUDA(c, cudaMemcpyAsync(cuth.data(), s->cut.p, sizeof(double) * na,
-                                        cudaMemcpyDeviceToHost, c->stream));
-            KTG_CUDA(c, lal_sync(c));
-            std::vector<int64_t> fsegs;
-            for (int32_t k = 0; k < na; ++k) {
-                fsegs.push_back(ab[k]);
-                fsegs.push_back(ab[k] + mh[k]);
-                fsegs.push_back(ab[k] + mh[k]);
-                fsegs.push_back(ae[k]);
-            }
-            if ((r2 = seg_sort(c, s->keys.p, s->keys_tmp.p, fsegs, s->seg))) return r2;
-            k_keys_to_cells<<<gcell, kT, 0, c->stream>>>(L, s->keys.p, s->cells.p);
-            ++c->launches;
+            if ((r2 = sort_segs(c, steps, steps_tmp,
+                                Segs{nullptr, nullptr, d64(o_hsoff), nsteps}, 2 * na, max_steps,
+                                &sorted)))
+                return r2;
+            Stripes S{d64(o_st), i32p(a_count), dbl(a_sa), dbl(a_sb), dbl(a_cap), dbl(a_used),
+                      reinterpret_cast<unsigned long long *>(slab + a_lo),
+                      reinterpret_cast<unsigned long long *>(slab + a_hi)};
+            k_half_stripes_cta<<<2 * na, kWideT, kHalfStripesSmem, c->stream>>>(
+                L, F, d64(o_hsoff), sorted, nsteps, d64(o_heoff), dbl(a_pe), dbl(a_pp),
+                d64(o_cap), frac, c->density_limit, S, c->status);
+            // 5. fill order, fill, stripe ranges, positions
+            k_fill_order<<<gcell, kT, 0, c->stream>>>(L, order, s->cells.p);
+            c->launches += 2;
             if (exact) {
-                if ((r2 = fx_prefix(run)) || (r2 = s->sbeg.ensure(c, stripes + 1))) return r2;
-                k_fill_fx<<<2 * na, kT, 0, c->stream>>>(L, S, s->pre.p, inv_scale, s->sbeg.p);
-                k_assign_fx<<<gcell, kT, 0, c->stream>>>(L, s->cells.p, S, s->sbeg.p,
-                                                         s->stripe_of.p);
-                c->launches += 2;
+                if ((r2 = fx_prefix(run))) return r2;
+                k_fill_fx<<<2 * na, 1024, kFillSmem, c->stream>>>(L, S, s->pre.p, scale, sbeg);
+                k_stripe_ends<<<dim3(16, std::min(2 * na, 65535)), kT, 0, c->stream>>>(
+                    L, C, s->cells.p, S, sbeg);
+                k_place_fx<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, sbeg);
+                c->launches += 3;
             } else {
+                if ((r2 = s->stripe_of.ensure(c, n + 1))) return r2;
                 k_fill<<<blocks_for(2 * na), kT, 0, c->stream>>>(L, C, s->cells.p, S,
                                                                  s->stripe_of.p);
-                ++c->launches;
+                k_stripe_minmax<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, s->stripe_of.p);
+                k_new_pos<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, s->stripe_of.p);
+                c->launches += 3;
             }
-            k_stripe_minmax<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, s->stripe_of.p);
-            k_new_pos<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, s->stripe_of.p);
-            c->launches += 2;
             KTG_CUDA(c, cudaGetLastError());
             // children
-            std::vector<double> halfbox(8 * na);
-            KTG_CUDA(c, cudaMemcpyAsync(halfbox.data(), s->half_box.p, sizeof(double) * 8 * na,
+            std::vector<char> back(8 * i64 + i32);
+            KTG_CUDA(c, cudaMemcpyAsync(back.data(), slab + a_halves, back.size(),
                                         cudaMemcpyDeviceToHost, c->stream));
             KTG_CUDA(c, lal_sync(c));
+            const double *halfbox = reinterpret_cast<const double *>(back.data());
+            const int32_t *mh = reinterpret_cast<const int32_t *>(back.data() + 8 * i64);
             hb.clear();
             he.clear();
             hv.clear();

@@ -219,6 +219,31 @@ def test_lal_profile_branches(kind, subtree, gpu_ctx):
     assert np.mean(gx != x) > 0.1
 
 
+@pytest.mark.parametrize("exact", [1, 0])
+@pytest.mark.parametrize("cells,subtree", [(2047, 0), (2048, 0), (2049, 0), (2049, 2048),
+                                           (4096, 0), (4097, 2048), (6150, 2048)])
+def test_lal_level_sorts_at_tile_edges(cells, subtree, exact, gpu_ctx):
+    """Level-by-level blocks around one tile of the sort (2048 keys), two and
+    three, with many equal centres, and centres a few ulp apart whose distances
+    from the cutline round to the same value: those fill by index."""
+    raw = synth.generate(synth.spec_tiny(seed=cells, macros=2, cells=cells, nets=cells + 30))
+    nl = netlist.flatten(raw)
+    n = nl.num_movable
+    rng = np.random.default_rng(cells)
+    lx, ly, ux, uy = raw.die
+    x = lx + 0.12 * (ux - lx) * np.abs(rng.standard_normal(n))
+    y = 0.5 * (ly + uy) + 0.08 * (uy - ly) * rng.standard_normal(n)
+    x = np.where(rng.random(n) < 0.3, np.round(x / 8.0) * 8.0, x)
+    near = rng.random(n) < 0.3
+    x[near] = lx + 2.0 + np.spacing(4.0) * rng.integers(0, 60, int(near.sum()))
+    gx, gy = run_gpu(gpu_ctx, nl, 8, 1.0, x, y, subtree=subtree, exact=exact)
+    gpu_ctx.set_option("lal_subtree_cells", 2048)
+    gpu_ctx.set_option("lal_exact_sums", 1)
+    ox, oy = run_oracle(nl, 8, 1.0, x, y)
+    assert np.array_equal(gx, ox) and np.array_equal(gy, oy)
+    assert np.mean(gx != x) > 0.1
+
+
 @pytest.mark.parametrize("cells,macros,rows,seed,spread", [(60000, 150, 400, 2, 0.05),
                                                            (60000, 150, 400, 2, 0.2),
                                                            (100000, 250, 500, 3, 0.25)])
