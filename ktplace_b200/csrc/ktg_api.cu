@@ -92,7 +92,6 @@ void free_netlist(ktg_ctx *c) {
     dev_free(c->height);
     dev_free(c->area);
     dev_free(c->row_cnt);
-    dev_free(c->heavy_rows);
     dev_free(c->block_sum);
     c->have_netlist = false;
 }
@@ -104,8 +103,7 @@ void free_systems(ktg_ctx *c) {
         dev_free(s.val);
         dev_free(s.diag);
         dev_free(s.rhs);
-        dev_free(s.lo);
-        dev_free(s.hi);
+        dev_free(s.bound);
         dev_free(s.r);
         dev_free(s.z);
         dev_free(s.p);
@@ -604,12 +602,10 @@ int ktg_upload_netlist(ktg_ctx *c, const ktg_netlist_view *nl) {
     if ((rc = dev_alloc(c, &c->area, n))) return rc;
     const int64_t bpa = (n + 255) / 256;
     if ((rc = dev_alloc(c, &c->row_cnt, 2 * n))) return rc;
-    if ((rc = dev_alloc(c, &c->heavy_rows, 1 + 2 * n))) return rc;
     if ((rc = dev_alloc(c, &c->block_sum, 2 * bpa))) return rc;
     if ((rc = reserve_systems(c, n, c->cap_nnz))) return rc;
     for (auto &s2 : c->sys) {
-        if ((rc = dev_alloc(c, &s2.lo, N))) return rc;
-        if ((rc = dev_alloc(c, &s2.hi, N))) return rc;
+        if ((rc = dev_alloc(c, &s2.bound, N))) return rc;
     }
     if ((rc = reserve_partials(c, (N + 255) / 256 + 64))) return rc;
     if ((rc = upload(c, c->var_of_vertex, nl->var_of_vertex, V))) return rc;
@@ -805,10 +801,14 @@ int ktg_download_bound_pins(ktg_ctx *c, int axis, uint32_t *lo, uint32_t *hi) {
     int rc = set_device(c);
     if (rc) return rc;
     if ((rc = sync(c))) return rc;
-    if (lo && c->N)
-        KTG_CUDA(c, cudaMemcpy(lo, c->sys[axis].lo, sizeof(uint32_t) * c->N, cudaMemcpyDeviceToHost));
-    if (hi && c->N)
-        KTG_CUDA(c, cudaMemcpy(hi, c->sys[axis].hi, sizeof(uint32_t) * c->N, cudaMemcpyDeviceToHost));
+    std::vector<int4> bound(c->N);
+    if ((lo || hi) && c->N)
+        KTG_CUDA(c, cudaMemcpy(bound.data(), c->sys[axis].bound, sizeof(int4) * c->N,
+                               cudaMemcpyDeviceToHost));
+    for (int64_t k = 0; k < c->N; ++k) {
+        if (lo) lo[k] = static_cast<uint32_t>(bound[k].y);
+        if (hi) hi[k] = static_cast<uint32_t>(bound[k].z);
+    }
     return KTG_OK;
 }
 

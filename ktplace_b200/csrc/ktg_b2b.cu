@@ -2,23 +2,21 @@
 //
 // Replaces LinearSystems::buildB2B / buildB2BAxis (globalPlacer/simpl/
 // simpl_lss.cc:11-114) and simplPlacer::Impl::getHpwl (simpl_placer.cc:
-// 256-275). Five launches build both axes at once:
+// 256-275). Four launches build both axes at once:
 //
 //   k_bound_pins  one lane per net, pins staged by the warp: first-index
 //                 argmin/argmax of the pin coordinate for x and y
 //                 (simpl_lss.cc:32-45) and, from the same pass, the net's
 //                 half perimeter (HPWL of the inputs).
-//   k_row_count   one thread per (axis, movable cell): number of movable
+//   k_row_count   four lanes per (axis, movable cell): number of movable
 //                 other ends of its B2B edges (simpl_lss.cc:75-83), plus a
 //                 per-block total.
 //   k_scan_blocks one block: exclusive scan of the block totals -> the first
 //                 CSR slot of every block and nnz per axis.
-//   k_fill        one thread per (axis, movable cell): block scan of the row
-//                 counts -> row_ptr, then the row's edges in the reference's
-//                 order (simpl_lss.cc:47-73, 89-113) so that diag and rhs are
-//                 summed exactly as the reference sums them; rows with many
-//                 movable other ends go to k_fill_heavy (a warp per row,
-//                 the same edges, sums and roundings).
+//   k_fill        a CTA per (axis, 64 movable cells): row_ptr, then the rows'
+//                 edges in the reference's order (simpl_lss.cc:47-73, 89-113),
+//                 computed a thread each and summed in order, so that diag and
+//                 rhs are rounded exactly as the reference rounds them.
 //
 // Bit-exactness: the library is compiled with -fmad=false (no FMA
 // contraction, like the reference's -ffp-contract=off) and CUDA's IEEE
@@ -87,8 +85,7 @@ constexpr int kPinChunk = 64;
 template <bool WithBounds, int R = kSimpl>
 __global__ void __launch_bounds__(kBuildThreads)
     k_bound_pins(NetlistDev nl, const double *__restrict__ x, const double *__restrict__ y,
-                 uint32_t *__restrict__ lo_x, uint32_t *__restrict__ hi_x,
-                 uint32_t *__restrict__ lo_y, uint32_t *__restrict__ hi_y,
+                 int4 *__restrict__ bound_x, int4 *__restrict__ bound_y,
                  double *__restrict__ partials, unsigned *__restrict__ ticket,
                  double *__restrict__ hpwl_out, double *__restrict__ terms = nullptr) {
     __shared__ double scratch[40];
@@ -152,10 +149,8 @@ __global__ void __launch_bounds__(kBuildThreads)
     double term = 0.0;
     if (k < nl.N) {
         if (WithBounds) {
-            lo_x[k] = lx;
-            hi_x[k] = hx;
-            lo_y[k] = ly;
-            hi_y[k] = hy;
+            bound_x[k] = make_int4(s, static_cast<int32_t>(lx), static_cast<int32_t>(hx), e - s);
+            bound_y[k] = make_int4(s, static_cast<int32_t>(ly), static_cast<int32_t>(hy), e - s);
         }
         // getHalfPerimeter: 0 for an empty box; nets with < 2 pins add 0.
         if (e - s >= 2 && !(bx0 > bx1 || by0 > by1)) term = (bx1 - bx0) + (by1 - by0);
@@ -196,56 +191,11 @@ __global__ void __launch_bounds__(1024)
     if (threadIdx.x == 0) *out = total;
 }
 
-// Edges of movable cell i's row on one axis, in the reference's order.
-// Visit(cell_var, other_pos_of_cell, there, own_offset, w, raw own offset,
-// raw other offset) for every edge.
-template <int R = kSimpl, typename Visit>
-__device__ __forceinline__ void for_each_edge(const NetlistDev &nl, const double *pos,
-                                              const double *fixed, const double *off,
-                                              const uint32_t *lo, const uint32_t *hi,
-                                              double floor_len, int32_t i, Visit &&visit) {
-    const double own_pos = pos[i];
-    const int32_t e0 = nl.pin_start[i];
-    const int32_t e1 = nl.pin_start[i + 1];
-    for (int32_t e = e0; e < e1; ++e) {
-        const int2 ref = nl.pin_ref[e];
-        const int32_t k = ref.x;
-        const uint32_t q = static_cast<uint32_t>(ref.y);
-        const uint32_t l = lo[k];
-        const uint32_t h = hi[k];
-        if (l == h) continue;
-        const int32_t s = nl.net_start[k];
-        // Kraftwerk2's base, w * 2 / (p - 1), is exactly twice w / (p - 1)
-        const double base = R == kKraftwerk2 ? 2.0 * nl.net_base[k] : nl.net_base[k];
-        const double own_raw = off[s + q];
-        const double own = own_pos + own_raw;
-        const double own_offset = own - own_pos;
-        auto edge = [&](uint32_t t) {
-            const int32_t p = s + static_cast<int32_t>(t);
-            const int32_t var = nl.pin_var[p];
-            if (R == kKraftwerk2 && var == i) return;  // a second pin of the row's own cell
-            const double cp = cell_pos(pos, fixed, var, nl.pin_cell[p]);
-            const double there = cp + off[p];
-            const double w = base / ref_max(fabs(own - there), floor_len);
-            visit(var, cp, there, own_offset, w, own_raw, off[p]);
-        };
-        if (q == l || q == h) {
-            const int32_t deg = nl.net_start[k + 1] - s;
-            for (int32_t t = 0; t < deg; ++t)
-                if (static_cast<uint32_t>(t) != q) edge(static_cast<uint32_t>(t));
-        } else {
-            edge(l);
-            edge(h);
-        }
-    }
-}
-
 struct AxisArgs {
     const double *pos;
     const double *fixed;
     const double *off;
-    const uint32_t *lo;
-    const uint32_t *hi;
+    const int4 *bound;
     double floor_len;
     const double *anchor;
     int32_t *row_ptr;
@@ -255,37 +205,42 @@ struct AxisArgs {
     double *rhs;
 };
 
-// Count of movable other ends per row; per-block totals for the scan.
+// Count of movable other ends per row; per-block totals for the scan. Chains of
+// dependent gathers (pin, bound pins, net) bound it, so a row's pins are split
+// over kCountLanes lanes and one 16-byte record per net and axis answers for its
+// first pin, bound pins and degree: 45 -> 31 us at 211k cells, 14 -> 8 at 12k.
+constexpr int kCountLanes = 4;
+
 template <int R = kSimpl>
-__global__ void __launch_bounds__(kBuildThreads)
+__global__ void __launch_bounds__(kBuildThreads *kCountLanes)
     k_row_count(NetlistDev nl, AxisArgs ax, AxisArgs ay, int32_t blocks_per_axis,
                 int32_t *__restrict__ row_cnt, int64_t *__restrict__ block_sum_out) {
-    __shared__ int32_t warp_tot[kBuildThreads / kWarp];
+    __shared__ int32_t warp_tot[kBuildThreads * kCountLanes / kWarp];
     const int axis = blockIdx.x >= blocks_per_axis ? 1 : 0;
     const AxisArgs &a = axis ? ay : ax;
-    const int32_t i = (blockIdx.x - axis * blocks_per_axis) * blockDim.x + threadIdx.x;
+    const int32_t i = (blockIdx.x - axis * blocks_per_axis) * kBuildThreads +
+                      static_cast<int32_t>(threadIdx.x) / kCountLanes;
+    const int sub = threadIdx.x % kCountLanes;
     int32_t cnt = 0;
     if (i < nl.n) {
         const int32_t e0 = nl.pin_start[i];
         const int32_t e1 = nl.pin_start[i + 1];
-        for (int32_t e = e0; e < e1; ++e) {
+        for (int32_t e = e0 + sub; e < e1; e += kCountLanes) {
             const int2 ref = nl.pin_ref[e];
             const int32_t k = ref.x;
-            const uint32_t q = static_cast<uint32_t>(ref.y);
-            const uint32_t l = a.lo[k];
-            const uint32_t h = a.hi[k];
+            const int32_t q = ref.y;
+            const int4 net = a.bound[k];
+            const int32_t s = net.x, l = net.y, h = net.z;
             if (l == h) continue;
-            const int32_t s = nl.net_start[k];
             if (R == kKraftwerk2) {
                 // movable other ends that are not the row's own cell
-                const auto other = [&](uint32_t t) {
-                    const int32_t v = nl.pin_var[s + static_cast<int32_t>(t)];
+                const auto other = [&](int32_t t) {
+                    const int32_t v = nl.pin_var[s + t];
                     return v >= 0 && v != i ? 1 : 0;
                 };
                 if (q == l || q == h) {
-                    const int32_t deg = nl.net_start[k + 1] - s;
-                    for (int32_t t = 0; t < deg; ++t)
-                        if (static_cast<uint32_t>(t) != q) cnt += other(static_cast<uint32_t>(t));
+                    for (int32_t t = 0; t < net.w; ++t)
+                        if (t != q) cnt += other(t);
                 } else {
                     cnt += other(l) + other(h);
                 }
@@ -295,16 +250,18 @@ __global__ void __launch_bounds__(kBuildThreads)
                 cnt += (nl.pin_var[s + l] >= 0 ? 1 : 0) + (nl.pin_var[s + h] >= 0 ? 1 : 0);
             }
         }
-        row_cnt[axis * nl.n + i] = cnt;
     }
     int32_t v = cnt;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = 1; o < kCountLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (i < nl.n && sub == 0) row_cnt[axis * nl.n + i] = v;
+#pragma unroll
+    for (int o = kCountLanes; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
         int64_t t = 0;
-        for (int w = 0; w < kBuildThreads / kWarp; ++w) t += warp_tot[w];
+        for (int w = 0; w < kBuildThreads * kCountLanes / kWarp; ++w) t += warp_tot[w];
         block_sum_out[blockIdx.x] = t;
     }
 }
@@ -368,186 +325,210 @@ __global__ void __launch_bounds__(1024)
     }
 }
 
-// Row pointers from a block scan of the counts, then the row's entries.
-// Kraftwerk2: alpha < 0 leaves the right-hand side at zero (withRhs false).
-// Rows with at least this many movable other ends (the bound pins of large
-// nets) are filled by k_fill_heavy, one warp per row, instead of by one
-// thread: their edges are the long serial chains of dependent gathers that
-// would otherwise set the kernel's time.
-constexpr int32_t kHeavyRow = 32;
-
-template <int R = kSimpl>
-__global__ void __launch_bounds__(kBuildThreads, 4)
-    k_fill(NetlistDev nl, AxisArgs ax, AxisArgs ay, int32_t blocks_per_axis, double alpha,
-           const int32_t *__restrict__ row_cnt, const int64_t *__restrict__ block_first,
-           int64_t cap, const int *__restrict__ status, int32_t *__restrict__ heavy) {
-    __shared__ int32_t warp_tot[kBuildThreads / kWarp];
-    const int axis = blockIdx.x >= blocks_per_axis ? 1 : 0;
-    const AxisArgs &a = axis ? ay : ax;
-    const int32_t i = (blockIdx.x - axis * blocks_per_axis) * blockDim.x + threadIdx.x;
-    const int32_t cnt = (i < nl.n) ? row_cnt[axis * nl.n + i] : 0;
-    // block exclusive scan of cnt
-    int32_t incl = cnt;
-    const int lane = threadIdx.x & 31;
+// Exclusive scan over the CTA (kBuildThreads threads); the total goes to *total.
+__device__ __forceinline__ int32_t block_excl(int32_t v, int32_t *warp_tot, int32_t *total) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int32_t incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += t;
     }
-    if (lane == 31) warp_tot[threadIdx.x >> 5] = incl;
+    if (lane == 31) warp_tot[wid] = incl;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        const int32_t w = threadIdx.x < kBuildThreads / kWarp ? warp_tot[threadIdx.x] : 0;
-        int32_t wi = w;
+    int32_t before = 0, all = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t t = __shfl_up_sync(0xffffffffu, wi, o);
-            if (threadIdx.x >= o) wi += t;
-        }
-        if (threadIdx.x < kBuildThreads / kWarp) warp_tot[threadIdx.x] = wi - w;
+    for (int w = 0; w < kBuildThreads / kWarp; ++w) {
+        const int32_t t = warp_tot[w];
+        if (w < wid) before += t;
+        all += t;
     }
     __syncthreads();
-    if (i >= nl.n) return;
+    *total = all;
+    return before + incl - v;
+}
+
+// Row pointers from a block scan of the counts, then the rows' entries, for
+// kFillRows rows a CTA. Gathers bound it: four dependent ones per edge, all
+// through L1/L2. A thread takes a pin of the rows (its bound pins, its weight,
+// how many edges it has), then an edge; edge numbers come from a scan of the
+// counts, so neighbouring threads read neighbouring pins of a net and write
+// neighbouring entries, whatever the rows' lengths. The weights and right-hand
+// terms go to shared memory, from where one thread per row and sum adds them in
+// edge order. Both axes take 148 us at 211k cells (47% of the issue slots, a
+// third of the stalls on gathers; six CTAs per SM instead of five cost spills
+// and gained nothing), 19 at 12k and 15 at 300; one thread per row (a warp for
+// rows of 32 ends and more) took 218 + 75 and 79 + 29.
+// Kraftwerk2: alpha < 0 leaves the right-hand side at zero (withRhs false).
+constexpr int kFillRows = 64;
+constexpr int kFillEdges = 4 * kBuildThreads;  // edges in shared memory at once
+static_assert(kBuildThreads % kFillRows == 0 && 2 * kFillRows <= kBuildThreads, "");
+
+template <int R = kSimpl>
+__global__ void __launch_bounds__(kBuildThreads, 5)
+    k_fill(NetlistDev nl, AxisArgs ax, AxisArgs ay, int32_t blocks_per_axis,
+           int32_t groups_per_axis, double alpha, const int32_t *__restrict__ row_cnt,
+           const int64_t *__restrict__ block_first, int64_t cap, const int *__restrict__ status) {
+    constexpr int kWarps = kBuildThreads / kWarp;
+    constexpr int kPer = kFillEdges / kBuildThreads;
+    __shared__ double s_w[kFillEdges], s_term[kFillEdges];
+    __shared__ double s_own[kBuildThreads], s_off[kBuildThreads], s_base[kBuildThreads];
+    __shared__ double s_pos[kFillRows];
+    __shared__ int32_t s_first[kBuildThreads];                  // the net's first pin
+    __shared__ int32_t s_lo[kBuildThreads], s_hi[kBuildThreads];  // hi < 0: every pin but lo
+    __shared__ int32_t s_edge[kBuildThreads + 1];
+    __shared__ uint8_t s_row[kBuildThreads];
+    __shared__ int32_t s_pin[kFillRows + 1];
+    __shared__ int32_t s_cnt[kPer * kWarps];
+    __shared__ int32_t warp_tot[kWarps];
+    __shared__ int64_t s_slot;
+    static_assert(kPer * kWarps == kWarp, "one lane per count below");
     if (*status != kStatusOk) return;  // capacity exceeded: leave the buffers alone
-    int64_t slot = block_first[blockIdx.x] + warp_tot[threadIdx.x >> 5] + (incl - cnt);
-    a.row_ptr[i] = static_cast<int32_t>(slot);
-    if (cnt >= kHeavyRow) {  // left for k_fill_heavy (the order of the list is free)
-        heavy[1 + atomicAdd(heavy, 1)] = axis * nl.n + i;
-        return;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int axis = blockIdx.x >= groups_per_axis ? 1 : 0;
+    const AxisArgs &a = axis ? ay : ax;
+    const int32_t g = blockIdx.x - axis * groups_per_axis;
+    const int32_t i0 = g * kFillRows;
+    const int rows = min(kFillRows, nl.n - i0);
+    {
+        const int32_t b = i0 / kBuildThreads;
+        const int32_t i = b * kBuildThreads + tid;
+        int32_t all;
+        const int32_t before =
+            block_excl(i < nl.n ? row_cnt[axis * nl.n + i] : 0, warp_tot, &all);
+        const int64_t slot = block_first[axis * blocks_per_axis + b] + before;
+        if (i == i0) s_slot = slot;
+        if (i >= i0 && i < i0 + rows) a.row_ptr[i] = static_cast<int32_t>(slot);
     }
-    double dg = 0.0;
-    double rh = 0.0;
-    for_each_edge<R>(nl, a.pos, a.fixed, a.off, a.lo, a.hi, a.floor_len, i,
-                     [&](int32_t var, double cp, double there, double own_offset, double w,
-                         double own_raw, double other_raw) {
-                         dg += w;
-                         if (var >= 0) {
-                             if (slot < cap) {
-                                 a.col[slot] = var;
-                                 a.val[slot] = -w;
-                             }
-                             ++slot;
-                             // Kraftwerk2: w * (otherOffset - ownOffset)
-                             rh += R == kKraftwerk2 ? w * (other_raw - own_raw)
-                                                    : w * ((there - cp) - own_offset);
-                         } else {
-                             // Kraftwerk2: w * (at[other] - ownOffset)
-                             rh += R == kKraftwerk2 ? w * (there - own_raw)
-                                                    : w * (there - own_offset);
-                         }
-                     });
+    if (tid <= rows) s_pin[tid] = nl.pin_start[i0 + tid];
+    if (tid < rows) s_pos[tid] = a.pos[i0 + tid];
+    __syncthreads();
+    int64_t slot = s_slot;
+    // thread r sums row r's weights, thread kFillRows + r its right-hand terms
+    const int row = tid % kFillRows;
+    const bool adds = tid < 2 * kFillRows && row < rows;
+    double sum = 0.0;
+    for (int32_t pc = s_pin[0]; pc < s_pin[rows]; pc += kBuildThreads) {
+        const int pins = min(kBuildThreads, s_pin[rows] - pc);
+        int32_t ne = 0;
+        if (tid < pins) {
+            const int2 ref = nl.pin_ref[pc + tid];
+            const int32_t k = ref.x, q = ref.y;
+            const int4 net = a.bound[k];
+            const int32_t s = net.x, l = net.y, h = net.z, deg = net.w;
+            // Kraftwerk2's base, w * 2 / (p - 1), is exactly twice w / (p - 1)
+            const double base = R == kKraftwerk2 ? 2.0 * nl.net_base[k] : nl.net_base[k];
+            const double own_raw = a.off[s + q];
+            int lo = 0, hi = rows;  // last row starting at or before the pin
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (s_pin[mid] <= pc + tid) lo = mid;
+                else hi = mid;
+            }
+            const double own_pos = s_pos[lo];
+            const double own = own_pos + own_raw;
+            const bool bound = q == l || q == h;
+            ne = l == h ? 0 : bound ? deg - 1 : 2;
+            s_first[tid] = s;
+            s_lo[tid] = bound ? q : l;
+            s_hi[tid] = bound ? -1 : h;
+            s_base[tid] = base;
+            s_own[tid] = own;
+            s_off[tid] = R == kKraftwerk2 ? own_raw : own - own_pos;
+            if (R == kKraftwerk2) s_row[tid] = static_cast<uint8_t>(lo);
+        }
+        int32_t edges;
+        const int32_t first = block_excl(ne, warp_tot, &edges);
+        s_edge[tid] = first;
+        if (tid == 0) s_edge[kBuildThreads] = edges;
+        __syncthreads();
+        for (int32_t c0 = 0; c0 < edges; c0 += kFillEdges) {
+            int32_t var[kPer];
+            double w[kPer];
+            unsigned entry[kPer];
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) {
+                const int32_t j = c0 + u * kBuildThreads + tid;
+                var[u] = -1;
+                w[u] = 0.0;
+                double term = 0.0;
+                bool has = j < edges;
+                if (has) {
+                    int lo = 0, hi = pins;  // the pin of edge j
+                    while (hi - lo > 1) {
+                        const int mid = (lo + hi) >> 1;
+                        if (s_edge[mid] <= j) lo = mid;
+                        else hi = mid;
+                    }
+                    const int32_t at = j - s_edge[lo], lq = s_lo[lo], hq = s_hi[lo];
+                    const int32_t t = hq < 0 ? at + (at >= lq ? 1 : 0) : at == 0 ? lq : hq;
+                    const int32_t p = s_first[lo] + t;
+                    var[u] = nl.pin_var[p];
+                    // a second pin of the row's own cell is no edge
+                    if (R == kKraftwerk2) has = var[u] != i0 + s_row[lo];
+                    if (has) {
+                        const double cp = var[u] >= 0 ? a.pos[var[u]] : a.fixed[nl.pin_cell[p]];
+                        const double other_raw = a.off[p];
+                        const double there = cp + other_raw;
+                        w[u] = s_base[lo] / ref_max(fabs(s_own[lo] - there), a.floor_len);
+                        // Kraftwerk2: w * (otherOffset - ownOffset), w * (at[other] - ownOffset)
+                        term = var[u] < 0          ? w[u] * (there - s_off[lo])
+                               : R == kKraftwerk2 ? w[u] * (other_raw - s_off[lo])
+                                                  : w[u] * ((there - cp) - s_off[lo]);
+                    }
+                }
+                // (an edge left out adds 0 below, which changes no sum)
+                s_w[u * kBuildThreads + tid] = w[u];
+                s_term[u * kBuildThreads + tid] = term;
+                entry[u] = __ballot_sync(0xffffffffu, has && var[u] >= 0);
+                if (lane == 0) s_cnt[u * kWarps + wid] = __popc(entry[u]);
+            }
+            __syncthreads();
+            int32_t incl = s_cnt[lane];
+            const int32_t mine = incl;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) {
+                const int32_t before = __shfl_sync(0xffffffffu, incl - mine, u * kWarps + wid);
+                if (!((entry[u] >> lane) & 1u)) continue;
+                const int64_t to = slot + before + __popc(entry[u] & ((1u << lane) - 1u));
+                if (to < cap) {
+                    a.col[to] = var[u];
+                    a.val[to] = -w[u];
+                }
+            }
+            slot += __shfl_sync(0xffffffffu, incl, 31);
+            if (adds) {
+                const int p0 = max(s_pin[row], pc) - pc, p1 = min(s_pin[row + 1], pc + pins) - pc;
+                if (p0 < p1) {
+                    const int j0 = max(s_edge[p0], c0) - c0;
+                    const int j1 = min(p1 < pins ? s_edge[p1] : edges, c0 + kFillEdges) - c0;
+                    const double *src = tid < kFillRows ? s_w : s_term;
+                    for (int j = j0; j < j1; ++j) sum += src[j];
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+    }
+    if (!adds) return;
+    const int32_t i = i0 + row;
+    const bool diag = tid < kFillRows;
     if (R == kKraftwerk2) {
-        a.diag[i] = dg;
-        a.rhs[i] = alpha < 0.0 ? 0.0 : rh;
+        if (diag) a.diag[i] = sum;
+        else a.rhs[i] = alpha < 0.0 ? 0.0 : sum;
         return;
     }
     if (alpha > 0.0) {
-        const double p = a.pos[i];
-        const double w = alpha / ref_max(fabs(p - a.anchor[i]), a.floor_len);
-        dg += w;
-        rh += w * a.anchor[i];
+        const double w = alpha / ref_max(fabs(s_pos[row] - a.anchor[i]), a.floor_len);
+        sum += diag ? w : w * a.anchor[i];
     }
-    a.diag[i] = ref_max(dg, 1e-12);
-    a.rhs[i] = rh;
-}
-
-// One warp per heavy row: the same edges in the same order as for_each_edge,
-// 32 at a time. Each lane computes one edge (gathers, weight, the rhs term)
-// and, when the other end is movable, writes its CSR entry at its rank among
-// this chunk's entries; then every lane adds the chunk's w and rhs terms in
-// edge order, so diag and rhs round exactly as in k_fill.
-template <int R = kSimpl>
-__global__ void __launch_bounds__(kBuildThreads)
-    k_fill_heavy(NetlistDev nl, AxisArgs ax, AxisArgs ay, double alpha, int64_t cap,
-                 const int *__restrict__ status, const int32_t *__restrict__ heavy) {
-    const int lane = threadIdx.x & 31;
-    const int32_t warps = static_cast<int32_t>((gridDim.x * blockDim.x) >> 5);
-    const int32_t count = heavy[0];
-    if (*status != kStatusOk) return;
-    for (int32_t h = static_cast<int32_t>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); h < count;
-         h += warps) {
-        const int32_t code = heavy[1 + h];
-        const int axis = code >= nl.n ? 1 : 0;
-        const int32_t i = code - (axis ? nl.n : 0);
-        const AxisArgs &a = axis ? ay : ax;
-        const double own_pos = a.pos[i];
-        int64_t slot = a.row_ptr[i];
-        double dg = 0.0, rh = 0.0;
-        const int32_t e0 = nl.pin_start[i], e1 = nl.pin_start[i + 1];
-        for (int32_t e = e0; e < e1; ++e) {
-            const int2 ref = nl.pin_ref[e];
-            const int32_t k = ref.x;
-            const uint32_t q = static_cast<uint32_t>(ref.y);
-            const uint32_t l = a.lo[k], hb = a.hi[k];
-            if (l == hb) continue;
-            const int32_t s0 = nl.net_start[k];
-            const double base = R == kKraftwerk2 ? 2.0 * nl.net_base[k] : nl.net_base[k];
-            const double own_raw = a.off[s0 + q];
-            const double own = own_pos + own_raw;
-            const double own_offset = own - own_pos;
-            const bool bound = q == l || q == hb;
-            // the pin's edges: every other pin t of the net, or its lo and hi
-            const int32_t ne = bound ? nl.net_start[k + 1] - s0 : 2;
-            for (int32_t t0 = 0; t0 < ne; t0 += 32) {
-                const int32_t j = t0 + lane;
-                bool has = false, entry = false;
-                int32_t var = -1;
-                double w = 0.0, term = 0.0;
-                if (j < ne) {
-                    const uint32_t t = bound ? static_cast<uint32_t>(j) : (j == 0 ? l : hb);
-                    if (!bound || t != q) {
-                        const int32_t p = s0 + static_cast<int32_t>(t);
-                        var = nl.pin_var[p];
-                        if (!(R == kKraftwerk2 && var == i)) {
-                            has = true;
-                            const double cp = cell_pos(a.pos, a.fixed, var, nl.pin_cell[p]);
-                            const double other_raw = a.off[p];
-                            const double there = cp + other_raw;
-                            w = base / ref_max(fabs(own - there), a.floor_len);
-                            if (var >= 0) {
-                                entry = true;
-                                term = R == kKraftwerk2 ? w * (other_raw - own_raw)
-                                                        : w * ((there - cp) - own_offset);
-                            } else {
-                                term = R == kKraftwerk2 ? w * (there - own_raw)
-                                                        : w * (there - own_offset);
-                            }
-                        }
-                    }
-                }
-                const unsigned em = __ballot_sync(0xffffffffu, entry);
-                if (entry) {
-                    const int64_t at = slot + __popc(em & ((1u << lane) - 1u));
-                    if (at < cap) {
-                        a.col[at] = var;
-                        a.val[at] = -w;
-                    }
-                }
-                slot += __popc(em);
-                const unsigned hm = __ballot_sync(0xffffffffu, has);
-                for (unsigned m = hm; m; m &= m - 1) {  // edge order = lane order
-                    const int src = __ffs(m) - 1;
-                    dg += __shfl_sync(0xffffffffu, w, src);
-                    rh += __shfl_sync(0xffffffffu, term, src);
-                }
-            }
-        }
-        if (lane == 0) {
-            if (R == kKraftwerk2) {
-                a.diag[i] = dg;
-                a.rhs[i] = alpha < 0.0 ? 0.0 : rh;
-            } else {
-                if (alpha > 0.0) {
-                    const double p = a.pos[i];
-                    const double wa = alpha / ref_max(fabs(p - a.anchor[i]), a.floor_len);
-                    dg += wa;
-                    rh += wa * a.anchor[i];
-                }
-                a.diag[i] = ref_max(dg, 1e-12);
-                a.rhs[i] = rh;
-            }
-        }
-    }
+    if (diag) a.diag[i] = ref_max(sum, 1e-12);
+    else a.rhs[i] = sum;
 }
 
 // Kraftwerk2's adjustments after buildSystem: diag += move_weight and
@@ -584,7 +565,7 @@ int launch_build(ktg_ctx *c, const double *x, const double *y, double alpha, con
     KTG_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     if (c->N > 0) {
         k_bound_pins<true, R><<<net_blocks, kBuildThreads, 0, c->stream>>>(
-            nl, x, y, c->sys[0].lo, c->sys[0].hi, c->sys[1].lo, c->sys[1].hi, c->partials,
+            nl, x, y, c->sys[0].bound, c->sys[1].bound, c->partials,
             c->counters + 0, c->scalars + 0);
         ++c->launches;
     } else {
@@ -594,22 +575,20 @@ int launch_build(ktg_ctx *c, const double *x, const double *y, double alpha, con
     for (int axis = 0; axis < 2; ++axis) {
         ktg::AxisSystem &s = c->sys[axis];
         a[axis] = AxisArgs{axis ? y : x, axis ? c->fixed_y : c->fixed_x, axis ? c->off_y : c->off_x,
-                           s.lo, s.hi, axis ? floor_y : floor_x, axis ? ay : ax,
+                           s.bound, axis ? floor_y : floor_x, axis ? ay : ax,
                            s.row_ptr, s.col, s.val, s.diag, s.rhs};
     }
     if (n > 0) {
-        k_row_count<R><<<2 * bpa, kBuildThreads, 0, c->stream>>>(nl, a[0], a[1], bpa,
-                                                                 c->row_cnt, c->block_sum);
+        k_row_count<R><<<2 * bpa, kBuildThreads * kCountLanes, 0, c->stream>>>(
+            nl, a[0], a[1], bpa, c->row_cnt, c->block_sum);
         k_scan_blocks<<<1, 1024, 0, c->stream>>>(c->block_sum, bpa, n, c->cap_nnz,
                                                  c->sys[0].row_ptr, c->sys[1].row_ptr,
                                                  c->nnz_dev, c->status);
-        KTG_CUDA(c, cudaMemsetAsync(c->heavy_rows, 0, sizeof(int32_t), c->stream));
-        k_fill<R><<<2 * bpa, kBuildThreads, 0, c->stream>>>(nl, a[0], a[1], bpa, alpha,
+        const int32_t gpa = (n + kFillRows - 1) / kFillRows;
+        k_fill<R><<<2 * gpa, kBuildThreads, 0, c->stream>>>(nl, a[0], a[1], bpa, gpa, alpha,
                                                             c->row_cnt, c->block_sum, c->cap_nnz,
-                                                            c->status, c->heavy_rows);
-        k_fill_heavy<R><<<8 * c->num_sms, kBuildThreads, 0, c->stream>>>(
-            nl, a[0], a[1], alpha, c->cap_nnz, c->status, c->heavy_rows);
-        c->launches += 4;
+                                                            c->status);
+        c->launches += 3;
     } else {
         KTG_CUDA(c, cudaMemsetAsync(c->sys[0].row_ptr, 0, sizeof(int32_t), c->stream));
         KTG_CUDA(c, cudaMemsetAsync(c->sys[1].row_ptr, 0, sizeof(int32_t), c->stream));
@@ -660,7 +639,7 @@ int launch_hpwl(ktg_ctx *c, const double *x, const double *y, double *out_dev) {
             c->hpwl_terms_cap = c->N;
         }
         k_bound_pins<false><<<net_blocks, kBuildThreads, 0, c->stream>>>(
-            nl, x, y, nullptr, nullptr, nullptr, nullptr, c->partials, c->counters + 0, out_dev,
+            nl, x, y, nullptr, nullptr, c->partials, c->counters + 0, out_dev,
             c->hpwl_terms);
         k_hpwl_ref_order<<<1, 1024, 0, c->stream>>>(c->hpwl_terms, c->N, out_dev);
         c->launches += 2;
@@ -668,7 +647,7 @@ int launch_hpwl(ktg_ctx *c, const double *x, const double *y, double *out_dev) {
         return KTG_OK;
     }
     k_bound_pins<false><<<net_blocks, kBuildThreads, 0, c->stream>>>(
-        nl, x, y, nullptr, nullptr, nullptr, nullptr, c->partials, c->counters + 0, out_dev);
+        nl, x, y, nullptr, nullptr, c->partials, c->counters + 0, out_dev);
     ++c->launches;
     KTG_CUDA(c, cudaGetLastError());
     return KTG_OK;

@@ -7,7 +7,7 @@
 //              pin_start[n+1] i32, pin_ref[Pm] int2 (net, pin),
 //              width/height/area[n] f64
 //   systems  : per axis row_ptr[n+1] i32, col[cap] i32, val[cap] f64,
-//              diag[n], rhs[n] f64, bound pins lo/hi[N] u32
+//              diag[n], rhs[n] f64, bound pins [N] i32 x 4
 //   PCG      : per axis r, z, p, ap [n] f64, positions x/y, anchors [n] f64
 //   density  : occ_fx[bins] i64 fixed point, avail[bins] f64
 #pragma once
@@ -59,8 +59,7 @@ struct AxisSystem {
     double *val = nullptr;       // [cap]
     double *diag = nullptr;      // [n]
     double *rhs = nullptr;       // [n]
-    uint32_t *lo = nullptr;      // [N]
-    uint32_t *hi = nullptr;      // [N]
+    int4 *bound = nullptr;       // [N] net's first pin, low and high bound pin, pins
     double *r = nullptr, *z = nullptr, *p = nullptr, *ap = nullptr, *s = nullptr;  // [n]
     // mixed precision: FP32 copy of val and the inner vectors
     float *val32 = nullptr;                                                 // [cap]
@@ -156,7 +155,6 @@ struct ktg_ctx {
     double *x = nullptr, *y = nullptr, *ax = nullptr, *ay = nullptr;  // [max(n, sys_cap_n)]
     int64_t stage_cap = 0;
     int32_t *row_cnt = nullptr;      // [2n]
-    int32_t *heavy_rows = nullptr;   // [1 + 2n] B2B rows filled one warp each: count, rows
     int64_t *block_sum = nullptr;    // [2 * blocks]
     int64_t *nnz_dev = nullptr;      // [2]
     double *partials = nullptr;      // reduction partials
