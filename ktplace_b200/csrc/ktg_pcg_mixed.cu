@@ -13,6 +13,7 @@
 // A round that fails to halve the true residual is reported as a stall; the
 // C ABI then finishes the solve with the FP64 kernel from the current x.
 #include "ktg_agg.h"
+#include "ktg_allreduce.cuh"
 #include "ktg_common.cuh"
 #include "ktg_context.h"
 #include "ktg_spmv.cuh"
@@ -57,7 +58,8 @@ struct MixArgs {
     double inner_tol;
     int64_t max_inner;
     int32_t max_outer;
-    double *part;  // [8 slots][2 axes][grid]
+    double *part;  // [6 slots][2 axes][grid]
+    unsigned long long *slots;  // the Chronopoulos-Gear form's sums
     unsigned *bar_count;
     unsigned *bar_gen;
     int *status;
@@ -78,7 +80,7 @@ struct MixArgs {
     int32_t trace_cap;
 };
 
-enum MixSlot { kTRR = 0, kTBB = 1, kIRZ0 = 2, kIPAP = 3, kIRR = 4, kIRZ = 5, kIZW = 6, kTZR = 7 };
+enum MixSlot { kTRR = 0, kTBB = 1, kIRZ0 = 2, kIPAP = 3, kIRR = 4, kIRZ = 5 };
 
 __device__ __forceinline__ double *mslot(const MixArgs &A, int slot, int axis) {
     return A.part + (static_cast<size_t>(slot) * 2 + axis) * gridDim.x;
@@ -421,6 +423,19 @@ enum MixPre { kPreJacobi = 0, kPreLearned = 1, kPreAgg = 2 };
 //   aggregation: the system is renumbered so that every aggregate lies in
 //     one block's rows; u = (block inverse) r reads the block's own slice
 //     after a __syncthreads, with no extra grid barrier.
+//
+// The sums of an iteration are one record exchange (ktg_allreduce.cuh), after
+// which one lane per axis advances the scalars. Arrival counter, partials read
+// back by every thread and scalars in every thread took 7.8 us of a 23 us
+// iteration at 47k cells.
+struct CgAxis {
+    double b_norm, true_resid, target, gamma, alpha, ztr, zts;
+    float alpha32, beta32, cu;  // cu: the coefficient c of z in the next u
+    unsigned active, stalled, live, in_live, ok, first;
+    int32_t outer;
+    int64_t inner;
+};
+
 template <int PRE>
 __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
     extern __shared__ __align__(16) double dyn[];
@@ -498,11 +513,9 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
         sx[l] = sax[axis].x[i];
         if (coarse) szaz[l] = __ldg(A.zaz + r0 + l);
     }
-    double einv[2] = {0.0, 0.0};
-    if (coarse) {
-        einv[0] = __ldg(A.coarse_einv);
-        einv[1] = __ldg(A.coarse_einv + 1);
-    }
+    __shared__ CgAxis st[2];
+    if (threadIdx.x < 2) st[threadIdx.x] = CgAxis{};
+    AllReduce<kSumWords> red{A.slots, A.status, 0u, total_deadline, A.barrier_timeout_ns};
     __syncthreads();
 
     // u = M r for own rows with the aggregation preconditioner: the block
@@ -553,18 +566,12 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
             });
     };
 
-    double b_norm[2] = {0.0, 0.0}, true_resid[2] = {0.0, 0.0}, prev_resid[2] = {0.0, 0.0};
-    bool active[2] = {false, false}, stalled[2] = {false, false};
-    int32_t outer[2] = {0, 0};
-    int64_t inner[2] = {0, 0};
-
     stamp(1);
     for (int round = 0;; ++round) {
         stamp(2);
         // ---- FP64 residual r = b - A x; r32, and u (Jacobi) or D^-1/2 r -----
         {
-            // rr x, bb x, rr y, bb y, z.r x, z.r y
-            double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // rr, bb, z.r per axis
             warp_tile_spmv<double>(
                 r0, n0, R, kAllAxes, wb, tile64,
                 [&](int pass, const int32_t *&rp, const int32_t *&col, const double *&val,
@@ -591,73 +598,57 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
                     }
                     const double zr = coarse ? static_cast<double>(szaz[l].x) * r : 0.0;
                     if (axis) {  // per-axis sums in registers (no runtime array index)
-                        acc[2] += r * r;
-                        acc[3] += b * b;
+                        acc[3] += r * r;
+                        acc[4] += b * b;
                         acc[5] += zr;
                     } else {
                         acc[0] += r * r;
                         acc[1] += b * b;
-                        acc[4] += zr;
+                        acc[2] += zr;
                     }
                 });
             if (PRE == kPreAgg) apply_blocks(kAllAxes);
-            const int sl[6] = {kTRR, kTBB, kTRR, kTBB, kTZR, kTZR};
-            const int ax[6] = {0, 0, 1, 1, 0, 1};
-            mstore<6>(A, acc, sl, ax, scratch);
-        }
-        if (!sync()) return;
-        bool live[2];
-        double r_norm[2];
-        // coarse state per axis: z^T r and z^T s by recurrence, and the
-        // coefficient c of z in the current u
-        double ztr[2] = {0.0, 0.0}, zts[2] = {0.0, 0.0};
-        float cu[2] = {0.0f, 0.0f};
-        {
-            double s[6];
-            const int sl[6] = {kTRR, kTBB, kTRR, kTBB, kTZR, kTZR};
-            const int ax[6] = {0, 0, 1, 1, 0, 1};
-            mreduce<6>(A, s, sl, ax, scratch);
-            if (coarse) {
-#pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    ztr[a] = s[4 + a];
-                    cu[a] = static_cast<float>(einv[a] * ztr[a]);
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < 2; ++a) {
+            const bool fine = red.sum<true, 3>(acc, scratch, [&](int a, const double(&t)[3]) {
+                if ((threadIdx.x & 31) != 0) return;
+                CgAxis &v = st[a];
                 if (round == 0) {
-                    b_norm[a] = sqrt(s[a * 2 + 1]);
-                    active[a] = b_norm[a] > 0.0;
+                    v.b_norm = sqrt(t[1]);
+                    v.active = v.b_norm > 0.0;
                 }
-                r_norm[a] = sqrt(s[a * 2 + 0]);
-                if (active[a]) {
-                    prev_resid[a] = true_resid[a];
-                    true_resid[a] = r_norm[a] / b_norm[a];
-                    if (round > 0 && outer[a] > 0 && !(true_resid[a] < 0.5 * prev_resid[a]) &&
-                        true_resid[a] > A.tol)
-                        stalled[a] = true;
+                const double r_norm = sqrt(t[0]);
+                if (v.active) {
+                    const double before = v.true_resid;
+                    v.true_resid = r_norm / v.b_norm;
+                    if (round > 0 && v.outer > 0 && !(v.true_resid < 0.5 * before) &&
+                        v.true_resid > A.tol)
+                        v.stalled = 1;
                 }
-                live[a] = active[a] && !stalled[a] && true_resid[a] > A.tol &&
-                          outer[a] < A.max_outer && inner[a] < A.max_inner;
-            }
-            if (blockIdx.x == 0 && threadIdx.x == 0 && round > 0 && round - 1 < A.hist_cap) {
-                if (A.hist_x) A.hist_x[round - 1] = true_resid[0];
-                if (A.hist_y) A.hist_y[round - 1] = true_resid[1];
-            }
+                v.live = v.active && !v.stalled && v.true_resid > A.tol &&
+                         v.outer < A.max_outer && v.inner < A.max_inner;
+                // inner stop: the round's reduction inner_tol, or as soon as the
+                // correction is good enough to finish (half the tolerance left over)
+                v.target = fmax(A.inner_tol * r_norm, kFinish * A.tol * v.b_norm);
+                v.in_live = v.live;
+                v.first = 1;
+                // coarse state: z^T r and z^T s by recurrence
+                v.zts = 0.0;
+                v.ztr = t[2];
+                v.cu = coarse ? static_cast<float>(__ldg(A.coarse_einv + a) * t[2]) : 0.0f;
+                double *hist = a ? A.hist_y : A.hist_x;
+                if (blockIdx.x == 0 && round > 0 && round - 1 < A.hist_cap && hist)
+                    hist[round - 1] = v.true_resid;
+            });
+            if (!fine) return;
         }
+        const bool live[2] = {st[0].live != 0, st[1].live != 0};
         if (!(live[0] || live[1])) break;
         if (pre) {
             apply_m(axis_mask(live[0], live[1]));
             if (!sync()) return;
         }
         // ---- inner FP32 PCG (Chronopoulos-Gear) -------------------------------
+        float cu[2] = {st[0].cu, st[1].cu};
         bool in_live[2] = {live[0], live[1]}, first[2] = {true, true};
-        double gamma_prev[2] = {0.0, 0.0}, alpha_prev[2] = {0.0, 0.0};
-        // inner stop: the round's reduction inner_tol, or as soon as the
-        // correction is good enough to finish (half the tolerance left over)
-        const double target[2] = {fmax(A.inner_tol * r_norm[0], kFinish * A.tol * b_norm[0]),
-                                  fmax(A.inner_tol * r_norm[1], kFinish * A.tol * b_norm[1])};
         stamp(3);
         for (;;) {
             // gamma, delta, rr, z.w per axis
@@ -701,66 +692,44 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
                         acc[3] += zw;
                     }
                 });
-            if (coarse) {  // one block sum for both axes (each value summed as alone)
-                const int sl[8] = {kIRZ, kIPAP, kIRR, kIZW, kIRZ, kIPAP, kIRR, kIZW};
-                const int ax[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-                mstore<8>(A, acc, sl, ax, scratch);
-            } else {
-                double a6[6] = {acc[0], acc[1], acc[2], acc[4], acc[5], acc[6]};
-                const int sl[6] = {kIRZ, kIPAP, kIRR, kIRZ, kIPAP, kIRR};
-                const int ax[6] = {0, 0, 0, 1, 1, 1};
-                mstore<6>(A, a6, sl, ax, scratch);
-            }
             stamp(4);
-            if (!sync()) return;
-            float alpha[2] = {0.0f, 0.0f}, beta[2] = {0.0f, 0.0f};
-            float cu_next[2] = {cu[0], cu[1]};
-            bool ok[2] = {false, false};
-            {
-                double s[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                if (coarse) {
-                    const int sl[8] = {kIRZ, kIPAP, kIRR, kIZW, kIRZ, kIPAP, kIRR, kIZW};
-                    const int ax[8] = {0, 0, 0, 0, 1, 1, 1, 1};
-                    mreduce<8>(A, s, sl, ax, scratch);
-                } else {
-                    double s6[6];
-                    const int sl[6] = {kIRZ, kIPAP, kIRR, kIRZ, kIPAP, kIRR};
-                    const int ax[6] = {0, 0, 0, 1, 1, 1};
-                    mreduce<6>(A, s6, sl, ax, scratch);
-                    s[0] = s6[0], s[1] = s6[1], s[2] = s6[2];
-                    s[4] = s6[3], s[5] = s6[4], s[6] = s6[5];
+            const bool fine = red.sum<false, 4>(acc, scratch, [&](int a, const double(&t)[4]) {
+                CgAxis &v = st[a];
+                if ((threadIdx.x & 31) != 0 || !v.in_live) return;
+                const double gamma = t[0], delta = t[1], rr = t[2], zw = t[3];
+                v.ok = 0;
+                v.in_live = 0;
+                if (!(sqrt(rr) > v.target) || v.inner >= A.max_inner || !(gamma > 0.0)) return;
+                double b = 0.0, pap = delta;
+                if (!v.first) {
+                    b = gamma / v.gamma;
+                    pap = delta - b * gamma / v.alpha;
                 }
-                const double gamma[2] = {s[0], s[4]}, delta[2] = {s[1], s[5]};
-                const double rr[2] = {s[2], s[6]}, zw[2] = {s[3], s[7]};
+                if (!(pap > 0.0)) return;
+                const double al = gamma / pap;
+                v.in_live = v.ok = 1;
+                v.alpha32 = static_cast<float>(al);
+                v.beta32 = static_cast<float>(b);
+                v.gamma = gamma;
+                v.alpha = al;
+                if (coarse) {  // s = w + beta s, r -= alpha s, projected on z
+                    v.zts = v.first ? zw : zw + b * v.zts;
+                    v.ztr -= al * v.zts;
+                    v.cu = static_cast<float>(__ldg(A.coarse_einv + a) * v.ztr);
+                }
+                v.first = 0;
+                ++v.inner;
+            });
+            if (!fine) return;
+            bool ok[2];
+            float alpha[2], beta[2], cu_next[2];
 #pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    if (!in_live[a]) continue;
-                    const double res = sqrt(rr[a]);
-                    if (!(res > target[a]) || inner[a] >= A.max_inner || !(gamma[a] > 0.0)) {
-                        in_live[a] = false;
-                        continue;
-                    }
-                    double b = 0.0, pap = delta[a];
-                    if (!first[a]) {
-                        b = gamma[a] / gamma_prev[a];
-                        pap = delta[a] - b * gamma[a] / alpha_prev[a];
-                    }
-                    if (!(pap > 0.0)) {
-                        in_live[a] = false;
-                        continue;
-                    }
-                    const double al = gamma[a] / pap;
-                    ok[a] = true;
-                    alpha[a] = static_cast<float>(al);
-                    beta[a] = static_cast<float>(b);
-                    gamma_prev[a] = gamma[a];
-                    alpha_prev[a] = al;
-                    if (coarse) {  // s = w + beta s, r -= alpha s, projected on z
-                        zts[a] = first[a] ? zw[a] : zw[a] + b * zts[a];
-                        ztr[a] -= al * zts[a];
-                        cu_next[a] = static_cast<float>(einv[a] * ztr[a]);
-                    }
-                }
+            for (int a = 0; a < 2; ++a) {
+                in_live[a] = in_live[a] && st[a].in_live;
+                ok[a] = in_live[a];
+                alpha[a] = st[a].alpha32;
+                beta[a] = st[a].beta32;
+                cu_next[a] = st[a].cu;
             }
             stamp(5);
             if (!(ok[0] || ok[1])) break;
@@ -793,7 +762,6 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
 #pragma unroll
             for (int a = 0; a < 2; ++a) {
                 if (!ok[a]) continue;
-                ++inner[a];
                 first[a] = false;
                 cu[a] = cu_next[a];
             }
@@ -813,22 +781,20 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
             sx[l] += static_cast<double>(sdd[l]);
             sax[axis].x[i] = sx[l];
         }
-#pragma unroll
-        for (int a = 0; a < 2; ++a)
-            if (live[a]) ++outer[a];
+        if (threadIdx.x < 2 && st[threadIdx.x].live) ++st[threadIdx.x].outer;
         if (!sync()) return;
     }
     stamp(7);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         ktg_mixed_info inf;
-        inf.resid_x = true_resid[0];
-        inf.resid_y = true_resid[1];
-        inf.inner_x = inner[0];
-        inf.inner_y = inner[1];
-        inf.outer_x = outer[0];
-        inf.outer_y = outer[1];
+        inf.resid_x = st[0].true_resid;
+        inf.resid_y = st[1].true_resid;
+        inf.inner_x = st[0].inner;
+        inf.inner_y = st[1].inner;
+        inf.outer_x = st[0].outer;
+        inf.outer_y = st[1].outer;
         inf.status = kStatusOk;
-        inf.stalled = (stalled[0] ? 1 : 0) | (stalled[1] ? 2 : 0);
+        inf.stalled = (st[0].stalled ? 1 : 0) | (st[1].stalled ? 2 : 0);
         inf.fp64_iters_x = 0;
         inf.fp64_iters_y = 0;
         *A.info = inf;
@@ -871,8 +837,15 @@ int launch_solve_mixed(ktg_ctx *c, double *x, double *y, double tol, double inne
     }
     MixArgs A;
     A.total_rows = static_cast<int32_t>(2 * nsys);
-    const int64_t want = (A.total_rows + 1023) / 1024;
-    const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(c->num_sms, want)));
+    // Blocks: 1,024 rows each, but small systems spread over up to 48 blocks of
+    // 256 rows or more, and once two solves no longer fit side by side
+    // one takes every SM (47k cells: 92 blocks took 11.5 us per product with
+    // its partial sums, 148 take 5.6).
+    const int64_t rows = A.total_rows, all = std::min(c->num_sms, 32 * kSumGroups);
+    int64_t want = rows <= 1024 ? 1 : std::max<int64_t>((rows + 1023) / 1024,
+                                                      std::min<int64_t>(48, rows / 256));
+    if (2 * want > all) want = all;
+    const int grid = static_cast<int>(std::max<int64_t>(1, std::min(all, want)));
     A.rows_per_block = static_cast<int32_t>((A.total_rows + grid - 1) / grid);
     if (A.rows_per_block == 0) A.rows_per_block = 1;
     A.blk_start = nullptr;
@@ -942,6 +915,7 @@ int launch_solve_mixed(ktg_ctx *c, double *x, double *y, double tol, double inne
     A.max_inner = max_inner;
     A.max_outer = max_outer;
     A.part = c->partials;
+    A.slots = c->sliced.slots;
     A.bar_count = c->counters + 2;
     A.bar_gen = c->counters + 3;
     A.status = c->status;
@@ -953,6 +927,10 @@ int launch_solve_mixed(ktg_ctx *c, double *x, double *y, double tol, double inne
     A.total_timeout_ns = 120000000000ull;
     KTG_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     KTG_CUDA(c, cudaMemsetAsync(c->counters + 2, 0, sizeof(unsigned), c->stream));
+    if (cg_form && grid > 1)
+        KTG_CUDA(c, cudaMemsetAsync(A.slots, 0xff,
+                                    sizeof(unsigned long long) * kSumSets * 2 * kSumWords * grid,
+                                    c->stream));
     void *args[] = {&A};
     KTG_CUDA(c, cudaLaunchCooperativeKernel((void *)fn, dim3(grid), dim3(kMixThreads), args, dyn,
                                             c->stream));

@@ -23,7 +23,7 @@
 //    and results are the same from run to run.
 //  * A row longer than `width` entries takes 2, 4, ... 32 lanes, so that no
 //    warp's slices outlast the others' (a 48-entry row on one lane did).
-//  * The two reductions per iteration are the barriers (AllReduce below), and
+//  * The two reductions per iteration are the barriers (ktg_allreduce.cuh), and
 //    the iteration's scalars are advanced by one lane per axis.
 //
 // The copy costs one pass over the CSR system and doubles as the solve's first
@@ -35,6 +35,7 @@
 // 600k 99.8 -> 70.2, 1M 158 -> 114. What bounds a step at 211k: 32k cycles of
 // gathers in the average block (28k wavefronts) and 38k in the slowest, 7k for
 // each reduction, 3k for the update.
+#include "ktg_allreduce.cuh"
 #include "ktg_common.cuh"
 #include "ktg_context.h"
 
@@ -48,15 +49,9 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMaxWidth = 24;              // entries per lane, at most (a warp per row aside)
 constexpr int kMinWidth = 8;               // even, as all widths
 constexpr int kBuckets = 2 + 3 * kMaxWidth;
-constexpr int kGroups = 5;                 // records a lane polls: at most 160 blocks
-constexpr int kRecord = 4;                 // words of a block's record
-constexpr int kSets = 4;
 constexpr int kSmallRows = 256;            // rows a block of a small system owns, at least
 constexpr int kSmallBlocks = 48;           // and blocks it has, at most
 constexpr size_t kSmemBudget = 124 * 1024;
-// A partial sum that has not been written yet. Arithmetic produces only the
-// canonical NaN, and a sum that carries this pattern is replaced by it.
-constexpr unsigned long long kUnset = ~0ull;
 
 struct SlicedAxis {
     const int32_t *rp;
@@ -96,164 +91,6 @@ struct SlicedArgs {
     uint64_t barrier_timeout_ns;
     uint64_t total_timeout_ns;
     const ktg_mixed_info *gate;  // see launch_solve
-};
-
-// K (1 or 2) words of a record.
-template <bool Acquire, int K>
-__device__ __forceinline__ void ld_words(const unsigned long long *p, unsigned long long (&u)[K]) {
-    if constexpr (K == 1) {
-        if constexpr (Acquire)
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(u[0]) : "l"(p) : "memory");
-        else
-            asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(u[0]) : "l"(p) : "memory");
-    } else {
-        if constexpr (Acquire)
-            asm volatile("ld.acquire.gpu.global.v2.u64 {%0, %1}, [%2];"
-                         : "=l"(u[0]), "=l"(u[1]) : "l"(p) : "memory");
-        else
-            asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
-                         : "=l"(u[0]), "=l"(u[1]) : "l"(p) : "memory");
-    }
-}
-
-__device__ __forceinline__ void st_relaxed_u64(unsigned long long *p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
-__device__ __forceinline__ void fence_acq_rel_gpu() {
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-}
-
-// Warp totals of K values per lane: lane k < K returns the total of value k.
-// While more than one value is left a step hands half of them to the partner
-// lane instead of exchanging all, so K values cost P - 1 + (5 - log2 P)
-// exchanges (P: K rounded up to a power of two) instead of 5 K.
-template <int K>
-__device__ __forceinline__ double warp_sums(const double (&v)[K]) {
-    constexpr int P = K == 1 ? 1 : K == 2 ? 2 : K <= 4 ? 4 : 8;
-    const int lane = threadIdx.x & 31;
-    double t[P];
-#pragma unroll
-    for (int k = 0; k < P; ++k) t[k] = k < K ? v[k] : 0.0;
-#pragma unroll
-    for (int h = P / 2; h >= 1; h >>= 1) {
-        const bool up = (lane & h) != 0;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const double give = up ? t[k] : t[k + h];
-            const double keep = up ? t[k + h] : t[k];
-            t[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
-        }
-    }
-#pragma unroll
-    for (int o = P; o < 32; o <<= 1) t[0] += __shfl_xor_sync(0xffffffffu, t[0], o);
-    return t[0];  // lane l: value l mod P
-}
-
-// Grid-wide sums that are also a grid barrier, one hop through L2: every block
-// stores its partial sums in a record of its own and polls all blocks'
-// records; the totals are added in a fixed order, the same in every block.
-// Warp a does it all for axis a (a lane polls up to kGroups records) and goes
-// straight on to that axis's scalars, so a reduction costs the block two
-// __syncthreads. 211k cells, 148 blocks: 4.5k cycles after the last arrival;
-// an arrival counter with a generation word, a read of the partials by all
-// threads and the scalars in every thread took 7k.
-//
-// A word is written and later set back to kUnset by its owner. Set b % kSets
-// serves reduction b: a block that has passed reduction b knows that every
-// block has arrived at it and so has read all records of b - 1, and resets its
-// own of that set. The reset is published by its next fence, at most two
-// reductions later, and the set is used again three later. Reductions without
-// Publish carry no fence: they order only the reads before them (whose values
-// the sums depend on) against later writes.
-struct AllReduce {
-    unsigned long long *slots;  // [kSets][grid][kRecord]: words 2 a, 2 a + 1 of axis a
-    int *status;
-    unsigned round;
-    uint64_t total_deadline;
-    uint64_t barrier_timeout;
-
-    // v: K values per thread and axis. In warp a every lane calls
-    // finish(a, totals of axis a) before the block goes on. Publish: other
-    // blocks read what this block wrote before the call. Returns false in every
-    // thread when a wait gave up. scratch holds 4 * 33 doubles.
-    template <bool Publish, int K, class Finish>
-    __device__ bool sum(const double (&v)[2 * K], double *scratch, Finish finish) {
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        const int nw = blockDim.x >> 5;
-        const int grid = gridDim.x;
-        const double wsum = warp_sums<2 * K>(v);
-        if (lane < 2 * K) scratch[lane * 33 + wid] = wsum;
-        __syncthreads();
-        int bad = 0;
-        if (wid < 2) {
-            double t[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) t[k] = lane < nw ? scratch[(wid * K + k) * 33 + lane] : 0.0;
-            double mine = warp_sums<K>(t);
-            if (grid > 1) {
-                unsigned long long *set =
-                    slots + static_cast<size_t>(round % kSets) * grid * kRecord + 2 * wid;
-                if (lane < K) {
-                    unsigned long long u =
-                        static_cast<unsigned long long>(__double_as_longlong(mine));
-                    if (u == kUnset) u = 0x7ff8000000000000ull;
-                    if (Publish) fence_acq_rel_gpu();
-                    st_relaxed_u64(set + static_cast<size_t>(blockIdx.x) * kRecord + lane, u);
-                }
-                unsigned long long u[kGroups][K];
-                unsigned wait = 0;
-#pragma unroll
-                for (int g = 0; g < kGroups; ++g) {
-#pragma unroll
-                    for (int k = 0; k < K; ++k) u[g][k] = 0ull;
-                    if (g * 32 + lane < grid) wait |= 1u << g;
-                }
-                uint64_t deadline = 0;
-                for (uint32_t spins = 1; wait; ++spins) {
-#pragma unroll
-                    for (int g = 0; g < kGroups; ++g)
-                        if ((wait >> g) & 1u)
-                            ld_words<Publish>(set + static_cast<size_t>(g * 32 + lane) * kRecord,
-                                              u[g]);
-#pragma unroll
-                    for (int g = 0; g < kGroups; ++g) {
-                        bool have = true;
-#pragma unroll
-                        for (int k = 0; k < K; ++k) have = have && u[g][k] != kUnset;
-                        if (have) wait &= ~(1u << g);
-                    }
-                    if (wait && (spins & 63u) == 0u) {
-                        const uint64_t now = global_timer_ns();
-                        if (deadline == 0) deadline = min(now + barrier_timeout, total_deadline);
-                        if (ld_relaxed_gpu(status) != kStatusOk || now > deadline) {
-                            atomicCAS(status, kStatusOk, kStatusTimeout);
-                            bad = 1;
-                            break;
-                        }
-                    }
-                }
-                __syncwarp();
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    t[k] = __longlong_as_double(static_cast<long long>(u[0][k]));
-#pragma unroll
-                    for (int g = 1; g < kGroups; ++g)
-                        t[k] += __longlong_as_double(static_cast<long long>(u[g][k]));
-                }
-                mine = warp_sums<K>(t);
-                if (round > 0 && lane < 2)
-                    st_relaxed_u64(slots + (static_cast<size_t>((round - 1) % kSets) * grid +
-                                            blockIdx.x) * kRecord + 2 * wid + lane,
-                                   kUnset);
-            }
-#pragma unroll
-            for (int k = 0; k < K; ++k) t[k] = __shfl_sync(0xffffffffu, mine, k);
-            finish(wid, t);
-        }
-        ++round;
-        return !__syncthreads_or(bad);
-    }
 };
 
 // Entry loads of the sliced copy: read once per iteration, so they bypass L1
@@ -338,7 +175,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_sliced(SlicedArgs A) {
     const size_t moff = static_cast<size_t>(blockIdx.x) * cap_slices;
     uint2 *const slices = A.S.slices + moff;
     uint2 *const mine = A.S.dealt + moff;
-    AllReduce red{A.S.slots, A.status, 0u, global_timer_ns() + A.total_timeout_ns,
+    AllReduce<2> red{A.S.slots, A.status, 0u, global_timer_ns() + A.total_timeout_ns,
                   A.barrier_timeout_ns};
     const uint64_t stream = evict_first_policy();
     __syncthreads();
@@ -754,7 +591,7 @@ int64_t sliced_entries(int64_t nnz_both, int num_sms) {
 // Slices of a block of `rows` rows: a warp per row at worst, and one end mark.
 int64_t sliced_slices(int64_t rows, int num_sms) { return rows + 2 * num_sms; }
 
-int64_t sliced_slots(int num_sms) { return int64_t(kSets) * kRecord * num_sms; }
+int64_t sliced_slots(int num_sms) { return int64_t(kSumSets) * 2 * kSumWords * num_sms; }
 
 int launch_solve_sliced(ktg_ctx *c, double *x, double *y, double tol, int64_t max_iter,
                         ktg_solve_info *info_dev, double *hist_x, double *hist_y,
@@ -777,7 +614,7 @@ int launch_solve_sliced(ktg_ctx *c, double *x, double *y, double tol, int64_t ma
             ? kThreads
             : std::min<int64_t>(kThreads, std::max<int64_t>(kSmallRows,
                                                             (total + kSmallBlocks - 1) / kSmallBlocks));
-    const int64_t most = std::min(c->num_sms, 32 * kGroups);
+    const int64_t most = std::min(c->num_sms, 32 * kSumGroups);
     const int grid = static_cast<int>(
         std::max<int64_t>(1, std::min<int64_t>(most, (total + rows - 1) / rows)));
     A.rows_per_block = static_cast<int32_t>(std::max<int64_t>(1, (total + grid - 1) / grid));
@@ -819,7 +656,7 @@ int launch_solve_sliced(ktg_ctx *c, double *x, double *y, double tol, int64_t ma
     A.total_timeout_ns = 120000000000ull;   // 120 s for the whole solve
     KTG_CUDA(c, cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
     KTG_CUDA(c, cudaMemsetAsync(c->sliced.slots, 0xff,
-                                sizeof(unsigned long long) * kSets * kRecord * grid, c->stream));
+                                sizeof(unsigned long long) * kSumSets * 4 * grid, c->stream));
     void *args[] = {&A};
     KTG_CUDA(c, cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(fn), dim3(grid),
                                             dim3(threads), args, bytes, c->stream));

@@ -68,3 +68,29 @@ def test_mixed_stall_falls_back_to_fp64(gpu_ctx):
     r = gpu_ctx.solve_mixed(x, y, TOL, inner_tol=0.999, max_outer=3)
     assert r["fp64_iters"][0] > 0 or r["fp64_iters"][1] > 0
     assert true_resid(sx, r["x"]) <= 10 * TOL
+
+
+@pytest.mark.parametrize("precond", [0, 2])
+@pytest.mark.parametrize("cells", [512, 513, 3000, 6145, 24577, 37888, 37889])
+def test_mixed_block_counts(cells, precond, gpu_ctx):
+    """Sizes around the changes of the block count (1,024 rows in one block, 48
+    small blocks, 1,024 rows each, every SM): the true residual meets the
+    tolerance, without the FP64 fallback."""
+    from ktplace_b200 import netlist, synth
+    nl = netlist.flatten(synth.generate(synth.SynthSpec(
+        num_movable=cells, num_nets=cells + cells // 20 + 8, num_pads=64,
+        num_rows=max(8, int(cells ** 0.5)), seed=cells)))
+    rng = np.random.default_rng(cells)
+    lx, ly, ux, uy = nl.die
+    x, ax = rng.uniform(lx, ux, (2, nl.num_movable))
+    y, ay = rng.uniform(ly, uy, (2, nl.num_movable))
+    fx, fy = nl.floors()
+    gpu_ctx.upload_netlist(nl)
+    gpu_ctx.set_option("precond", precond)
+    gpu_ctx.build_b2b(x, y, 0.3, ax, ay, fx, fy)
+    sx, sy = gpu_ctx.system(0), gpu_ctx.system(1)
+    r = gpu_ctx.solve_mixed(x, y, TOL)
+    gpu_ctx.set_option("precond", 0)
+    assert true_resid(sx, r["x"]) <= TOL * 1.0001
+    assert true_resid(sy, r["y"]) <= TOL * 1.0001
+    assert list(r["fp64_iters"]) == [0, 0]
