@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
         // ---- FP64 residual r = b - A x; r32, and u (Jacobi) or D^-1/2 r -----
         {
             double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // rr, bb, z.r per axis
-            warp_tile_spmv<double>(
+            warp_tile_spmv<double, true>(
                 r0, n0, R, kAllAxes, wb, tile64,
                 [&](int pass, const int32_t *&rp, const int32_t *&col, const double *&val,
                     const double *&in) {

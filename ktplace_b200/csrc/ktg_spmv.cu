@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kSpmvThreads)
     warp_row_bounds(R, wb, [&](int32_t l) {
         return int64_t(__ldg(rp + r0 + l)) - base + int64_t(kRowCost) * l;
     });
-    warp_tile_spmv<double>(
+    warp_tile_spmv<double, true>(
         r0, INT32_MAX, R, kAllAxes, wb, tilebuf,
         [&](int, const int32_t *&trp, const int32_t *&tcol, const double *&tval,
             const double *&tin) {

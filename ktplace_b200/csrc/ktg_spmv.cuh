@@ -3,8 +3,7 @@
 // Each warp takes 32 consecutive rows of its block and streams their
 // (contiguous) nonzeros in chunks of kTileChunk, every lane loading
 // consecutive entries: coalesced column and value loads and kTileQ
-// independent gathers in flight per lane (FP32 tiles issue the next chunk's
-// column loads behind them). The products go to the warp's
+// independent gathers in flight per lane. The products go to the warp's
 // slice of shared memory and each lane adds its own row's products in
 // storage order onto the row's first term, carrying the running sum across
 // chunks, so every row sum is the same sequence of roundings as a
@@ -83,11 +82,22 @@ __device__ __forceinline__ unsigned axis_mask(bool a0, bool a1) {
 //   csr(pass, rp, col, val, in): the axis's CSR arrays and gathered vector;
 //   start(l, pass, i) -> T: the row's first term (diag * own value);
 //   emit(l, pass, i, sum): the finished row sum.
-// tilebuf holds kTileChunk elements per warp, 16-byte aligned.
-template <typename T, class Csr, class Start, class Emit>
+//   gather(in, c) -> T: entry c of the vector (L2 unless said otherwise).
+// tilebuf holds kTileChunk elements per warp, 16-byte aligned. kAhead: the next
+// chunk's columns load while the chunk's own gathers are in flight, one memory
+// round trip per chunk instead of two (3% off the FP32 solves at 211k cells, 4%
+// off the FP64 product at 500k rows); the register-capped FP64 solves keep the
+// plain order, the extra registers cost them about as much.
+struct FarGather {
+    template <typename T>
+    __device__ T operator()(const T *in, int32_t c) const { return __ldcg(in + c); }
+};
+
+template <typename T, bool kAhead = sizeof(T) == 4, class Csr, class Start, class Emit,
+          class Gather = FarGather>
 __device__ __forceinline__ void warp_tile_spmv(int32_t r0, int32_t n0, int32_t R, unsigned live,
                                                const int32_t *wb, T *tilebuf, Csr csr, Start start,
-                                               Emit emit) {
+                                               Emit emit, Gather gather = {}) {
     using P2 = typename TilePair<T>::type;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -130,12 +140,6 @@ __device__ __forceinline__ void warp_tile_spmv(int32_t r0, int32_t n0, int32_t R
                     cl[q] = k < k_end ? __ldg(col + k) : -1;
                 }
             };
-            // FP32 tiles load the next chunk's columns while the chunk's own
-            // gathers are in flight (one memory round trip per chunk instead
-            // of two; 3% off the FP32 solves at 211k cells). The FP64 tiles
-            // keep the plain order: with their 8-byte products the extra
-            // registers cost the register-capped FP64 solve about as much.
-            constexpr bool kAhead = sizeof(T) == 4;
             if (kAhead) load_cols(k_begin);
 #pragma unroll 1
             for (int32_t k0 = k_begin; k0 < k_end; k0 += kTileChunk) {
@@ -144,7 +148,7 @@ __device__ __forceinline__ void warp_tile_spmv(int32_t r0, int32_t n0, int32_t R
 #pragma unroll
                 for (int q = 0; q < kTileQ; ++q) {
                     const int32_t k = k0 + lane + 32 * q;
-                    pr[q] = cl[q] >= 0 ? __ldg(val + k) * __ldcg(in + cl[q]) : T(0);
+                    pr[q] = cl[q] >= 0 ? __ldg(val + k) * gather(in, cl[q]) : T(0);
                 }
                 if (kAhead) load_cols(k0 + kTileChunk);
 #pragma unroll
