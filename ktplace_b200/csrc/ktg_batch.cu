@@ -11,6 +11,8 @@
 //     so uneven sizes balance without any grid-wide synchronisation;
 //   * FP64 Jacobi-PCG (the reference's method), or FP32 Jacobi-PCG inside FP64
 //     iterative refinement (true FP64 residual as the convergence test);
+//     the latter on a renumbered FP32 copy of the system (Jagged), with the
+//     search direction in every CTA's shared memory;
 //   * per system the device records iterations, the final residual and the
 //     solve latency (%globaltimer from dequeue to done).
 // The launch only enqueues work, so the whole batch solve is captured once
@@ -24,6 +26,7 @@
 #include <new>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "ktg_common.cuh"
@@ -50,7 +53,6 @@ struct BatchArgs {
     const int32_t *rp;     // system k's row_ptr (local offsets) at row_base + k
     const int32_t *col;
     const double *val;
-    const float *val32;
     const double *diag;
     const double *rhs;
     double *x;
@@ -63,14 +65,19 @@ struct BatchArgs {
     float *z32;
     float *p32;
     float *ap32;
+    // the mixed solve's copy of the systems (Jagged)
+    int32_t *jcol;
+    float *jval;
+    float *diag32;
+    int32_t *perm, *inv, *len, *start, *next;
     unsigned *queue;
     ktg_batch_result *results;
     double tol;
     double inner_tol;
     int64_t max_iter;
     int32_t max_outer;
-    int32_t mixed;
     uint64_t total_timeout_ns;
+    int32_t near_bytes;  // dynamic shared memory: room for p
 };
 
 // Cluster-wide deterministic sum of K values per thread. Partials are double
@@ -85,13 +92,20 @@ __device__ __forceinline__ void cluster_sum(double (&v)[K], double *part, int &b
         for (int k = 0; k < K; ++k) mine[k] = v[k];
     }
     cl.sync();
-    const unsigned nb = cl.num_blocks();
+    const int nb = static_cast<int>(cl.num_blocks()), lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {  // one read per value, added in rank order
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-        double t = 0.0;
-        for (unsigned q = 0; q < nb; ++q) t += *cl.map_shared_rank(mine + k, q);
-        v[k] = t;
+        for (int k = 0; k < K; ++k) {
+            const double q = lane < nb ? *cl.map_shared_rank(mine + k, lane) : 0.0;
+            double t = 0.0;
+            for (int r = 0; r < nb; ++r) t += __shfl_sync(0xffffffffu, q, r);
+            if (lane == 0) scratch[k] = t;
+        }
     }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = scratch[k];
+    __syncthreads();
     buf ^= 1;
 }
 
@@ -114,12 +128,334 @@ __device__ __forceinline__ T row_dot(const int32_t *rp, const int32_t *col, cons
     return acc;
 }
 
+// Rows a thread handles at a time in the vector phases: their loads are issued
+// together.
+constexpr int kBatchRows = 4;
+
+template <class Row>
+__device__ __forceinline__ void each_rows(int32_t a, int32_t b, Row row) {
+    const int32_t step = kBatchRows * blockDim.x, last = (kBatchRows - 1) * blockDim.x;
+    int32_t i = a + static_cast<int32_t>(threadIdx.x);
+    for (; i + last < b; i += step) row(i, std::integral_constant<int, kBatchRows>());
+    for (; i < b; i += blockDim.x) row(i, std::integral_constant<int, 1>());
+}
+
+// The search direction p that the products gather: every CTA of the cluster
+// keeps all of it in shared memory when it fits (`near`); a CTA stores its rows
+// into each. Random gathers from L2 run at 0.9 per clock and SM, those from
+// shared memory at about 9, and they bound the solve.
+// FP32 copy of a CTA's rows for the inner products of the mixed solve. The rows
+// are renumbered by length (longest first, stable) and dealt to the warps in
+// units: a long row (long_row) (its entries in order; the warp forms
+// the products 128 at a time and every lane adds them in that order), or 32
+// shorter rows, a lane each (entries step by step, those of the rows that have
+// one next to each other, so nothing is padded). Either way a row's terms are
+// added in storage order. The whole inner solve runs in this numbering. The
+// warp tiles it replaces waited for a row pointer, a column and a value per 128
+// entries and for the longest row of each 32: 66k cycles a product for 8,550
+// rows, now 34k, bound by instruction issue (the copy costs 40k once). 24
+// systems of 5k to 48k rows on clusters of 4 x 1,024: 11.5 -> 7.1 ms.
+constexpr int kLenBuckets = 64;   // rows of 63 entries and more are one bucket
+constexpr int kSliceCost = 4;     // a unit's own cost, in steps
+// Rows taken by a whole warp. One lane needs a round trip to L2 per eight entries,
+// a warp one per 128 but two instructions of every lane per entry: up to 128
+// rows a warp the round trips count (5,016 rows on 4 CTAs: 17.4 us an iteration
+// with long rows by lanes, 13.2 by warps), beyond that the instructions do
+// (34,219 rows: 34k cycles a product with the longest rows alone by warps, 48k
+// with all from 32 entries on).
+__device__ __forceinline__ int long_row(int32_t rows, int warps) {
+    return rows > 128 * warps ? kLenBuckets - 1 : 32;
+}
+
+struct Jagged {
+    int32_t a, rows;      // first row of the CTA (in the renumbered system), rows
+    int32_t *col;         // of the system
+    float *val;
+    float *diag, *ap;     // from here on by renumbered row of the system
+    int32_t *perm, *inv;  // row of a number, number of a row
+    int32_t *len, *start; // entries of a row; first entry of unit s at start[a + s]
+    int32_t *next;        // the unit its warp takes after s (-1: none) at next[a + s]
+    int32_t *first;       // shared memory: the first unit of each warp, then the
+                          // number of long rows (units of one row, the first ones)
+
+    __device__ static int bucket(int32_t n) {
+        return kLenBuckets - 1 - (n < kLenBuckets ? n : kLenBuckets - 1);
+    }
+
+    // Row (from a on) of lane q in unit s; -1: none.
+    __device__ int32_t row_of(int32_t s, int32_t longs, int q) const {
+        if (s < longs) return q == 0 ? s : -1;
+        const int32_t r = longs + 32 * (s - longs) + q;
+        return r < rows ? r : -1;
+    }
+
+    // hist: [warps][kLenBuckets], tot: [kLenBuckets] in shared memory.
+    __device__ __noinline__ void build(const int32_t *rp, const int32_t *scol, const double *sval,
+                          const double *sdiag, int32_t *hist, int32_t *tot,
+                          cg::cluster_group &cl) const {
+        const int tid = threadIdx.x, nt = blockDim.x;
+        const int lane = tid & 31, wid = tid >> 5, nw = nt >> 5;
+        const unsigned below = (1u << lane) - 1u;
+        __syncthreads();
+        for (int k = tid; k < nw * kLenBuckets; k += nt) hist[k] = 0;
+        __syncthreads();
+        const int32_t w0 = static_cast<int32_t>(static_cast<int64_t>(rows) * wid / nw);
+        const int32_t w1 = static_cast<int32_t>(static_cast<int64_t>(rows) * (wid + 1) / nw);
+        int32_t *mine = hist + wid * kLenBuckets;
+        for (int32_t l = w0 + lane; l < w1; l += 32)
+            atomicAdd(mine + bucket(rp[a + l + 1] - rp[a + l]), 1);
+        __syncthreads();
+        for (int k = tid; k < kLenBuckets; k += nt) {
+            int32_t t = 0;
+            for (int w = 0; w < nw; ++w) t += hist[w * kLenBuckets + k];
+            tot[k] = t;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            constexpr int kPer = kLenBuckets / 32;
+            int32_t sum = 0;
+            for (int q = 0; q < kPer; ++q) sum += tot[lane * kPer + q];
+            int32_t incl = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            int32_t run = incl - sum;
+            for (int q = 0; q < kPer; ++q) {
+                const int32_t t = tot[lane * kPer + q];
+                tot[lane * kPer + q] = run;
+                run += t;
+            }
+            __syncwarp();
+            if (lane == 0) first[32] = tot[bucket(long_row(rows, nw)) + 1];
+        }
+        __syncthreads();
+        for (int k = tid; k < kLenBuckets; k += nt) {
+            int32_t run = tot[k];
+            for (int w = 0; w < nw; ++w) {
+                const int32_t t = hist[w * kLenBuckets + k];
+                hist[w * kLenBuckets + k] = run;
+                run += t;
+            }
+        }
+        __syncthreads();
+        for (int32_t l0 = w0; l0 < w1; l0 += 32) {
+            const int32_t l = l0 + lane;
+            const bool in = l < w1;
+            const int32_t n = in ? rp[a + l + 1] - rp[a + l] : 0;
+            const int bk = in ? bucket(n) : -1;
+            const unsigned same = __match_any_sync(0xffffffffu, bk);
+            const int rank = __popc(same & below);
+            const int32_t to = in ? a + mine[bk] + rank : 0;
+            __syncwarp();
+            if (in && rank == 0) mine[bk] += __popc(same);
+            __syncwarp();
+            if (in) {
+                perm[to] = a + l;
+                inv[a + l] = to;
+                len[to] = n;
+                diag[to] = static_cast<float>(sdiag[a + l]);
+            }
+        }
+        __syncthreads();
+        const int32_t longs = first[32], slices = longs + (rows - longs + 31) / 32;
+        for (int32_t s = wid; s < slices; s += nw) {
+            const int32_t r = row_of(s, longs, lane);
+            const int32_t n = r >= 0 ? len[a + r] : 0;
+            const int32_t t = __reduce_add_sync(0xffffffffu, n);
+            if (lane == 0) start[a + s] = t;
+        }
+        __syncthreads();
+        if (wid == 0) {
+            int32_t run = rows > 0 ? rp[a] : 0;
+            for (int32_t s0 = 0; s0 < slices; s0 += 32) {
+                const int32_t t = s0 + lane < slices ? start[a + s0 + lane] : 0;
+                int32_t incl = t;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += u;
+                }
+                if (s0 + lane < slices) start[a + s0 + lane] = run + incl - t;
+                run += __shfl_sync(0xffffffffu, incl, 31);
+            }
+        }
+        // slices, longest first, to the warp with least to do (lane w: warp w)
+        if (wid == nw - 1) {
+            uint32_t load = 0;
+            int32_t last = -1;
+            if (lane < nw) first[lane] = -1;
+            for (int32_t s0 = 0; s0 < slices; s0 += 32) {
+                const int32_t u = s0 + lane;
+                const int32_t longest = u >= slices ? 0
+                                        : u < longs ? len[a + u] / 4
+                                                    : len[a + row_of(u, longs, 0)];
+                const int32_t here = slices - s0 < 32 ? slices - s0 : 32;
+                for (int32_t q = 0; q < here; ++q) {
+                    const uint32_t cost = __shfl_sync(0xffffffffu, longest, q) + kSliceCost;
+                    // (loads stay below 2^26 steps: 2^31 entries of 32 a step)
+                    const uint32_t least =
+                        __reduce_min_sync(0xffffffffu, lane < nw ? load << 5 | lane : ~0u);
+                    if (lane == (least & 31u)) {
+                        if (last < 0) first[lane] = s0 + q;
+                        else next[a + last] = s0 + q;
+                        last = s0 + q;
+                        load += cost;
+                    }
+                }
+            }
+            if (last >= 0) next[a + last] = -1;
+        }
+        cl.sync();  // every CTA's inv
+        for (int32_t s = wid; s < slices; s += nw) {
+            if (s < longs) {
+                const int32_t n = len[a + s], e = rp[perm[a + s]], at = start[a + s];
+                for (int32_t j = lane; j < n; j += 32) {
+                    col[at + j] = __ldcg(inv + scol[e + j]);
+                    val[at + j] = static_cast<float>(sval[e + j]);
+                }
+                continue;
+            }
+            const int32_t r = row_of(s, longs, lane);
+            const int32_t n = r >= 0 ? len[a + r] : 0, e = r >= 0 ? rp[perm[a + r]] : 0;
+            const int32_t most = __reduce_max_sync(0xffffffffu, n);
+            int32_t at = start[a + s];
+#pragma unroll 4
+            for (int32_t j = 0; j < most; ++j) {
+                const unsigned m = __ballot_sync(0xffffffffu, j < n);
+                if (j < n) {
+                    const int32_t to = at + __popc(m & below);
+                    col[to] = __ldcg(inv + scol[e + j]);
+                    val[to] = static_cast<float>(sval[e + j]);
+                }
+                at += __popc(m);
+            }
+        }
+        __syncthreads();
+    }
+
+    // ap = A p for the CTA's rows; returns the thread's part of p^T A p. p is in
+    // shared memory (Near) or global. A lane's entries are loaded kDeep at a
+    // time, one group ahead, across slices: L2's latency is what there is to
+    // hide. Not inlined: it needs the registers to itself.
+    template <bool Near>
+    __device__ __noinline__ double product(const float *far_p) const {
+        extern __shared__ __align__(16) double near_mem[];
+        const float *near_p = reinterpret_cast<const float *>(near_mem);
+        auto gather = [&](int32_t k) { return Near ? near_p[k] : __ldcg(far_p + k); };
+        double w = 0.0;
+        constexpr int kDeep = 8;
+        const int lane = threadIdx.x & 31;
+        const unsigned below = (1u << lane) - 1u;
+        int32_t c[kDeep];
+        float v[kDeep];
+        const int32_t longs = first[32];
+        auto head = [&](int32_t s, int32_t &n, int32_t &at, int32_t &after) {
+            const int32_t r = s >= 0 ? row_of(s, longs, lane) : -1;
+            n = r >= 0 ? len[a + r] : 0;
+            at = s >= 0 ? start[a + s] : 0;
+            after = s >= 0 ? next[a + s] : -1;
+        };
+        // entries j, j + 1, ... of slice rows of n entries each from `at` on, or
+        // of rows of one length (even): then step j lies at at + 32 j
+        auto load = [&](int32_t j, int32_t n, int32_t &at, bool even) {
+            if (even) {
+                const int32_t *ce = col + at + 32 * j + lane;
+                const float *ve = val + at + 32 * j + lane;
+#pragma unroll
+                for (int k = 0; k < kDeep; ++k) {
+                    c[k] = j + k < n ? __ldcg(ce + 32 * k) : -1;
+                    v[k] = j + k < n ? __ldcg(ve + 32 * k) : 0.0f;
+                }
+                return;
+            }
+#pragma unroll
+            for (int k = 0; k < kDeep; ++k) {
+                const bool has = j + k < n;
+                const unsigned m = __ballot_sync(0xffffffffu, has);
+                const int32_t e = at + __popc(m & below);
+                c[k] = has ? __ldcg(col + e) : -1;
+                v[k] = has ? __ldcg(val + e) : 0.0f;
+                at += __popc(m);
+            }
+        };
+        auto same = [&](int32_t n) {
+            return __reduce_max_sync(0xffffffffu, n) == __reduce_min_sync(0xffffffffu, n);
+        };
+        int32_t s = first[threadIdx.x >> 5], n, at, after;
+        head(s, n, at, after);
+        while (s >= 0 && s < longs) {  // a warp's long rows come first
+            const int32_t many = __shfl_sync(0xffffffffu, n, 0);
+            const float p = gather(a + s);
+            float sum = diag[a + s] * p;
+            for (int32_t j = 0; j < many; j += 128) {
+                float t[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int32_t e = j + 32 * k + lane;
+                    c[k] = e < many ? __ldcg(col + at + e) : -1;
+                    t[k] = e < many ? __ldcg(val + at + e) : 0.0f;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (c[k] >= 0) t[k] = t[k] * gather(c[k]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int32_t here = min(32, many - j - 32 * k);
+                    for (int32_t q = 0; q < here; ++q) sum += __shfl_sync(0xffffffffu, t[k], q);
+                }
+            }
+            if (lane == 0) {
+                ap[a + s] = sum;
+                w += static_cast<double>(p) * sum;
+            }
+            s = after;
+            head(s, n, at, after);
+        }
+        bool even = same(n);
+        load(0, n, at, even);
+        while (s >= 0) {
+            int32_t next_n, next_at, next_after;
+            head(after, next_n, next_at, next_after);
+            const int32_t r = row_of(s, longs, lane), i = a + r;
+            const bool on = r >= 0;
+            const int32_t most = __reduce_max_sync(0xffffffffu, n);
+            const float p = on ? gather(i) : 0.0f;
+            float sum = on ? diag[i] * p : 0.0f;
+            for (int32_t j = 0; j < most; j += kDeep) {
+#pragma unroll
+                for (int k = 0; k < kDeep; ++k)
+                    if (c[k] >= 0) sum += v[k] * gather(c[k]);
+                if (j + kDeep < most) {
+                    load(j + kDeep, n, at, even);
+                } else {
+                    even = same(next_n);
+                    load(0, next_n, next_at, even);
+                }
+            }
+            if (on) {
+                ap[i] = sum;
+                w += static_cast<double>(p) * sum;
+            }
+            s = after;
+            n = next_n;
+            at = next_at;
+            after = next_after;
+        }
+        return w;
+    }
+};
+
+template <bool Mixed>
 __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
     cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) double near_mem[];
     __shared__ double scratch[33 * 4];
     __shared__ double part[2 * 4];
     __shared__ __align__(16) double tilebuf[32 * kTileChunk];  // warp tiles, <= 32 warps
     __shared__ int32_t wb[32 + 1];
+    __shared__ int32_t first_slice[33];
+    __shared__ Jagged J;
+    __shared__ float *peers[16];  // p of every CTA of the cluster
     __shared__ int s_job;
     __shared__ int s_stop;
     int buf = 0;
@@ -141,12 +477,14 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
         const SysDesc S = A.sys[sid];
         const uint64_t t0 = global_timer_ns();
         const int32_t n = S.n;
-        const int32_t a = static_cast<int32_t>((static_cast<int64_t>(n) * rank) / nb);
-        const int32_t b = static_cast<int32_t>((static_cast<int64_t>(n) * (rank + 1)) / nb);
+        // the CTA's rows (from a multiple of four on: p is stored by fours)
+        auto split = [&](unsigned q) {
+            return q == nb ? n : static_cast<int32_t>(static_cast<int64_t>(n) * q / nb) & ~3;
+        };
+        const int32_t a = split(rank), b = split(rank + 1);
         const int32_t *rp = A.rp + S.row_base + sid;
         const int32_t *col = A.col + S.nnz_base;
         const double *val = A.val + S.nnz_base;
-        const float *val32 = A.val32 + S.nnz_base;
         const double *dg = A.diag + S.row_base;
         const double *rhs = A.rhs + S.row_base;
         double *x = A.x + S.row_base;
@@ -163,7 +501,7 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
         res.status = late ? KTG_ERR_TIMEOUT : KTG_OK;
         double resid = 0.0;
 
-        if (!A.mixed) {
+        if constexpr (!Mixed) {
             double *z = A.z + S.row_base;
             double *p = A.p + S.row_base;
             double *ap = A.ap + S.row_base;
@@ -191,7 +529,7 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
                 if (rank == 0 && threadIdx.x == 0) s_stop = global_timer_ns() > deadline ? 1 : 0;
                 double w[1] = {0.0};
                 double pcur = 0.0;
-                warp_tile_spmv<double>(
+                warp_tile_spmv<double, true>(
                     a, INT32_MAX, b - a, kAllAxes, wb, tilebuf,
                     [&](int, const int32_t *&trp, const int32_t *&tcol, const double *&tval,
                         const double *&tin) {
@@ -246,24 +584,52 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
             }
             res.iters = it;
         } else {
+            // r = b - A x for the CTA's rows
+            auto residual = [&](auto emit) {
+                warp_tile_spmv<double, true>(
+                    a, INT32_MAX, b - a, kAllAxes, wb, tilebuf,
+                    [&](int, const int32_t *&trp, const int32_t *&tcol, const double *&tval,
+                        const double *&tin) {
+                        trp = rp;
+                        tcol = col;
+                        tval = val;
+                        tin = x;
+                    },
+                    [&](int32_t, int, int32_t i) { return dg[i] * __ldcg(x + i); },
+                    [&](int32_t, int, int32_t i, double s) { emit(i, rhs[i], rhs[i] - s); });
+            };
             float *d = A.d32 + S.row_base;
             float *ri = A.ri32 + S.row_base;
             float *z = A.z32 + S.row_base;
             float *p = A.p32 + S.row_base;
             float *ap = A.ap32 + S.row_base;
+            if (threadIdx.x == 0)
+                J = Jagged{a, b - a, A.jcol + S.nnz_base, A.jval + S.nnz_base,
+                           A.diag32 + S.row_base, ap, A.perm + S.row_base, A.inv + S.row_base,
+                           A.len + S.row_base, A.start + S.row_base, A.next + S.row_base,
+                           first_slice};
+            __syncthreads();
+            float *const near_p = reinterpret_cast<float *>(near_mem);
+            const bool near = static_cast<int64_t>(n) * 4 <= A.near_bytes;
+            if (threadIdx.x < nb) peers[threadIdx.x] = cl.map_shared_rank(near_p, threadIdx.x);
+            __syncthreads();
+            auto put = [&](int32_t i, float t) {
+                if (near)
+                    for (unsigned q = 0; q < nb; ++q) peers[q][i] = t;
+                else
+                    __stcg(p + i, t);
+            };
+            auto own = [&](int32_t i) { return near ? near_p[i] : __ldcg(p + i); };
             double bnorm = 0.0, prev = 0.0;
             int64_t inner = 0;
             int32_t outer = 0;
             for (int round = 0;; ++round) {
                 double v[2] = {0.0, 0.0};  // rr, bb
-                for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) {
-                    const double s = row_dot<double, double>(rp, col, val, x, i, dg[i] * __ldcg(x + i));
-                    const double bi = rhs[i];
-                    const double rr = bi - s;
+                residual([&](int32_t i, double bi, double rr) {
                     r[i] = rr;
                     v[0] += rr * rr;
                     v[1] += bi * bi;
-                }
+                });
                 cluster_sum<2>(v, part, buf, scratch, cl);
                 if (round == 0) bnorm = sqrt(v[1]);
                 const double rnorm = sqrt(v[0]);
@@ -275,14 +641,17 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
                     if (stalled && resid > A.tol) res.status = 1;  // stalled: caller may retry in FP64
                     break;
                 }
+                if (round == 0)
+                    J.build(rp, col, val, dg, reinterpret_cast<int32_t *>(tilebuf),
+                            reinterpret_cast<int32_t *>(scratch), cl);
                 double q[2] = {0.0, 0.0};  // rz, rr (inner)
                 for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) {
-                    const float rf = static_cast<float>(r[i]);
-                    const float zf = rf / static_cast<float>(dg[i]);
+                    const float rf = static_cast<float>(r[J.perm[i]]);
+                    const float zf = rf / J.diag[i];
                     ri[i] = rf;
                     d[i] = 0.0f;
                     z[i] = zf;
-                    __stcg(p + i, zf);
+                    put(i, zf);
                     q[0] += static_cast<double>(rf) * zf;
                     q[1] += static_cast<double>(rf) * rf;
                 }
@@ -293,48 +662,55 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
                 bool live = rho > 0.0;
                 while (live && iresid > target && inner < A.max_iter) {
                     double w[1] = {0.0};
-                    float pcur = 0.0f;
-                    warp_tile_spmv<float>(
-                        a, INT32_MAX, b - a, kAllAxes, wb, reinterpret_cast<float *>(tilebuf),
-                        [&](int, const int32_t *&trp, const int32_t *&tcol, const float *&tval,
-                            const float *&tin) {
-                            trp = rp;
-                            tcol = col;
-                            tval = val32;
-                            tin = p;
-                        },
-                        [&](int32_t, int, int32_t i) {
-                            pcur = __ldcg(p + i);
-                            return static_cast<float>(dg[i]) * pcur;
-                        },
-                        [&](int32_t, int, int32_t i, float s) {
-                            ap[i] = s;
-                            w[0] += static_cast<double>(pcur) * s;
-                        });
+                    w[0] = near ? J.product<true>(p) : J.product<false>(p);
                     cluster_sum<1>(w, part, buf, scratch, cl);
                     ++inner;
                     if (!(w[0] > 0.0)) break;
                     const float alpha = static_cast<float>(rho / w[0]);
                     double u[2] = {0.0, 0.0};
-                    for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) {
-                        d[i] += alpha * __ldcg(p + i);
-                        const float rr = ri[i] - alpha * ap[i];
-                        const float zz = rr / static_cast<float>(dg[i]);
-                        ri[i] = rr;
-                        z[i] = zz;
-                        u[0] += static_cast<double>(rr) * rr;
-                        u[1] += static_cast<double>(rr) * zz;
-                    }
+                    each_rows(a, b, [&](int32_t i0, auto count) {
+                        float xv[kBatchRows], rv[kBatchRows], av[kBatchRows], dv[kBatchRows];
+#pragma unroll
+                        for (int k = 0; k < count(); ++k) {
+                            const int32_t i = i0 + k * blockDim.x;
+                            xv[k] = d[i];
+                            rv[k] = ri[i];
+                            av[k] = ap[i];
+                            dv[k] = J.diag[i];
+                        }
+#pragma unroll
+                        for (int k = 0; k < count(); ++k) {
+                            const int32_t i = i0 + k * blockDim.x;
+                            d[i] = xv[k] + alpha * own(i);
+                            const float rr = rv[k] - alpha * av[k];
+                            const float zz = rr / dv[k];
+                            ri[i] = rr;
+                            z[i] = zz;
+                            u[0] += static_cast<double>(rr) * rr;
+                            u[1] += static_cast<double>(rr) * zz;
+                        }
+                    });
                     cluster_sum<2>(u, part, buf, scratch, cl);
                     iresid = sqrt(u[0]);
                     if (!(u[1] > 0.0)) break;
                     const float beta = static_cast<float>(u[1] / rho);
                     rho = u[1];
-                    for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x)
-                        __stcg(p + i, z[i] + beta * __ldcg(p + i));
+                    const int32_t b4 = near ? a + (b - a) / 4 * 4 : a;
+                    for (int32_t i = a + 4 * static_cast<int32_t>(threadIdx.x); i < b4;
+                         i += 4 * blockDim.x) {
+                        float4 t = *reinterpret_cast<const float4 *>(near_p + i);
+                        t.x = z[i] + beta * t.x;
+                        t.y = z[i + 1] + beta * t.y;
+                        t.z = z[i + 2] + beta * t.z;
+                        t.w = z[i + 3] + beta * t.w;
+                        for (unsigned q = 0; q < nb; ++q)
+                            *reinterpret_cast<float4 *>(peers[q] + i) = t;
+                    }
+                    for (int32_t i = b4 + static_cast<int32_t>(threadIdx.x); i < b; i += blockDim.x)
+                        put(i, z[i] + beta * own(i));
                     cl.sync();
                 }
-                for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) x[i] += d[i];
+                for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) x[J.perm[i]] += d[i];
                 ++outer;
                 cl.sync();
             }
@@ -357,6 +733,7 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
 struct ktg_batch {
     int device = 0;
     int num_sms = 0;
+    int near_limit = 0;         // dynamic shared memory a CTA of the mixed solve can have
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
     std::string err;
@@ -373,7 +750,10 @@ struct ktg_batch {
     int32_t *rp = nullptr;  // rows + num_sys entries
     int32_t *col = nullptr;
     double *val = nullptr;
-    float *val32 = nullptr;
+    int32_t *jcol = nullptr;  // the mixed solve's copy, built by it
+    float *jval = nullptr, *diag32 = nullptr;
+    int32_t *perm = nullptr, *inv = nullptr, *len = nullptr, *start = nullptr,
+            *next = nullptr;
     double *diag = nullptr, *rhs = nullptr, *x = nullptr, *x0 = nullptr;
     double *r = nullptr, *z = nullptr, *p = nullptr, *ap = nullptr;
     float *d32 = nullptr, *ri32 = nullptr, *z32 = nullptr, *p32 = nullptr, *ap32 = nullptr;
@@ -452,7 +832,10 @@ int reserve(ktg_batch *b, int64_t rows, int64_t nnz, int64_t nsys) {
             (rc = grow(b, &b->p, 0, cap)) || (rc = grow(b, &b->ap, 0, cap)) ||
             (rc = grow(b, &b->d32, 0, cap)) || (rc = grow(b, &b->ri32, 0, cap)) ||
             (rc = grow(b, &b->z32, 0, cap)) || (rc = grow(b, &b->p32, 0, cap)) ||
-            (rc = grow(b, &b->ap32, 0, cap)))
+            (rc = grow(b, &b->ap32, 0, cap)) || (rc = grow(b, &b->diag32, 0, cap)) ||
+            (rc = grow(b, &b->perm, 0, cap)) || (rc = grow(b, &b->inv, 0, cap)) ||
+            (rc = grow(b, &b->len, 0, cap)) || (rc = grow(b, &b->start, 0, cap)) ||
+            (rc = grow(b, &b->next, 0, cap)))
             return rc;
         b->cap_rows = cap;
     }
@@ -471,17 +854,11 @@ int reserve(ktg_batch *b, int64_t rows, int64_t nnz, int64_t nsys) {
     if (nnz > b->cap_nnz) {
         const int64_t cap = std::max(nnz, 2 * b->cap_nnz);
         if ((rc = grow(b, &b->col, b->nnz, cap)) || (rc = grow(b, &b->val, b->nnz, cap)) ||
-            (rc = grow(b, &b->val32, b->nnz, cap)))
+            (rc = grow(b, &b->jcol, 0, cap)) || (rc = grow(b, &b->jval, 0, cap)))
             return rc;
         b->cap_nnz = cap;
     }
     return KTG_OK;
-}
-
-__global__ void k_batch_f32(const double *a, float *b, int64_t n) {
-    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-        b[i] = static_cast<float>(a[i]);
 }
 
 __global__ void k_stamp(unsigned long long *t) { *t = ktg::global_timer_ns(); }
@@ -561,8 +938,8 @@ void ktg_batch_destroy(ktg_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
-    void *ptrs[] = {b->d_sys, b->d_order, b->rp, b->col, b->val, b->val32, b->diag, b->rhs,
-                    b->x, b->x0, b->r, b->z, b->p, b->ap, b->d32, b->ri32, b->z32, b->p32,
+    void *ptrs[] = {b->d_sys, b->d_order, b->rp, b->col, b->val, b->jcol, b->jval, b->diag32,
+                    b->perm, b->inv, b->len, b->start, b->next, b->diag, b->rhs, b->x, b->x0, b->r, b->z, b->p, b->ap, b->d32, b->ri32, b->z32, b->p32,
                     b->ap32, b->queue, b->queue2, b->results, b->d_minfo, b->d_sinfo,
                     b->d_stamp};
     for (void *p : ptrs)
@@ -615,11 +992,6 @@ int ktg_batch_add_system(ktg_batch *b, int64_t n, const int64_t *row_ptr, const 
         KTG_BCUDA(b, cudaMemcpyAsync(b->rhs + base, rhs, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
         KTG_BCUDA(b, cudaMemcpyAsync(b->x + base, x0, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
         KTG_BCUDA(b, cudaMemcpyAsync(b->x0 + base, x0, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
-    }
-    if (m) {
-        k_batch_f32<<<static_cast<int>(std::min<int64_t>((m + 255) / 256, 4096)), 256, 0, b->stream>>>(
-            b->val + ebase, b->val32 + ebase, m);
-        ++b->launches;
     }
     KTG_BCUDA(b, cudaStreamSynchronize(b->stream));
     b->sys.push_back(ktg::SysDesc{base, ebase, static_cast<int32_t>(n), 0});
@@ -748,9 +1120,45 @@ int ktg_batch_reset_x(ktg_batch *b) {
     return KTG_OK;
 }
 
+static void (*batch_kernel(int mixed))(ktg::BatchArgs) {
+    return mixed ? ktg::k_batch_pcg<true> : ktg::k_batch_pcg<false>;
+}
+
+// Shared memory for the mixed solve's search direction in each class: the
+// largest system's, or as much as there is (larger systems then gather from
+// L2). The FP64 solve has none: 8 bytes a row leave it too little L1 (24 systems
+// of 5k to 48k rows on 4 x 1,024: 20.7 ms with, 13.7 without).
+static int near_room(ktg_batch *b, int mixed, int *small, int *large) {
+    *small = *large = 0;
+    if (!mixed) return KTG_OK;
+    int &near_limit = b->near_limit;
+    if (near_limit == 0) {
+        cudaFuncAttributes fa;
+        int most = 0;
+        KTG_BCUDA(b, cudaFuncGetAttributes(&fa, batch_kernel(mixed)));
+        KTG_BCUDA(b, cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                            b->device));
+        const int limit = (most - static_cast<int>(fa.sharedSizeBytes)) / 256 * 256;
+        KTG_BCUDA(b, cudaFuncSetAttribute(batch_kernel(mixed),
+                                          cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+        near_limit = limit;
+    }
+    const std::vector<char> off = offloaded(b);
+    int64_t n[2] = {0, 0};
+    for (size_t i = 0; i < b->sys.size(); ++i) {
+        int64_t &m = n[b->split_rows > 0 && b->sys[i].n >= b->split_rows ? 1 : 0];
+        if (!off[i]) m = std::max<int64_t>(m, b->sys[i].n);
+    }
+    for (int k = 0; k < 2; ++k)
+        *(k ? large : small) = static_cast<int>(std::min<int64_t>(
+            near_limit, (n[k] * 4 + 255) / 256 * 256));
+    return KTG_OK;
+}
+
 // How many clusters of `cluster` CTAs of `threads` threads can be resident
 // at once on the whole device.
-static int resident_clusters(ktg_batch *b, int cluster, int threads, int *out) {
+static int resident_clusters(ktg_batch *b, int mixed, int cluster, int threads, int near_bytes,
+                             int *out) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -759,21 +1167,35 @@ static int resident_clusters(ktg_batch *b, int cluster, int threads, int *out) {
     attr[0].val.clusterDim.z = 1;
     cfg.blockDim = dim3(threads);
     cfg.gridDim = dim3(cluster);
+    cfg.dynamicSmemBytes = near_bytes;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (cluster > 8)
-        KTG_BCUDA(b, cudaFuncSetAttribute(ktg::k_batch_pcg,
+        KTG_BCUDA(b, cudaFuncSetAttribute(batch_kernel(mixed),
                                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    KTG_BCUDA(b, cudaOccupancyMaxActiveClusters(out, ktg::k_batch_pcg, &cfg));
+    KTG_BCUDA(b, cudaOccupancyMaxActiveClusters(out, batch_kernel(mixed), &cfg));
     if (*out < 1) return berr(b, KTG_ERR_CUDA, "cluster shape cannot be resident");
     return KTG_OK;
+}
+
+// The same with the search direction in shared memory, or without where the
+// shape is then not resident.
+static int near_clusters(ktg_batch *b, int mixed, int cluster, int threads, int *near_bytes,
+                         int *out) {
+    if (*near_bytes > 0) {
+        if (resident_clusters(b, mixed, cluster, threads, *near_bytes, out) == KTG_OK) return KTG_OK;
+        (void)cudaGetLastError();
+        b->err.clear();
+        *near_bytes = 0;
+    }
+    return resident_clusters(b, mixed, cluster, threads, 0, out);
 }
 
 // One persistent launch over the systems order[first, first + count): `clusters`
 // clusters of `cluster` CTAs of `threads` threads draining `queue`.
 static int enqueue_class(ktg_batch *b, int first, int count, unsigned *queue, int cluster,
-                         int threads, int clusters, double tol, int64_t max_iter, int mixed,
-                         double inner_tol, cudaStream_t st) {
+                         int threads, int clusters, int near_bytes, double tol, int64_t max_iter,
+                         int mixed, double inner_tol, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -781,17 +1203,18 @@ static int enqueue_class(ktg_batch *b, int first, int count, unsigned *queue, in
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = near_bytes;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(std::max(1, std::min(clusters, count)) * cluster);
-    ktg::BatchArgs A{b->d_sys, b->d_order + first, count, b->rp, b->col, b->val, b->val32,
+    ktg::BatchArgs A{b->d_sys, b->d_order + first, count, b->rp, b->col, b->val,
                      b->diag, b->rhs, b->x, b->r, b->z, b->p, b->ap, b->d32, b->ri32, b->z32,
-                     b->p32, b->ap32, queue, b->results, tol, inner_tol, max_iter, 50, mixed,
-                     120000000000ull};
+                     b->p32, b->ap32, b->jcol, b->jval, b->diag32, b->perm, b->inv, b->len,
+                     b->start, b->next, queue, b->results, tol, inner_tol, max_iter, 50,
+                     120000000000ull, near_bytes};
     KTG_BCUDA(b, cudaMemsetAsync(queue, 0, sizeof(unsigned), st));
-    KTG_BCUDA(b, cudaLaunchKernelEx(&cfg, ktg::k_batch_pcg, A));
+    KTG_BCUDA(b, cudaLaunchKernelEx(&cfg, batch_kernel(mixed), A));
     return KTG_OK;
 }
 
@@ -805,21 +1228,25 @@ static int batch_enqueue(ktg_batch *b, double tol, int64_t max_iter, int mixed, 
                          cudaStream_t st) {
     const int ns = b->num_queued;
     const int nl = b->num_large;
-    int res_small = 0;
-    int rc = resident_clusters(b, b->cluster, b->threads, &res_small);
+    int res_small = 0, near_small = 0, near_large = 0;
+    int rc = near_room(b, mixed, &near_small, &near_large);
     if (rc) return rc;
+    if (nl < ns &&
+        (rc = near_clusters(b, mixed, b->cluster, b->threads, &near_small, &res_small)))
+        return rc;
     if (nl == 0) {
-        rc = enqueue_class(b, 0, ns, b->queue, b->cluster, b->threads, res_small, tol, max_iter,
-                           mixed, inner_tol, st);
+        rc = enqueue_class(b, 0, ns, b->queue, b->cluster, b->threads, res_small, near_small, tol,
+                           max_iter, mixed, inner_tol, st);
         b->graph_kernels = 1;
         return rc;
     }
     int res_large = 0;
-    if ((rc = resident_clusters(b, b->split_cluster, b->split_threads, &res_large))) return rc;
+    if ((rc = near_clusters(b, mixed, b->split_cluster, b->split_threads, &near_large, &res_large)))
+        return rc;
     const int large_clusters = std::min({b->split_clusters, res_large, nl});
     if (nl == ns) {
         rc = enqueue_class(b, 0, ns, b->queue2, b->split_cluster, b->split_threads, large_clusters,
-                           tol, max_iter, mixed, inner_tol, st);
+                           near_large, tol, max_iter, mixed, inner_tol, st);
         b->graph_kernels = 1;
         return rc;
     }
@@ -843,10 +1270,10 @@ static int batch_enqueue(ktg_batch *b, double tol, int64_t max_iter, int mixed, 
         rc = berr(b, KTG_ERR_CUDA, "stream fork failed");
     if (!rc)
         rc = enqueue_class(b, 0, nl, b->queue2, b->split_cluster, b->split_threads, large_clusters,
-                           tol, max_iter, mixed, inner_tol, side);
+                           near_large, tol, max_iter, mixed, inner_tol, side);
     if (!rc)
-        rc = enqueue_class(b, nl, ns - nl, b->queue, b->cluster, b->threads, small_clusters, tol,
-                           max_iter, mixed, inner_tol, st);
+        rc = enqueue_class(b, nl, ns - nl, b->queue, b->cluster, b->threads, small_clusters,
+                           near_small, tol, max_iter, mixed, inner_tol, st);
     if (!rc && (cudaEventRecord(join, side) != cudaSuccess ||
                 cudaStreamWaitEvent(st, join, 0) != cudaSuccess))
         rc = berr(b, KTG_ERR_CUDA, "stream join failed");
@@ -1032,7 +1459,7 @@ int ktg_batch_autotune(ktg_batch *b, double tol, int precision, double inner_tol
         for (int t : kThreads) {
             if ((rc = ktg_batch_set_shape(b, c, t))) break;
             int resident = 0;
-            if (resident_clusters(b, c, t, &resident) != KTG_OK) {
+            if (resident_clusters(b, precision, c, t, 0, &resident) != KTG_OK) {
                 b->err.clear();
                 continue;  // shape not launchable on this device
             }
@@ -1119,7 +1546,7 @@ int ktg_batch_autotune_split(ktg_batch *b, double tol, int precision, double inn
         for (const auto &sh : kShapes) {
             if (rc) break;
             int resident = 0;
-            if (resident_clusters(b, sh[0], sh[1], &resident) != KTG_OK) {
+            if (resident_clusters(b, precision, sh[0], sh[1], 0, &resident) != KTG_OK) {
                 b->err.clear();
                 continue;  // shape not launchable on this device
             }

@@ -285,3 +285,44 @@ def test_upload_second_axis_larger_keeps_first(systems):
     for s, v, got in ((s0, v0, r["x"]), (s1, v1, r["y"])):
         ref = oracle.port_pcg_axis(s, v, TOL, MAX_ITER)
         assert np.linalg.norm(got - ref["x"]) <= 1e-9 * np.linalg.norm(ref["x"])
+
+
+@pytest.mark.parametrize("cluster,threads", [(1, 1024), (2, 128), (4, 1024), (16, 512)])
+def test_batch_mixed_renumbered_rows(cluster, threads):
+    """The mixed solve's renumbered copy at its edges: fewer rows than CTAs or
+    than a slice, rows that are not a multiple of four per CTA, empty rows, a row
+    longer than the length buckets, and a system too large for shared memory
+    (its search direction stays in global memory): the true residual meets the
+    tolerance and a second solve gives the same bits."""
+    rng = np.random.default_rng(cluster)
+    cases = []
+    for n in (1, 2, 3, 5, 31, 33, 257, 1029, 60007):
+        deg = np.minimum(rng.integers(0, 9, n), n - 1)
+        deg[rng.integers(0, n, max(1, n // 50))] = 0
+        if n > 1000:
+            deg[n // 3] = 700
+        rows = np.repeat(np.arange(n), deg)
+        cols = (rows + rng.integers(1, max(2, n), rows.shape[0])) % n
+        keep = cols != rows
+        a, b = rows[keep], cols[keep]
+        w = rng.uniform(0.1, 1.0, a.shape[0])
+        r, c, v = np.concatenate([a, b]), np.concatenate([b, a]), -np.concatenate([w, w])
+        order = np.argsort(r, kind="stable")
+        r, c, v = r[order], c[order], v[order]
+        diag = rng.uniform(0.5, 1.5, n) + np.bincount(r, weights=-v, minlength=n)
+        rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))])
+        cases.append((dict(row_ptr=rp.astype(np.int64), col=c.astype(np.int32), val=v, diag=diag,
+                           rhs=rng.standard_normal(n)), rng.standard_normal(n)))
+    b, ids = make_batch(cases)
+    b.set_shape(cluster, threads)
+    got = []
+    for _ in range(2):
+        b.reset_x()
+        b.solve(TOL, MAX_ITER, precision=1, inner_tol=1e-3)
+        got.append([b.get_x(i, s["diag"].shape[0]) for (s, _), i in zip(cases, ids)])
+    res = b.results()
+    for (s, _), sid, x, again in zip(cases, ids, *got):
+        assert res[sid]["status"] == 0, res[sid]
+        assert true_resid(s, x) <= TOL * 1.0001
+        assert np.array_equal(x, again)
+    b.close()
