@@ -6,11 +6,12 @@
 // every iteration, the stopping test -- runs inside one kernel, so there is no
 // host round trip per iteration. Each block owns a contiguous slice of the
 // combined row space [x rows | y rows] (one 1024-thread block per SM); in
-// the textbook form three grid barriers per iteration separate
+// the textbook form (the default, form 3 with 32 lanes, is in
+// ktg_pcg_sliced.cu) three grid barriers per iteration separate
 //   A: Ap = A p and p.Ap partials
 //   B: x += a p, r -= a Ap, z = r / diag, and r.r, r.z partials
 //   C: p = z + b p
-// and the default form (3) folds C into A, gathering z and updating p and
+// and form 3 folds C into A, gathering z and updating p and
 // A p = A z + b A p there, for two barriers per iteration.
 // When a block's rows fit, its slices of x, r, z, p and Ap live in shared
 // memory for the whole solve, so phases B and C never leave the SM and only
@@ -18,8 +19,7 @@
 // L1 instead: every KB of shared memory comes out of the L1 that holds the
 // SpMV's gathers in flight (a block with 30 KB more shared memory solved
 // the 211k system in 8.6 ms instead of 5.8).
-// SpMV runs in one of three shapes (option "pcg_lanes"): warp tiles (the
-// default: each warp takes a range of the block's rows balanced by
+// SpMV runs in one of three shapes (option "pcg_lanes"): warp tiles (each warp takes a range of the block's rows balanced by
 // nonzeros and streams their nonzeros 32 rows at a time with coalesced
 // loads, each lane adding its row's products in storage order), one thread
 // per row (same row sums, four gathers in flight), or four lanes per row.
