@@ -463,8 +463,8 @@ def run_ours(args):
                           "other_ms": statistics.median(step_ms) - solve_med},
             "solve_variants": variants,
             "learned_step": learned_step,
-            "roofline": {"kernel": "k_pcg<1, 32, 0, 1> (persistent cooperative PCG, x+y, "
-                                   "warp-tile SpMV, two grid barriers per iteration)",
+            "roofline": {"kernel": "k_pcg_sliced<4> (persistent cooperative PCG, x+y, rows "
+                                   "sorted by length over lanes, two grid sums per iteration)",
                          "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": NCU_TRAFFIC_BYTES["k_pcg"], "algorithmic_bytes": byts,
