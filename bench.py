@@ -260,7 +260,7 @@ def spmv_bytes(n: int, m: int) -> float:
 # DRAM bytes (read + write) per launch of the dominant kernel on this
 # workload, from an ncu capture of bench.py --profile-once (dram__bytes_read.sum +
 # dram__bytes_write.sum of the k_pcg launch).
-NCU_TRAFFIC_BYTES = {"k_pcg": 100.221184e6 + 14.856192e6}
+NCU_TRAFFIC_BYTES = {"k_pcg": 3805.376256e6 + 39.944192e6}
 
 
 def measured_peak():
@@ -468,10 +468,11 @@ def run_ours(args):
                          "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "traffic": NCU_TRAFFIC_BYTES["k_pcg"], "algorithmic_bytes": byts,
-                         "note": "working set is L2-resident: traffic << algorithmic bytes",
-                         "limiter": "L1TEX data pipe: 57% of peak over the whole solve in the ncu "
+                         "note": "the entries' loads leave L2 first: about half of their "
+                                 "stream comes from DRAM, the vectors stay in L2",
+                         "limiter": "L1TEX data pipe: 47% of peak over the whole solve in the ncu "
                                     "capture (random 8-byte gathers, one LSU wavefront each); "
-                                    "L2 39%, DRAM 0.2% (ncu of bench.py --profile-once)"},
+                                    "L2 23%, DRAM 11% (ncu of bench.py --profile-once)"},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},
