@@ -356,11 +356,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_sliced(SlicedArgs A) {
     // step instead of 120; 211k cells: 31.8 instead of 30).
     auto gather = [](const double *p) { return NV > 1 ? *p : __ldcg(p); };
     // ||r|| / ||b|| > tol; the squares decide unless they are close (the exact
-    // form's square root and division are on every step's critical path)
+    // form's square root and division are on every step's critical path). A
+    // negative tolerance, which nothing meets, has no square to compare with.
     auto resid = [](double rr, double bn) { return sqrt(rr) / bn; };
     auto above_tol = [&](double rr, double bn) {
         const double lim = A.tol * bn, q = lim * lim;
-        if (q > 1e-280 && q < 1e280) {
+        if (lim > 0.0 && q > 1e-280 && q < 1e280) {
             if (rr > q * (1.0 + 1e-10)) return true;
             if (rr < q * (1.0 - 1e-10)) return false;
         }

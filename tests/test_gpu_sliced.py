@@ -94,3 +94,18 @@ def test_axes_apart(gpu_ctx, port_built):
         assert np.linalg.norm(got["x"] - ref["x"]) <= SOL_RTOL * np.linalg.norm(ref["x"]), kind
         scale = max(np.linalg.norm(ref["y"]), 1e-300)
         assert np.linalg.norm(got["y"] - ref["y"]) <= 1e-9 * scale, kind
+
+
+@pytest.mark.parametrize("tol", [-3e-2, -1.0, 0.0])
+@pytest.mark.parametrize("n", [300, 2050])
+def test_tolerance_that_nothing_meets(n, tol, gpu_ctx, port_built):
+    """Zero and negative tolerances run all the iterations that are allowed."""
+    sx, sy = random_system(n, [2, 6, 10], 11), random_system(n, [4, 8], 12)
+    x0, y0 = np.random.default_rng(13).standard_normal((2, n))
+    gpu_ctx.upload_system(0, sx)
+    gpu_ctx.upload_system(1, sy)
+    got = gpu_ctx.solve(x0, y0, tol, 6)
+    ref = oracle.port_solve_both(sx, x0, sy, y0, tol, 6)
+    assert ref["iters"] == 6 and got["iters"] == 6
+    for k in ("x", "y"):
+        assert np.linalg.norm(got[k] - ref[k]) <= SOL_RTOL * np.linalg.norm(ref[k])
