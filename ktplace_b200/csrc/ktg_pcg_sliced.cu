@@ -517,7 +517,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_sliced(SlicedArgs A) {
 #pragma unroll 2
         for (int32_t j = threadIdx.x; j < R; j += blockDim.x) {
             const int axis = vax[j];
-            const bool on = st.ok[axis] != 0u;
+            // (an axis that is done keeps its last ok and alpha)
+            const bool on = ((mask >> axis) & 1u) && st.ok[axis] != 0u;
             const double a = st.alpha[axis];
             const double apv = vap[j], d = vd[j], ri = vr[j];
             if (!on) continue;
