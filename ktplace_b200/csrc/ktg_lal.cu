@@ -3156,6 +3156,7 @@ __global__ void k_clamp_die(CellsDev C, int32_t n, double lx, double ly, double 
 struct LalState {
     std::vector<double> rowy, spans, obst;
     std::vector<double> side[4];  // obstacles' lx, ly, ux, uy, each sorted
+    int64_t odd = 0;              // obstacles that are in none of the four
     std::vector<int64_t> rowspan;
     double die[4] = {0, 0, 0, 0};
     DevBuf<double> d_rowy, d_spans, d_obst;
@@ -3174,14 +3175,18 @@ struct LalState {
     bool subtree_attr = false;
     bool wide_attr = false;
     // Upper bound on the obstacles that overlap `box`: the lesser of those that
-    // meet its x range and those that meet its y range.
+    // meet its x range and those that meet its y range. An obstacle whose sides
+    // are not in order passes the kernels' overlap test where its upper side lies
+    // above the box's lower and its lower side below the box's upper, so every
+    // box counts all of these; a box without extent counts all obstacles.
     int64_t obstacle_bound(const double *box) const {
-        auto meet = [&](int k) {
+        auto meet = [&](int k) -> int64_t {
+            if (!(box[k] < box[k + 2])) return static_cast<int64_t>(side[k].size());
             const auto past = std::lower_bound(side[k].begin(), side[k].end(), box[k + 2]);
             const auto before = std::upper_bound(side[k + 2].begin(), side[k + 2].end(), box[k]);
             return (past - side[k].begin()) - (before - side[k + 2].begin());
         };
-        return std::max<int64_t>(0, std::min(meet(0), meet(1)));
+        return odd + std::min(meet(0), meet(1));
     }
     // Upper bound on the profile's steps and edges of `box`: the rows it can
     // meet (as box_rows) and their spans.
@@ -3238,9 +3243,13 @@ int set_free_space(ktg_ctx *c, int64_t nrows, const double *rowy, const int64_t 
     s->spans.assign(spans, spans + 2 * S);
     s->obst.assign(obst, obst + 4 * nobst);
     for (int k = 0; k < 4; ++k) s->side[k].clear();
+    s->odd = 0;
     for (int64_t o = 0; o < nobst; ++o) {
         const double *q = obst + 4 * o;
-        if (!(q[0] <= q[2]) || !(q[1] <= q[3])) continue;  // overlaps no box
+        if (!(q[0] <= q[2]) || !(q[1] <= q[3])) {
+            ++s->odd;
+            continue;
+        }
         for (int k = 0; k < 4; ++k) s->side[k].push_back(q[k]);
     }
     for (int k = 0; k < 4; ++k) std::sort(s->side[k].begin(), s->side[k].end());

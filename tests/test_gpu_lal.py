@@ -261,3 +261,39 @@ def test_lal_handed_off_blocks(cells, macros, rows, seed, spread, gpu_ctx):
     for _ in range(4):
         got = run_gpu(gpu_ctx, nl, bins, 1.0, x, y)
         assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("subtree", [0, 2048])
+@pytest.mark.parametrize("kind", ["lx_past_ux", "ly_past_uy", "not_a_number"])
+def test_lal_obstacles_with_sides_out_of_order(kind, subtree, gpu_ctx):
+    """Obstacles whose lower side lies past their upper one, or is no number,
+    inside the blocks: their edges cut stripes as every obstacle's do, so the
+    room for stripes has to count them."""
+    raw = synth.generate(synth.spec_tiny(seed=8, macros=2, cells=420, nets=450))
+    nl = netlist.flatten(raw)
+    x, y = clustered(raw, nl.num_movable, 31, 0.15)
+    g = grid.build_grid(nl, 8, 1.0)
+    fs = grid.build_free_space(nl)
+    rng = np.random.default_rng(6)
+    lx, ly, ux, uy = fs.die
+    px, py = rng.uniform(lx, ux, 1900), rng.uniform(ly, uy, 1900)
+    swap = 0.5 * np.array([[1, 0, 0, 1], [0, 1, 1, 0], [0, 0, 1, 1]])[
+        ["lx_past_ux", "ly_past_uy", "not_a_number"].index(kind)]
+    fs.obstacles = np.stack([px, py, px, py], 1) + swap
+    if kind == "not_a_number":
+        fs.obstacles[:, 0] = np.nan
+    gpu_ctx.set_option("lal_subtree_cells", subtree)
+    gpu_ctx.set_option("lal_exact_sums", 1)
+    gpu_ctx.upload_netlist(nl)
+    gpu_ctx.set_grid(g)
+    gpu_ctx.set_free_space(fs)
+    try:
+        gx, gy = gpu_ctx.lal(x, y)
+    finally:
+        gpu_ctx.set_option("lal_subtree_cells", 2048)
+    gd = dict(origin=(g.origin_x, g.origin_y), dx=g.dx, dy=g.dy, nx=g.nx, ny=g.ny, avail=g.avail)
+    L = lal_ref.LAL(nl.width, nl.height, gd, lal_ref.free_rows(fs.row_y, fs.row_span, fs.spans),
+                    fs.obstacles, fs.die, g.density_limit)
+    ox, oy = L.legalize(x, y)
+    assert np.array_equal(gx, np.array(ox)) and np.array_equal(gy, np.array(oy))
+    assert np.mean(gx != x) > 0.1
