@@ -3158,6 +3158,7 @@ struct LalState {
     std::vector<double> side[4];  // obstacles' lx, ly, ux, uy, each sorted
     int64_t odd = 0;              // obstacles that are in none of the four
     std::vector<int64_t> rowspan;
+    bool rows_sorted = true;  // by y start, which are all numbers
     double die[4] = {0, 0, 0, 0};
     DevBuf<double> d_rowy, d_spans, d_obst;
     DevBuf<int64_t> d_rowspan;
@@ -3188,8 +3189,9 @@ struct LalState {
         };
         return odd + std::min(meet(0), meet(1));
     }
-    // Upper bound on the profile's steps and edges of `box`: the rows it can
-    // meet (as box_rows) and their spans.
+    // Upper bound on the profile's steps and edges of `box` and of its halves: the
+    // rows it can meet (as box_rows) and their spans. Where rows start at no
+    // number, box_rows finds others for a half than for the box: all of them then.
     void profile_bound(const double *box, bool vertical, int64_t &steps, int64_t &edges) const {
         const int64_t R = static_cast<int64_t>(rowy.size() / 2);
         int64_t lo = 0, hi = R;  // first row with box.ly < y end
@@ -3198,13 +3200,14 @@ struct LalState {
             if (box[1] < rowy[2 * mid + 1]) hi = mid;
             else lo = mid + 1;
         }
-        const int64_t r0 = lo;
+        int64_t r0 = lo;
         hi = R;  // first row from r0 with y start >= box.uy
         while (lo < hi) {
             const int64_t mid = (lo + hi) >> 1;
             if (rowy[2 * mid] < box[3]) lo = mid + 1;
             else hi = mid;
         }
+        if (!rows_sorted) r0 = 0, lo = R;
         const int64_t sp = R ? rowspan[lo] - rowspan[r0] : 0;
         steps = vertical ? 2 * sp : 0;
         edges = (vertical ? 2 * sp : 2 * (lo - r0)) + 2;
@@ -3240,6 +3243,8 @@ int set_free_space(ktg_ctx *c, int64_t nrows, const double *rowy, const int64_t 
     const int64_t S = nrows > 0 ? rowspan[nrows] : 0;
     s->rowy.assign(rowy, rowy + 2 * nrows);
     s->rowspan.assign(rowspan, rowspan + nrows + 1);
+    s->rows_sorted = true;
+    for (int64_t r = 0; r < nrows; ++r) s->rows_sorted = s->rows_sorted && !std::isnan(rowy[2 * r]);
     s->spans.assign(spans, spans + 2 * S);
     s->obst.assign(obst, obst + 4 * nobst);
     for (int k = 0; k < 4; ++k) s->side[k].clear();

@@ -297,3 +297,33 @@ def test_lal_obstacles_with_sides_out_of_order(kind, subtree, gpu_ctx):
     ox, oy = L.legalize(x, y)
     assert np.array_equal(gx, np.array(ox)) and np.array_equal(gy, np.array(oy))
     assert np.mean(gx != x) > 0.1
+
+
+@pytest.mark.parametrize("subtree", [0, 2048])
+def test_lal_rows_that_start_at_no_number(subtree, gpu_ctx):
+    """Rows whose start is no number break the order that the row searches rely
+    on, so a half box can find more of them than its block: the room for its
+    profile has to hold. Positions stay finite and inside the die."""
+    raw = synth.generate(synth.spec_tiny(seed=8, macros=2, cells=900, nets=950))
+    nl = netlist.flatten(raw)
+    x, y = clustered(raw, nl.num_movable, 31, 0.15)
+    g = grid.build_grid(nl, 8, 1.0)
+    fs = grid.build_free_space(nl)
+    lx, ly, ux, uy = fs.die
+    rows = 4000
+    edge = np.linspace(ly, uy, rows + 1)
+    fs.row_y = np.stack([edge[:-1], edge[1:]], 1)
+    fs.row_y[np.random.default_rng(3).integers(0, rows, rows // 3), 0] = np.nan
+    fs.spans = np.tile([[lx, ux]], (rows, 1))
+    fs.row_span = np.arange(rows + 1, dtype=np.int64)
+    gpu_ctx.set_option("lal_subtree_cells", subtree)
+    gpu_ctx.set_option("lal_exact_sums", 1)
+    gpu_ctx.upload_netlist(nl)
+    gpu_ctx.set_grid(g)
+    gpu_ctx.set_free_space(fs)
+    try:
+        gx, gy = gpu_ctx.lal(x, y)
+    finally:
+        gpu_ctx.set_option("lal_subtree_cells", 2048)
+    assert np.all((gx >= lx) & (gx <= ux) & (gy >= ly) & (gy <= uy))
+    assert np.mean(gx != x) > 0.1
