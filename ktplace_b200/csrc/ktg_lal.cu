@@ -617,6 +617,7 @@ struct Level {
     int32_t *m;
     double *low_area, *high_area, *cut;
     double *half_box;      // [8 na]: low box, high box
+    int32_t *redo;         // set by k_fill_order: nothing filled or placed yet
 };
 
 // The per-cell kernels below run on a 2-D grid: y strides over the active
@@ -783,6 +784,7 @@ __global__ void k_block_split(Level L, CellsDev C, const int32_t *cells, const l
         for (int32_t p = b + m; p < e; ++p) high += C.area[cells[p]];
     }
     if (lane != 0) return;
+    if (blk == 0) *L.redo = 0;
     L.m[blk] = m;
     L.low_area[blk] = low;
     L.high_area[blk] = high;
@@ -1362,7 +1364,12 @@ __global__ void __launch_bounds__(kWideT) k_half_stripes_cta(Level L, Free F, co
 // (centre, id): the distance is monotone in that order, so the low half keeps
 // it, the high half reverses it, and cells at the same (rounded) distance go by
 // id. A run of one centre is in id order already; a run of several centres is
-// ranked by counting.
+// ranked by counting, which costs the square of its length: past kMixedRun cells
+// the level is left unfilled, and the host sorts by (distance, id) and fills it
+// (150k cells within 60 ulp of one x: 5.6 ms in all, 12.9 with ranks by counting;
+// 5.4 with one x for all of them).
+constexpr int kMixedRun = 256;
+
 __global__ void k_fill_order(Level L, const Key *keys, int32_t *cells) {
     for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
         const int32_t b = L.b[blk], e = L.e[blk], mid = b + L.m[blk];
@@ -1400,6 +1407,10 @@ __global__ void k_fill_order(Level L, const Key *keys, int32_t *cells) {
             const unsigned long long id = keys[p].b;
             int32_t rank = p - rs;
             if (re - rs > 1 && keys[rs].a != keys[re - 1].a) {
+                if (re - rs > kMixedRun) {
+                    *L.redo = 1;
+                    continue;
+                }
                 rank = 0;
                 for (int32_t q = rs; q < re; ++q) rank += keys[q].b < id ? 1 : 0;
             }
@@ -1408,9 +1419,23 @@ __global__ void k_fill_order(Level L, const Key *keys, int32_t *cells) {
     }
 }
 
+// The keys of that order, from the keys sorted by (centre, id).
+__global__ void k_distance_keys(Level L, const Key *keys, Key *out) {
+    for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
+        const int32_t b = L.b[blk], e = L.e[blk], mid = b + L.m[blk];
+        const double cut = L.cut[blk];
+        for (int32_t p = b + blockIdx.x * blockDim.x + threadIdx.x; p < e;
+             p += gridDim.x * blockDim.x) {
+            const double c = unord(keys[p].a);
+            out[p] = Key{ord(-(p < mid ? cut - c : c - cut)), keys[p].b};
+        }
+    }
+}
+
 // One thread per half: greedy fill in the sorted order (nonlinearScale,
 // simpl_lal.cc:332-340).
 __global__ void k_fill(Level L, CellsDev C, const int32_t *cells, Stripes S, int32_t *stripe_of) {
+    if (*L.redo) return;
     const int32_t h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= 2 * L.na) return;
     const int32_t blk = h >> 1;
@@ -1446,6 +1471,7 @@ __global__ void __launch_bounds__(1024) k_fill_fx(Level L, Stripes S, const long
                                                   double scale, int32_t *sbeg) {
     extern __shared__ long long win[];
     __shared__ int32_t s_done;
+    if (*L.redo) return;
     const int lane = threadIdx.x & 31;
     const int32_t h = blockIdx.x;
     const int32_t blk = h >> 1;
@@ -1503,6 +1529,7 @@ __global__ void __launch_bounds__(1024) k_fill_fx(Level L, Stripes S, const long
 // the runs at a stripe's ends can hold them.
 __global__ void k_stripe_ends(Level L, CellsDev C, const int32_t *cells, Stripes S,
                               const int32_t *sbeg) {
+    if (*L.redo) return;
     const int lane = threadIdx.x & 31;
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int32_t h = blockIdx.y; h < 2 * L.na; h += gridDim.y) {
@@ -1564,6 +1591,7 @@ __device__ __forceinline__ void place_cell(const CellsDev &C, const Stripes &S, 
 // the cell's new position.
 __global__ void k_place_fx(Level L, CellsDev C, const int32_t *cells, Stripes S,
                            const int32_t *sbeg) {
+    if (*L.redo) return;
     for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
         const int32_t b = L.b[blk], e = L.e[blk], mid = b + L.m[blk];
         const bool v = L.vert[blk] != 0;
@@ -1585,6 +1613,7 @@ __global__ void k_place_fx(Level L, CellsDev C, const int32_t *cells, Stripes S,
 
 __global__ void k_stripe_minmax(Level L, CellsDev C, const int32_t *cells, Stripes S,
                                 const int32_t *stripe_of) {
+    if (*L.redo) return;
     for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
         const int32_t b = L.b[blk], e = L.e[blk];
         const bool v = L.vert[blk] != 0;
@@ -1601,6 +1630,7 @@ __global__ void k_stripe_minmax(Level L, CellsDev C, const int32_t *cells, Strip
 
 __global__ void k_new_pos(Level L, CellsDev C, const int32_t *cells, Stripes S,
                           const int32_t *stripe_of) {
+    if (*L.redo) return;
     for (int32_t blk = blockIdx.y; blk < L.na; blk += gridDim.y) {
         const int32_t b = L.b[blk], e = L.e[blk];
         const bool v = L.vert[blk] != 0;
@@ -3652,14 +3682,15 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
             };
             const size_t n_steps = std::max(st, hst) + 1, n_edges = std::max(ed, hed) + 1,
                          n_st = stripes + 1;
-            const size_t a_blob = carve(blob.size()), a_halves = carve(8 * i64 + i32),
+            const size_t a_blob = carve(blob.size()), a_halves = carve(8 * i64 + i32 + 4),
                          a_low = carve(i64), a_high = carve(i64), a_cut = carve(i64),
                          a_nsteps = carve(2 * i64), a_count = carve(2 * i32),
                          a_steps = carve(sizeof(Key) * n_steps),
                          a_tmp = carve(sizeof(Key) * n_steps), a_pe = carve(8 * n_edges),
                          a_pp = carve(8 * n_edges), a_sa = carve(8 * n_st), a_sb = carve(8 * n_st),
                          a_cap = carve(8 * n_st), a_used = carve(8 * n_st), a_lo = carve(8 * n_st),
-                         a_hi = carve(8 * n_st), a_beg = carve(4 * n_st);
+                         a_hi = carve(8 * n_st), a_beg = carve(4 * n_st),
+                         a_ranges = carve(4 * i32);
             if ((r2 = s->level.ensure(c, static_cast<int64_t>(need)))) return r2;
             char *const slab = s->level.p;
             auto dbl = [&](size_t at) { return reinterpret_cast<double *>(slab + at); };
@@ -3686,7 +3717,8 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
             KTG_CUDA(c, cudaMemcpyAsync(slab + a_blob, blob.data(), blob.size(),
                                         cudaMemcpyHostToDevice, c->stream));
             Level L{na, d32(o_b), d32(o_e), dbl(a_blob + o_box), d32(o_v), dbl(a_blob + o_room),
-                    i32p(a_halves + 8 * i64), dbl(a_low), dbl(a_high), dbl(a_cut), dbl(a_halves)};
+                    i32p(a_halves + 8 * i64), dbl(a_low), dbl(a_high), dbl(a_cut), dbl(a_halves),
+                    i32p(a_halves + 8 * i64 + i32)};
             const dim3 gcell(std::min(64, blocks_for(maxlen)), std::min(na, 65535));
             // 1. cells by centre
             Key *order, *sorted;
@@ -3723,31 +3755,56 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
                 L, F, d64(o_hsoff), sorted, nsteps, d64(o_heoff), dbl(a_pe), dbl(a_pp),
                 d64(o_cap), frac, c->density_limit, S, c->status);
             // 5. fill order, fill, stripe ranges, positions
+            auto fill = [&]() -> int {
+                int r3;
+                if (exact) {
+                    if ((r3 = fx_prefix(run))) return r3;
+                    k_fill_fx<<<2 * na, 1024, kFillSmem, c->stream>>>(L, S, s->pre.p, scale, sbeg);
+                    k_stripe_ends<<<dim3(16, std::min(2 * na, 65535)), kT, 0, c->stream>>>(
+                        L, C, s->cells.p, S, sbeg);
+                    k_place_fx<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, sbeg);
+                } else {
+                    if ((r3 = s->stripe_of.ensure(c, n + 1))) return r3;
+                    k_fill<<<blocks_for(2 * na), kT, 0, c->stream>>>(L, C, s->cells.p, S,
+                                                                     s->stripe_of.p);
+                    k_stripe_minmax<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S,
+                                                                 s->stripe_of.p);
+                    k_new_pos<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, s->stripe_of.p);
+                }
+                c->launches += 3;
+                KTG_CUDA(c, cudaGetLastError());
+                return KTG_OK;
+            };
             k_fill_order<<<gcell, kT, 0, c->stream>>>(L, order, s->cells.p);
             c->launches += 2;
-            if (exact) {
-                if ((r2 = fx_prefix(run))) return r2;
-                k_fill_fx<<<2 * na, 1024, kFillSmem, c->stream>>>(L, S, s->pre.p, scale, sbeg);
-                k_stripe_ends<<<dim3(16, std::min(2 * na, 65535)), kT, 0, c->stream>>>(
-                    L, C, s->cells.p, S, sbeg);
-                k_place_fx<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, sbeg);
-                c->launches += 3;
-            } else {
-                if ((r2 = s->stripe_of.ensure(c, n + 1))) return r2;
-                k_fill<<<blocks_for(2 * na), kT, 0, c->stream>>>(L, C, s->cells.p, S,
-                                                                 s->stripe_of.p);
-                k_stripe_minmax<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, s->stripe_of.p);
-                k_new_pos<<<gcell, kT, 0, c->stream>>>(L, C, s->cells.p, S, s->stripe_of.p);
-                c->launches += 3;
-            }
-            KTG_CUDA(c, cudaGetLastError());
+            if ((r2 = fill())) return r2;
             // children
-            std::vector<char> back(8 * i64 + i32);
+            std::vector<char> back(8 * i64 + i32 + 4);
             KTG_CUDA(c, cudaMemcpyAsync(back.data(), slab + a_halves, back.size(),
                                         cudaMemcpyDeviceToHost, c->stream));
             KTG_CUDA(c, lal_sync(c));
             const double *halfbox = reinterpret_cast<const double *>(back.data());
             const int32_t *mh = reinterpret_cast<const int32_t *>(back.data() + 8 * i64);
+            if (mh[na]) {  // long runs of one distance: the halves sorted, then filled
+                std::vector<int32_t> ranges(4 * na);  // of the halves: first, end
+                for (int32_t k = 0; k < na; ++k) {
+                    ranges[2 * k] = ab[k];
+                    ranges[2 * k + 1] = ranges[2 * na + 2 * k] = ab[k] + mh[k];
+                    ranges[2 * na + 2 * k + 1] = ae[k];
+                }
+                KTG_CUDA(c, cudaMemcpyAsync(slab + a_ranges, ranges.data(), 4 * i32,
+                                            cudaMemcpyHostToDevice, c->stream));
+                KTG_CUDA(c, cudaMemsetAsync(L.redo, 0, sizeof(int32_t), c->stream));
+                Key *const by = order == s->keys.p ? s->keys_tmp.p : s->keys.p;
+                k_distance_keys<<<gcell, kT, 0, c->stream>>>(L, order, by);
+                if ((r2 = sort_segs(c, by, order,
+                                    Segs{i32p(a_ranges), i32p(a_ranges) + 2 * na, nullptr, nullptr},
+                                    2 * na, maxlen, &order)))
+                    return r2;
+                k_keys_to_cells<<<gcell, kT, 0, c->stream>>>(L, order, s->cells.p);
+                c->launches += 2;
+                if ((r2 = fill())) return r2;
+            }
             hb.clear();
             he.clear();
             hv.clear();

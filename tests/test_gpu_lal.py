@@ -327,3 +327,47 @@ def test_lal_rows_that_start_at_no_number(subtree, gpu_ctx):
         gpu_ctx.set_option("lal_subtree_cells", 2048)
     assert np.all((gx >= lx) & (gx <= ux) & (gy >= ly) & (gy <= uy))
     assert np.mean(gx != x) > 0.1
+
+
+def piled(raw, n, seed, ulps):
+    """Centres within `ulps` ulp of one x, far from the cutline: thousands of them
+    at each rounded distance."""
+    rng = np.random.default_rng(seed)
+    lx, ly, ux, uy = raw.die
+    x = lx + 2.0 + np.spacing(4.0) * rng.integers(0, ulps, n)
+    y = 0.5 * (ly + uy) + 0.1 * (uy - ly) * rng.standard_normal(n)
+    return x, y
+
+
+@pytest.mark.parametrize("exact", [1, 0])
+@pytest.mark.parametrize("subtree", [0, 2048])
+def test_lal_long_runs_of_one_distance(subtree, exact, gpu_ctx):
+    raw = synth.generate(synth.spec_tiny(seed=12, macros=2, cells=5200, nets=5230))
+    nl = netlist.flatten(raw)
+    x, y = piled(raw, nl.num_movable, 3, 60)
+    far = np.random.default_rng(4).random(nl.num_movable) < 0.2
+    x[far] = clustered(raw, nl.num_movable, 5, 0.2)[0][far]
+    gx, gy = run_gpu(gpu_ctx, nl, 8, 1.0, x, y, subtree=subtree, exact=exact)
+    gpu_ctx.set_option("lal_subtree_cells", 2048)
+    gpu_ctx.set_option("lal_exact_sums", 1)
+    ox, oy = run_oracle(nl, 8, 1.0, x, y)
+    assert np.array_equal(gx, ox) and np.array_equal(gy, oy)
+
+
+def test_lal_long_runs_cost_no_square(gpu_ctx):
+    """A pile of 150k cells takes at most the time of two legalizations with one
+    centre for all of them: only the levels with such runs sort and fill again."""
+    raw = synth.generate(synth.SynthSpec(num_movable=150000, num_nets=151000, num_pads=400,
+                                         num_rows=500, utilization=0.6, num_macros=0, seed=5))
+    nl = netlist.flatten(raw)
+    bins = grid.default_bins_per_axis(nl.num_movable)
+    ms = {}
+    for ulps in (1, 60):
+        x, y = piled(raw, nl.num_movable, 7, ulps)
+        took = []
+        for _ in range(4):
+            run_gpu(gpu_ctx, nl, bins, 1.0, x, y)
+            took.append(gpu_ctx.lal_stats()["ms_total"])
+        ms[ulps] = min(took[1:])
+    print(ms)
+    assert ms[60] <= 2.0 * ms[1], ms
