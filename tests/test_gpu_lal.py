@@ -371,3 +371,19 @@ def test_lal_long_runs_cost_no_square(gpu_ctx):
         ms[ulps] = min(took[1:])
     print(ms)
     assert ms[60] <= 2.0 * ms[1], ms
+
+
+@pytest.mark.parametrize("cells", [700, 1300, 1900])
+def test_lal_halves_go_to_other_ctas(cells, gpu_ctx):
+    """The queue is used: every region is one block of the first launch, so more
+    one-CTA blocks than regions are halves that were handed off. Without the
+    level-by-level path in between, and bit-identical to it."""
+    raw = synth.generate(synth.spec_tiny(seed=cells, macros=2, cells=cells, nets=cells + 30))
+    nl = netlist.flatten(raw)
+    x, y = clustered(raw, nl.num_movable, 3, 0.03)
+    want = run_gpu(gpu_ctx, nl, 16, 1.0, x, y, subtree=0)
+    gx, gy = run_gpu(gpu_ctx, nl, 16, 1.0, x, y)
+    st = gpu_ctx.lal_stats()
+    assert st["big_levels"] == 0 and st["subtree_handed_back"] == 0
+    assert st["subtree_blocks"] > st["regions"], st
+    assert np.array_equal(gx, want[0]) and np.array_equal(gy, want[1])
