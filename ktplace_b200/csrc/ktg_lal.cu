@@ -3475,17 +3475,29 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
     auto run_subtree = [&](const std::vector<SubTask> &tasks, std::vector<SubTask> &left) -> int {
         const int32_t nt = static_cast<int32_t>(tasks.size());
         const int32_t cap = nt * kHandSlots;
-        const int grid = std::min(c->num_sms, cap);
+        // CTAs: as many as the queue can keep busy, one for every part of at most
+        // kHandOff cells that the blocks halve into; the rest would hold their SMs
+        // waiting, and other streams' work out (a block of 100 cells: 1, not 48)
+        int64_t parts = 0;
+        for (const SubTask &t : tasks) {
+            int64_t k = 1;
+            for (int32_t size = t.e - t.b; size > kHandOff; size = (size + 1) / 2) k *= 2;
+            parts += k;
+        }
+        const int grid = static_cast<int>(std::min<int64_t>(c->num_sms, parts));
+        // scratch for them, and for what a larger batch of this design may take
+        const int64_t room = std::max<int64_t>(
+            grid, std::min<int64_t>(c->num_sms, 2 * static_cast<int64_t>(n) / kHandOff + 1));
         const double t0 = now_ms();
         int r2;
         const bool grow = s->ready.cap < cap;
         if ((r2 = s->tasks.ensure(c, kQueueHead + sizeof(SubTask) * static_cast<int64_t>(cap))) ||
             (r2 = s->ready.ensure(c, cap)) || (r2 = s->tfail.ensure(c, cap)) ||
-            (r2 = s->swork.ensure(c, c->num_sms * (kDescBytes + 6 * 8 * kStripeCap))))
+            (r2 = s->swork.ensure(c, room * (kDescBytes + 6 * 8 * kStripeCap))))
             return r2;
-        double *const strp = reinterpret_cast<double *>(s->swork.p + c->num_sms * kDescBytes);
+        double *const strp = reinterpret_cast<double *>(s->swork.p + grid * kDescBytes);
         auto *const strlh =
-            reinterpret_cast<unsigned long long *>(strp + c->num_sms * 4 * kStripeCap);
+            reinterpret_cast<unsigned long long *>(strp + grid * 4 * kStripeCap);
         if (grow || s->epoch == 0xffffffffu) {
             KTG_CUDA(c, cudaMemsetAsync(s->ready.p, 0, sizeof(unsigned) * s->ready.cap, c->stream));
             s->epoch = 0;

@@ -387,3 +387,21 @@ def test_lal_halves_go_to_other_ctas(cells, gpu_ctx):
     assert st["big_levels"] == 0 and st["subtree_handed_back"] == 0
     assert st["subtree_blocks"] > st["regions"], st
     assert np.array_equal(gx, want[0]) and np.array_equal(gy, want[1])
+
+
+def test_lal_scratch_of_a_small_design(port_built):
+    """A design whose blocks keep a few CTAs busy takes scratch for those, not for
+    one on every SM (0.8 MB each)."""
+    import torch
+    from ktplace_b200.gpu import Context
+    raw = synth.generate(synth.spec_tiny(seed=5, macros=2, cells=300, nets=330))
+    nl = netlist.flatten(raw)
+    x, y = clustered(raw, nl.num_movable, 3, 0.03)
+    taken = []
+    for _ in range(2):  # the first one also loads the kernels
+        with Context(0) as ctx:
+            before = torch.cuda.mem_get_info()[0]
+            run_gpu(ctx, nl, 16, 1.0, x, y)
+            assert ctx.lal_stats()["subtree_blocks"] >= 1
+            taken.append(before - torch.cuda.mem_get_info()[0])
+    assert taken[1] <= 48 * 2**20, taken
