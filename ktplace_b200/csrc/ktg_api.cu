@@ -121,6 +121,7 @@ void free_systems(ktg_ctx *c) {
     dev_free(c->sliced_rows);
     dev_free(c->sliced_nnz);
     c->sliced = ktg::SlicedSystem{};
+    c->sliced_cap = 0;
     dev_free(c->x);
     dev_free(c->y);
     dev_free(c->ax);
@@ -232,15 +233,20 @@ int reserve_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
             if ((rc = dev_alloc(c, &s.val32, nnz))) return rc;
             if ((rc = dev_alloc(c, &s.s32, nnz))) return rc;
         }
-        const int64_t entries = ktg::sliced_entries(2 * nnz, c->num_sms);  // a multiple of 32
-        if ((rc = dev_alloc(c, &c->sliced_nnz, entries * 12))) return rc;
-        c->sliced.val = reinterpret_cast<double *>(c->sliced_nnz);
-        c->sliced.col = reinterpret_cast<int32_t *>(c->sliced.val + entries);
         c->val32_valid = false;
         c->precond_ready = false;
         c->agg_ready = false;
         c->coarse_z_ready = false;
         c->sys_cap_nnz = nnz;
+    }
+    // the sliced copy pads for the blocks that a solve of these rows takes
+    const int64_t entries = ktg::sliced_entries(
+        2 * c->sys_cap_nnz, ktg::sliced_blocks(2 * c->sys_cap_n, c->num_sms));  // a multiple of 32
+    if (entries > c->sliced_cap) {
+        if ((rc = dev_alloc(c, &c->sliced_nnz, entries * 12))) return rc;
+        c->sliced.val = reinterpret_cast<double *>(c->sliced_nnz);
+        c->sliced.col = reinterpret_cast<int32_t *>(c->sliced.val + entries);
+        c->sliced_cap = entries;
     }
     return KTG_OK;
 }

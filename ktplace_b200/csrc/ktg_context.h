@@ -117,6 +117,7 @@ struct ktg_ctx {
     ktg::AxisSystem sys[2];
     ktg::SlicedSystem sliced;  // scratch of the default FP64 solve
     char *sliced_rows = nullptr, *sliced_nnz = nullptr;  // its two allocations
+    int64_t sliced_cap = 0;                              // entries of the second
     bool have_system = false;  // both axes valid with sys_n rows
     bool axis_valid[2] = {false, false};
     bool val32_valid = false;  // sys[*].val32 mirrors sys[*].val
@@ -208,7 +209,8 @@ int launch_solve(ktg_ctx *ctx, double *x, double *y, double tol, int64_t max_ite
 int launch_solve_sliced(ktg_ctx *ctx, double *x, double *y, double tol, int64_t max_iter,
                         ktg_solve_info *info_dev, double *hist_x, double *hist_y,
                         int64_t hist_cap);
-int64_t sliced_entries(int64_t nnz_both, int num_sms);
+int sliced_blocks(int64_t rows, int num_sms);
+int64_t sliced_entries(int64_t nnz_both, int blocks);
 int64_t sliced_slices(int64_t rows, int num_sms);
 int64_t sliced_slots(int num_sms);
 int launch_occupancy(ktg_ctx *ctx, const double *x, const double *y, double *occ_dev,

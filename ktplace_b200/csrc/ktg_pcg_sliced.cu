@@ -586,9 +586,32 @@ size_t sliced_smem(int nv, int64_t rows_per_block) {
 
 }  // namespace
 
-int64_t sliced_entries(int64_t nnz_both, int num_sms) {
-    return 32 * region_base(nnz_both, num_sms);
+// Blocks of a solve over `rows` rows of both axes.
+static int sliced_grid(int64_t rows, int num_sms) {
+    // One up to kThreads rows (its sums need no barrier: 5.1 us a step at 600
+    // rows, 7.5 us on three blocks). Then kSmallBlocks of kSmallRows to kThreads
+    // rows (2,000 rows: 7.0 us a step with 256 rows a block, 9.4 with 1,024;
+    // 24,000 rows: 9.7 and 10.1), and beyond that kThreads rows a block: a third of
+    // the SMs serves a small system as well as all of them, and leaves room for
+    // solves on other streams.
+    const int64_t per =
+        rows <= kThreads
+            ? kThreads
+            : std::min<int64_t>(kThreads, std::max<int64_t>(kSmallRows,
+                                                            (rows + kSmallBlocks - 1) / kSmallBlocks));
+    const int64_t most = std::min(num_sms, 32 * kSumGroups);
+    return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(most, (rows + per - 1) / per)));
 }
+
+// The most blocks of a solve over up to `rows` rows (sliced_grid can fall by one
+// where the rows of a block grow).
+int sliced_blocks(int64_t rows, int num_sms) {
+    const int64_t small = std::min<int64_t>(kSmallBlocks, (rows + kSmallRows - 1) / kSmallRows);
+    const int64_t blocks = rows <= kThreads ? 1 : std::max(small, (rows + kThreads - 1) / kThreads);
+    return static_cast<int>(std::min<int64_t>(std::min(num_sms, 32 * kSumGroups), blocks));
+}
+
+int64_t sliced_entries(int64_t nnz_both, int blocks) { return 32 * region_base(nnz_both, blocks); }
 
 // Slices of a block of `rows` rows: a warp per row at worst, and one end mark.
 int64_t sliced_slices(int64_t rows, int num_sms) { return rows + 2 * num_sms; }
@@ -605,20 +628,7 @@ int launch_solve_sliced(ktg_ctx *c, double *x, double *y, double tol, int64_t ma
     }
     A.n = static_cast<int32_t>(c->sys_n);
     const int64_t total = 2 * c->sys_n;
-    // Blocks: one up to kThreads rows (its sums need no barrier: 5.1 us a step
-    // at 600 rows, 7.5 us on three blocks). Then kSmallBlocks of kSmallRows to
-    // kThreads rows (2,000 rows: 7.0 us a step with 256 rows a block, 9.4 with
-    // 1,024; 24,000 rows: 9.7 and 10.1), and beyond that kThreads rows a block:
-    // a third of the SMs serves a small system as well as all of them, and
-    // leaves room for solves on other streams.
-    const int64_t rows =
-        total <= kThreads
-            ? kThreads
-            : std::min<int64_t>(kThreads, std::max<int64_t>(kSmallRows,
-                                                            (total + kSmallBlocks - 1) / kSmallBlocks));
-    const int64_t most = std::min(c->num_sms, 32 * kSumGroups);
-    const int grid = static_cast<int>(
-        std::max<int64_t>(1, std::min<int64_t>(most, (total + rows - 1) / rows)));
+    const int grid = sliced_grid(total, c->num_sms);
     A.rows_per_block = static_cast<int32_t>(std::max<int64_t>(1, (total + grid - 1) / grid));
     A.slices_per_block = A.rows_per_block + 1;
     const int threads = grid > 1 && A.rows_per_block <= kSmallRows ? kThreads / 2 : kThreads;

@@ -109,3 +109,24 @@ def test_tolerance_that_nothing_meets(n, tol, gpu_ctx, port_built):
     assert ref["iters"] == 6 and got["iters"] == 6
     for k in ("x", "y"):
         assert np.linalg.norm(got[k] - ref[k]) <= SOL_RTOL * np.linalg.norm(ref[k])
+
+
+def test_scratch_follows_the_blocks(port_built):
+    """The copy is padded per block of the solve, so a small design's context takes
+    little memory; rows may outgrow it when the entries do not."""
+    import torch
+    from ktplace_b200 import netlist, synth
+    from ktplace_b200.gpu import Context
+    nl = netlist.flatten(synth.generate(synth.spec_tiny(seed=1, cells=300, nets=330)))
+    taken = []
+    for _ in range(2):  # the first one also loads the library
+        with Context(0) as ctx:
+            before = torch.cuda.mem_get_info()[0]
+            ctx.upload_netlist(nl)
+            taken.append(before - torch.cuda.mem_get_info()[0])
+    assert taken[1] <= 6 * 2**20, taken
+    with Context(0) as ctx:
+        check(ctx, 300, [100, 200, 60])
+        check(ctx, 24_001, [0, 2], seed=4)
+        check(ctx, 160_001, [0, 2, 0, 0], seed=5)
+        check(ctx, 300, [100, 200, 60])
