@@ -25,7 +25,7 @@ namespace ktg {
 // Bits of ktg_ctx::attr_bits.
 constexpr unsigned kAttrOccupancy = 1u;  // k_occ_accum<true> opt-in shared memory
 constexpr unsigned kAttrMixed = 2u;      // k_pcg_mixed_cg opt-in shared memory
-constexpr unsigned kAttrSliced = 4u;     // k_pcg_sliced opt-in shared memory
+constexpr unsigned kAttrSliced = 4u;     // k_pcg_sliced<...> opt-in shared memory, four bits
 
 struct AggState;  // aggregation preconditioner buffers (ktg_agg.cu)
 struct LalState;  // free space and scratch of the look-ahead legalizer (ktg_lal.cu)

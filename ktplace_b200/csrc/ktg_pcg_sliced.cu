@@ -649,11 +649,11 @@ int launch_solve_sliced(ktg_ctx *c, double *x, double *y, double tol, int64_t ma
     while (sliced_smem(vecs[pick], A.rows_per_block) > kSmemBudget) --pick;
     const Kernel fn = kernels[pick];
     const size_t bytes = sliced_smem(vecs[pick], A.rows_per_block);
-    if (!(c->attr_bits & kAttrSliced)) {
-        for (const Kernel k : kernels)
-            KTG_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(kSmemBudget)));
-        c->attr_bits |= kAttrSliced;
+    // per variant, as it comes up: the attribute loads the kernel
+    if (!(c->attr_bits & (kAttrSliced << pick))) {
+        KTG_CUDA(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(kSmemBudget)));
+        c->attr_bits |= kAttrSliced << pick;
     }
     A.tol = tol;
     A.max_iter = max_iter;
