@@ -533,7 +533,8 @@ int ktg_upload_netlist(ktg_ctx *c, const ktg_netlist_view *nl) {
         int32_t m = 0;
         for (int64_t p = nl->net_start[k]; p < nl->net_start[k + 1]; ++p) m += pin_var[p] >= 0;
         net_mov[k] = m;
-        // Bound rows (2) get m-1 movable ends, the others at most 2 each.
+        // Bound rows (2) get m-1 movable ends, the others at most 2 each, where
+        // every pin belongs to one row entry (else see below).
         if (m > 1) cap += 4 * static_cast<int64_t>(m) - 6;
         range += 4 * static_cast<int64_t>(m);
     }
@@ -545,11 +546,16 @@ int ktg_upload_netlist(ktg_ctx *c, const ktg_netlist_view *nl) {
             return set_error(c, KTG_ERR_ARG, "pin_ref out of range");
         pin_ref[e] = make_int2(k, q);
     }
+    std::vector<bool> listed(P);
+    bool twice = false;  // a cell lists a pin more than once: its edges count each time
     for (int64_t i = 0; i < n; ++i)
         for (int64_t e = nl->pin_start[i]; e < nl->pin_start[i + 1]; ++e) {
             const int64_t p = nl->net_start[nl->pin_net[e]] + nl->pin_q[e];
             if (pin_var[p] != i) return set_error(c, KTG_ERR_ARG, "pin_ref does not point to its cell");
+            twice = twice || listed[p];
+            listed[p] = true;
         }
+    if (twice) cap = range;
     if (range > lim) return set_error(c, KTG_ERR_RANGE, "B2B systems exceed 32-bit indices");
     std::vector<double> area(n);
     double total_area = 0.0;

@@ -95,3 +95,32 @@ def test_build_at_tile_edges(n, kraftwerk2, gpu_ctx):
             assert np.array_equal(got[k], np.asarray(want[k])), (axis, k)
         for k in ("col", "val"):
             assert np.array_equal(got[k][:m], np.asarray(want[k])), (axis, k)
+
+
+def test_pins_listed_twice(gpu_ctx):
+    """A cell may list a pin more than once; each listing adds its edges to the
+    row, beyond what the nets' pins alone would give."""
+    raw = design(65, 9)
+    fixed = np.nonzero(raw.fixed)[0].astype(raw.pin_cell.dtype)
+    pads = np.tile(fixed[:2], 200)  # nets of fixed pins: room for the listings
+    starts = raw.net_start[-1] + 2 * np.arange(1, 201)
+    zeros = np.zeros(len(pads))
+    raw = dataclasses.replace(
+        raw, net_start=np.concatenate([raw.net_start, starts.astype(raw.net_start.dtype)]),
+        pin_cell=np.concatenate([raw.pin_cell, pads]),
+        pin_fox=np.concatenate([raw.pin_fox, zeros]), pin_foy=np.concatenate([raw.pin_foy, zeros]),
+        net_weight=np.concatenate([raw.net_weight, np.ones(200)]))
+    nl = netlist.flatten(raw)
+    n = nl.num_movable
+    times = np.where(np.arange(len(nl.pin_net)) % 3 == 0, 2, 1)
+    cell = np.repeat(np.repeat(np.arange(n), np.diff(nl.pin_start)), times)
+    nl.pin_net, nl.pin_q = np.repeat(nl.pin_net, times), np.repeat(nl.pin_q, times)
+    nl.pin_start = np.concatenate([[0], np.cumsum(np.bincount(cell, minlength=n))])
+    x, y, ax, ay = np.random.default_rng(2).uniform(0.0, 500.0, (4, n))
+    gpu_ctx.upload_netlist(nl)
+    gpu_ctx.build_b2b(x, y, 0.3, ax, ay, 3.0, 2.0)
+    for axis, (pos, anchor, floor) in enumerate(((x, ax, 3.0), (y, ay, 2.0))):
+        want = restated(nl, pos, axis, 0.3, anchor, floor, False)
+        got = gpu_ctx.system(axis)
+        for k, v in want.items():
+            assert np.array_equal(got[k], np.asarray(v)), (axis, k)
