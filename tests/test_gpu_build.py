@@ -124,3 +124,25 @@ def test_pins_listed_twice(gpu_ctx):
         got = gpu_ctx.system(axis)
         for k, v in want.items():
             assert np.array_equal(got[k], np.asarray(v)), (axis, k)
+
+
+@pytest.mark.parametrize("nets", [2047, 2048, 2049, 4097])
+def test_bound_pins_come_back_in_parts(nets, gpu_ctx):
+    """Downloaded 2,048 nets at a time; the first lowest and first highest pin."""
+    raw = design(64, 3)
+    rng = np.random.default_rng(nets)
+    pins = rng.choice(np.nonzero(~raw.fixed)[0], (nets, 3))
+    raw = dataclasses.replace(
+        raw, net_start=(3 * np.arange(nets + 1)).astype(raw.net_start.dtype),
+        pin_cell=pins.ravel().astype(raw.pin_cell.dtype), pin_fox=rng.uniform(-2.0, 2.0, 3 * nets),
+        pin_foy=rng.uniform(-2.0, 2.0, 3 * nets), net_weight=np.ones(nets))
+    nl = netlist.flatten(raw, kraftwerk2=True)  # (pins of one cell stay apart)
+    n = nl.num_movable
+    x, y = rng.uniform(0.0, 500.0, (2, n))
+    gpu_ctx.upload_netlist(nl)
+    gpu_ctx.build_b2b(x, y, 0.0, None, None, 3.0, 2.0)
+    for axis, (pos, off) in enumerate(((x, nl.off_x), (y, nl.off_y))):
+        at = (pos[nl.var_of_vertex[nl.pin_cell]] + off).reshape(-1, 3)
+        lo, hi = gpu_ctx.bound_pins(axis)
+        assert nl.num_nets == nets
+        assert np.array_equal(lo, np.argmin(at, 1)) and np.array_equal(hi, np.argmax(at, 1))
