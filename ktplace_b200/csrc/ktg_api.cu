@@ -93,6 +93,7 @@ void free_netlist(ktg_ctx *c) {
     dev_free(c->area);
     dev_free(c->row_cnt);
     dev_free(c->block_sum);
+    for (auto &s : c->sys) dev_free(s.bound);
     c->have_netlist = false;
 }
 
@@ -103,7 +104,6 @@ void free_systems(ktg_ctx *c) {
         dev_free(s.val);
         dev_free(s.diag);
         dev_free(s.rhs);
-        dev_free(s.bound);
         dev_free(s.r);
         dev_free(s.z);
         dev_free(s.p);
@@ -131,10 +131,9 @@ void free_systems(ktg_ctx *c) {
     c->stage_cap = 0;
     c->have_system = false;
     c->axis_valid[0] = c->axis_valid[1] = false;
+    c->val32_valid = c->precond_ready = c->agg_ready = c->coarse_z_ready = false;
 }
 
-// Makes room for systems of `rows` rows and `nnz` entries per axis and for
-// per-net bound pins of the current netlist.
 // A larger array that keeps the first `keep` elements of the old one (the
 // copy is stream-ordered; cudaFree waits for it).
 template <typename T>
@@ -196,7 +195,7 @@ int reserve_sliced_rows(ktg_ctx *c, int64_t rows) {
 // that hold a system (row pointers, columns, values, diagonal, right-hand
 // side) keep their contents when they grow, so an axis installed earlier
 // stays valid; the solver scratch is just reallocated.
-int reserve_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
+int grow_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
     int rc;
     if (rows > c->sys_cap_n) {
         const int64_t old = c->sys_cap_n;
@@ -249,6 +248,15 @@ int reserve_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
         c->sliced_cap = entries;
     }
     return KTG_OK;
+}
+
+int reserve_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
+    const int rc = grow_systems(c, rows, nnz);
+    if (rc) {  // some arrays are gone: the systems go with them, the next call starts afresh
+        free_systems(c);
+        (void)cudaGetLastError();  // reported
+    }
+    return rc;
 }
 
 int reserve_partials(ktg_ctx *c, int64_t count) {

@@ -43,3 +43,48 @@ def test_host_side_errors(gpu_ctx):
     x = np.zeros(4)
     with pytest.raises(KtgError):
         gpu_ctx.solve_mixed(x, x, TOL, inner_tol=1.5)
+
+
+def test_out_of_memory_leaves_no_system_behind(port_built):
+    """A larger system that does not fit takes the smaller one with it (its arrays
+    had to make way): no later call runs on what is left, and the context takes
+    systems again."""
+    import torch
+    import oracle
+    from ktplace_b200 import _lib
+    from ktplace_b200._lib import KtgError
+    from ktplace_b200.gpu import Context
+    from test_gpu_sliced import random_system
+    n = 500
+    small = [random_system(n, [2, 6, 10], k) for k in (1, 2)]
+    m = 8_000_000
+    rng = np.random.default_rng(3)
+    large = dict(row_ptr=np.linspace(0, m, n + 1).astype(np.int64),
+                 col=rng.integers(0, n, m).astype(np.int32), val=np.full(m, -1e-3),
+                 diag=np.full(n, 1e3), rhs=np.ones(n))
+    x0, y0 = rng.standard_normal((2, n))
+    ref = oracle.port_solve_both(small[0], x0, small[1], y0, TOL, 1000)
+    with Context(0) as ctx:
+        for axis in (0, 1):
+            ctx.upload_system(axis, small[axis])
+        ctx.solve(x0, y0, TOL, 1000)
+        torch.cuda.empty_cache()
+        room = torch.cuda.mem_get_info()[0] - 300 * 2**20
+        held = torch.empty(room, dtype=torch.uint8, device="cuda")
+        try:
+            with pytest.raises(KtgError):
+                ctx.upload_system(0, large)
+            for call in (lambda: ctx.solve(x0, y0, TOL, 10), lambda: ctx.spmv(0, x0),
+                         lambda: ctx.solve_mixed(x0, y0, TOL)):
+                with pytest.raises(KtgError) as e:
+                    call()
+                assert e.value.code == _lib.KTG_ERR_STATE
+        finally:
+            del held
+            torch.cuda.empty_cache()
+        for axis in (0, 1):
+            ctx.upload_system(axis, small[axis])
+        got = ctx.solve(x0, y0, TOL, 1000)
+        assert got["iters"] == ref["iters"]
+        for k in ("x", "y"):
+            assert np.linalg.norm(got[k] - ref[k]) <= 1e-9 * np.linalg.norm(ref[k])
