@@ -431,7 +431,7 @@ enum MixPre { kPreJacobi = 0, kPreLearned = 1, kPreAgg = 2 };
 struct CgAxis {
     double b_norm, true_resid, target, gamma, alpha, ztr, zts;
     float alpha32, beta32, cu;  // cu: the coefficient c of z in the next u
-    unsigned active, stalled, live, in_live, ok, first;
+    unsigned active, stalled, live, in_live, first;
     int32_t outer;
     int64_t inner;
 };
@@ -697,7 +697,6 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
                 CgAxis &v = st[a];
                 if ((threadIdx.x & 31) != 0 || !v.in_live) return;
                 const double gamma = t[0], delta = t[1], rr = t[2], zw = t[3];
-                v.ok = 0;
                 v.in_live = 0;
                 if (!(sqrt(rr) > v.target) || v.inner >= A.max_inner || !(gamma > 0.0)) return;
                 double b = 0.0, pap = delta;
@@ -707,7 +706,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) k_pcg_mixed_cg(MixArgs A) {
                 }
                 if (!(pap > 0.0)) return;
                 const double al = gamma / pap;
-                v.in_live = v.ok = 1;
+                v.in_live = 1;
                 v.alpha32 = static_cast<float>(al);
                 v.beta32 = static_cast<float>(b);
                 v.gamma = gamma;
