@@ -88,8 +88,13 @@ __device__ __forceinline__ double warp_sums(const double (&v)[K]) {
 // block has arrived at it and so has read all records of b - 1, and resets its
 // own of that set. The reset is published by its next fence, at most two
 // reductions later, and the set is used again three later. Reductions without
-// Publish carry no fence: they order only the reads before them (whose values
-// the sums depend on) against later writes.
+// Publish carry no fence, so they establish no order between blocks that the
+// memory model would promise for accesses at large. Callers use them only to
+// keep a later overwrite behind earlier reads, and only where every value read
+// goes into a sum: the writer holds a total computed from it, and a load whose
+// value has been used cannot return a later store. (The solves' gathers qualify;
+// those of an axis that is done do not enter a sum, but nothing writes its
+// entries any more.) Reads of what others wrote need Publish.
 //
 // A record holds W words of each axis.
 template <int W>
