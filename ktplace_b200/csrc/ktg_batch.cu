@@ -12,7 +12,8 @@
 //   * FP64 Jacobi-PCG (the reference's method), or FP32 Jacobi-PCG inside FP64
 //     iterative refinement (true FP64 residual as the convergence test);
 //     the latter on a renumbered FP32 copy of the system (Jagged), with the
-//     search direction in every CTA's shared memory;
+//     search direction in every CTA's shared memory, where that pays (jagged_pays,
+//     near_clusters), else on the system itself in warp tiles;
 //   * per system the device records iterations, the final residual and the
 //     solve latency (%globaltimer from dequeue to done).
 // The launch only enqueues work, so the whole batch solve is captured once
@@ -53,6 +54,7 @@ struct BatchArgs {
     const int32_t *rp;     // system k's row_ptr (local offsets) at row_base + k
     const int32_t *col;
     const double *val;
+    const float *val32;
     const double *diag;
     const double *rhs;
     double *x;
@@ -77,12 +79,16 @@ struct BatchArgs {
     int64_t max_iter;
     int32_t max_outer;
     uint64_t total_timeout_ns;
-    int32_t near_bytes;  // dynamic shared memory: room for p
 };
 
 // Cluster-wide deterministic sum of K values per thread. Partials are double
-// buffered in shared memory so one cluster barrier per reduction suffices.
-template <int K>
+// buffered in shared memory so one cluster barrier per reduction suffices. Every
+// thread reads all of them, or (ByWarp) one warp reads each once for the others:
+// 16 CTAs of 512 threads, 2,000 rows, 0.91 against 0.70 ms a solve; 4 CTAs, 52,000
+// rows, 22.4 against 23.8.
+constexpr int kPortable = 8;  // CTAs of a portable cluster
+
+template <int K, bool ByWarp>
 __device__ __forceinline__ void cluster_sum(double (&v)[K], double *part, int &buf,
                                             double *scratch, cg::cluster_group &cl) {
     block_sum_k<K>(v, scratch);
@@ -93,19 +99,28 @@ __device__ __forceinline__ void cluster_sum(double (&v)[K], double *part, int &b
     }
     cl.sync();
     const int nb = static_cast<int>(cl.num_blocks()), lane = threadIdx.x & 31;
-    if (threadIdx.x < 32) {  // one read per value, added in rank order
+    if constexpr (!ByWarp) {
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            const double q = lane < nb ? *cl.map_shared_rank(mine + k, lane) : 0.0;
             double t = 0.0;
-            for (int r = 0; r < nb; ++r) t += __shfl_sync(0xffffffffu, q, r);
-            if (lane == 0) scratch[k] = t;
+            for (int q = 0; q < nb; ++q) t += *cl.map_shared_rank(mine + k, q);
+            v[k] = t;
         }
-    }
-    __syncthreads();
+    } else {
+        if (threadIdx.x < 32) {
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = scratch[k];
-    __syncthreads();
+            for (int k = 0; k < K; ++k) {
+                const double q = lane < nb ? *cl.map_shared_rank(mine + k, lane) : 0.0;
+                double t = 0.0;
+                for (int r = 0; r < nb; ++r) t += __shfl_sync(0xffffffffu, q, r);
+                if (lane == 0) scratch[k] = t;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = scratch[k];
+        __syncthreads();
+    }
     buf ^= 1;
 }
 
@@ -140,9 +155,20 @@ __device__ __forceinline__ void each_rows(int32_t a, int32_t b, Row row) {
     for (; i < b; i += blockDim.x) row(i, std::integral_constant<int, 1>());
 }
 
-// The search direction p that the products gather: every CTA of the cluster
-// keeps all of it in shared memory when it fits (`near`); a CTA stores its rows
-// into each. Random gathers from L2 run at 0.9 per clock and SM, those from
+// Whether the renumbered copy and the direction in shared memory pay for a system.
+// Few rows a CTA do not make up for building the copy (ms a solve, without and with:
+// 300 rows 1 x 512 0.27 and 0.38, 1,000 rows 4 x 512 0.50 and 0.56, 2 x 512 0.58 and
+// 0.58, 1 x 512 0.78 and 0.72; 5,000 rows 8 x 512 1.14 and 1.06), and in clusters of
+// 16 storing every CTA's rows to all others takes what the gathers save (16 x 512:
+// 10,000 rows 1.92 and 2.01, 48,000 rows 7.5 and 9.9).
+constexpr int kJaggedRows = 600;  // of a CTA
+
+__host__ __device__ inline bool jagged_pays(int64_t rows, int cluster) {
+    return cluster <= kPortable && rows >= static_cast<int64_t>(kJaggedRows) * cluster;
+}
+
+// The search direction p that its products gather lies whole in every CTA's shared
+// memory; a CTA stores its rows into each. Random gathers from L2 run at 0.9 per clock and SM, those from
 // shared memory at about 9, and they bound the solve.
 // FP32 copy of a CTA's rows for the inner products of the mixed solve. The rows
 // are renumbered by length (longest first, stable) and dealt to the warps in
@@ -151,9 +177,9 @@ __device__ __forceinline__ void each_rows(int32_t a, int32_t b, Row row) {
 // shorter rows, a lane each (entries step by step, those of the rows that have
 // one next to each other, so nothing is padded). Either way a row's terms are
 // added in storage order. The whole inner solve runs in this numbering. The
-// warp tiles it replaces waited for a row pointer, a column and a value per 128
+// warp tiles wait for a row pointer, a column and a value per 128
 // entries and for the longest row of each 32: 66k cycles a product for 8,550
-// rows, now 34k, bound by instruction issue (the copy costs 40k once). 24
+// rows, this 34k, bound by instruction issue (the copy costs 40k once). 24
 // systems of 5k to 48k rows on clusters of 4 x 1,024: 11.5 -> 7.1 ms.
 constexpr int kLenBuckets = 64;   // rows of 63 entries and more are one bucket
 constexpr int kSliceCost = 4;     // a unit's own cost, in steps
@@ -334,14 +360,13 @@ struct Jagged {
     }
 
     // ap = A p for the CTA's rows; returns the thread's part of p^T A p. p is in
-    // shared memory (Near) or global. A lane's entries are loaded kDeep at a
+    // shared memory. A lane's entries are loaded kDeep at a
     // time, one group ahead, across slices: L2's latency is what there is to
     // hide. Not inlined: it needs the registers to itself.
-    template <bool Near>
-    __device__ __noinline__ double product(const float *far_p) const {
+    __device__ __noinline__ double product() const {
         extern __shared__ __align__(16) double near_mem[];
         const float *near_p = reinterpret_cast<const float *>(near_mem);
-        auto gather = [&](int32_t k) { return Near ? near_p[k] : __ldcg(far_p + k); };
+        auto gather = [&](int32_t k) { return near_p[k]; };
         double w = 0.0;
         constexpr int kDeep = 8;
         const int lane = threadIdx.x & 31;
@@ -445,8 +470,14 @@ struct Jagged {
     }
 };
 
-template <bool Mixed>
+// kNear: the mixed solve where some system's p is kept in shared memory; apart from
+// kTiles, whose registers it does not fit (52,000 rows, 4 x 512: 22.4 ms, with the
+// code for both 23.1). kTilesWide: kTiles for clusters beyond kPortable.
+enum Solve { kFp64 = 0, kTiles = 1, kTilesWide = 2, kNear = 3 };
+
+template <int Kind>
 __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
+    constexpr bool kByWarp = Kind != kTiles;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) double near_mem[];
     __shared__ double scratch[33 * 4];
@@ -501,7 +532,7 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
         res.status = late ? KTG_ERR_TIMEOUT : KTG_OK;
         double resid = 0.0;
 
-        if constexpr (!Mixed) {
+        if constexpr (Kind == kFp64) {
             double *z = A.z + S.row_base;
             double *p = A.p + S.row_base;
             double *ap = A.ap + S.row_base;
@@ -518,7 +549,7 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
                 v[1] += ri * zi;
                 v[2] += ri * ri;
             }
-            cluster_sum<3>(v, part, buf, scratch, cl);
+            cluster_sum<3, kByWarp>(v, part, buf, scratch, cl);
             const double bnorm = sqrt(v[0]);
             bool active = bnorm > 0.0 && !late;
             double rho = v[1];
@@ -546,7 +577,7 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
                         ap[i] = s;
                         w[0] += pcur * s;
                     });
-                cluster_sum<1>(w, part, buf, scratch, cl);
+                cluster_sum<1, kByWarp>(w, part, buf, scratch, cl);
                 if (*cl.map_shared_rank(&s_stop, 0)) {
                     res.status = KTG_ERR_TIMEOUT;
                     break;
@@ -565,7 +596,7 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
                         u[1] += ri * zi;
                     }
                 }
-                cluster_sum<2>(u, part, buf, scratch, cl);
+                cluster_sum<2, kByWarp>(u, part, buf, scratch, cl);
                 ++it;
                 if (!ok) {
                     active = false;
@@ -598,121 +629,173 @@ __global__ void __launch_bounds__(1024) k_batch_pcg(BatchArgs A) {
                     [&](int32_t, int, int32_t i) { return dg[i] * __ldcg(x + i); },
                     [&](int32_t, int, int32_t i, double s) { emit(i, rhs[i], rhs[i] - s); });
             };
-            float *d = A.d32 + S.row_base;
-            float *ri = A.ri32 + S.row_base;
-            float *z = A.z32 + S.row_base;
-            float *p = A.p32 + S.row_base;
-            float *ap = A.ap32 + S.row_base;
-            if (threadIdx.x == 0)
-                J = Jagged{a, b - a, A.jcol + S.nnz_base, A.jval + S.nnz_base,
-                           A.diag32 + S.row_base, ap, A.perm + S.row_base, A.inv + S.row_base,
-                           A.len + S.row_base, A.start + S.row_base, A.next + S.row_base,
-                           first_slice};
-            __syncthreads();
-            float *const near_p = reinterpret_cast<float *>(near_mem);
-            const bool near = static_cast<int64_t>(n) * 4 <= A.near_bytes;
-            if (threadIdx.x < nb) peers[threadIdx.x] = cl.map_shared_rank(near_p, threadIdx.x);
-            __syncthreads();
-            auto put = [&](int32_t i, float t) {
-                if (near)
-                    for (unsigned q = 0; q < nb; ++q) peers[q][i] = t;
-                else
-                    __stcg(p + i, t);
-            };
-            auto own = [&](int32_t i) { return near ? near_p[i] : __ldcg(p + i); };
-            double bnorm = 0.0, prev = 0.0;
             int64_t inner = 0;
             int32_t outer = 0;
-            for (int round = 0;; ++round) {
-                double v[2] = {0.0, 0.0};  // rr, bb
-                residual([&](int32_t i, double bi, double rr) {
-                    r[i] = rr;
-                    v[0] += rr * rr;
-                    v[1] += bi * bi;
-                });
-                cluster_sum<2>(v, part, buf, scratch, cl);
-                if (round == 0) bnorm = sqrt(v[1]);
-                const double rnorm = sqrt(v[0]);
-                prev = resid;
-                resid = bnorm > 0.0 ? rnorm / bnorm : 0.0;
-                const bool stalled = round > 0 && !(resid < 0.5 * prev);
-                if (!(bnorm > 0.0) || late || resid <= A.tol || outer >= A.max_outer ||
-                    inner >= A.max_iter || stalled) {
-                    if (stalled && resid > A.tol) res.status = 1;  // stalled: caller may retry in FP64
-                    break;
+            // A copy of the solve for each place of p, so that neither has the
+            // other's pointers in registers.
+            auto solve = [&](auto place) {
+                constexpr bool Near = decltype(place)::value;
+                float *d = A.d32 + S.row_base;
+                float *ri = A.ri32 + S.row_base;
+                float *z = A.z32 + S.row_base;
+                float *p = A.p32 + S.row_base;
+                float *ap = A.ap32 + S.row_base;
+                const float *val32 = A.val32 + S.nnz_base;
+                float *const near_p = reinterpret_cast<float *>(near_mem);
+                if constexpr (Near) {
+                    if (threadIdx.x == 0)
+                        J = Jagged{a, b - a, A.jcol + S.nnz_base, A.jval + S.nnz_base,
+                                   A.diag32 + S.row_base, ap, A.perm + S.row_base,
+                                   A.inv + S.row_base, A.len + S.row_base, A.start + S.row_base,
+                                   A.next + S.row_base, first_slice};
+                    if (threadIdx.x < nb)
+                        peers[threadIdx.x] = cl.map_shared_rank(near_p, threadIdx.x);
+                    __syncthreads();
                 }
-                if (round == 0)
-                    J.build(rp, col, val, dg, reinterpret_cast<int32_t *>(tilebuf),
-                            reinterpret_cast<int32_t *>(scratch), cl);
-                double q[2] = {0.0, 0.0};  // rz, rr (inner)
-                for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) {
-                    const float rf = static_cast<float>(r[J.perm[i]]);
-                    const float zf = rf / J.diag[i];
-                    ri[i] = rf;
-                    d[i] = 0.0f;
-                    z[i] = zf;
-                    put(i, zf);
-                    q[0] += static_cast<double>(rf) * zf;
-                    q[1] += static_cast<double>(rf) * rf;
-                }
-                cluster_sum<2>(q, part, buf, scratch, cl);
-                double rho = q[0];
-                double iresid = sqrt(q[1]);
-                const double target = A.inner_tol * rnorm;
-                bool live = rho > 0.0;
-                while (live && iresid > target && inner < A.max_iter) {
-                    double w[1] = {0.0};
-                    w[0] = near ? J.product<true>(p) : J.product<false>(p);
-                    cluster_sum<1>(w, part, buf, scratch, cl);
-                    ++inner;
-                    if (!(w[0] > 0.0)) break;
-                    const float alpha = static_cast<float>(rho / w[0]);
-                    double u[2] = {0.0, 0.0};
-                    each_rows(a, b, [&](int32_t i0, auto count) {
-                        float xv[kBatchRows], rv[kBatchRows], av[kBatchRows], dv[kBatchRows];
-#pragma unroll
-                        for (int k = 0; k < count(); ++k) {
-                            const int32_t i = i0 + k * blockDim.x;
-                            xv[k] = d[i];
-                            rv[k] = ri[i];
-                            av[k] = ap[i];
-                            dv[k] = J.diag[i];
-                        }
-#pragma unroll
-                        for (int k = 0; k < count(); ++k) {
-                            const int32_t i = i0 + k * blockDim.x;
-                            d[i] = xv[k] + alpha * own(i);
-                            const float rr = rv[k] - alpha * av[k];
-                            const float zz = rr / dv[k];
-                            ri[i] = rr;
-                            z[i] = zz;
-                            u[0] += static_cast<double>(rr) * rr;
-                            u[1] += static_cast<double>(rr) * zz;
-                        }
+                auto put = [&](int32_t i, float t) {
+                    if constexpr (Near)
+                        for (unsigned q = 0; q < nb; ++q) peers[q][i] = t;
+                    else
+                        __stcg(p + i, t);
+                };
+                auto own = [&](int32_t i) {
+                    if constexpr (Near) return near_p[i];
+                    else return __ldcg(p + i);
+                };
+                auto row = [&](int32_t i) {
+                    if constexpr (Near) return J.perm[i];
+                    else return i;
+                };
+                auto diagonal = [&](int32_t i) {
+                    if constexpr (Near) return J.diag[i];
+                    else return static_cast<float>(dg[i]);
+                };
+                double bnorm = 0.0, prev = 0.0;
+                for (int round = 0;; ++round) {
+                    double v[2] = {0.0, 0.0};  // rr, bb
+                    residual([&](int32_t i, double bi, double rr) {
+                        r[i] = rr;
+                        v[0] += rr * rr;
+                        v[1] += bi * bi;
                     });
-                    cluster_sum<2>(u, part, buf, scratch, cl);
-                    iresid = sqrt(u[0]);
-                    if (!(u[1] > 0.0)) break;
-                    const float beta = static_cast<float>(u[1] / rho);
-                    rho = u[1];
-                    const int32_t b4 = near ? a + (b - a) / 4 * 4 : a;
-                    for (int32_t i = a + 4 * static_cast<int32_t>(threadIdx.x); i < b4;
-                         i += 4 * blockDim.x) {
-                        float4 t = *reinterpret_cast<const float4 *>(near_p + i);
-                        t.x = z[i] + beta * t.x;
-                        t.y = z[i + 1] + beta * t.y;
-                        t.z = z[i + 2] + beta * t.z;
-                        t.w = z[i + 3] + beta * t.w;
-                        for (unsigned q = 0; q < nb; ++q)
-                            *reinterpret_cast<float4 *>(peers[q] + i) = t;
+                    cluster_sum<2, kByWarp>(v, part, buf, scratch, cl);
+                    if (round == 0) bnorm = sqrt(v[1]);
+                    const double rnorm = sqrt(v[0]);
+                    prev = resid;
+                    resid = bnorm > 0.0 ? rnorm / bnorm : 0.0;
+                    const bool stalled = round > 0 && !(resid < 0.5 * prev);
+                    if (!(bnorm > 0.0) || late || resid <= A.tol || outer >= A.max_outer ||
+                        inner >= A.max_iter || stalled) {
+                        // stalled: caller may retry in FP64
+                        if (stalled && resid > A.tol) res.status = 1;
+                        break;
                     }
-                    for (int32_t i = b4 + static_cast<int32_t>(threadIdx.x); i < b; i += blockDim.x)
-                        put(i, z[i] + beta * own(i));
+                    if constexpr (Near)
+                        if (round == 0)
+                            J.build(rp, col, val, dg, reinterpret_cast<int32_t *>(tilebuf),
+                                    reinterpret_cast<int32_t *>(scratch), cl);
+                    double q[2] = {0.0, 0.0};  // rz, rr (inner)
+                    for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) {
+                        const float rf = static_cast<float>(r[row(i)]);
+                        const float zf = rf / diagonal(i);
+                        ri[i] = rf;
+                        d[i] = 0.0f;
+                        z[i] = zf;
+                        put(i, zf);
+                        q[0] += static_cast<double>(rf) * zf;
+                        q[1] += static_cast<double>(rf) * rf;
+                    }
+                    cluster_sum<2, kByWarp>(q, part, buf, scratch, cl);
+                    double rho = q[0];
+                    double iresid = sqrt(q[1]);
+                    const double target = A.inner_tol * rnorm;
+                    bool live = rho > 0.0;
+                    while (live && iresid > target && inner < A.max_iter) {
+                        double w[1] = {0.0};
+                        if constexpr (Near) {
+                            w[0] = J.product();
+                        } else {
+                            float pcur = 0.0f;
+                            warp_tile_spmv<float>(
+                                a, INT32_MAX, b - a, kAllAxes, wb,
+                                reinterpret_cast<float *>(tilebuf),
+                                [&](int, const int32_t *&trp, const int32_t *&tcol,
+                                    const float *&tval, const float *&tin) {
+                                    trp = rp;
+                                    tcol = col;
+                                    tval = val32;
+                                    tin = p;
+                                },
+                                [&](int32_t, int, int32_t i) {
+                                    pcur = __ldcg(p + i);
+                                    return diagonal(i) * pcur;
+                                },
+                                [&](int32_t, int, int32_t i, float s) {
+                                    ap[i] = s;
+                                    w[0] += static_cast<double>(pcur) * s;
+                                });
+                        }
+                        cluster_sum<1, kByWarp>(w, part, buf, scratch, cl);
+                        ++inner;
+                        if (!(w[0] > 0.0)) break;
+                        const float alpha = static_cast<float>(rho / w[0]);
+                        double u[2] = {0.0, 0.0};
+                        each_rows(a, b, [&](int32_t i0, auto count) {
+                            float xv[kBatchRows], rv[kBatchRows], av[kBatchRows], dv[kBatchRows];
+#pragma unroll
+                            for (int k = 0; k < count(); ++k) {
+                                const int32_t i = i0 + k * blockDim.x;
+                                xv[k] = d[i];
+                                rv[k] = ri[i];
+                                av[k] = ap[i];
+                                dv[k] = diagonal(i);
+                            }
+#pragma unroll
+                            for (int k = 0; k < count(); ++k) {
+                                const int32_t i = i0 + k * blockDim.x;
+                                d[i] = xv[k] + alpha * own(i);
+                                const float rr = rv[k] - alpha * av[k];
+                                const float zz = rr / dv[k];
+                                ri[i] = rr;
+                                z[i] = zz;
+                                u[0] += static_cast<double>(rr) * rr;
+                                u[1] += static_cast<double>(rr) * zz;
+                            }
+                        });
+                        cluster_sum<2, kByWarp>(u, part, buf, scratch, cl);
+                        iresid = sqrt(u[0]);
+                        if (!(u[1] > 0.0)) break;
+                        const float beta = static_cast<float>(u[1] / rho);
+                        rho = u[1];
+                        int32_t first = a;
+                        if constexpr (Near) {
+                            first = a + (b - a) / 4 * 4;
+                            for (int32_t i = a + 4 * static_cast<int32_t>(threadIdx.x); i < first;
+                                 i += 4 * blockDim.x) {
+                                float4 t = *reinterpret_cast<const float4 *>(near_p + i);
+                                t.x = z[i] + beta * t.x;
+                                t.y = z[i + 1] + beta * t.y;
+                                t.z = z[i + 2] + beta * t.z;
+                                t.w = z[i + 3] + beta * t.w;
+                                for (unsigned q = 0; q < nb; ++q)
+                                    *reinterpret_cast<float4 *>(peers[q] + i) = t;
+                            }
+                        }
+                        for (int32_t i = first + static_cast<int32_t>(threadIdx.x); i < b;
+                             i += blockDim.x)
+                            put(i, z[i] + beta * own(i));
+                        cl.sync();
+                    }
+                    for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) x[row(i)] += d[i];
+                    ++outer;
                     cl.sync();
                 }
-                for (int32_t i = a + threadIdx.x; i < b; i += blockDim.x) x[J.perm[i]] += d[i];
-                ++outer;
-                cl.sync();
+            };
+            if constexpr (Kind == kNear) {
+                if (jagged_pays(n, static_cast<int>(nb))) solve(std::true_type());
+                else solve(std::false_type());
+            } else {
+                solve(std::false_type());
             }
             res.iters = inner;
             res.outer = outer;
@@ -750,6 +833,7 @@ struct ktg_batch {
     int32_t *rp = nullptr;  // rows + num_sys entries
     int32_t *col = nullptr;
     double *val = nullptr;
+    float *val32 = nullptr;   // values for the mixed solve on the CSR system
     int32_t *jcol = nullptr;  // the mixed solve's copy, built by it
     float *jval = nullptr, *diag32 = nullptr;
     int32_t *perm = nullptr, *inv = nullptr, *len = nullptr, *start = nullptr,
@@ -854,11 +938,17 @@ int reserve(ktg_batch *b, int64_t rows, int64_t nnz, int64_t nsys) {
     if (nnz > b->cap_nnz) {
         const int64_t cap = std::max(nnz, 2 * b->cap_nnz);
         if ((rc = grow(b, &b->col, b->nnz, cap)) || (rc = grow(b, &b->val, b->nnz, cap)) ||
-            (rc = grow(b, &b->jcol, 0, cap)) || (rc = grow(b, &b->jval, 0, cap)))
+            (rc = grow(b, &b->val32, b->nnz, cap)) || (rc = grow(b, &b->jcol, 0, cap)) || (rc = grow(b, &b->jval, 0, cap)))
             return rc;
         b->cap_nnz = cap;
     }
     return KTG_OK;
+}
+
+__global__ void k_batch_f32(const double *a, float *b, int64_t n) {
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+        b[i] = static_cast<float>(a[i]);
 }
 
 __global__ void k_stamp(unsigned long long *t) { *t = ktg::global_timer_ns(); }
@@ -938,7 +1028,7 @@ void ktg_batch_destroy(ktg_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
-    void *ptrs[] = {b->d_sys, b->d_order, b->rp, b->col, b->val, b->jcol, b->jval, b->diag32,
+    void *ptrs[] = {b->d_sys, b->d_order, b->rp, b->col, b->val, b->val32, b->jcol, b->jval, b->diag32,
                     b->perm, b->inv, b->len, b->start, b->next, b->diag, b->rhs, b->x, b->x0, b->r, b->z, b->p, b->ap, b->d32, b->ri32, b->z32, b->p32,
                     b->ap32, b->queue, b->queue2, b->results, b->d_minfo, b->d_sinfo,
                     b->d_stamp};
@@ -992,6 +1082,11 @@ int ktg_batch_add_system(ktg_batch *b, int64_t n, const int64_t *row_ptr, const 
         KTG_BCUDA(b, cudaMemcpyAsync(b->rhs + base, rhs, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
         KTG_BCUDA(b, cudaMemcpyAsync(b->x + base, x0, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
         KTG_BCUDA(b, cudaMemcpyAsync(b->x0 + base, x0, sizeof(double) * n, cudaMemcpyHostToDevice, b->stream));
+    }
+    if (m) {
+        k_batch_f32<<<static_cast<int>(std::min<int64_t>((m + 255) / 256, 4096)), 256, 0, b->stream>>>(
+            b->val + ebase, b->val32 + ebase, m);
+        ++b->launches;
     }
     KTG_BCUDA(b, cudaStreamSynchronize(b->stream));
     b->sys.push_back(ktg::SysDesc{base, ebase, static_cast<int32_t>(n), 0});
@@ -1120,38 +1215,63 @@ int ktg_batch_reset_x(ktg_batch *b) {
     return KTG_OK;
 }
 
-static void (*batch_kernel(int mixed))(ktg::BatchArgs) {
-    return mixed ? ktg::k_batch_pcg<true> : ktg::k_batch_pcg<false>;
+static void (*batch_kernel(int mixed, int cluster, int near_bytes))(ktg::BatchArgs) {
+    return !mixed                      ? ktg::k_batch_pcg<ktg::kFp64>
+           : near_bytes > 0            ? ktg::k_batch_pcg<ktg::kNear>
+           : cluster <= ktg::kPortable ? ktg::k_batch_pcg<ktg::kTiles>
+                                       : ktg::k_batch_pcg<ktg::kTilesWide>;
 }
 
-// Shared memory for the mixed solve's search direction in each class: the
-// largest system's, or as much as there is (larger systems then gather from
-// L2). The FP64 solve has none: 8 bytes a row leave it too little L1 (24 systems
-// of 5k to 48k rows on 4 x 1,024: 20.7 ms with, 13.7 without).
-static int near_room(ktg_batch *b, int mixed, int *small, int *large) {
-    *small = *large = 0;
+// What a class would keep in shared memory: the search directions of its mixed
+// solves, room for the largest that pays (bytes; none where a system's direction does
+// not fit, since that one decides the class's time), and its systems in rows.
+struct NearPlan {
+    int bytes = 0;
+    int64_t most = 0;          // rows of the largest system
+    int64_t all = 0, big = 0;  // rows of all, and of those of at least half as many
+};
+
+// A system's own cost, in rows: a solve of 300 rows takes as long as 1,000 more do
+// (8 x 512: 0.3 ms, and 0.2 us a row).
+constexpr int64_t kSystemRows = 1000;
+
+// The FP64 solve keeps nothing there: 8 bytes a row leave it too little L1 (24
+// systems of 5k to 48k rows on 4 x 1,024: 20.7 ms with, 13.7 without).
+static int near_room(ktg_batch *b, int mixed, NearPlan *plan) {
     if (!mixed) return KTG_OK;
     int &near_limit = b->near_limit;
     if (near_limit == 0) {
+        const auto kernel = ktg::k_batch_pcg<ktg::kNear>;
         cudaFuncAttributes fa;
         int most = 0;
-        KTG_BCUDA(b, cudaFuncGetAttributes(&fa, batch_kernel(mixed)));
+        KTG_BCUDA(b, cudaFuncGetAttributes(&fa, kernel));
         KTG_BCUDA(b, cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin,
                                             b->device));
         const int limit = (most - static_cast<int>(fa.sharedSizeBytes)) / 256 * 256;
-        KTG_BCUDA(b, cudaFuncSetAttribute(batch_kernel(mixed),
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+        KTG_BCUDA(b, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          limit));
         near_limit = limit;
     }
     const std::vector<char> off = offloaded(b);
-    int64_t n[2] = {0, 0};
+    auto in_class = [&](size_t i) { return b->split_rows > 0 && b->sys[i].n >= b->split_rows; };
+    int64_t near[2] = {0, 0};
     for (size_t i = 0; i < b->sys.size(); ++i) {
-        int64_t &m = n[b->split_rows > 0 && b->sys[i].n >= b->split_rows ? 1 : 0];
-        if (!off[i]) m = std::max<int64_t>(m, b->sys[i].n);
+        if (off[i]) continue;
+        const int k = in_class(i) ? 1 : 0;
+        const int64_t n = b->sys[i].n;
+        plan[k].most = std::max(plan[k].most, n);
+        if (ktg::jagged_pays(n, k ? b->split_cluster : b->cluster)) near[k] = std::max(near[k], n);
+    }
+    for (size_t i = 0; i < b->sys.size(); ++i) {
+        if (off[i]) continue;
+        NearPlan &p = plan[in_class(i) ? 1 : 0];
+        const int64_t rows = b->sys[i].n + kSystemRows;
+        p.all += rows;
+        if (2 * static_cast<int64_t>(b->sys[i].n) >= p.most) p.big += rows;
     }
     for (int k = 0; k < 2; ++k)
-        *(k ? large : small) = static_cast<int>(std::min<int64_t>(
-            near_limit, (n[k] * 4 + 255) / 256 * 256));
+        if (plan[k].most * 4 <= near_limit)
+            plan[k].bytes = static_cast<int>((near[k] * 4 + 255) / 256 * 256);
     return KTG_OK;
 }
 
@@ -1171,22 +1291,34 @@ static int resident_clusters(ktg_batch *b, int mixed, int cluster, int threads, 
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (cluster > 8)
-        KTG_BCUDA(b, cudaFuncSetAttribute(batch_kernel(mixed),
+        KTG_BCUDA(b, cudaFuncSetAttribute(batch_kernel(mixed, cluster, near_bytes),
                                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    KTG_BCUDA(b, cudaOccupancyMaxActiveClusters(out, batch_kernel(mixed), &cfg));
+    KTG_BCUDA(b, cudaOccupancyMaxActiveClusters(out, batch_kernel(mixed, cluster, near_bytes), &cfg));
     if (*out < 1) return berr(b, KTG_ERR_CUDA, "cluster shape cannot be resident");
     return KTG_OK;
 }
 
-// The same with the search direction in shared memory, or without where the
-// shape is then not resident.
-static int near_clusters(ktg_batch *b, int mixed, int cluster, int threads, int *near_bytes,
-                         int *out) {
-    if (*near_bytes > 0) {
-        if (resident_clusters(b, mixed, cluster, threads, *near_bytes, out) == KTG_OK) return KTG_OK;
+// The same for a class's plan: with the search directions in shared memory, or
+// without (*near_bytes 0) where the shape is then not resident, or where fewer
+// clusters are and that costs more than it gives: the class is mostly systems much
+// smaller than its largest, which gain little, and they would take well longer than
+// the largest does (8 x 512: 2 systems of 45k rows and 200 of 5k 8.4 ms without, 13.1
+// with; 200 of 40k rows 30.7 and 28.3; 4 x 512: the first 14.3 and 8.6).
+static int near_clusters(ktg_batch *b, int mixed, int cluster, int threads, const NearPlan &plan,
+                         int *near_bytes, int *out) {
+    *near_bytes = 0;
+    if (plan.bytes > 0) {
+        int with = 0, without = 0;
+        if (resident_clusters(b, mixed, cluster, threads, plan.bytes, &with) == KTG_OK &&
+            (resident_clusters(b, mixed, cluster, threads, 0, &without) != KTG_OK ||
+             with >= without || 2 * plan.big >= plan.all || 4 * plan.all <= 5 * with * plan.most)) {
+            b->err.clear();
+            *near_bytes = plan.bytes;
+            *out = with;
+            return KTG_OK;
+        }
         (void)cudaGetLastError();
         b->err.clear();
-        *near_bytes = 0;
     }
     return resident_clusters(b, mixed, cluster, threads, 0, out);
 }
@@ -1208,13 +1340,13 @@ static int enqueue_class(ktg_batch *b, int first, int count, unsigned *queue, in
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3(std::max(1, std::min(clusters, count)) * cluster);
-    ktg::BatchArgs A{b->d_sys, b->d_order + first, count, b->rp, b->col, b->val,
+    ktg::BatchArgs A{b->d_sys, b->d_order + first, count, b->rp, b->col, b->val, b->val32,
                      b->diag, b->rhs, b->x, b->r, b->z, b->p, b->ap, b->d32, b->ri32, b->z32,
                      b->p32, b->ap32, b->jcol, b->jval, b->diag32, b->perm, b->inv, b->len,
                      b->start, b->next, queue, b->results, tol, inner_tol, max_iter, 50,
-                     120000000000ull, near_bytes};
+                     120000000000ull};
     KTG_BCUDA(b, cudaMemsetAsync(queue, 0, sizeof(unsigned), st));
-    KTG_BCUDA(b, cudaLaunchKernelEx(&cfg, batch_kernel(mixed), A));
+    KTG_BCUDA(b, cudaLaunchKernelEx(&cfg, batch_kernel(mixed, cluster, near_bytes), A));
     return KTG_OK;
 }
 
@@ -1229,10 +1361,11 @@ static int batch_enqueue(ktg_batch *b, double tol, int64_t max_iter, int mixed, 
     const int ns = b->num_queued;
     const int nl = b->num_large;
     int res_small = 0, near_small = 0, near_large = 0;
-    int rc = near_room(b, mixed, &near_small, &near_large);
+    NearPlan plan[2];  // of the systems below the split, and from it on
+    int rc = near_room(b, mixed, plan);
     if (rc) return rc;
     if (nl < ns &&
-        (rc = near_clusters(b, mixed, b->cluster, b->threads, &near_small, &res_small)))
+        (rc = near_clusters(b, mixed, b->cluster, b->threads, plan[0], &near_small, &res_small)))
         return rc;
     if (nl == 0) {
         rc = enqueue_class(b, 0, ns, b->queue, b->cluster, b->threads, res_small, near_small, tol,
@@ -1241,7 +1374,8 @@ static int batch_enqueue(ktg_batch *b, double tol, int64_t max_iter, int mixed, 
         return rc;
     }
     int res_large = 0;
-    if ((rc = near_clusters(b, mixed, b->split_cluster, b->split_threads, &near_large, &res_large)))
+    if ((rc = near_clusters(b, mixed, b->split_cluster, b->split_threads, plan[1], &near_large,
+                            &res_large)))
         return rc;
     const int large_clusters = std::min({b->split_clusters, res_large, nl});
     if (nl == ns) {

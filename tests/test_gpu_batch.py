@@ -326,3 +326,79 @@ def test_batch_mixed_renumbered_rows(cluster, threads):
         assert true_resid(s, x) <= TOL * 1.0001
         assert np.array_equal(x, again)
     b.close()
+
+
+def uneven_system(n, rng, long_row):
+    """Empty rows, rows of up to 16 entries and one of `long_row`."""
+    deg = np.minimum(rng.integers(0, 9, n), n - 1)
+    deg[rng.integers(0, n, max(1, n // 50))] = 0
+    if n > 1000:
+        deg[n // 3] = long_row
+    rows = np.repeat(np.arange(n), deg)
+    cols = (rows + rng.integers(1, max(2, n), rows.shape[0])) % n
+    keep = cols != rows
+    a, b = rows[keep], cols[keep]
+    w = rng.uniform(0.1, 1.0, a.shape[0])
+    r, c, v = np.concatenate([a, b]), np.concatenate([b, a]), -np.concatenate([w, w])
+    order = np.argsort(r, kind="stable")
+    r, c, v = r[order], c[order], v[order]
+    diag = rng.uniform(0.5, 1.5, n) + np.bincount(r, weights=-v, minlength=n)
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))])
+    return (dict(row_ptr=rp.astype(np.int64), col=c.astype(np.int32), val=v, diag=diag,
+                 rhs=rng.standard_normal(n)), rng.standard_normal(n))
+
+
+@pytest.mark.parametrize("mix", ["rule", "largest_that_fits", "one_too_large", "many_small"])
+@pytest.mark.parametrize("cluster,threads", [(1, 1024), (2, 256), (4, 1024), (8, 512), (16, 512)])
+def test_batch_mixed_either_layout(cluster, threads, mix):
+    """The mixed solve on the system itself and on its renumbered copy, side by
+    side in one launch: around 600 rows a CTA, with a system whose direction just
+    fits in shared memory or does not, and with more small systems than clusters.
+    True residuals meet the tolerance, and a second solve, and one after another
+    shape's, give the same bits."""
+    rng = np.random.default_rng(cluster)
+    edge = 600 * cluster
+    sizes = {"rule": [edge - 1, edge, edge + 3, 40, edge + 1601, 1],
+             "largest_that_fits": [49_401, edge - 5, 30_002],
+             "one_too_large": [52_003, edge + 5, edge - 1],
+             "many_small": [20_011] + [1201 + k for k in range(60)]}[mix]
+    cases = [uneven_system(n, rng, 150 + 550 * (k % 2)) for k, n in enumerate(sizes)]
+    b, ids = make_batch(cases)
+    got = []
+    for shape in ((cluster, threads), (cluster, threads), (2, 512), (cluster, threads)):
+        b.set_shape(*shape)
+        b.reset_x()
+        b.solve(TOL, MAX_ITER, precision=1, inner_tol=1e-3)
+        if shape == (cluster, threads):
+            got.append([b.get_x(i, s["diag"].shape[0]) for (s, _), i in zip(cases, ids)])
+    res = b.results()
+    for (s, _), sid, x, again, third in zip(cases, ids, *got):
+        assert res[sid]["status"] == 0, res[sid]
+        assert true_resid(s, x) <= TOL * 1.0001
+        assert np.array_equal(x, again) and np.array_equal(x, third)
+    b.close()
+
+
+@pytest.mark.parametrize("cluster,threads", [(1, 1024), (4, 1024), (8, 512)])
+def test_batch_mixed_beyond_shared_memory_costs_no_more(cluster, threads):
+    """Systems whose search direction does not fit in shared memory: the FP32
+    iterations read half the bytes of the FP64 ones, so the mixed solve of the
+    same systems takes no longer than the FP64 solve and its extra rounds."""
+    import time
+    rng = np.random.default_rng(7)
+    cases = [uneven_system(60_007, rng, 40) for _ in range(4)]
+    b, _ = make_batch(cases)
+    b.set_shape(cluster, threads)
+    ms, per = {}, {}
+    for precision in (0, 1):
+        took = []
+        for _ in range(4):
+            b.reset_x()
+            t = time.perf_counter()
+            b.solve(TOL, MAX_ITER, precision=precision, inner_tol=1e-3)
+            its = max(r["iters"] for r in b.results())
+            took.append(time.perf_counter() - t)
+        ms[precision] = min(took[1:])
+        per[precision] = ms[precision] / its
+    b.close()
+    assert per[1] <= 1.25 * per[0], (ms, per)
