@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -821,16 +822,14 @@ int ktg_download_bound_pins(ktg_ctx *c, int axis, uint32_t *lo, uint32_t *hi) {
     int rc = set_device(c);
     if (rc) return rc;
     if ((rc = sync(c))) return rc;
-    if (!lo && !hi) return KTG_OK;
-    int4 part[2048];  // no allocation that could fail
-    for (int64_t k0 = 0; k0 < c->N; k0 += 2048) {
-        const int64_t cnt = std::min<int64_t>(2048, c->N - k0);
-        KTG_CUDA(c, cudaMemcpy(part, c->sys[axis].bound + k0, sizeof(int4) * cnt,
-                               cudaMemcpyDeviceToHost));
-        for (int64_t k = 0; k < cnt; ++k) {
-            if (lo) lo[k0 + k] = static_cast<uint32_t>(part[k].y);
-            if (hi) hi[k0 + k] = static_cast<uint32_t>(part[k].z);
-        }
+    if ((!lo && !hi) || c->N == 0) return KTG_OK;
+    const std::unique_ptr<int4[]> bound(new (std::nothrow) int4[c->N]);
+    if (!bound) return set_error(c, KTG_ERR_NOMEM, "out of host memory");
+    KTG_CUDA(c, cudaMemcpy(bound.get(), c->sys[axis].bound, sizeof(int4) * c->N,
+                           cudaMemcpyDeviceToHost));
+    for (int64_t k = 0; k < c->N; ++k) {
+        if (lo) lo[k] = static_cast<uint32_t>(bound[k].y);
+        if (hi) hi[k] = static_cast<uint32_t>(bound[k].z);
     }
     return KTG_OK;
 }
