@@ -555,15 +555,20 @@ int ktg_upload_netlist(ktg_ctx *c, const ktg_netlist_view *nl) {
             return set_error(c, KTG_ERR_ARG, "pin_ref out of range");
         pin_ref[e] = make_int2(k, q);
     }
-    std::vector<bool> listed(P);
-    bool twice = false;  // a cell lists a pin more than once: its edges count each time
+    // A cell that lists a pin more than once has its edges each time. Listed pins
+    // are marked where their cell is looked up (variables take 30 bits).
+    constexpr int32_t kListed = 1 << 30;
+    bool twice = false;
     for (int64_t i = 0; i < n; ++i)
         for (int64_t e = nl->pin_start[i]; e < nl->pin_start[i + 1]; ++e) {
             const int64_t p = nl->net_start[nl->pin_net[e]] + nl->pin_q[e];
-            if (pin_var[p] != i) return set_error(c, KTG_ERR_ARG, "pin_ref does not point to its cell");
-            twice = twice || listed[p];
-            listed[p] = true;
+            if ((pin_var[p] & ~kListed) != i)
+                return set_error(c, KTG_ERR_ARG, "pin_ref does not point to its cell");
+            twice = twice || (pin_var[p] & kListed);
+            pin_var[p] |= kListed;
         }
+    for (int64_t p = 0; p < P; ++p)
+        if (pin_var[p] >= 0) pin_var[p] &= ~kListed;
     if (twice) cap = range;
     if (range > lim) return set_error(c, KTG_ERR_RANGE, "B2B systems exceed 32-bit indices");
     std::vector<double> area(n);
