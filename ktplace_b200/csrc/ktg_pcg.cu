@@ -6,8 +6,8 @@
 // every iteration, the stopping test -- runs inside one kernel, so there is no
 // host round trip per iteration. Each block owns a contiguous slice of the
 // combined row space [x rows | y rows] (one 1024-thread block per SM); in
-// the textbook form (the default, form 3 with 32 lanes, is in
-// ktg_pcg_sliced.cu) three grid barriers per iteration separate
+// the textbook form (the default, form 3 with 32 lanes, is in ktg_pcg_sliced.cu
+// but for solves of a few iterations) three grid barriers per iteration separate
 //   A: Ap = A p and p.Ap partials
 //   B: x += a p, r -= a Ap, z = r / diag, and r.r, r.z partials
 //   C: p = z + b p
@@ -19,10 +19,10 @@
 // L1 instead: every KB of shared memory comes out of the L1 that holds the
 // SpMV's gathers in flight (a block with 30 KB more shared memory solved
 // the 211k system in 8.6 ms instead of 5.8).
-// SpMV runs in one of three shapes (option "pcg_lanes"): warp tiles (each warp takes a range of the block's rows balanced by
-// nonzeros and streams their nonzeros 32 rows at a time with coalesced
-// loads, each lane adding its row's products in storage order), one thread
-// per row (same row sums, four gathers in flight), or four lanes per row.
+// SpMV runs in one of three shapes (option "pcg_lanes"): warp tiles (each warp
+// takes a range of the block's rows balanced by nonzeros and streams their
+// nonzeros 32 rows at a time with coalesced loads, each lane adding its row's
+// products in storage order), one thread per row (same row sums, four gathers in flight), or four lanes per row.
 // The first two give the same row sums; their solves are bit-identical in
 // form 2 and agree to rounding in the others (dot-product partials group
 // rows by thread differently).
@@ -1017,10 +1017,13 @@ struct Variant {
 // form 0: textbook three-barrier PCG; form 1: Chronopoulos-Gear two-barrier;
 // form 2: textbook PCG with the reference's summation order everywhere
 // (bit-identical to the reference's solve); form 3: textbook PCG with A p by
-// recurrence, two barriers (with 32 lanes, the default, it is the sliced kernel
-// of ktg_pcg_sliced.cu).
+// recurrence, two barriers (with 32 lanes, the default, for solves of at most
+// few_steps iterations; the others run in ktg_pcg_sliced.cu).
 Variant pick_variant(int form, bool smem, int lanes) {
     if (form == 3) {
+        if (lanes == 32)
+            return {smem ? k_pcg<true, 32, false, true> : k_pcg<false, 32, false, true>,
+                    kVecsPerRow};
         if (smem) return {lanes == 4 ? k_pcg<true, 4, false, true> : k_pcg<true, 1, false, true>,
                           kVecsPerRow};
         return {lanes == 4 ? k_pcg<false, 4, false, true> : k_pcg<false, 1, false, true>,
@@ -1043,6 +1046,16 @@ Variant pick_variant(int form, bool smem, int lanes) {
 
 int lanes_index(int lanes) { return lanes == 4 ? 1 : lanes == 32 ? 2 : 0; }
 
+// Iterations up to which a solve of n rows per axis on the systems themselves is
+// done before the sliced solve has made up for its copy (-1: none). us a solve
+// here and sliced: 1,000 rows 0 iterations 34 and 32; 12k 0: 38 and 42, 1: 59 and
+// 53; 49k 1: 60 and 70, 2: 80 and 84; 100k 2: 92 and 103, 4: 142 and 137; 211k 4:
+// 204 and 218, 8: 347 and 331; 1M 4: 802 and 958, 8: 1,444 and 1,417.
+int64_t few_steps(int64_t n) {
+    if (n < 10000) return -1;
+    return std::min<int64_t>(n < 700000 ? 4 : 7, n / 24000);
+}
+
 }  // namespace
 
 int pcg_lanes_default = 32;
@@ -1053,7 +1066,7 @@ int launch_solve(ktg_ctx *c, double *x, double *y, double tol, int64_t max_iter,
     const int64_t nsys = c->sys_n;
     const int lanes = c->pcg_lanes > 0 ? c->pcg_lanes : pcg_lanes_default;
     const int form = c->pcg_form >= 0 ? c->pcg_form : pcg_form_default;
-    if (form == 3 && lanes == 32) {
+    if (form == 3 && lanes == 32 && max_iter > few_steps(nsys)) {
         const int rc = launch_solve_sliced(c, x, y, tol, max_iter, info_dev, hist_x, hist_y,
                                            hist_cap);
         if (rc) return rc;

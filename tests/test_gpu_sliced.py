@@ -130,3 +130,42 @@ def test_scratch_follows_the_blocks(port_built):
         check(ctx, 24_001, [0, 2], seed=4)
         check(ctx, 160_001, [0, 2, 0, 0], seed=5)
         check(ctx, 300, [100, 200, 60])
+
+
+@pytest.mark.parametrize("n", [9_999, 10_000, 24_003, 110_001, 720_007])
+def test_solves_of_few_iterations(n, gpu_ctx, port_built):
+    """Either side of the line below which a capped solve runs on the systems
+    themselves: the iterates are the same ones."""
+    sx, sy = random_system(n, [2, 6, 10], 21), random_system(n, [4, 8], 22)
+    x0, y0 = np.random.default_rng(23).standard_normal((2, n))
+    gpu_ctx.upload_system(0, sx)
+    gpu_ctx.upload_system(1, sy)
+    for steps in (0, 1, 2, 4, 5, 7, 8):
+        got = gpu_ctx.solve(x0, y0, TOL, steps, hist_cap=8)
+        ref = oracle.port_solve_both(sx, x0, sy, y0, TOL, steps)
+        assert got["iters"] == ref["iters"] == steps
+        for k in ("x", "y"):
+            assert np.linalg.norm(got[k] - ref[k]) <= SOL_RTOL * np.linalg.norm(ref[k])
+
+
+def test_few_iterations_need_no_copy(gpu_ctx, port_built):
+    """A solve that may take no step costs the first residual, two and a half steps
+    at most; making the sliced copy takes more than four."""
+    import time
+    import torch
+    n = 1_000_000
+    sx = random_system(n, [6, 8, 10], 31)
+    gpu_ctx.upload_system(0, sx)
+    gpu_ctx.upload_system(1, sx)
+    x0, y0 = np.random.default_rng(32).standard_normal((2, n))
+    dx, dy = torch.tensor(x0, device="cuda"), torch.tensor(y0, device="cuda")
+    took = {}
+    for steps in (0, 10, 20):
+        for rep in range(6):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            gpu_ctx.solve_dev(dx, dy, 0.0, steps)
+            torch.cuda.synchronize()
+            if rep:
+                took[steps] = min(took.get(steps, 1.0), time.perf_counter() - t)
+    assert took[0] <= 2.5 * (took[20] - took[10]) / 10, took
