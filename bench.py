@@ -240,14 +240,18 @@ class ClockSampler:
 
 
 def pcg_bytes(n: int, m: int, iters: int) -> float:
-    """Algorithmic bytes of one axis's PCG: start pass + iters iterations.
-    Iteration: val f64 + col i32 per entry, row_ptr, 14 n-vector passes (SpMV
-    reads diag and p and writes Ap; update reads x, p, r, Ap, diag and writes
-    x, r, z; direction reads z, p and writes p). Start: one SpMV on x plus
-    reading diag, x, rhs and writing r, z, p."""
-    it = 12.0 * m + 4.0 * (n + 1) + 8.0 * n * 14
-    start = 12.0 * m + 4.0 * (n + 1) + 8.0 * n * 6
-    return start + iters * it
+    """Algorithmic bytes of one axis's default solve (k_pcg_sliced): its set-up,
+    `iters` iterations and the write-back. m entries are 12 bytes each (f64
+    value, i32 column), the vectors f64.
+    Iteration: the entries and 13 passes over n-vectors. The product reads z
+    (the gathered vector counts once), diag, p, A p and x and writes p, A p and
+    x; the update reads A p, diag and r and writes r and z.
+    Set-up: the entries are read and written once each; per row three reads of
+    the row pointers (12 bytes), diag, x and their copies (32), the start
+    records written and gathered (32), the permutation written and read (8),
+    the axis (1), and diag, x, rhs, r and z of the first residual (40).
+    Write-back: permutation, x, p, and x in row order (28 bytes a row)."""
+    return 24.0 * m + 153.0 * n + iters * (12.0 * m + 8.0 * 13 * n)
 
 
 def spmv_bytes(n: int, m: int) -> float:
