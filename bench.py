@@ -276,6 +276,27 @@ def measured_peak():
         return 6650.0, "fallback"
 
 
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+            "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config", "e2e",
+            "gpu_launches", "clocks", "result", "result_vs_reference", "breakdown", "roofline",
+            "cpu_baseline")
+LEGS = {"learned_step": ("ms", "e2e_ms"), "batch": ("ms_per_batch", "systems_per_s"),
+        "kraftwerk2": ("gpu_ms",), "bookshelf": ("ms",), "lal": ("gpu_ms", "e2e_ms")}
+
+
+def headline(line: dict) -> dict:
+    """The line for standard output: the step's own figures, and of the other legs
+    one or two each. Everything measured is some 20 KB, more than a reader that
+    keeps the end of the output gets whole; it goes to standard error."""
+    out = {k: line[k] for k in HEADLINE}
+    out["roofline"] = {k: v for k, v in line["roofline"].items() if k not in ("note", "limiter")}
+    out["legs"] = {name: {k: line[name][k] for k in keys if k in line[name]}
+                   for name, keys in LEGS.items() if line.get(name)}
+    if line.get("solve_variants"):
+        out["legs"]["solve_ms"] = {k: v["ms"] for k, v in line["solve_variants"].items()}
+    return out
+
+
 def run_ours(args):
     import torch
     rank, world, local = dist_env()
@@ -488,7 +509,8 @@ def run_ours(args):
             "lal": lal_line,
             "clocks": clk,
         }
-        print(json.dumps(line))
+        print(json.dumps({"detail": line}), file=sys.stderr)
+        print(json.dumps(headline(line)))
     ctx.close()
     if dist:
         dist.barrier()
