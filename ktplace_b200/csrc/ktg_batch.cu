@@ -834,7 +834,10 @@ struct ktg_batch {
     int32_t *col = nullptr;
     double *val = nullptr;
     float *val32 = nullptr;   // values for the mixed solve on the CSR system
-    int32_t *jcol = nullptr;  // the mixed solve's copy, built by it
+    // the mixed solve's copies, built by it: one allocation for so many rows, entries
+    char *jagged = nullptr;
+    int64_t jagged_rows = 0, jagged_nnz = 0;
+    int32_t *jcol = nullptr;
     float *jval = nullptr, *diag32 = nullptr;
     int32_t *perm = nullptr, *inv = nullptr, *len = nullptr, *start = nullptr,
             *next = nullptr;
@@ -916,10 +919,7 @@ int reserve(ktg_batch *b, int64_t rows, int64_t nnz, int64_t nsys) {
             (rc = grow(b, &b->p, 0, cap)) || (rc = grow(b, &b->ap, 0, cap)) ||
             (rc = grow(b, &b->d32, 0, cap)) || (rc = grow(b, &b->ri32, 0, cap)) ||
             (rc = grow(b, &b->z32, 0, cap)) || (rc = grow(b, &b->p32, 0, cap)) ||
-            (rc = grow(b, &b->ap32, 0, cap)) || (rc = grow(b, &b->diag32, 0, cap)) ||
-            (rc = grow(b, &b->perm, 0, cap)) || (rc = grow(b, &b->inv, 0, cap)) ||
-            (rc = grow(b, &b->len, 0, cap)) || (rc = grow(b, &b->start, 0, cap)) ||
-            (rc = grow(b, &b->next, 0, cap)))
+            (rc = grow(b, &b->ap32, 0, cap)))
             return rc;
         b->cap_rows = cap;
     }
@@ -938,10 +938,39 @@ int reserve(ktg_batch *b, int64_t rows, int64_t nnz, int64_t nsys) {
     if (nnz > b->cap_nnz) {
         const int64_t cap = std::max(nnz, 2 * b->cap_nnz);
         if ((rc = grow(b, &b->col, b->nnz, cap)) || (rc = grow(b, &b->val, b->nnz, cap)) ||
-            (rc = grow(b, &b->val32, b->nnz, cap)) || (rc = grow(b, &b->jcol, 0, cap)) || (rc = grow(b, &b->jval, 0, cap)))
+            (rc = grow(b, &b->val32, b->nnz, cap)))
             return rc;
         b->cap_nnz = cap;
     }
+    return KTG_OK;
+}
+
+// The arrays of the renumbered copies, in one allocation when a mixed solve first
+// wants them (grown with every system that was added they took a fifth of the time
+// of adding 24).
+int reserve_jagged(ktg_batch *b) {
+    if (b->cap_rows <= b->jagged_rows && b->cap_nnz <= b->jagged_nnz) return KTG_OK;
+    if (b->jagged) cudaFree(b->jagged);
+    b->jagged = nullptr;
+    b->jagged_rows = b->jagged_nnz = 0;
+    const int64_t per_row = (b->cap_rows * 4 + 255) / 256 * 256;
+    const int64_t per_entry = (b->cap_nnz * 4 + 255) / 256 * 256;
+    KTG_BCUDA(b, cudaMalloc(&b->jagged, 6 * per_row + 2 * per_entry + 256));
+    char *at = b->jagged;
+    auto take = [&](auto **p, int64_t bytes) {
+        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(at);
+        at += bytes;
+    };
+    take(&b->jcol, per_entry);
+    take(&b->jval, per_entry);
+    take(&b->diag32, per_row);
+    take(&b->perm, per_row);
+    take(&b->inv, per_row);
+    take(&b->len, per_row);
+    take(&b->start, per_row);
+    take(&b->next, per_row);
+    b->jagged_rows = b->cap_rows;
+    b->jagged_nnz = b->cap_nnz;
     return KTG_OK;
 }
 
@@ -1028,9 +1057,9 @@ void ktg_batch_destroy(ktg_batch *b) {
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->graph) cudaGraphExecDestroy(b->graph);
-    void *ptrs[] = {b->d_sys, b->d_order, b->rp, b->col, b->val, b->val32, b->jcol, b->jval, b->diag32,
-                    b->perm, b->inv, b->len, b->start, b->next, b->diag, b->rhs, b->x, b->x0, b->r, b->z, b->p, b->ap, b->d32, b->ri32, b->z32, b->p32,
-                    b->ap32, b->queue, b->queue2, b->results, b->d_minfo, b->d_sinfo,
+    void *ptrs[] = {b->d_sys, b->d_order, b->rp, b->col, b->val, b->val32, b->jagged,
+                    b->diag, b->rhs, b->x, b->x0, b->r, b->z, b->p, b->ap, b->d32, b->ri32, b->z32,
+                    b->p32, b->ap32, b->queue, b->queue2, b->results, b->d_minfo, b->d_sinfo,
                     b->d_stamp};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -1521,11 +1550,14 @@ int ktg_batch_solve(ktg_batch *b, double tol, int64_t max_iter, int precision, d
             cudaGraphExecDestroy(b->graph);
             b->graph = nullptr;
         }
+        NearPlan plan[2];
+        int rc = near_room(b, precision, plan);
+        if (!rc && plan[0].bytes + plan[1].bytes > 0) rc = reserve_jagged(b);
+        if (rc) return rc;
         // Capture the whole batch solve once on a private stream.
         cudaStream_t cap;
         KTG_BCUDA(b, cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
         cudaGraph_t g = nullptr;
-        int rc = KTG_OK;
         if (cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaStreamDestroy(cap);
             return berr(b, KTG_ERR_CUDA, "stream capture failed to start");

@@ -402,3 +402,28 @@ def test_batch_mixed_beyond_shared_memory_costs_no_more(cluster, threads):
         per[precision] = ms[precision] / its
     b.close()
     assert per[1] <= 1.25 * per[0], (ms, per)
+
+
+def test_batch_copies_come_with_the_first_mixed_solve():
+    """Adding systems and FP64 solves take no memory for the renumbered copies; a
+    mixed solve does, and again after more systems were added."""
+    import torch
+    from ktplace_b200.gpu import Batch
+    rng = np.random.default_rng(5)
+    cases = [uneven_system(30_011, rng, 40) for _ in range(12)]
+    b = Batch(0)
+    b.set_shape(4, 1024)
+    ids, free = [], []
+    for first, last, precision in ((0, 8, 0), (8, 8, 1), (8, 12, 1)):
+        ids += [b.add_system(*cases[k]) for k in range(first, last)]
+        b.reset_x()
+        b.solve(TOL, MAX_ITER, precision=precision, inner_tol=1e-3)
+        res = b.results()
+        for (s, _), sid in zip(cases, ids):
+            assert res[sid]["status"] == 0
+            assert true_resid(s, b.get_x(sid, 30_011)) <= TOL * 1.0001
+        free.append(torch.cuda.mem_get_info()[0])
+    b.close()
+    per_row, per_entry = 24, 8
+    nnz = sum(len(s["col"]) for s, _ in cases[:8])
+    assert free[0] - free[1] >= 0.9 * (per_row * 8 * 30_011 + per_entry * nnz)
