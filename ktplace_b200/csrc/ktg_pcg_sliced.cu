@@ -517,8 +517,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_sliced(SlicedArgs A) {
 #pragma unroll 2
         for (int32_t j = threadIdx.x; j < R; j += blockDim.x) {
             const int axis = vax[j];
-            // (an axis that is done keeps its last ok and alpha)
-            const bool on = ((mask >> axis) & 1u) && st.ok[axis] != 0u;
+            const bool on = st.ok[axis] != 0u;
             const double a = st.alpha[axis];
             const double apv = vap[j], d = vd[j], ri = vr[j];
             if (!on) continue;
@@ -550,6 +549,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_pcg_sliced(SlicedArgs A) {
                     if (ok) st.rr[a] = t[0];
                     st.active[a] = go;
                     st.live[a] = more;
+                    if (!more) st.ok[a] = 0u;  // its rows are left alone from here on
                 }
             }))
             return;
