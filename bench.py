@@ -263,8 +263,8 @@ def spmv_bytes(n: int, m: int) -> float:
 
 # DRAM bytes (read + write) per launch of the dominant kernel on this
 # workload, from an ncu capture of bench.py --profile-once (dram__bytes_read.sum +
-# dram__bytes_write.sum of the k_pcg launch).
-NCU_TRAFFIC_BYTES = {"k_pcg": 3805.376256e6 + 39.944192e6}
+# dram__bytes_write.sum of the k_pcg_sliced launch).
+NCU_TRAFFIC_BYTES = {"k_pcg_sliced": 3753.058304e6 + 40.552704e6}
 
 
 def measured_peak():
@@ -492,12 +492,12 @@ def run_ours(args):
                                    "sorted by length over lanes, two grid sums per iteration)",
                          "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_kind": peak_kind,
-                         "traffic": NCU_TRAFFIC_BYTES["k_pcg"], "algorithmic_bytes": byts,
+                         "traffic": NCU_TRAFFIC_BYTES["k_pcg_sliced"], "algorithmic_bytes": byts,
                          "note": "the entries' loads leave L2 first: about half of their "
                                  "stream comes from DRAM, the vectors stay in L2",
-                         "limiter": "L1TEX data pipe: 47% of peak over the whole solve in the ncu "
+                         "limiter": "L1TEX data pipe: 48% of peak over the whole solve in the ncu "
                                     "capture (random 8-byte gathers, one LSU wavefront each); "
-                                    "L2 23%, DRAM 11% (ncu of bench.py --profile-once)"},
+                                    "L2 49%, DRAM 11% (profiles/k_pcg_sliced_synth211k.md)"},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h},

@@ -127,8 +127,8 @@ def test_pins_listed_twice(gpu_ctx):
 
 
 @pytest.mark.parametrize("nets", [2047, 2048, 2049, 4097])
-def test_bound_pins_come_back_in_parts(nets, gpu_ctx):
-    """Downloaded 2,048 nets at a time; the first lowest and first highest pin."""
+def test_bound_pins_download(nets, gpu_ctx):
+    """The first lowest and the first highest pin of every net."""
     raw = design(64, 3)
     rng = np.random.default_rng(nets)
     pins = rng.choice(np.nonzero(~raw.fixed)[0], (nets, 3))
