@@ -119,9 +119,8 @@ def gather_to_root(plan: ShardPlan, rank: int, out, group=None):
 class BatchShardSolver:
     """The GPU solver of one rank's share of a batch of netlists: each owned
     netlist's x and y B2B systems are built on this rank's GPU and loaded into
-    one Batch, which is autotuned once (cluster shape and the pairs sent to the
-    whole GPU, both again for those that are left, then the size split) and
-    solved by graph replay. `make_unit(u)` returns
+    one Batch, which is autotuned once (cluster shape, then the pairs sent to the
+    whole GPU, then the size split) and solved by graph replay. `make_unit(u)` returns
     (netlist, x, y, anchor_x, anchor_y, alpha) for netlist u; a unit's host
     result is its x solution followed by its y solution.
     """
@@ -159,19 +158,17 @@ class BatchShardSolver:
                 self.batch.add_from_context(ctx, x, y)
                 self.rows.append(nl.num_movable)
         if self.autotune:
-            # the largest systems decide the shape until they are sent to the whole
-            # GPU; without them another is best, and another threshold with it (64
-            # netlists: 31 ms a batch on 8 x 512, chosen with all of them, 27 on
-            # 4 x 1,024)
-            for _ in range(2):
-                c, t, _ = self.batch.autotune(self.tol, precision=self.precision,
-                                              inner_tol=self.inner_tol, probe_iter=40)
-                self.shape = (c, t)
-                self.offload, _, _ = self.batch.autotune_offload(
-                    self.tol, precision=self.precision, inner_tol=self.inner_tol,
-                    max_iter=self.max_iter)
-                if not self.offload["pairs"]:
-                    break
+            # The shape is chosen with the pairs that the whole GPU takes anyway, those
+            # whose search directions do not fit in shared memory, out of the queue:
+            # they decided it (64 netlists: 8 x 512, 31 ms a batch once they had left;
+            # 4 x 1,024 without them, 27).
+            self.batch.set_offload(50_000 if self.precision == 1 else 0)
+            c, t, _ = self.batch.autotune(self.tol, precision=self.precision,
+                                          inner_tol=self.inner_tol, probe_iter=40)
+            self.shape = (c, t)
+            self.offload, _, _ = self.batch.autotune_offload(
+                self.tol, precision=self.precision, inner_tol=self.inner_tol,
+                max_iter=self.max_iter)
             self.split, _, _ = self.batch.autotune_split(self.tol, precision=self.precision,
                                                          inner_tol=self.inner_tol,
                                                          max_iter=self.max_iter)
