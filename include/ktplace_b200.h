@@ -525,9 +525,10 @@ int ktg_bookshelf_geometry(const ktg_bookshelf *b, double *die4, double *obstacl
  *   "pcg_lanes"  SpMV shape in the PCG: 32 = warp tiles (each warp streams
  *                the nonzeros of its range of rows 32 rows at a time, each
  *                lane adding its row's products in storage order; the ranges
- *                are balanced by nonzeros) and, in form 3, a copy of the
- *                system with the rows of each block sorted by length and dealt
- *                over 1 to 32 lanes each, 1 = one thread per row (the same
+ *                are balanced by nonzeros) and, in form 3 for solves of more
+ *                than a few iterations, a copy of the system with the rows of
+ *                each block sorted by length and dealt over 1 to 32 lanes
+ *                each, 1 = one thread per row (the same
  *                row sums: the same solve bit for bit in form 2, to rounding
  *                in the others), 4 = four lanes per row; 0 = default (32)
  *   "pcg_form"   0: textbook PCG (three grid barriers per iteration),
