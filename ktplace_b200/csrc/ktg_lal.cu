@@ -1717,6 +1717,7 @@ struct SubArgs {
     double frac, limit_density;
     int32_t exact;           // areas sum exactly: prefix sums and binary searches
     double scale, inv_scale; // 2^q, 2^-q
+    int32_t rows_local;      // a block with more rows reads them where they are (-1: all do)
 };
 
 __device__ __forceinline__ bool sub_less(uint32_t a2, unsigned long long a0, unsigned long long a1,
@@ -2485,7 +2486,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                 box_rows(A.F, T.box, row0, r1);
                 rows = r1 - row0;
             }
-            if (rows <= kRowsLocal) {
+            if (rows <= A.rows_local) {
                 for (int i = tid; i < rows; i += nt) {
                     const int64_t f = first_span(A.F, row0 + i, T.box[0]);
                     int64_t e = f, hi = A.F.rowspan[row0 + i + 1];
@@ -3112,7 +3113,7 @@ __global__ void __launch_bounds__(kSubThreads, 1) k_subtree(SubArgs A) {
                     h.level = d.level;
                     h.vert = d.vert;
                     h.r0 = row0;
-                    h.r1 = rows <= kRowsLocal ? row0 + rows : -1;
+                    h.r1 = rows <= A.rows_local ? row0 + rows : -1;
                 }
                 __threadfence();
                 for (int q = 0; q < 2; ++q) atomicExch(A.ready + s_slot + q, A.epoch);
@@ -3189,6 +3190,11 @@ struct LalState {
     int64_t odd = 0;              // obstacles that are in none of the four
     std::vector<int64_t> rowspan;
     bool rows_sorted = true;  // by y start, which are all numbers
+    // The row ends ascend, and in each row the spans' starts and ends: a search
+    // among a block's own rows and spans then finds what one among all of them
+    // finds. Rows that overlap may break the order, and a binary search over
+    // another window then ends at another row, so blocks read all rows in place.
+    bool windows = true;
     double die[4] = {0, 0, 0, 0};
     DevBuf<double> d_rowy, d_spans, d_obst;
     DevBuf<int64_t> d_rowspan;
@@ -3274,7 +3280,14 @@ int set_free_space(ktg_ctx *c, int64_t nrows, const double *rowy, const int64_t 
     s->rowy.assign(rowy, rowy + 2 * nrows);
     s->rowspan.assign(rowspan, rowspan + nrows + 1);
     s->rows_sorted = true;
-    for (int64_t r = 0; r < nrows; ++r) s->rows_sorted = s->rows_sorted && !std::isnan(rowy[2 * r]);
+    s->windows = true;
+    for (int64_t r = 0; r < nrows; ++r) {
+        s->rows_sorted = s->rows_sorted && !std::isnan(rowy[2 * r]);
+        s->windows = s->windows && rowy[2 * std::max<int64_t>(r - 1, 0) + 1] <= rowy[2 * r + 1];
+        for (int64_t k = rowspan[r]; k < rowspan[r + 1]; ++k)
+            for (int q = 0; q < 2; ++q)
+                s->windows = s->windows && spans[2 * std::max(k - 1, rowspan[r]) + q] <= spans[2 * k + q];
+    }
     s->spans.assign(spans, spans + 2 * S);
     s->obst.assign(obst, obst + 4 * nobst);
     for (int k = 0; k < 4; ++k) s->side[k].clear();
@@ -3517,7 +3530,7 @@ int launch_lal(ktg_ctx *c, double *x, double *y, int32_t max_level, int32_t min_
         SubArgs A{slots, nt, cap, reinterpret_cast<SubQueue *>(s->tasks.p), s->ready.p, ++s->epoch,
                   s->tfail.p, s->cells.p, C, F, reinterpret_cast<SubDesc *>(s->swork.p), strp,
                   strlh, max_level, min_cells, stripe_extra, frac, c->density_limit,
-                  exact ? 1 : 0, scale, inv_scale};
+                  exact ? 1 : 0, scale, inv_scale, s->windows ? kRowsLocal : -1};
         k_subtree<<<grid, kSubThreads, kSubSmem, c->stream>>>(A);
         ++c->launches;
         KTG_CUDA(c, cudaGetLastError());

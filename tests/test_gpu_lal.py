@@ -405,3 +405,39 @@ def test_lal_scratch_of_a_small_design(port_built):
             assert ctx.lal_stats()["subtree_blocks"] >= 1
             taken.append(before - torch.cuda.mem_get_info()[0])
     assert taken[1] <= 48 * 2**20, taken
+
+
+@pytest.mark.parametrize("subtree", [0, 300, 2048])
+@pytest.mark.parametrize("cells,seed", [(600, 5), (2500, 6)])
+def test_lal_rows_that_overlap(cells, seed, subtree, gpu_ctx):
+    """Rows in order of their starts whose ends are not: a search by row end finds
+    the oracle's row only over all rows, not over those that a block can meet.
+    Bit-identical positions on every path."""
+    raw = synth.generate(synth.spec_tiny(seed=seed, macros=2, cells=cells, nets=cells + 30))
+    nl = netlist.flatten(raw)
+    x, y = clustered(raw, nl.num_movable, 31, 0.15)
+    g = grid.build_grid(nl, 8, 1.0)
+    fs = grid.build_free_space(nl)
+    lx, ly, ux, uy = fs.die
+    rng = np.random.default_rng(seed)
+    rows = 150
+    start = np.linspace(ly, uy, rows + 1)[:-1]
+    fs.row_y = np.stack([start, start + rng.uniform(0.1, 3.0, rows) * (uy - ly) / rows], 1)
+    fs.spans = np.sort(rng.uniform(lx, ux, (rows, 4)), axis=1).reshape(-1, 2)
+    fs.row_span = 2 * np.arange(rows + 1, dtype=np.int64)
+    assert np.any(np.diff(fs.row_y[:, 1]) < 0)
+    gpu_ctx.set_option("lal_subtree_cells", subtree)
+    gpu_ctx.set_option("lal_exact_sums", 1)
+    gpu_ctx.upload_netlist(nl)
+    gpu_ctx.set_grid(g)
+    gpu_ctx.set_free_space(fs)
+    try:
+        gx, gy = gpu_ctx.lal(x, y)
+    finally:
+        gpu_ctx.set_option("lal_subtree_cells", 2048)
+    gd = dict(origin=(g.origin_x, g.origin_y), dx=g.dx, dy=g.dy, nx=g.nx, ny=g.ny, avail=g.avail)
+    L = lal_ref.LAL(nl.width, nl.height, gd, lal_ref.free_rows(fs.row_y, fs.row_span, fs.spans),
+                    fs.obstacles, fs.die, g.density_limit)
+    ox, oy = L.legalize(x, y)
+    assert np.array_equal(gx, np.array(ox)) and np.array_equal(gy, np.array(oy))
+    assert np.mean(gx != x) > 0.1
