@@ -105,23 +105,7 @@ void free_systems(ktg_ctx *c) {
         dev_free(s.val);
         dev_free(s.diag);
         dev_free(s.rhs);
-        dev_free(s.r);
-        dev_free(s.z);
-        dev_free(s.p);
-        dev_free(s.ap);
-        dev_free(s.s);
-        dev_free(s.val32);
-        dev_free(s.d32);
-        dev_free(s.r32);
-        dev_free(s.z32);
-        dev_free(s.p32);
-        dev_free(s.ap32);
-        dev_free(s.s32);
-        dev_free(s.rs32);
     }
-    dev_free(c->sliced_rows);
-    dev_free(c->sliced_nnz);
-    c->sliced = ktg::SlicedSystem{};
     c->sliced_cap = 0;
     dev_free(c->x);
     dev_free(c->y);
@@ -133,6 +117,13 @@ void free_systems(ktg_ctx *c) {
     c->have_system = false;
     c->axis_valid[0] = c->axis_valid[1] = false;
     c->val32_valid = c->precond_ready = c->agg_ready = c->coarse_z_ready = false;
+}
+
+void free_scratch(ktg_ctx *c) {
+    for (ktg::Scratch *m : {&c->solve_rows, &c->solve_nnz}) {
+        dev_free(m->p);
+        m->bytes = 0;
+    }
 }
 
 // A larger array that keeps the first `keep` elements of the old one (the
@@ -155,41 +146,69 @@ int dev_grow_keep(ktg_ctx *c, T **p, int64_t keep, int64_t count) {
     return KTG_OK;
 }
 
-// The per-row scratch of the default FP64 solve, in one allocation.
-int reserve_sliced_rows(ktg_ctx *c, int64_t rows) {
-    const int64_t slices = ktg::sliced_slices(2 * rows, c->num_sms);
+// Cuts pieces out of one device allocation: the pieces are named, then measured
+// (first pass, null base), then placed.
+struct Pieces {
+    char *base;
     int64_t at = 0;
-    auto take = [&](int64_t bytes) {
-        const int64_t here = at;
-        at += (bytes + 255) / 256 * 256;
-        return here;
-    };
-    const int64_t vec = sizeof(double) * 2 * rows;
-    const int64_t diag = take(vec), x = take(vec), r = take(vec), z = take(vec), p = take(vec),
-                  ap = take(vec), start = take(sizeof(ktg::Start) * 2 * rows),
-                  perm = take(sizeof(int32_t) * 2 * rows), axis = take(2 * rows),
-                  lists = take(sizeof(uint2) * slices), dealt = take(sizeof(uint2) * slices),
-                  widths = take(sizeof(uint32_t) * slices), owner = take(slices),
-                  slots = take(sizeof(uint64_t) * ktg::sliced_slots(c->num_sms));
-    const int rc = dev_alloc(c, &c->sliced_rows, at);
-    if (rc) return rc;
-    char *m = c->sliced_rows;
-    ktg::SlicedSystem &s = c->sliced;
-    s.diag = reinterpret_cast<double *>(m + diag);
-    s.x = reinterpret_cast<double *>(m + x);
-    s.r = reinterpret_cast<double *>(m + r);
-    s.z = reinterpret_cast<double *>(m + z);
-    s.p = reinterpret_cast<double *>(m + p);
-    s.ap = reinterpret_cast<double *>(m + ap);
-    s.start = reinterpret_cast<ktg::Start *>(m + start);
-    s.perm = reinterpret_cast<int32_t *>(m + perm);
-    s.axis = reinterpret_cast<uint8_t *>(m + axis);
-    s.slices = reinterpret_cast<uint2 *>(m + lists);
-    s.dealt = reinterpret_cast<uint2 *>(m + dealt);
-    s.widths = reinterpret_cast<uint32_t *>(m + widths);
-    s.owner = reinterpret_cast<uint8_t *>(m + owner);
-    s.slots = reinterpret_cast<unsigned long long *>(m + slots);
+    template <typename T>
+    void take(T *&p, int64_t count) {
+        if (base) p = reinterpret_cast<T *>(base + at);
+        at += (static_cast<int64_t>(sizeof(T)) * count + 255) / 256 * 256;
+    }
+};
+
+// Scratch holds nothing between calls, so a context keeps its memory from one
+// netlist or system to the next where it is large enough: freeing and mapping it
+// again cost more than the rest of a small design's upload (60 netlists of 2 to
+// 20,000 cells, each after another system: 0.43 ms in the middle, 1.36 without).
+// Memory that is over four times what is needed, and 256 MB more, goes back.
+template <typename F>
+int alloc_pieces(ktg_ctx *c, ktg::Scratch &mem, F &&cut) {
+    Pieces size{nullptr};
+    cut(size);
+    if (mem.bytes < size.at || mem.bytes > 4 * size.at + (256ll << 20)) {
+        mem.bytes = 0;
+        const int rc = dev_alloc(c, &mem.p, size.at);
+        if (rc) return rc;
+        mem.bytes = size.at;
+    }
+    Pieces place{mem.p};
+    cut(place);
     return KTG_OK;
+}
+
+// The solvers' scratch by rows, in one allocation.
+int reserve_solve_rows(ktg_ctx *c, int64_t rows) {
+    return alloc_pieces(c, c->solve_rows, [&](Pieces &m) {
+        ktg::SlicedSystem &s = c->sliced;
+        const int64_t slices = ktg::sliced_slices(2 * rows, c->num_sms);
+        for (double **v : {&s.diag, &s.x, &s.r, &s.z, &s.p, &s.ap}) m.take(*v, 2 * rows);
+        m.take(s.start, 2 * rows);
+        m.take(s.perm, 2 * rows);
+        m.take(s.axis, 2 * rows);
+        m.take(s.slices, slices);
+        m.take(s.dealt, slices);
+        m.take(s.widths, slices);
+        m.take(s.owner, slices);
+        m.take(s.slots, ktg::sliced_slots(c->num_sms));
+        for (auto &t : c->sys) {
+            for (double **v : {&t.r, &t.z, &t.p, &t.ap, &t.s}) m.take(*v, rows);
+            for (float **v : {&t.d32, &t.r32, &t.z32, &t.p32, &t.ap32, &t.rs32}) m.take(*v, rows);
+        }
+    });
+}
+
+// The solvers' scratch by entries, in one allocation.
+int reserve_solve_nnz(ktg_ctx *c, int64_t nnz, int64_t sliced) {
+    return alloc_pieces(c, c->solve_nnz, [&](Pieces &m) {
+        m.take(c->sliced.val, sliced);
+        m.take(c->sliced.col, sliced);
+        for (auto &s : c->sys) {
+            m.take(s.val32, nnz);
+            m.take(s.s32, nnz);
+        }
+    });
 }
 
 // Room for systems of `rows` rows and `nnz` entries per axis. The arrays
@@ -204,19 +223,8 @@ int grow_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
             if ((rc = dev_grow_keep(c, &s.row_ptr, old > 0 ? old + 1 : 0, rows + 1))) return rc;
             if ((rc = dev_grow_keep(c, &s.diag, old, rows))) return rc;
             if ((rc = dev_grow_keep(c, &s.rhs, old, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.r, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.z, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.p, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.ap, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.s, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.d32, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.r32, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.z32, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.p32, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.ap32, rows))) return rc;
-            if ((rc = dev_alloc(c, &s.rs32, rows))) return rc;
         }
-        if ((rc = reserve_sliced_rows(c, rows))) return rc;
+        if ((rc = reserve_solve_rows(c, rows))) return rc;
         if ((rc = dev_alloc(c, &c->x, rows))) return rc;
         if ((rc = dev_alloc(c, &c->y, rows))) return rc;
         if ((rc = dev_alloc(c, &c->ax, rows))) return rc;
@@ -224,29 +232,26 @@ int grow_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
         c->sys_cap_n = rows;
         c->stage_cap = rows;
     }
-    if (nnz > c->sys_cap_nnz) {
+    const bool more = nnz > c->sys_cap_nnz;
+    if (more) {
         const int64_t old = c->sys_cap_nnz;
         for (auto &s : c->sys) {
             // room to read the last entries four at a time
             if ((rc = dev_grow_keep(c, &s.col, old, nnz + 3))) return rc;
             if ((rc = dev_grow_keep(c, &s.val, old, nnz + 3))) return rc;
-            if ((rc = dev_alloc(c, &s.val32, nnz))) return rc;
-            if ((rc = dev_alloc(c, &s.s32, nnz))) return rc;
         }
-        c->val32_valid = false;
-        c->precond_ready = false;
-        c->agg_ready = false;
-        c->coarse_z_ready = false;
         c->sys_cap_nnz = nnz;
     }
     // the sliced copy pads for the blocks that a solve of these rows takes
     const int64_t entries = ktg::sliced_entries(
         2 * c->sys_cap_nnz, ktg::sliced_blocks(2 * c->sys_cap_n, c->num_sms));  // a multiple of 32
-    if (entries > c->sliced_cap) {
-        if ((rc = dev_alloc(c, &c->sliced_nnz, entries * 12))) return rc;
-        c->sliced.val = reinterpret_cast<double *>(c->sliced_nnz);
-        c->sliced.col = reinterpret_cast<int32_t *>(c->sliced.val + entries);
-        c->sliced_cap = entries;
+    if (more || entries > c->sliced_cap) {
+        if ((rc = reserve_solve_nnz(c, c->sys_cap_nnz, std::max(entries, c->sliced_cap)))) return rc;
+        c->sliced_cap = std::max(entries, c->sliced_cap);
+        c->val32_valid = false;
+        c->precond_ready = false;
+        c->agg_ready = false;
+        c->coarse_z_ready = false;
     }
     return KTG_OK;
 }
@@ -255,6 +260,7 @@ int reserve_systems(ktg_ctx *c, int64_t rows, int64_t nnz) {
     const int rc = grow_systems(c, rows, nnz);
     if (rc) {  // some arrays are gone: the systems go with them, the next call starts afresh
         free_systems(c);
+        free_scratch(c);
         (void)cudaGetLastError();  // reported
     }
     return rc;
@@ -378,6 +384,7 @@ void ktg_destroy(ktg_ctx *c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     free_netlist(c);
     free_systems(c);
+    free_scratch(c);
     ktg::free_agg(c);
     ktg::free_lal(c);
     dev_free(c->coarse_head_w);

@@ -53,6 +53,11 @@ struct SlicedSystem {
     unsigned long long *slots = nullptr;              // the grid-wide sums
 };
 
+struct Scratch {
+    char *p = nullptr;
+    int64_t bytes = 0;
+};
+
 struct AxisSystem {
     int32_t *row_ptr = nullptr;  // [n+1]
     int32_t *col = nullptr;      // [cap]
@@ -116,8 +121,9 @@ struct ktg_ctx {
     // systems
     ktg::AxisSystem sys[2];
     ktg::SlicedSystem sliced;  // scratch of the default FP64 solve
-    char *sliced_rows = nullptr, *sliced_nnz = nullptr;  // its two allocations
-    int64_t sliced_cap = 0;                              // entries of the second
+    // the solvers' scratch, by rows and by entries (sys[*].r .. rs32, sliced)
+    ktg::Scratch solve_rows, solve_nnz;
+    int64_t sliced_cap = 0;  // entries of the sliced copy
     bool have_system = false;  // both axes valid with sys_n rows
     bool axis_valid[2] = {false, false};
     bool val32_valid = false;  // sys[*].val32 mirrors sys[*].val

@@ -88,3 +88,54 @@ def test_out_of_memory_leaves_no_system_behind(port_built):
         assert got["iters"] == ref["iters"]
         for k in ("x", "y"):
             assert np.linalg.norm(got[k] - ref[k]) <= 1e-9 * np.linalg.norm(ref[k])
+
+
+def test_scratch_from_one_design_to_the_next():
+    """The solvers' scratch stays with the context from one netlist or system to
+    another where it is large enough, with the results of a fresh context, and goes
+    back where it is far larger than what the next one needs."""
+    import torch
+    from ktplace_b200 import netlist, synth
+    from ktplace_b200.gpu import Context
+    from test_gpu_sliced import random_system
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    def run(ctx, design):
+        if isinstance(design, list):
+            n = len(design[0]["diag"])
+            for axis in (0, 1):
+                ctx.upload_system(axis, design[axis])
+        else:
+            n = design.num_movable
+            ctx.upload_netlist(design)
+            x, y = 100.0 * np.random.default_rng(n).random((2, n))
+            ctx.build_b2b(x, y, 0.2, y, x)
+        x0, y0 = np.random.default_rng(n + 1).standard_normal((2, n))
+        out = []
+        for precond in (0, 2):
+            ctx.set_option("precond", precond)
+            got = ctx.solve(x0, y0, 1e-7, 500), ctx.solve_mixed(x0, y0, 1e-6)
+            out += [v for g in got for v in (g["x"], g["y"])]
+        return out
+
+    raw = [synth.generate(synth.spec_tiny(seed=k, macros=0, cells=n, nets=n + 20))
+           for k, n in enumerate((300, 3000))]
+    designs = [netlist.flatten(raw[0]), [random_system(20_000, [2, 6, 10], k) for k in (1, 2)],
+               netlist.flatten(raw[0]), netlist.flatten(raw[1]),
+               [random_system(777, [0, 4, 300], k) for k in (3, 4)], netlist.flatten(raw[0])]
+    with Context(0) as ctx:
+        for design in designs:
+            got = run(ctx, design)
+            with Context(0) as fresh:
+                for a, b in zip(got, run(fresh, design)):
+                    assert np.array_equal(a, b)
+        n, m = 500, 30_000_000
+        ctx.upload_system(0, dict(row_ptr=np.linspace(0, m, n + 1).astype(np.int64),
+                                  col=np.resize(np.arange(n, dtype=np.int32), m),
+                                  val=np.full(m, -1e-6), diag=np.ones(n), rhs=np.ones(n)))
+        before = free()
+        run(ctx, designs[0])
+        assert free() - before > 1_500_000_000  # of 0.72 GB of systems, 1.2 GB of scratch
