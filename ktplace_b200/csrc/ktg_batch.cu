@@ -44,7 +44,7 @@ struct SysDesc {
     int64_t row_base;  // first row in the concatenated vectors
     int64_t nnz_base;  // first entry in col/val
     int32_t n;
-    int32_t pad;
+    int32_t nnz;
 };
 
 struct BatchArgs {
@@ -165,6 +165,23 @@ constexpr int kJaggedRows = 600;  // of a CTA
 
 __host__ __device__ inline bool jagged_pays(int64_t rows, int cluster) {
     return cluster <= kPortable && rows >= static_cast<int64_t>(kJaggedRows) * cluster;
+}
+
+// Whether they pay for a launch whose systems are all like this one; beside one for
+// which they do, the rule above holds (the tiles are slower in the kernel that has
+// both). With more than 512 threads the tiles are faster and the copy's warps have less
+// each: it pays from 1,400 rows and 8,500 entries a CTA on, and not for chains (speed
+// with the copy against without, 1,024 threads, clusters 1, 2, 4, 8: 800 rows a CTA of 3
+// entries 0.83, 0.84, 0.72, 0.78, of 8 0.91, 0.88, 0.87, 0.97; 1,400 of 3 0.96, 0.90,
+// 0.88, 1.07, of 8 1.02, 1.00, 1.10, 1.17; 3,000 of 2 0.95, 0.99, 0.93, 0.87, of 3 1.07,
+// 1.04, 1.15, 1.12). With up to 512, rows of few entries pay later in clusters of 4 and
+// more (512 threads: 800 rows of 3 1.06, 1.06, 0.86, 0.92, of 8 1.10, 1.05, 1.09, 1.10;
+// 1,000 of 3 1.14, 1.14, 0.98, 0.99).
+inline bool jagged_pays_alone(int64_t rows, int64_t nnz, int cluster, int threads) {
+    if (!jagged_pays(rows, cluster)) return false;
+    if (threads > 512)
+        return rows >= 1400ll * cluster && nnz >= 8500ll * cluster && 2 * nnz >= 5 * rows;
+    return cluster < 4 || rows >= 1000ll * cluster || nnz >= 6 * rows;
 }
 
 // The search direction p that its products gather lies whole in every CTA's shared
@@ -1118,7 +1135,7 @@ int ktg_batch_add_system(ktg_batch *b, int64_t n, const int64_t *row_ptr, const 
         ++b->launches;
     }
     KTG_BCUDA(b, cudaStreamSynchronize(b->stream));
-    b->sys.push_back(ktg::SysDesc{base, ebase, static_cast<int32_t>(n), 0});
+    b->sys.push_back(ktg::SysDesc{base, ebase, static_cast<int32_t>(n), static_cast<int32_t>(m)});
     b->cost.push_back(m + n);
     b->rows += n;
     b->nnz += m;
@@ -1284,12 +1301,16 @@ static int near_room(ktg_batch *b, int mixed, NearPlan *plan) {
     const std::vector<char> off = offloaded(b);
     auto in_class = [&](size_t i) { return b->split_rows > 0 && b->sys[i].n >= b->split_rows; };
     int64_t near[2] = {0, 0};
+    bool alone[2] = {false, false};
     for (size_t i = 0; i < b->sys.size(); ++i) {
         if (off[i]) continue;
         const int k = in_class(i) ? 1 : 0;
         const int64_t n = b->sys[i].n;
         plan[k].most = std::max(plan[k].most, n);
-        if (ktg::jagged_pays(n, k ? b->split_cluster : b->cluster)) near[k] = std::max(near[k], n);
+        const int cluster = k ? b->split_cluster : b->cluster;
+        if (ktg::jagged_pays(n, cluster)) near[k] = std::max(near[k], n);
+        alone[k] = alone[k] || ktg::jagged_pays_alone(n, b->sys[i].nnz, cluster,
+                                                      k ? b->split_threads : b->threads);
     }
     for (size_t i = 0; i < b->sys.size(); ++i) {
         if (off[i]) continue;
@@ -1299,7 +1320,7 @@ static int near_room(ktg_batch *b, int mixed, NearPlan *plan) {
         if (2 * static_cast<int64_t>(b->sys[i].n) >= p.most) p.big += rows;
     }
     for (int k = 0; k < 2; ++k)
-        if (plan[k].most * 4 <= near_limit)
+        if (alone[k] && plan[k].most * 4 <= near_limit)
             plan[k].bytes = static_cast<int>((near[k] * 4 + 255) / 256 * 256);
     return KTG_OK;
 }

@@ -427,3 +427,41 @@ def test_batch_copies_come_with_the_first_mixed_solve():
     per_row, per_entry = 24, 8
     nnz = sum(len(s["col"]) for s, _ in cases[:8])
     assert free[0] - free[1] >= 0.9 * (per_row * 8 * 30_011 + per_entry * nnz)
+
+
+@pytest.mark.parametrize("cluster,threads", [(1, 1024), (4, 512), (4, 1024), (8, 512), (8, 1024)])
+def test_batch_mixed_layout_by_entries(cluster, threads):
+    """Rows and entries a CTA on both sides of where the renumbered copy starts to
+    pay for the shape, chains among them, in one launch."""
+    rng = np.random.default_rng(cluster + threads)
+    cases = []
+    for per in (599, 601, 999, 1001, 1399, 1401, 3001):
+        for deg in (2, 3, 6, 13):
+            n = per * cluster + 2
+            if deg == 2:
+                a = np.arange(n - 1)
+                b = a + 1
+            else:
+                a = rng.integers(0, n, n * deg // 2)
+                b = (a + rng.integers(1, n, a.shape[0])) % n
+            w = rng.uniform(0.1, 1.0, a.shape[0])
+            r, c, v = np.concatenate([a, b]), np.concatenate([b, a]), -np.concatenate([w, w])
+            order = np.argsort(r, kind="stable")
+            r, c, v = r[order], c[order], v[order]
+            diag = rng.uniform(0.5, 1.5, n) + np.bincount(r, weights=-v, minlength=n)
+            rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))])
+            cases.append((dict(row_ptr=rp.astype(np.int64), col=c.astype(np.int32), val=v,
+                               diag=diag, rhs=rng.standard_normal(n)), rng.standard_normal(n)))
+    b, ids = make_batch(cases)
+    b.set_shape(cluster, threads)
+    got = []
+    for _ in range(2):
+        b.reset_x()
+        b.solve(TOL, MAX_ITER, precision=1, inner_tol=1e-3)
+        got.append([b.get_x(i, s["diag"].shape[0]) for (s, _), i in zip(cases, ids)])
+    res = b.results()
+    for (s, _), sid, x, again in zip(cases, ids, *got):
+        assert res[sid]["status"] == 0, res[sid]
+        assert true_resid(s, x) <= TOL * 1.0001
+        assert np.array_equal(x, again)
+    b.close()
