@@ -123,7 +123,10 @@ int ktg_set_pointer_mode(ktg_ctx *ctx, int mode);
 
 /* Uploads the netlist topology once per design; it stays device-resident.
  * Replaces the per-call reads of Netlist in buildB2B and getHpwl
- * (simpl_lss.cc:11-27, simpl_placer.cc:256-275). */
+ * (simpl_lss.cc:11-27, simpl_placer.cc:256-275). The solvers' scratch stays
+ * with the context from one netlist or system to the next and is given back
+ * with the context, or where it is over four times what is needed, and 256 MB
+ * more. */
 int ktg_upload_netlist(ktg_ctx *ctx, const ktg_netlist_view *nl);
 
 /* ---- B2B assembly --------------------------------------------------------- */
@@ -270,7 +273,9 @@ int ktg_occupancy(ktg_ctx *ctx, const double *x, const double *y, double *occ,
  *                           obstacles, as FreeSpace::build leaves them)
  *   obstacles [4*num_obstacles]  lx ly ux uy of the fixed blocks
  *   die       [4]           lx ly ux uy
- * KTG_ERR_ARG on unsorted rows or a row_span that is not ascending. */
+ * Rows may overlap; where their y ends then do not ascend, legalization takes
+ * a slower path. KTG_ERR_ARG on unsorted rows or a row_span that is not
+ * ascending. */
 int ktg_set_free_space(ktg_ctx *ctx, int64_t num_rows, const double *row_y,
                        const int64_t *row_span, const double *spans, int64_t num_obstacles,
                        const double *obstacles, const double *die);
